@@ -1,11 +1,13 @@
 // Newton systems of tet meshes generated on the GPU (include/b200gen.h):
 // kinetic + stable Neo-Hookean (PSD-projected) + ground barrier + Dirichlet
 // vertices, straight into device triplet buffers. The arithmetic restates the
-// host generator (csrc/scene/scene_gen.cpp: snh_derivatives, jacobi_eigen,
-// the kinetic / elastic / ground / fixed passes) per element; results agree
-// with it to rounding (FMA contraction on the device).
+// host generator (csrc/scene/scene_gen.cpp: snh_derivatives, the kinetic /
+// elastic / ground / fixed passes) per element, with the closed-form PSD
+// projection of b2s_snh.cuh in place of its 9x9 Jacobi; results agree with it
+// to rounding.
 #include "b2s_fixed_reduce.cuh"
 #include "b2s_internal.cuh"
+#include "b2s_snh.cuh"
 
 #include "../../include/b200gen.h"
 
@@ -35,112 +37,6 @@ struct DevMesh
     b2gen_material     mat{};
     int                device = 0;
 };
-
-// ---- stable Neo-Hookean: dPsi/dF and the PSD-projected d2Psi/dF2 -----------
-__device__ void jacobi_eigen9(double* a, double* w, double* v)
-{
-    for(int i = 0; i < 81; ++i)
-        v[i] = 0.0;
-    for(int i = 0; i < 9; ++i)
-        v[i * 9 + i] = 1.0;
-    for(int sweep = 0; sweep < 60; ++sweep)
-    {
-        double off = 0.0, diag = 0.0;
-        for(int p = 0; p < 9; ++p)
-        {
-            diag += a[p * 9 + p] * a[p * 9 + p];
-            for(int q = p + 1; q < 9; ++q)
-                off += a[p * 9 + q] * a[p * 9 + q];
-        }
-        if(off <= 1e-30 * (diag + 1e-300))
-            break;
-        for(int p = 0; p < 9; ++p)
-            for(int q = p + 1; q < 9; ++q)
-            {
-                const double apq = a[p * 9 + q];
-                if(fabs(apq) < 1e-300)
-                    continue;
-                const double app = a[p * 9 + p], aqq = a[q * 9 + q];
-                const double theta = (aqq - app) / (2.0 * apq);
-                const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                const double c = 1.0 / sqrt(t * t + 1.0), s = t * c;
-                for(int k = 0; k < 9; ++k)
-                {
-                    const double akp = a[k * 9 + p], akq = a[k * 9 + q];
-                    a[k * 9 + p] = c * akp - s * akq;
-                    a[k * 9 + q] = s * akp + c * akq;
-                }
-                for(int k = 0; k < 9; ++k)
-                {
-                    const double apk = a[p * 9 + k], aqk = a[q * 9 + k];
-                    a[p * 9 + k] = c * apk - s * aqk;
-                    a[q * 9 + k] = s * apk + c * aqk;
-                }
-                for(int k = 0; k < 9; ++k)
-                {
-                    const double vkp = v[k * 9 + p], vkq = v[k * 9 + q];
-                    v[k * 9 + p] = c * vkp - s * vkq;
-                    v[k * 9 + q] = s * vkp + c * vkq;
-                }
-            }
-    }
-    for(int i = 0; i < 9; ++i)
-        w[i] = a[i * 9 + i];
-}
-
-// F column-major; P = dPsi/dF, H = d2Psi/dF2 (vec(F) column-major), PSD
-__device__ void snh_derivatives(const double F[9], double mu, double lambda, double P[9], double H[81])
-{
-    const double f0[3] = {F[0], F[1], F[2]}, f1[3] = {F[3], F[4], F[5]}, f2[3] = {F[6], F[7], F[8]};
-    auto cross = [](const double* a, const double* b, double* c) {
-        c[0] = a[1] * b[2] - a[2] * b[1];
-        c[1] = a[2] * b[0] - a[0] * b[2];
-        c[2] = a[0] * b[1] - a[1] * b[0];
-    };
-    double g[9];
-    cross(f1, f2, g);
-    cross(f2, f0, g + 3);
-    cross(f0, f1, g + 6);
-    const double J = f0[0] * g[0] + f0[1] * g[1] + f0[2] * g[2];
-    const double s = lambda * (J - 1.0) - mu;
-    for(int i = 0; i < 9; ++i)
-        P[i] = mu * F[i] + s * g[i];
-    for(int i = 0; i < 9; ++i)
-        for(int j = 0; j < 9; ++j)
-            H[i * 9 + j] = (i == j ? mu : 0.0) + lambda * g[i] * g[j];
-    // d2J/df_a df_b: (0,1) = -[f2]x, (0,2) = [f1]x, (1,2) = -[f0]x (and transposes)
-    auto put_cross = [&](int bi, int bj, const double* a, double sign) {
-        const double m[9] = {0, -a[2], a[1], a[2], 0, -a[0], -a[1], a[0], 0};  // row-major [a]x
-        for(int r = 0; r < 3; ++r)
-            for(int c = 0; c < 3; ++c)
-            {
-                const double v = sign * s * m[r * 3 + c];
-                H[(bi * 3 + r) * 9 + (bj * 3 + c)] += v;
-                H[(bj * 3 + c) * 9 + (bi * 3 + r)] += v;
-            }
-    };
-    put_cross(0, 1, f2, -1.0);
-    put_cross(0, 2, f1, +1.0);
-    put_cross(1, 2, f0, -1.0);
-    double a[81], w[9], v[81];
-    for(int i = 0; i < 81; ++i)
-        a[i] = H[i];
-    jacobi_eigen9(a, w, v);
-    bool neg = false;
-    for(int i = 0; i < 9; ++i)
-        neg |= (w[i] < 0.0);
-    if(!neg)
-        return;
-    for(int i = 0; i < 9; ++i)
-        for(int j = 0; j < 9; ++j)
-        {
-            double acc = 0.0;
-            for(int k = 0; k < 9; ++k)
-                if(w[k] > 0.0)
-                    acc += v[i * 9 + k] * w[k] * v[j * 9 + k];
-            H[i * 9 + j] = acc;
-        }
-}
 
 // a row-major 3x3 block of the pair (ra, rb) into slot k, upper orientation
 __device__ __forceinline__ void write_block(int64_t k, int32_t ra, int32_t rb, const double* Hab, int32_t* rows,
@@ -202,72 +98,163 @@ __global__ void k_mass(int nv, const int32_t* __restrict__ vt_start, const int32
     mass[v] = m;
 }
 
-__global__ void __launch_bounds__(GEN_BLOCK) k_elastic(int nv, int nt, const int32_t* __restrict__ tets,
-                                                       const double* __restrict__ vol,
-                                                       const double* __restrict__ G, const double* __restrict__ x,
-                                                       double mu, double lambda, double dt2, int32_t* rows,
-                                                       int32_t* cols, double* vals, double* __restrict__ tet_g)
+// the block of vertex pair (i, j) after the Dirichlet rule: rows and columns
+// of fixed vertices zero, the identity on their diagonal blocks
+__device__ __forceinline__ void apply_fixed(bool fix, bool diag, double* H)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if(t >= nt)
+    if(!fix)
         return;
-    const int32_t* T  = tets + (int64_t)t * 4;
-    const double*  Gs = G + (int64_t)t * 12;
-    double         F[9] = {0};
+#pragma unroll
+    for(int e = 0; e < 9; ++e)
+        H[e] = (diag && e % 4 == 0) ? 1.0 : 0.0;
+}
+
+// slot k of a tet's ten upper blocks -> its vertex pair (q, r), q <= r
+__device__ __forceinline__ int slot_q(int k) { return (0x3221110000ull >> (4 * k)) & 0xF; }
+__device__ __forceinline__ int slot_r(int k) { return (0x3323213210ull >> (4 * k)) & 0xF; }
+
+// One thread per tet: F, the stress for the gradient and the ten projected
+// Hessian blocks (b2s_snh.cuh: closed form, everything in registers). Bound by
+// the FP64 pipe and the 800 B of triplets written per tet. A 9x9 Jacobi per
+// tet, its two 648-byte arrays in local memory, took the whole system of
+// 480,000 tets 11.1 ms; with this kernel it takes 0.21 ms (1.9 TB/s). The
+// blocks go through shared memory, five slots at a time, so that a warp's
+// stores cover whole 360-byte runs: written thread by thread every 8-byte
+// store of a warp would touch 32 sectors. 46 KB and at most 128 registers:
+// four CTAs per SM. The Dirichlet rule is applied as the blocks are made, not
+// in a pass over the written triplets.
+constexpr int GEN_HALF = 5;             // slots staged together
+constexpr int GEN_RUN  = 9 * GEN_HALF;  // their doubles per tet (odd: no bank conflicts)
+__global__ void __launch_bounds__(GEN_BLOCK, 4) k_elastic(int nv, int nt, const int32_t* __restrict__ tets,
+                                                          const double* __restrict__ vol,
+                                                          const double* __restrict__ G, const double* __restrict__ x,
+                                                          const uint8_t* __restrict__ fixed, double mu, double lambda,
+                                                          double dt2, int32_t* rows, int32_t* cols, double* vals,
+                                                          double* __restrict__ tet_g)
+{
+    __shared__ double s_val[GEN_BLOCK / 32][32 * GEN_RUN];
+    __shared__ int4   s_tet[GEN_BLOCK];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int t0 = blockIdx.x * GEN_BLOCK + 32 * w;  // the warp's first tet
+    if(t0 >= nt)
+        return;
+    const int     n    = min(32, nt - t0);  // its tets; the lanes past them repeat the last one
+    const int     t    = t0 + min(lane, n - 1);
+    const int4    T4   = reinterpret_cast<const int4*>(tets)[t];
+    const int32_t T[4] = {T4.x, T4.y, T4.z, T4.w};
+    s_tet[threadIdx.x] = T4;
+    unsigned fx = 0;
+    if(fixed)
+#pragma unroll
+        for(int q = 0; q < 4; ++q)
+            fx |= fixed[T[q]] ? 1u << q : 0u;
+    double g[4][3];
+#pragma unroll
+    for(int i = 0; i < 6; ++i)
+    {
+        const double2 d = reinterpret_cast<const double2*>(G + (int64_t)t * 12)[i];
+        g[(2 * i) / 3][(2 * i) % 3]         = d.x;
+        g[(2 * i + 1) / 3][(2 * i + 1) % 3] = d.y;
+    }
+    double F[9] = {0};
+#pragma unroll
     for(int q = 0; q < 4; ++q)
-        for(int a = 0; a < 3; ++a)
-            for(int b = 0; b < 3; ++b)
-                F[a + 3 * b] += x[T[q] * 3 + a] * Gs[q * 3 + b];
-    double P[9], H[81];
-    snh_derivatives(F, mu, lambda, P, H);
-    const double s = vol[t] * dt2;
-    for(int q = 0; q < 4; ++q)
+#pragma unroll
         for(int a = 0; a < 3; ++a)
         {
-            double acc = 0.0;
+            const double xa = x[(int64_t)T[q] * 3 + a];
+#pragma unroll
             for(int b = 0; b < 3; ++b)
-                acc += P[a + 3 * b] * Gs[q * 3 + b];
-            tet_g[(int64_t)t * 12 + q * 3 + a] = s * acc;
+                F[a + 3 * b] += xa * g[q][b];
         }
-    int slot = 0;
+    double               P[9];
+    b2s::snh::Projected h;
+    b2s::snh::derivatives(F, mu, lambda, vol[t] * dt2, P, h);
+    if(lane < n)
+    {
+        double f[12];
+#pragma unroll
+        for(int i = 0; i < 12; ++i)
+            f[i] = P[i % 3] * g[i / 3][0] + P[i % 3 + 3] * g[i / 3][1] + P[i % 3 + 6] * g[i / 3][2];
+#pragma unroll
+        for(int i = 0; i < 6; ++i)
+            reinterpret_cast<double2*>(tet_g + (int64_t)t * 12)[i] = make_double2(f[2 * i], f[2 * i + 1]);
+    }
+    // the shape gradients in the V frame
+#pragma unroll
     for(int q = 0; q < 4; ++q)
-        for(int r = q; r < 4; ++r, ++slot)
+    {
+        const double a = g[q][0], b = g[q][1], c = g[q][2];
+#pragma unroll
+        for(int i = 0; i < 3; ++i)
+            g[q][i] = h.v[i][0] * a + h.v[i][1] * b + h.v[i][2] * c;
+    }
+    const int64_t slot0 = (int64_t)nv + (int64_t)t0 * 10;
+#pragma unroll
+    for(int half = 0; half < 2; ++half)
+    {
+        double* mine = s_val[w] + lane * GEN_RUN;
+#pragma unroll
+        for(int k = 0; k < GEN_HALF; ++k)
         {
-            double Hb[9];
-            for(int a = 0; a < 3; ++a)
-                for(int c = 0; c < 3; ++c)
-                {
-                    double acc = 0.0;
-                    for(int b = 0; b < 3; ++b)
-                    {
-                        const double gq = Gs[q * 3 + b];
-                        for(int d = 0; d < 3; ++d)
-                            acc += gq * H[(a + 3 * b) * 9 + (c + 3 * d)] * Gs[r * 3 + d];
-                    }
-                    Hb[a * 3 + c] = s * acc;
-                }
+            const int q = slot_q(GEN_HALF * half + k), r = slot_r(GEN_HALF * half + k);
+            double    Hb[9];
+            b2s::snh::block(h, g[q], g[r], Hb);
             if(q == r)  // exact symmetry of diagonal blocks
+            {
+#pragma unroll
                 for(int a = 0; a < 3; ++a)
+#pragma unroll
                     for(int c = a + 1; c < 3; ++c)
-                    {
-                        const double m = 0.5 * (Hb[a * 3 + c] + Hb[c * 3 + a]);
-                        Hb[a * 3 + c] = Hb[c * 3 + a] = m;
-                    }
-            write_block((int64_t)nv + (int64_t)t * 10 + slot, T[q], T[r], Hb, rows, cols, vals);
+                        Hb[a * 3 + c] = Hb[c * 3 + a] = 0.5 * (Hb[a * 3 + c] + Hb[c * 3 + a]);
+            }
+            apply_fixed((fx >> q & 1u) || (fx >> r & 1u), T[q] == T[r], Hb);
+            const bool tp = T[q] > T[r];
+#pragma unroll
+            for(int a = 0; a < 3; ++a)
+#pragma unroll
+                for(int c = 0; c < 3; ++c)
+                    mine[9 * k + c * 3 + a] = tp ? Hb[c * 3 + a] : Hb[a * 3 + c];  // column-major, upper orientation
         }
+        __syncwarp();
+        double* V = vals + slot0 * 9 + half * GEN_RUN;
+#pragma unroll 5
+        for(int i = 0; i < GEN_RUN; ++i)
+        {
+            const int e = i * 32 + lane, tt = e / GEN_RUN;
+            if(tt < n)
+                V[(int64_t)tt * (2 * GEN_RUN) + (e - tt * GEN_RUN)] = s_val[w][e];
+        }
+        __syncwarp();
+    }
+    const int32_t* ids = reinterpret_cast<const int32_t*>(s_tet + 32 * w);
+#pragma unroll
+    for(int i = 0; i < 10; ++i)
+    {
+        const int e = i * 32 + lane, tt = e / 10, k = e - tt * 10;
+        if(tt < n)
+        {
+            const int32_t va = ids[4 * tt + slot_q(k)], vb = ids[4 * tt + slot_r(k)];
+            rows[slot0 + e]  = min(va, vb);
+            cols[slot0 + e]  = max(va, vb);
+        }
+    }
 }
 
 // kinetic block and the gradient (kinetic, tets by index, ground) per vertex
 __global__ void k_vertex(int nv, int nt, const double* __restrict__ mass, const double* __restrict__ x,
                          const double* __restrict__ xt, const int32_t* __restrict__ vt_start,
-                         const int32_t* __restrict__ vt_list, const double* __restrict__ tet_g, int32_t* rows,
-                         int32_t* cols, double* vals, double* __restrict__ grad)
+                         const int32_t* __restrict__ vt_list, const double* __restrict__ tet_g,
+                         const uint8_t* __restrict__ fixed, int32_t* rows, int32_t* cols, double* vals,
+                         double* __restrict__ grad)
 {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if(v >= nv)
         return;
+    const bool   fix  = fixed && fixed[v];
     const double m    = mass[v];
-    const double H[9] = {m, 0, 0, 0, m, 0, 0, 0, m};
+    double       H[9] = {m, 0, 0, 0, m, 0, 0, 0, m};
+    apply_fixed(fix, true, H);
     write_block(v, v, v, H, rows, cols, vals);
     double g[3];
     for(int a = 0; a < 3; ++a)
@@ -279,18 +266,19 @@ __global__ void k_vertex(int nv, int nt, const double* __restrict__ mass, const 
             g[a] += tet_g[(int64_t)(tq >> 2) * 12 + (tq & 3) * 3 + a];
     }
     for(int a = 0; a < 3; ++a)
-        grad[(int64_t)v * 3 + a] = g[a];
+        grad[(int64_t)v * 3 + a] = fix ? 0.0 : g[a];
 }
 
 // ground barrier (normal +y) on the candidates: one diagonal block each
 __global__ void k_ground(int nv, int nt, int ng, const int32_t* __restrict__ ground, const double* __restrict__ x,
-                         double ground_y, double dhat, double kappa, double dt2, int32_t* rows, int32_t* cols,
-                         double* vals, double* __restrict__ grad)
+                         const uint8_t* __restrict__ fixed, double ground_y, double dhat, double kappa, double dt2,
+                         int32_t* rows, int32_t* cols, double* vals, double* __restrict__ grad)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= ng)
         return;
     const int32_t g   = ground[i];
+    const bool    fix = fixed && fixed[g];
     const double  d   = x[(int64_t)g * 3 + 1] - ground_y;
     double        k   = 0.0, gy = 0.0;
     if(d < dhat)
@@ -301,31 +289,12 @@ __global__ void k_ground(int nv, int nt, int ng, const int32_t* __restrict__ gro
         k               = fmax(0.0, dt2 * kappa * (b2 * 4.0 * D + 2.0 * b1));
         gy              = dt2 * kappa * b1 * 2.0 * d;
     }
-    const double H[9] = {0, 0, 0, 0, k, 0, 0, 0, 0};
+    double H[9] = {0, 0, 0, 0, k, 0, 0, 0, 0};
+    apply_fixed(fix, true, H);
     write_block((int64_t)nv + (int64_t)nt * 10 + i, g, g, H, rows, cols, vals);
     // one candidate per vertex: the add keeps the order kinetic, tets, ground
-    grad[(int64_t)g * 3 + 1] += gy;
-}
-
-// Dirichlet vertices: their rows / columns zero, diagonal I, gradient 0
-__global__ void k_fixed(int64_t T, int nv, const uint8_t* __restrict__ fixed, const int32_t* __restrict__ rows,
-                        const int32_t* __restrict__ cols, double* vals, double* grad)
-{
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if(s < T)
-    {
-        const int32_t i = rows[s], j = cols[s];
-        if(fixed[i] || fixed[j])
-        {
-            double* V = vals + s * 9;
-            for(int e = 0; e < 9; ++e)
-                V[e] = 0.0;
-            if(i == j)
-                V[0] = V[4] = V[8] = 1.0;
-        }
-    }
-    if(s < nv && fixed[s])
-        grad[s * 3] = grad[s * 3 + 1] = grad[s * 3 + 2] = 0.0;
+    if(!fix)
+        grad[(int64_t)g * 3 + 1] += gy;
 }
 
 int grid_of(int64_t n) { return (int)((n + GEN_BLOCK - 1) / GEN_BLOCK); }
@@ -514,25 +483,20 @@ int b2gen_system(b2gen_mesh* m, const double* d_x, const double* d_xtilde, int32
         cudaStream_t      st  = static_cast<cudaStream_t>(stream);
         const b2gen_material& c = m->mat;
         const double      dt2 = c.dt * c.dt;
+        const uint8_t*    fixed = m->fixed.size() > 0 ? m->fixed.data() : nullptr;  // Dirichlet rule in every pass
         k_elastic<<<grid_of(m->nt), GEN_BLOCK, 0, st>>>(m->nv, m->nt, m->tets.data(), m->vol.data(), m->grad.data(),
-                                                        d_x, c.mu, c.lambda, dt2, d_rows, d_cols, d_vals,
-                                                        m->tet_g.data());
+                                                        d_x, fixed, c.mu, c.lambda, dt2, d_rows, d_cols,
+                                                        d_vals, m->tet_g.data());
         B2S_CHECK_LAUNCH();
         k_vertex<<<grid_of(m->nv), GEN_BLOCK, 0, st>>>(m->nv, m->nt, m->mass.data(), d_x, d_xtilde,
-                                                       m->vt_start.data(), m->vt_list.data(), m->tet_g.data(), d_rows,
-                                                       d_cols, d_vals, d_grad);
+                                                       m->vt_start.data(), m->vt_list.data(), m->tet_g.data(), fixed,
+                                                       d_rows, d_cols, d_vals, d_grad);
         B2S_CHECK_LAUNCH();
         if(m->ng > 0)
         {
-            k_ground<<<grid_of(m->ng), GEN_BLOCK, 0, st>>>(m->nv, m->nt, m->ng, m->ground.data(), d_x, c.ground_y,
-                                                           c.dhat, c.kappa, dt2, d_rows, d_cols, d_vals, d_grad);
-            B2S_CHECK_LAUNCH();
-        }
-        if(m->fixed.size() > 0)
-        {
-            const int64_t T = b2gen_num_triplets(m);
-            k_fixed<<<grid_of(std::max<int64_t>(T, m->nv)), GEN_BLOCK, 0, st>>>(T, m->nv, m->fixed.data(), d_rows,
-                                                                                 d_cols, d_vals, d_grad);
+            k_ground<<<grid_of(m->ng), GEN_BLOCK, 0, st>>>(m->nv, m->nt, m->ng, m->ground.data(), d_x, fixed,
+                                                           c.ground_y, c.dhat, c.kappa, dt2, d_rows, d_cols, d_vals,
+                                                           d_grad);
             B2S_CHECK_LAUNCH();
         }
         B2S_CUDA(cudaStreamSynchronize(st));

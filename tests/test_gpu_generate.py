@@ -254,3 +254,77 @@ def test_contact_producer_against_the_host_routines(cuda):
             gref[3 * pairs[p][i]:3 * pairs[p][i] + 3] += G[3 * i:3 * i + 3]
     assert np.abs(grad.cpu().numpy() - gref).max() <= 1e-10 * np.abs(gref).max()
     gc.close()
+
+
+def _snh_hessian(F, mu, lam):
+    """dPsi/dF and the eigen-clamped d2Psi/dF2 (vec(F) column-major) by numpy."""
+    f = F.T.ravel()
+    f0, f1, f2 = f[:3], f[3:6], f[6:]
+    g = np.concatenate([np.cross(f1, f2), np.cross(f2, f0), np.cross(f0, f1)])
+    s = lam * (f0 @ g[:3] - 1.0) - mu
+    H = mu * np.eye(9) + lam * np.outer(g, g)
+    for i, j, a, sg in ((0, 1, f2, -1.0), (0, 2, f1, 1.0), (1, 2, f0, -1.0)):
+        M = sg * s * np.array([[0, -a[2], a[1]], [a[2], 0, -a[0]], [-a[1], a[0], 0]])
+        H[3 * i:3 * i + 3, 3 * j:3 * j + 3] += M
+        H[3 * j:3 * j + 3, 3 * i:3 * i + 3] += M.T
+    w, Q = np.linalg.eigh(H)
+    return mu * f + s * g, (Q * np.maximum(w, 0.0)) @ Q.T, np.abs(H).max()
+
+
+@pytest.mark.parametrize("n_tets", [1, 31, 33, 160, 421])
+def test_projected_hessian_at_special_states(cuda, n_tets):
+    """Separate tets (warps and CTAs with a remainder) at states where the
+    closed-form projection could go wrong: rest, rotations, inverted,
+    collapsed to a plane, a line and a point, repeated and tiny singular
+    values; some vertices fixed. Each block to 1e-13 of its tet's largest
+    unprojected entry (an eigenvalue of either side is off by a few eps |H|,
+    and clamping does not amplify it)."""
+    from libuipc_b200.gpu_scene import GpuTetMesh
+
+    rng = np.random.default_rng(7)
+    corner = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1.0]])
+    rest = (corner + 0.1 * rng.normal(size=(n_tets, 4, 3))) * 0.01
+    Fs = []
+    for t in range(n_tets):
+        Q = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+        u, v = rng.normal(size=(2, 3))
+        Fs.append([np.eye(3), Q, Q @ np.diag([1, 1, -1.0]), rng.normal(size=(3, 3)), Q @ np.diag([1.2, 0.7, 0]),
+                   Q @ np.diag([0, 0, 1.5]), np.outer(u, v), np.zeros((3, 3)), Q @ np.diag([2, 2, 0.3]) @ Q.T,
+                   Q @ np.diag([2, 1e-5, 1e-10]), np.eye(3) + 1e-6 * rng.normal(size=(3, 3))][t % 11])
+    x = np.einsum("tab,tqb->tqa", np.array(Fs), rest)
+    x += rng.normal(size=(n_tets, 1, 3)) * 0.01 * (np.arange(n_tets) % 2)[:, None, None]
+    tets = np.arange(4 * n_tets, dtype=np.int32).reshape(-1, 4)
+    tets = np.array([row[rng.permutation(4)] for row in tets])
+    perm = tets - 4 * np.arange(n_tets)[:, None]
+    fixed = rng.random(4 * n_tets) < 0.1
+    cfg = {"E": 1e6, "nu": 0.49, "rho": 1e3, "dt": 0.01, "kappa": 1e9, "dhat": 1e-3}
+    mu, lam = 1e6 / (2 * 1.49), 1e6 * 0.49 / (1.49 * 0.02)
+    mesh = GpuTetMesh(rest.reshape(-1, 3), tets, cfg, cuda, fixed=fixed)
+    try:
+        xd = to_dev(x.ravel(), cuda)
+        rows, cols, vals, _ = (a.cpu().numpy() for a in mesh.system(xd, xd))
+    finally:
+        mesh.close()
+    nv = 4 * n_tets
+    for t in range(n_tets):
+        X, xt = rest[t][perm[t]], x[t][perm[t]]
+        E = (X[1:] - X[0]).T
+        G = np.vstack([-np.linalg.inv(E).sum(0), np.linalg.inv(E)])  # shape gradients
+        F = (xt.T @ G)
+        _, H, big = _snh_hessian(F, mu, lam)
+        scale = np.linalg.det(E) / 6.0 * 1e-4  # signed, as the volume is
+        H = H.reshape(3, 3, 3, 3) * scale  # [b, a, d, c]
+        lim = 1e-13 * big * abs(scale) * np.abs(G).max() ** 2 * 9
+        k = nv + 10 * t
+        for q in range(4):
+            for r in range(q, 4):
+                i, j = tets[t, q], tets[t, r]
+                B = np.einsum("b,badc,d->ac", G[q], H, G[r])
+                if fixed[i] or fixed[j]:
+                    B = np.eye(3) * (i == j)
+                if i > j:
+                    i, j, B = j, i, B.T
+                assert rows[k] == i and cols[k] == j
+                got = vals[k].reshape(3, 3).T
+                assert np.abs(got - B).max() <= (0.0 if fixed[i] or fixed[j] else lim), (t % 11, q, r)
+                k += 1
