@@ -291,7 +291,8 @@ constexpr int SPMV_TILE = 1024;  // blocks per SpMV tile (the span of the transp
 void spmv_f64(b2s_solver* s, const Matrix& A, const double* x, double* y, double* d_dot);
 
 // reductions
-int  reduction_grid();
+int  reduction_grid();               // the largest grid (sizes the partials)
+int  reduction_grid(int64_t items);  // the grid for a sum over `items` elements
 void launch_dot(b2s_solver* s, const double* a, const double* b, int64_t n, double* d_out);
 // several dot products in one pass: d_out[k] = a[k] . b[k], k < m (FP64,
 // deterministic)

@@ -558,7 +558,7 @@ static void precond_launch(b2s_solver* s, int kind, const double* r, double* z, 
         return;
     if(kind == B2S_PRECOND_MAS)
         mas_apply_levels(s, r, sc ? &sc->converged : nullptr);
-    const int grid = reduction_grid();
+    const int grid = reduction_grid(nb);
     ensure_reduction(red, grid, 2);
     k_precond_finish<double, 3><<<grid, RED_BLOCK, 0, st>>>(nb, kind, mas_view(s), s->dinv.data(), r, z, sc,
                                                  red.partials.data(), red.counter.data());
@@ -718,7 +718,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
     auto true_residual = [&]() -> double
     {
         spmv_f64(s, A, x, P.tmp.data(), nullptr);
-        k_res_norms<<<reduction_grid(), RED_BLOCK, 0, st>>>(n, b, P.tmp.data(), s->red.partials.data(),
+        k_res_norms<<<reduction_grid(n), RED_BLOCK, 0, st>>>(n, b, P.tmp.data(), s->red.partials.data(),
                                                             s->red.counter.data(), s->dot_out.data());
         B2S_CHECK_LAUNCH();
         double h2[2];
@@ -907,7 +907,7 @@ static void precond_launch_f32(b2s_solver* s, int kind, const float* r, float* z
         return;
     if(kind == B2S_PRECOND_MAS)
         mas_apply_levels_f32(s, r, sc ? &sc->converged : nullptr, mixed_inverse_bf16());
-    const int grid = reduction_grid();
+    const int grid = reduction_grid(nb);
     ensure_reduction(red, grid, 2);
     k_precond_finish<float, 4><<<grid, RED_BLOCK, 0, s->stream>>>(nb, kind, mas_view(s), s->dinv.data(), r, z, sc,
                                                                red.partials.data(), red.counter.data());
@@ -1091,7 +1091,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
     {
         // z = P r, p = z; returns r.z (FP64 sum); also leaves r.r in dot_out[1]
         precond_launch_f32(s, k, P.r32.data(), P.z32.data(), nullptr, s->red);
-        k_dot2_f32<<<reduction_grid(), RED_BLOCK, 0, st>>>(n4, P.r32.data(), P.z32.data(), s->red.partials.data(),
+        k_dot2_f32<<<reduction_grid(n4), RED_BLOCK, 0, st>>>(n4, P.r32.data(), P.z32.data(), s->red.partials.data(),
                                                             s->red.counter.data(), s->dot_out.data());
         B2S_CHECK_LAUNCH();
         B2S_CUDA(cudaMemcpyAsync(P.p32.data(), P.z32.data(), sizeof(float) * n4, cudaMemcpyDeviceToDevice, st));
@@ -1118,7 +1118,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
     auto true_residual = [&]() -> double
     {
         spmv_f64(s, A, x, P.tmp.data(), nullptr);
-        k_res_norms<<<reduction_grid(), RED_BLOCK, 0, st>>>(n, b, P.tmp.data(), s->red.partials.data(),
+        k_res_norms<<<reduction_grid(n), RED_BLOCK, 0, st>>>(n, b, P.tmp.data(), s->red.partials.data(),
                                                             s->red.counter.data(), s->dot_out.data());
         B2S_CHECK_LAUNCH();
         double h2[2];

@@ -62,39 +62,49 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* partials, unsi
     __syncthreads();
     if(!is_last)
         return false;
-    // last block: sum the partials in block order, NV values in parallel warps
+    // last block: NV values side by side, G warps each (a fixed shape for a
+    // given grid). Every lane adds a strided subset in order, then a fixed
+    // tree; the loads go out 8 at a time, independent of one another. With one
+    // warp per value the 1184 partials of a full grid took five dependent
+    // rounds of loads at the end of every kernel with a sum.
     __threadfence();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __shared__ double res[NV];
-    for(int k = warp; k < NV; k += blockDim.x >> 5)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int G = nw > NV ? nw / NV : 1;
+    __shared__ double res[NV][RED_BLOCK / 32];
+    for(int job = warp; job < NV * G; job += nw)
     {
-        // each lane sums a strided subset in order, then a fixed-shape tree;
-        // the loads go out 8 at a time (independent), the adds keep the order
-        const volatile double* pk  = (const volatile double*)partials + (size_t)k * gridDim.x;
-        double                 acc = 0.0;
-        for(unsigned int b = lane; b < gridDim.x; b += 32 * 8)
+        const int              k = job / G, part = job - k * G;
+        const volatile double* pk   = (const volatile double*)partials + (size_t)k * gridDim.x;
+        const unsigned int     step = 32u * G;
+        double                 acc  = 0.0;
+        for(unsigned int b = 32 * part + lane; b < gridDim.x; b += step * 8)
         {
             double t[8];
 #pragma unroll
             for(int j = 0; j < 8; ++j)
-                t[j] = b + 32u * j < gridDim.x ? pk[b + 32u * j] : 0.0;
+                t[j] = b + step * j < gridDim.x ? pk[b + step * j] : 0.0;
 #pragma unroll
             for(int j = 0; j < 8; ++j)
-                if(b + 32u * j < gridDim.x)
+                if(b + step * j < gridDim.x)
                     acc += t[j];
         }
 #pragma unroll
         for(int o = 16; o > 0; o >>= 1)
             acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if(lane == 0)
-            res[k] = acc;
+            res[k][part] = acc;
     }
     __syncthreads();
     if(threadIdx.x != 0)
         return false;
 #pragma unroll
     for(int k = 0; k < NV; ++k)
-        total[k] = res[k];
+    {
+        double t = res[k][0];
+        for(int g = 1; g < G; ++g)
+            t += res[k][g];
+        total[k] = t;
+    }
     *counter = 0u;  // ready for the next launch
     return true;
 }
