@@ -226,12 +226,7 @@ int b2s_get_upper_bsr(b2s_solver* s, int32_t* rowptr, int32_t* colidx, double* v
                            B2S_CUDA(cudaMemcpyAsync(colidx, A.cols.data(), sizeof(int32_t) * A.nnz,
                                                     cudaMemcpyDefault, st));
                        if(vals && A.nnz)
-                       {
-                           // planes -> column-major blocks: one strided copy per component
-                           for(int q = 0; q < 9; ++q)
-                               B2S_CUDA(cudaMemcpy2DAsync(vals + q, 9 * sizeof(double), A.vals.data() + (size_t)q * A.stride,
-                                                          sizeof(double), sizeof(double), A.nnz, cudaMemcpyDefault, st));
-                       }
+                           b2s::copy_blocks_out(s, A, vals);
                        B2S_CUDA(cudaStreamSynchronize(st));
                    });
 }

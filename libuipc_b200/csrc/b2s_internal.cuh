@@ -285,6 +285,10 @@ void exclusive_scan(b2s_solver* s, const int32_t* in, int32_t* out, int64_t n, D
 void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const int32_t* rows,
                        const int32_t* cols, const double* vals, bool spmv_tiles);
 
+// the first nnz blocks of A as 9 doubles each (column-major) to `out`, host or
+// device memory, on the solver's stream
+void copy_blocks_out(b2s_solver* s, const Matrix& A, double* out);
+
 constexpr int SPMV_TILE = 1024;  // blocks per SpMV tile (the span of the transposed-half ranks)
 
 // y = A x (+ optional pAp into partial reduction slot)
