@@ -123,6 +123,8 @@ int b2s_destroy(b2s_solver* s)
     b2s::drop_graphs(s);
     if(s->pcg.h_sc)
         cudaFreeHost(s->pcg.h_sc);
+    if(s->asmb.h_info)
+        cudaFreeHost(s->asmb.h_info);
     if(s->ev_begin)
         cudaEventDestroy(s->ev_begin);
     if(s->ev_end)

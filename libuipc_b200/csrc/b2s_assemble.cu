@@ -389,18 +389,51 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_sort_rows(int32_t nb, const int32
 
 // Rows longer than ROW_CAP pairs (e.g. an affine body touched by thousands of
 // cloth vertices), listed by k_sort_rows: one CTA per row (persistent over the
-// list). Every key (column << 32 | source; unique) gets its rank by counting
-// the smaller keys, tile by tile through shared memory; a key is the head of
-// its column's run when no key has its column and a smaller source. O(L^2 / T)
-// work per row with T threads.
+// list). The keys (column << 32 | source; unique) are sorted LONG_TILE at a
+// time in shared memory (bitonic); with several tiles every key's rank is its
+// place in its tile plus a binary search in each of the others. Counting the
+// smaller keys of the whole row for every key, O(L^2), took 25 us a launch on
+// the rows of 25 bodies under a cloth of 128^2 vertices (1,200 pairs; 9 us now).
 constexpr int LONG_THREADS = 1024;
 constexpr int LONG_TILE    = 4096;
 
+__device__ __forceinline__ uint64_t pair_key(int2 q)
+{
+    return ((uint64_t)(uint32_t)q.x << 32) | (uint64_t)(uint32_t)q.y;
+}
+
+// keys [0, n) of s_key ascending (whole CTA); n <= LONG_TILE, the slots up to
+// the next power of two hold ~0
+__device__ __forceinline__ void sort_tile(uint64_t* s_key, int n)
+{
+    int size2 = 32;
+    while(size2 < n)
+        size2 <<= 1;
+    for(int i = n + (int)threadIdx.x; i < size2; i += LONG_THREADS)
+        s_key[i] = ~0ull;
+    __syncthreads();
+    for(int size = 2; size <= size2; size <<= 1)
+        for(int stride = size >> 1; stride > 0; stride >>= 1)
+        {
+            for(int i = threadIdx.x; i < size2 / 2; i += LONG_THREADS)
+            {
+                const int      lo = 2 * i - (i & (stride - 1));
+                const int      hi = lo + stride;
+                const bool     up = (lo & size) == 0;
+                const uint64_t a = s_key[lo], b = s_key[hi];
+                if((a > b) == up)
+                {
+                    s_key[lo] = b;
+                    s_key[hi] = a;
+                }
+            }
+            __syncthreads();
+        }
+}
+
 __global__ void __launch_bounds__(LONG_THREADS) k_sort_long_rows(const int32_t* __restrict__ long_rows,
-                                                                 const int32_t* __restrict__ row_start,
-                                                                 const int2* __restrict__ bucket,
-                                                                 int32_t* __restrict__ sorted_col,
-                                                                 int32_t* __restrict__ sorted_src,
+                                                                 const int32_t* __restrict__ row_start, int2* bucket,
+                                                                 int32_t* sorted_col, int32_t* sorted_src,
                                                                  int32_t* __restrict__ uniq_count)
 {
     __shared__ uint64_t s_key[LONG_TILE];
@@ -409,45 +442,79 @@ __global__ void __launch_bounds__(LONG_THREADS) k_sort_long_rows(const int32_t* 
     for(int e = blockIdx.x; e < n_long; e += gridDim.x)
     {
         const int32_t r = long_rows[1 + e], beg = row_start[r], L = row_start[r + 1] - beg;
-        int           heads = 0;
-        for(int base = 0; base < L; base += LONG_THREADS)
+        const bool    many = L > LONG_TILE;
+        // sort the tiles (one tile: straight to the result; several: in place)
+        for(int t0 = 0; t0 < L; t0 += LONG_TILE)
         {
-            const int      i    = base + (int)threadIdx.x;
-            uint64_t       me   = ~0ull;
-            if(i < L)
+            const int n = min(LONG_TILE, L - t0);
+            __syncthreads();  // the previous tile is written
+            for(int k = threadIdx.x; k < n; k += LONG_THREADS)
+                s_key[k] = pair_key(bucket[beg + t0 + k]);
+            __syncthreads();
+            sort_tile(s_key, n);
+            for(int k = threadIdx.x; k < n; k += LONG_THREADS)
             {
-                const int2 q = bucket[beg + i];
-                me           = ((uint64_t)(uint32_t)q.x << 32) | (uint64_t)(uint32_t)q.y;
-            }
-            const uint32_t col  = (uint32_t)(me >> 32);
-            int            rank = 0;
-            bool           head = true;
-            for(int t0 = 0; t0 < L; t0 += LONG_TILE)
-            {
-                const int n = min(LONG_TILE, L - t0);
-                __syncthreads();  // the previous tile is read
-                for(int k = threadIdx.x; k < n; k += LONG_THREADS)
+                const int32_t c = (int32_t)(s_key[k] >> 32), sr = (int32_t)(s_key[k] & 0xFFFFFFFFull);
+                if(many)
+                    bucket[beg + t0 + k] = make_int2(c, sr);
+                else
                 {
-                    const int2 q = bucket[beg + t0 + k];
-                    s_key[k]     = ((uint64_t)(uint32_t)q.x << 32) | (uint64_t)(uint32_t)q.y;
+                    sorted_col[beg + k] = c;
+                    sorted_src[beg + k] = sr;
                 }
-                __syncthreads();
-                if(i < L)
-                    for(int k = 0; k < n; ++k)
-                    {
-                        const uint64_t o = s_key[k];
-                        rank += o < me ? 1 : 0;
-                        head = head && !((uint32_t)(o >> 32) == col && o < me);
-                    }
-            }
-            if(i < L)
-            {
-                sorted_col[beg + rank] = (int32_t)col;
-                sorted_src[beg + rank] = (int32_t)(me & 0xFFFFFFFFull);
-                heads += head ? 1 : 0;
             }
         }
+        __syncthreads();
+        if(many)
+            for(int own = 0; own < L; own += LONG_TILE)
+            {
+                constexpr int PER = LONG_TILE / LONG_THREADS;
+                uint64_t      key[PER];
+                int           rank[PER];
+#pragma unroll
+                for(int j = 0; j < PER; ++j)
+                {
+                    const int i = own + j * LONG_THREADS + (int)threadIdx.x;
+                    key[j]      = i < L ? pair_key(bucket[beg + i]) : ~0ull;
+                    rank[j]     = i - own;
+                }
+                for(int t0 = 0; t0 < L; t0 += LONG_TILE)
+                {
+                    if(t0 == own)
+                        continue;
+                    const int n = min(LONG_TILE, L - t0);
+                    __syncthreads();  // the previous tile is read
+                    for(int k = threadIdx.x; k < n; k += LONG_THREADS)
+                        s_key[k] = pair_key(bucket[beg + t0 + k]);
+                    __syncthreads();
+#pragma unroll
+                    for(int j = 0; j < PER; ++j)
+                    {
+                        int lo = 0, hi = n;
+                        while(lo < hi)
+                        {
+                            const int m = (lo + hi) >> 1;
+                            if(s_key[m] < key[j])
+                                lo = m + 1;
+                            else
+                                hi = m;
+                        }
+                        rank[j] += lo;
+                    }
+                }
+#pragma unroll
+                for(int j = 0; j < PER; ++j)
+                    if(own + j * LONG_THREADS + (int)threadIdx.x < L)
+                    {
+                        sorted_col[beg + rank[j]] = (int32_t)(key[j] >> 32);
+                        sorted_src[beg + rank[j]] = (int32_t)(key[j] & 0xFFFFFFFFull);
+                    }
+            }
+        __syncthreads();  // the sorted row is visible to the CTA
         // the row's number of distinct columns
+        int heads = 0;
+        for(int i = threadIdx.x; i < L; i += LONG_THREADS)
+            heads += (i == 0 || sorted_col[beg + i] != sorted_col[beg + i - 1]) ? 1 : 0;
 #pragma unroll
         for(int o = 16; o > 0; o >>= 1)
             heads += __shfl_xor_sync(0xffffffffu, heads, o);
@@ -482,6 +549,8 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_mark_runs(int32_t nb, const int32
     for(int32_t r = blockIdx.x * (ASM_BLOCK / 32) + w; r < nb; r += warps_total)
     {
         const int32_t beg = row_start[r], L = row_start[r + 1] - beg;
+        if(L > ROW_CAP)
+            continue;  // k_mark_long_rows
         const int32_t obeg = rowptr[r];
         int           heads_before = 0;
         for(int base = 0; base < L; base += 32)
@@ -510,20 +579,76 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_mark_runs(int32_t nb, const int32
     }
 }
 
+// the same for the rows listed by k_sort_rows, one CTA per row: a warp stepping
+// through 20,000 pairs 32 at a time is a chain of 640 dependent rounds
+__global__ void __launch_bounds__(LONG_THREADS) k_mark_long_rows(const int32_t* __restrict__ long_rows,
+                                                                 const int32_t* __restrict__ row_start,
+                                                                 const int32_t* __restrict__ sorted_col,
+                                                                 const int32_t* __restrict__ rowptr,
+                                                                 int32_t* __restrict__ out_rows,
+                                                                 int32_t* __restrict__ out_cols,
+                                                                 int32_t* __restrict__ run_start,
+                                                                 int32_t* __restrict__ diag_index)
+{
+    __shared__ int s_warp[LONG_THREADS / 32];
+    const int      n_long = long_rows[0], lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for(int e = blockIdx.x; e < n_long; e += gridDim.x)
+    {
+        const int32_t r = long_rows[1 + e], beg = row_start[r], L = row_start[r + 1] - beg;
+        int64_t       o0 = rowptr[r];
+        if(threadIdx.x == 0)
+            diag_index[r] = sorted_col[beg] == r ? (int32_t)o0 : -1;
+        for(int base = 0; base < L; base += LONG_THREADS)
+        {
+            const int     k    = base + (int)threadIdx.x;
+            const int32_t c    = k < L ? sorted_col[beg + k] : 0;
+            const bool    head = k < L && (k == 0 || sorted_col[beg + k - 1] != c);
+            const unsigned hm  = __ballot_sync(0xffffffffu, head);
+            __syncthreads();  // s_warp of the previous round is read
+            if(lane == 0)
+                s_warp[w] = __popc(hm);
+            __syncthreads();
+            int before = 0, all = 0;
+#pragma unroll
+            for(int q = 0; q < LONG_THREADS / 32; ++q)
+            {
+                before += q < w ? s_warp[q] : 0;
+                all += s_warp[q];
+            }
+            if(head)
+            {
+                const int64_t o = o0 + before + __popc(hm & ((1u << lane) - 1u));
+                out_rows[o]     = r;
+                out_cols[o]     = c;
+                run_start[o]    = beg + k;
+            }
+            o0 += all;
+        }
+    }
+}
+
 // One thread per (unique block, column of its 3x3): the column's 3 values
 // summed over the run's sources in source order (the sorted order). The
 // three threads of a block read its sources' 72 contiguous bytes together;
 // four sources are fetched ahead, the additions stay in order from the first.
+// Runs longer than `run_cap` go to long_runs (count, then the blocks) instead.
 __global__ void __launch_bounds__(ASM_BLOCK) k_sum_runs(int64_t U, const int32_t* __restrict__ run_start,
                                                          const int32_t* __restrict__ sorted_src,
                                                          const double* __restrict__ src_vals,
-                                                         double* __restrict__ out_vals, int64_t S)
+                                                         double* __restrict__ out_vals, int64_t S, int run_cap,
+                                                         int32_t* long_runs)
 {
     for(int64_t t = (int64_t)blockIdx.x * ASM_BLOCK + threadIdx.x; t < 3 * U; t += (int64_t)gridDim.x * ASM_BLOCK)
     {
         const int64_t o = t / 3;
         const int     c = (int)(t - 3 * o);
         const int32_t b = run_start[o], e = run_start[o + 1];
+        if(e - b > run_cap)
+        {
+            if(c == 0)
+                long_runs[1 + atomicAdd(long_runs, 1)] = (int32_t)o;
+            continue;
+        }
         double        acc[3] = {};
         for(int32_t k = b; k < e; k += 4)
         {
@@ -547,6 +672,61 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_sum_runs(int64_t U, const int32_t
 #pragma unroll
         for(int q = 0; q < 3; ++q)
             out_vals[(int64_t)(3 * c + q) * S + o] = acc[q];
+    }
+}
+
+// The listed long runs (the diagonal blocks of an affine body collect one
+// source per contact), one warp each: 4 x 32 sources are gathered together
+// (coalesced, 9 doubles each) into shared memory, then lanes 0-8 add their
+// component over them, in source order from the first as k_sum_runs does. Its
+// one thread per column waited for memory once per four sources.
+constexpr int LONG_RUN       = 64;
+constexpr int LONG_RUN_WARPS = 4;
+__global__ void __launch_bounds__(LONG_RUN_WARPS * 32) k_sum_long_runs(const int32_t* __restrict__ long_runs,
+                                                                       const int32_t* __restrict__ run_start,
+                                                                       const int32_t* __restrict__ sorted_src,
+                                                                       const double* __restrict__ src_vals,
+                                                                       double* __restrict__ out_vals, int64_t S)
+{
+    constexpr int     CH = 128;
+    __shared__ double s_v[LONG_RUN_WARPS][CH * 9];
+    const int         lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int         n = long_runs[0];
+    for(int i = blockIdx.x * LONG_RUN_WARPS + w; i < n; i += gridDim.x * LONG_RUN_WARPS)
+    {
+        const int64_t o = long_runs[1 + i];
+        const int32_t b = run_start[o], e = run_start[o + 1];
+        double        acc = 0.0;
+        for(int32_t k0 = b; k0 < e; k0 += CH)
+        {
+            const int m = min(CH, e - k0);
+            int       src[CH / 32];
+#pragma unroll
+            for(int j = 0; j < CH / 32; ++j)
+                src[j] = 32 * j + lane < m ? sorted_src[k0 + 32 * j + lane] : -1;
+#pragma unroll
+            for(int j = 0; j < CH / 32; ++j)
+            {
+                double v[9];
+#pragma unroll
+                for(int q = 0; q < 9; ++q)
+                {
+                    const int t  = 32 * q + lane, k = t / 9;
+                    const int sk = __shfl_sync(0xffffffffu, src[j], k);
+                    v[q]         = sk >= 0 ? src_vals[(int64_t)sk * 9 + (t - 9 * k)] : 0.0;
+                }
+#pragma unroll
+                for(int q = 0; q < 9; ++q)
+                    s_v[w][288 * j + 32 * q + lane] = v[q];
+            }
+            __syncwarp();
+            if(lane < 9)
+                for(int k = 0; k < m; ++k)
+                    acc = k0 + k == b ? s_v[w][9 * k + lane] : acc + s_v[w][9 * k + lane];
+            __syncwarp();
+        }
+        if(lane < 9)
+            out_vals[(int64_t)lane * S + o] = acc;
     }
 }
 
@@ -604,6 +784,13 @@ __global__ void __launch_bounds__(OUT_BLOCKS) k_blocks_out(int64_t k0, int64_t n
     __syncthreads();
     for(int e = t; e < 9 * m; e += OUT_BLOCKS)
         out[9 * base + e] = s_b[e];
+}
+
+__global__ void k_publish(const int32_t* nnz, const int* err, const int32_t* n_long, int32_t* info)
+{
+    info[0] = *nnz;
+    info[1] = *err;
+    info[2] = n_long ? *n_long : 0;
 }
 
 int asm_grid(int64_t work, int block)
@@ -717,11 +904,16 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
         B2S_CHECK_LAUNCH();
     }
     exclusive_scan(s, w.uniq_count.data(), M.rowptr.data(), nb, w.scan_tmp);
-    int32_t U = 0;
-    int     herr = 0;
-    B2S_CUDA(cudaMemcpyAsync(&U, M.rowptr.data() + nb, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    B2S_CUDA(cudaMemcpyAsync(&herr, w.err.data(), sizeof(int), cudaMemcpyDeviceToHost, st));
+    // the sizes the host needs, written by the device straight into pinned host
+    // memory (a copy to pageable memory is ~9 us each, and a MAS build assembles
+    // five coarse levels)
+    if(!w.h_info)
+        B2S_CUDA(cudaMallocHost(&w.h_info, 3 * sizeof(int32_t)));
+    k_publish<<<1, 1, 0, st>>>(M.rowptr.data() + nb, w.err.data(), nb > 0 ? w.long_rows.data() : nullptr, w.h_info);
+    B2S_CHECK_LAUNCH();
     B2S_CUDA(cudaStreamSynchronize(st));
+    const int32_t U = w.h_info[0], n_long = w.h_info[2];
+    const int     herr = w.h_info[1];
     B2S_REQUIRE(!(herr & DERR_TRIPLET_INDEX), B2S_ERR_ARGUMENT,
                 "triplet column index outside [0, n_block_rows)");
     B2S_REQUIRE(!(herr & DERR_ROW_OVERFLOW), B2S_ERR_ARGUMENT,
@@ -742,15 +934,37 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
             nb, w.row_start.data(), w.sorted_col.data(), M.rowptr.data(), M.rows.data(), M.cols.data(),
             w.run_start.data(), M.diag_index.data());
         B2S_CHECK_LAUNCH();
+        if(n_long > 0)
+        {
+            k_mark_long_rows<<<std::min(n_long, NUM_SMS_HINT * 2), LONG_THREADS, 0, st>>>(
+                w.long_rows.data(), w.row_start.data(), w.sorted_col.data(), M.rowptr.data(), M.rows.data(),
+                M.cols.data(), w.run_start.data(), M.diag_index.data());
+            B2S_CHECK_LAUNCH();
+        }
         B2S_CUDA(cudaMemcpyAsync(w.run_start.data() + U, w.row_start.data() + nb, sizeof(int32_t),
                                  cudaMemcpyDeviceToDevice, st));
         if(U > 0)
         {
             // one pass in block order (no grid-stride loop): the CTAs in
             // flight cover neighbouring rows, whose sources share cache lines
-            k_sum_runs<<<(unsigned)((3 * U + ASM_BLOCK - 1) / ASM_BLOCK), ASM_BLOCK, 0, st>>>(
-                U, w.run_start.data(), w.sorted_src.data(), vals, M.vals.data(), M.stride);
+            // (runs above LONG_RUN are set apart only when there are long
+            // rows: elsewhere a run has at most ROW_CAP sources, and a few
+            // dozen in the meshes)
+            if(n_long > 0)
+            {
+                w.long_runs.resize((size_t)U + 1, 1.2);
+                B2S_CUDA(cudaMemsetAsync(w.long_runs.data(), 0, sizeof(int32_t), st));
+            }
+            k_sum_runs<<<(unsigned)((3 * (int64_t)U + ASM_BLOCK - 1) / ASM_BLOCK), ASM_BLOCK, 0, st>>>(
+                U, w.run_start.data(), w.sorted_src.data(), vals, M.vals.data(), M.stride,
+                n_long > 0 ? LONG_RUN : INT32_MAX, w.long_runs.data());
             B2S_CHECK_LAUNCH();
+            if(n_long > 0)
+            {
+                k_sum_long_runs<<<NUM_SMS_HINT, LONG_RUN_WARPS * 32, 0, st>>>(
+                    w.long_runs.data(), w.run_start.data(), w.sorted_src.data(), vals, M.vals.data(), M.stride);
+                B2S_CHECK_LAUNCH();
+            }
         }
     }
     M.has_trank = false;

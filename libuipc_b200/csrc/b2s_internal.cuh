@@ -145,8 +145,10 @@ struct AssemblyScratch
     DBuf<int32_t> sorted_col, sorted_src;
     DBuf<int32_t> run_start;  // [U+1] sorted position of each unique block's first source
     DBuf<int32_t> long_rows;  // [1 + nb]: count, then the rows too long for one warp
+    DBuf<int32_t> long_runs;  // [1 + U]: count, then the blocks whose run is summed by a warp
     DBuf<int32_t> scan_tmp;
     DBuf<int>     err;
+    int32_t*      h_info = nullptr;  // pinned: blocks, error bits, long rows of the last assembly
 };
 
 // ---------------------------------------------------------------------------
