@@ -17,8 +17,9 @@ namespace b2s
 namespace
 {
 constexpr int SCAN_BLOCK = 256;
-constexpr int SCAN_ITEMS = 4;  // elements per thread
+constexpr int SCAN_ITEMS = 16;  // elements per thread
 constexpr int SCAN_TILE  = SCAN_BLOCK * SCAN_ITEMS;
+constexpr int SCAN_DIRECT_TILES = 2048;  // tiles whose sums every block adds up by itself
 
 // block-wide inclusive scan of one int per thread (warp shuffles + smem)
 __device__ __forceinline__ int block_inclusive_scan(int v, int* warp_sums)
@@ -53,57 +54,86 @@ __device__ __forceinline__ int block_inclusive_scan(int v, int* warp_sums)
     return v;
 }
 
-// tile exclusive scan; writes out[i] (i < n) and the tile total into tile_sums
-__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(const int32_t* in, int32_t* out, int64_t n,
-                                                           int32_t* tile_sums)
+// the sum of each tile
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_sums(const int32_t* __restrict__ in, int64_t n,
+                                                          int32_t* __restrict__ tile_sums)
 {
     __shared__ int warp_sums[SCAN_BLOCK / 32];
-    const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    int           v[SCAN_ITEMS];
-    int           local = 0;
+    const int64_t  base = (int64_t)blockIdx.x * SCAN_TILE;
+    int            v    = 0;
 #pragma unroll
     for(int k = 0; k < SCAN_ITEMS; ++k)
     {
-        v[k] = (base + k < n) ? in[base + k] : 0;
-        local += v[k];
+        const int64_t j = base + k * SCAN_BLOCK + threadIdx.x;
+        v += j < n ? in[j] : 0;
     }
-    int incl = block_inclusive_scan(local, warp_sums);
-    int run  = incl - local;
-#pragma unroll
-    for(int k = 0; k < SCAN_ITEMS; ++k)
-    {
-        if(base + k < n)
-            out[base + k] = run;
-        run += v[k];
-    }
-    if(threadIdx.x == blockDim.x - 1)
-        tile_sums[blockIdx.x] = incl;
+    v = block_inclusive_scan(v, warp_sums);
+    if(threadIdx.x == SCAN_BLOCK - 1)
+        tile_sums[blockIdx.x] = v;
 }
 
-__global__ void k_scan_add(int32_t* out, int64_t n, const int32_t* tile_offsets)
+// out[0 .. n] of one tile, from the tiles before it: their sums (added up by
+// every block: at most SCAN_DIRECT_TILES of them) or their scanned offsets.
+// out must not alias in.
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(const int32_t* __restrict__ in, int32_t* __restrict__ out,
+                                                           int64_t n, const int32_t* __restrict__ tile_sums,
+                                                           const int32_t* __restrict__ tile_offsets)
 {
-    const int64_t i = (int64_t)blockIdx.x * SCAN_TILE + threadIdx.x;
-    const int32_t add = tile_offsets[blockIdx.x];
+    __shared__ int warp_sums[SCAN_BLOCK / 32], pre_sums[SCAN_BLOCK / 32];
+    __shared__ int s_in[SCAN_TILE + SCAN_TILE / 32];  // padded: a thread reads 16 in a row
+    __shared__ int s_pre;
+    const int64_t  base = (int64_t)blockIdx.x * SCAN_TILE;
+    int            p    = 0;
+    if(tile_offsets)
+        p = threadIdx.x == 0 ? tile_offsets[blockIdx.x] : 0;
+    else
+        for(int t = threadIdx.x; t < (int)blockIdx.x; t += SCAN_BLOCK)
+            p += tile_sums[t];
 #pragma unroll
     for(int k = 0; k < SCAN_ITEMS; ++k)
     {
-        int64_t j = i + (int64_t)k * SCAN_BLOCK;
+        const int     i = k * SCAN_BLOCK + threadIdx.x;
+        const int64_t j = base + i;
+        s_in[i + i / 32] = j < n ? in[j] : 0;
+    }
+    p = block_inclusive_scan(p, pre_sums);
+    if(threadIdx.x == SCAN_BLOCK - 1)
+        s_pre = p;
+    __syncthreads();
+    int local = 0;
+#pragma unroll
+    for(int k = 0; k < SCAN_ITEMS; ++k)
+    {
+        const int i = threadIdx.x * SCAN_ITEMS + k;
+        local += s_in[i + i / 32];
+    }
+    const int incl = block_inclusive_scan(local, warp_sums);
+    int       run  = s_pre + incl - local;
+#pragma unroll
+    for(int k = 0; k < SCAN_ITEMS; ++k)
+    {
+        const int i = threadIdx.x * SCAN_ITEMS + k, v = s_in[i + i / 32];
+        s_in[i + i / 32] = run;
+        run += v;
+    }
+    if(threadIdx.x == SCAN_BLOCK - 1 && base + SCAN_TILE >= n)
+        out[n] = run;
+    __syncthreads();
+#pragma unroll
+    for(int k = 0; k < SCAN_ITEMS; ++k)
+    {
+        const int     i = k * SCAN_BLOCK + threadIdx.x;
+        const int64_t j = base + i;
         if(j < n)
-            out[j] += add;
+            out[j] = s_in[i + i / 32];
     }
-}
-
-__global__ void k_write_total(int32_t* out, int64_t n, const int32_t* in, const int32_t* tile_offsets,
-                              int64_t last_tile)
-{
-    // out[n] = exclusive(out[n-1]) + in[n-1]; computed from the last element
-    if(threadIdx.x == 0 && blockIdx.x == 0)
-        out[n] = (n > 0) ? (out[n - 1] + in[n - 1]) : 0;
 }
 }  // namespace
 
-// Exclusive scan of n int32 into out[0..n] (out[n] = total). `in` may alias
-// `out` only when the caller keeps a copy of in[n-1]; here in != out always.
+// Exclusive scan of n int32 into out[0..n] (out[n] = total); in != out. One
+// launch up to SCAN_TILE elements, two up to SCAN_DIRECT_TILES tiles (every
+// block adds the sums before its own: 8 M elements at most 8 loads a thread),
+// beyond that the tile sums are scanned first.
 void exclusive_scan(b2s_solver* s, const int32_t* in, int32_t* out, int64_t n, DBuf<int32_t>& tmp)
 {
     cudaStream_t st = s->stream;
@@ -112,55 +142,30 @@ void exclusive_scan(b2s_solver* s, const int32_t* in, int32_t* out, int64_t n, D
         B2S_CUDA(cudaMemsetAsync(out, 0, sizeof(int32_t), st));
         return;
     }
-    const int64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    // recursion through a flat list of levels inside one scratch buffer
-    std::vector<int64_t> level_n{n};
-    while(level_n.back() > SCAN_TILE)
-        level_n.push_back((level_n.back() + SCAN_TILE - 1) / SCAN_TILE);
-    // scratch: for each level k >= 1 an array of level_n[k] sums + their scan (+1)
+    auto    tiles_of = [](int64_t m) { return (m + SCAN_TILE - 1) / SCAN_TILE; };
     int64_t need = 0;
-    std::vector<int64_t> off_sums, off_scan;
-    for(size_t k = 0; k < level_n.size(); ++k)
-    {
-        int64_t t = (level_n[k] + SCAN_TILE - 1) / SCAN_TILE;
-        off_sums.push_back(need);
-        need += t;
-        off_scan.push_back(need);
-        need += t + 1;
-    }
+    for(int64_t m = n; tiles_of(m) > 1; m = tiles_of(m))
+        need += 2 * tiles_of(m) + 1;
     tmp.resize(need + 1, 1.5);
-    // up-sweep: scan tiles at every level
-    const int32_t* cur_in  = in;
-    int32_t*       cur_out = out;
-    for(size_t k = 0; k < level_n.size(); ++k)
+    auto scan = [&](auto& self, const int32_t* src, int32_t* dst, int64_t m, int32_t* room) -> void
     {
-        int64_t nk = level_n[k];
-        int64_t t  = (nk + SCAN_TILE - 1) / SCAN_TILE;
-        k_scan_tiles<<<(unsigned)t, SCAN_BLOCK, 0, st>>>(cur_in, cur_out, nk, tmp.data() + off_sums[k]);
-        B2S_CHECK_LAUNCH();
-        cur_in  = tmp.data() + off_sums[k];
-        cur_out = tmp.data() + off_scan[k];
-        if(t == 1)
+        const int64_t t    = tiles_of(m);
+        int32_t*      sums = room;
+        int32_t*      offs = nullptr;
+        if(t > 1)
         {
-            // single tile: its exclusive scan is zero
-            B2S_CUDA(cudaMemsetAsync(cur_out, 0, sizeof(int32_t), st));
-            break;
+            k_scan_sums<<<(unsigned)t, SCAN_BLOCK, 0, st>>>(src, m, sums);
+            B2S_CHECK_LAUNCH();
+            if(t > SCAN_DIRECT_TILES)
+            {
+                offs = room + t;
+                self(self, sums, offs, t, room + 2 * t + 1);
+            }
         }
-    }
-    // down-sweep: add scanned tile offsets
-    for(int k = (int)level_n.size() - 1; k >= 0; --k)
-    {
-        int64_t nk = level_n[k];
-        int64_t t  = (nk + SCAN_TILE - 1) / SCAN_TILE;
-        if(t == 1)
-            continue;
-        int32_t* target = (k == 0) ? out : tmp.data() + off_scan[k - 1];
-        k_scan_add<<<(unsigned)t, SCAN_BLOCK, 0, st>>>(target, nk, tmp.data() + off_scan[k]);
+        k_scan_tiles<<<(unsigned)t, SCAN_BLOCK, 0, st>>>(src, dst, m, sums, offs);
         B2S_CHECK_LAUNCH();
-    }
-    (void)tiles;
-    k_write_total<<<1, 32, 0, st>>>(out, n, in, nullptr, 0);
-    B2S_CHECK_LAUNCH();
+    };
+    scan(scan, in, out, n, tmp.data());
 }
 
 namespace
@@ -199,9 +204,10 @@ __global__ void k_count_rows(const int32_t* __restrict__ rows, const int32_t* __
 }
 
 // (column, source) of every kept triplet into its row's bucket; the lanes of
-// a row take consecutive places from one atomic of the lowest of them
+// a row take consecutive places from one atomic of the lowest of them, which
+// counts row_count back down
 __global__ void k_scatter_rows(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols, int64_t T,
-                               int32_t nb, const int32_t* __restrict__ row_start, int32_t* __restrict__ row_fill,
+                               int32_t nb, const int32_t* __restrict__ row_start, int32_t* __restrict__ row_count,
                                int2* __restrict__ bucket, int* err)
 {
     const int     lane   = threadIdx.x & 31;
@@ -226,12 +232,12 @@ __global__ void k_scatter_rows(const int32_t* __restrict__ rows, const int32_t* 
         const int      leader = __ffs(peers) - 1;
         int32_t        pos    = 0;
         if(ok && lane == leader)
-            pos = atomicAdd(&row_fill[r], __popc(peers));
+            pos = atomicSub(&row_count[r], __popc(peers)) - __popc(peers);
         pos = __shfl_sync(0xffffffffu, pos, leader);
         if(!ok)
             continue;
         const int32_t k = pos + __popc(peers & ((1u << lane) - 1u));
-        if(k >= len)
+        if(k < 0 || k >= len)
         {
             atomicOr(err, DERR_ROW_OVERFLOW);
             continue;
@@ -251,7 +257,8 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_sort_rows(int32_t nb, const int32
                                                          const int2* __restrict__ bucket,
                                                          int32_t* __restrict__ sorted_col,
                                                          int32_t* __restrict__ sorted_src,
-                                                         int32_t* __restrict__ uniq_count, int32_t* long_rows)
+                                                         int32_t* __restrict__ uniq_count, int32_t* long_rows,
+                                                         int32_t* n_long)
 {
     __shared__ int32_t s_col[ASM_BLOCK / 32][ROW_CAP];
     __shared__ int32_t s_src[ASM_BLOCK / 32][ROW_CAP];
@@ -376,7 +383,7 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_sort_rows(int32_t nb, const int32
         {
             // longer than a warp's shared memory: sorted by k_sort_long_rows
             if(lane == 0)
-                long_rows[1 + atomicAdd(long_rows, 1)] = (int32_t)r;
+                long_rows[atomicAdd(n_long, 1)] = (int32_t)r;
             continue;
         }
 #pragma unroll
@@ -432,16 +439,17 @@ __device__ __forceinline__ void sort_tile(uint64_t* s_key, int n)
 }
 
 __global__ void __launch_bounds__(LONG_THREADS) k_sort_long_rows(const int32_t* __restrict__ long_rows,
+                                                                 const int32_t* __restrict__ n_rows,
                                                                  const int32_t* __restrict__ row_start, int2* bucket,
                                                                  int32_t* sorted_col, int32_t* sorted_src,
                                                                  int32_t* __restrict__ uniq_count)
 {
     __shared__ uint64_t s_key[LONG_TILE];
     __shared__ int      s_heads[LONG_THREADS / 32];
-    const int n_long = long_rows[0];
+    const int n_long = *n_rows;
     for(int e = blockIdx.x; e < n_long; e += gridDim.x)
     {
-        const int32_t r = long_rows[1 + e], beg = row_start[r], L = row_start[r + 1] - beg;
+        const int32_t r = long_rows[e], beg = row_start[r], L = row_start[r + 1] - beg;
         const bool    many = L > LONG_TILE;
         // sort the tiles (one tile: straight to the result; several: in place)
         for(int t0 = 0; t0 < L; t0 += LONG_TILE)
@@ -536,8 +544,10 @@ __global__ void __launch_bounds__(LONG_THREADS) k_sort_long_rows(const int32_t* 
 
 // One warp per row: every run of equal columns becomes one slot of the
 // block-upper BSR: its row, column and the position of its first source in
-// the sorted order (run_start; run_start[U] = T written by the caller).
-__global__ void __launch_bounds__(ASM_BLOCK) k_mark_runs(int32_t nb, const int32_t* __restrict__ row_start,
+// the sorted order (run_start; run_start[U] = the kept triplets). The stream's
+// padding past U gets row -1 / column 0 (never used: every reader checks).
+__global__ void __launch_bounds__(ASM_BLOCK) k_mark_runs(int32_t nb, int64_t U, int64_t S,
+                                                         const int32_t* __restrict__ row_start,
                                                          const int32_t* __restrict__ sorted_col,
                                                          const int32_t* __restrict__ rowptr,
                                                          int32_t* __restrict__ out_rows, int32_t* __restrict__ out_cols,
@@ -546,6 +556,16 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_mark_runs(int32_t nb, const int32
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int warps_total = gridDim.x * (ASM_BLOCK / 32);
+    if(blockIdx.x == 0 && threadIdx.x < 32)
+    {
+        if(U + lane < S)
+        {
+            out_rows[U + lane] = -1;
+            out_cols[U + lane] = 0;
+        }
+        if(lane == 0)
+            run_start[U] = row_start[nb];
+    }
     for(int32_t r = blockIdx.x * (ASM_BLOCK / 32) + w; r < nb; r += warps_total)
     {
         const int32_t beg = row_start[r], L = row_start[r + 1] - beg;
@@ -582,6 +602,7 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_mark_runs(int32_t nb, const int32
 // the same for the rows listed by k_sort_rows, one CTA per row: a warp stepping
 // through 20,000 pairs 32 at a time is a chain of 640 dependent rounds
 __global__ void __launch_bounds__(LONG_THREADS) k_mark_long_rows(const int32_t* __restrict__ long_rows,
+                                                                 const int32_t* __restrict__ n_rows,
                                                                  const int32_t* __restrict__ row_start,
                                                                  const int32_t* __restrict__ sorted_col,
                                                                  const int32_t* __restrict__ rowptr,
@@ -591,10 +612,10 @@ __global__ void __launch_bounds__(LONG_THREADS) k_mark_long_rows(const int32_t* 
                                                                  int32_t* __restrict__ diag_index)
 {
     __shared__ int s_warp[LONG_THREADS / 32];
-    const int      n_long = long_rows[0], lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int      n_long = *n_rows, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for(int e = blockIdx.x; e < n_long; e += gridDim.x)
     {
-        const int32_t r = long_rows[1 + e], beg = row_start[r], L = row_start[r + 1] - beg;
+        const int32_t r = long_rows[e], beg = row_start[r], L = row_start[r + 1] - beg;
         int64_t       o0 = rowptr[r];
         if(threadIdx.x == 0)
             diag_index[r] = sorted_col[beg] == r ? (int32_t)o0 : -1;
@@ -790,7 +811,7 @@ __global__ void k_publish(const int32_t* nnz, const int* err, const int32_t* n_l
 {
     info[0] = *nnz;
     info[1] = *err;
-    info[2] = n_long ? *n_long : 0;
+    info[2] = *n_long;
 }
 
 int asm_grid(int64_t work, int block)
@@ -862,43 +883,39 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
     M.valid             = false;
     M.generation += 1;
     M.nb                = nb;
-    w.err.resize(1);
-    B2S_CUDA(cudaMemsetAsync(w.err.data(), 0, sizeof(int), st));
-    w.row_count.resize((size_t)nb + 1, 1.25);
+    // row counts, then the error bits and the number of long rows: one fill
+    w.row_count.resize((size_t)nb + 3, 1.25);
     w.row_start.resize((size_t)nb + 1, 1.25);
-    w.row_fill.resize((size_t)nb + 1, 1.25);
+    int* const     err    = w.row_count.data() + nb + 1;
+    int32_t* const n_long_dev = w.row_count.data() + nb + 2;
     w.uniq_count.resize((size_t)nb + 1, 1.25);
     M.rowptr.resize((size_t)nb + 1, 1.25);
     M.diag_index.resize((size_t)std::max(nb, 1), 1.25);
-    B2S_CUDA(cudaMemsetAsync(w.row_count.data(), 0, sizeof(int32_t) * ((size_t)nb + 1), st));
-    B2S_CUDA(cudaMemsetAsync(w.row_fill.data(), 0, sizeof(int32_t) * ((size_t)nb + 1), st));
+    B2S_CUDA(cudaMemsetAsync(w.row_count.data(), 0, sizeof(int32_t) * ((size_t)nb + 3), st));
     if(T > 0)
     {
         w.bucket.resize(T, 1.25);
         w.sorted_col.resize(T, 1.25);
         w.sorted_src.resize(T, 1.25);
-        k_count_rows<<<asm_grid(T, ASM_BLOCK), ASM_BLOCK, 0, st>>>(rows, cols, T, nb, w.row_count.data(),
-                                                                   w.err.data());
+        k_count_rows<<<asm_grid(T, ASM_BLOCK), ASM_BLOCK, 0, st>>>(rows, cols, T, nb, w.row_count.data(), err);
         B2S_CHECK_LAUNCH();
     }
     exclusive_scan(s, w.row_count.data(), w.row_start.data(), nb, w.scan_tmp);
     if(T > 0)
     {
         k_scatter_rows<<<asm_grid(T, ASM_BLOCK), ASM_BLOCK, 0, st>>>(rows, cols, T, nb, w.row_start.data(),
-                                                                     w.row_fill.data(), w.bucket.data(),
-                                                                     w.err.data());
+                                                                     w.row_count.data(), w.bucket.data(), err);
         B2S_CHECK_LAUNCH();
     }
     if(nb > 0)
     {
-        w.long_rows.resize((size_t)nb + 1, 1.25);
-        B2S_CUDA(cudaMemsetAsync(w.long_rows.data(), 0, sizeof(int32_t), st));
+        w.long_rows.resize((size_t)nb, 1.25);
         k_sort_rows<<<asm_grid((int64_t)nb * 32, ASM_BLOCK), ASM_BLOCK, 0, st>>>(
             nb, w.row_start.data(), w.bucket.data(), w.sorted_col.data(),
-            w.sorted_src.data(), w.uniq_count.data(), w.long_rows.data());
+            w.sorted_src.data(), w.uniq_count.data(), w.long_rows.data(), n_long_dev);
         B2S_CHECK_LAUNCH();
-        // the long rows (count in long_rows[0], read on the device)
-        k_sort_long_rows<<<NUM_SMS_HINT * 2, LONG_THREADS, 0, st>>>(w.long_rows.data(), w.row_start.data(),
+        // the long rows (their number is read on the device)
+        k_sort_long_rows<<<NUM_SMS_HINT * 2, LONG_THREADS, 0, st>>>(w.long_rows.data(), n_long_dev, w.row_start.data(),
                                                                     w.bucket.data(), w.sorted_col.data(),
                                                                     w.sorted_src.data(), w.uniq_count.data());
         B2S_CHECK_LAUNCH();
@@ -909,7 +926,7 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
     // five coarse levels)
     if(!w.h_info)
         B2S_CUDA(cudaMallocHost(&w.h_info, 3 * sizeof(int32_t)));
-    k_publish<<<1, 1, 0, st>>>(M.rowptr.data() + nb, w.err.data(), nb > 0 ? w.long_rows.data() : nullptr, w.h_info);
+    k_publish<<<1, 1, 0, st>>>(M.rowptr.data() + nb, err, n_long_dev, w.h_info);
     B2S_CHECK_LAUNCH();
     B2S_CUDA(cudaStreamSynchronize(st));
     const int32_t U = w.h_info[0], n_long = w.h_info[2];
@@ -923,26 +940,21 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
     M.rows.resize(M.stride, 1.2);
     M.cols.resize(M.stride, 1.2);
     M.vals.resize((size_t)9 * M.stride, 1.2);
-    // padding past U: row -1 / col 0 (never used: every reader checks k < U)
-    B2S_CUDA(cudaMemsetAsync(M.rows.data() + U, 0xff, sizeof(int32_t) * (M.stride - U), st));
-    B2S_CUDA(cudaMemsetAsync(M.cols.data() + U, 0, sizeof(int32_t) * (M.stride - U), st));
     if(nb > 0)
     {
         // slots of the runs, then their sums (values as planes with stride M.stride)
         w.run_start.resize((size_t)U + 1, 1.2);
         k_mark_runs<<<asm_grid((int64_t)nb * 32, ASM_BLOCK), ASM_BLOCK, 0, st>>>(
-            nb, w.row_start.data(), w.sorted_col.data(), M.rowptr.data(), M.rows.data(), M.cols.data(),
+            nb, U, M.stride, w.row_start.data(), w.sorted_col.data(), M.rowptr.data(), M.rows.data(), M.cols.data(),
             w.run_start.data(), M.diag_index.data());
         B2S_CHECK_LAUNCH();
         if(n_long > 0)
         {
             k_mark_long_rows<<<std::min(n_long, NUM_SMS_HINT * 2), LONG_THREADS, 0, st>>>(
-                w.long_rows.data(), w.row_start.data(), w.sorted_col.data(), M.rowptr.data(), M.rows.data(),
-                M.cols.data(), w.run_start.data(), M.diag_index.data());
+                w.long_rows.data(), n_long_dev, w.row_start.data(), w.sorted_col.data(), M.rowptr.data(),
+                M.rows.data(), M.cols.data(), w.run_start.data(), M.diag_index.data());
             B2S_CHECK_LAUNCH();
         }
-        B2S_CUDA(cudaMemcpyAsync(w.run_start.data() + U, w.row_start.data() + nb, sizeof(int32_t),
-                                 cudaMemcpyDeviceToDevice, st));
         if(U > 0)
         {
             // one pass in block order (no grid-stride loop): the CTAs in
@@ -966,6 +978,11 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
                 B2S_CHECK_LAUNCH();
             }
         }
+    }
+    else
+    {
+        B2S_CUDA(cudaMemsetAsync(M.rows.data(), 0xff, sizeof(int32_t) * M.stride, st));
+        B2S_CUDA(cudaMemsetAsync(M.cols.data(), 0, sizeof(int32_t) * M.stride, st));
     }
     M.has_trank = false;
     if(spmv_tiles && U > 0)

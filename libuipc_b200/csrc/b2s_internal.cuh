@@ -140,11 +140,11 @@ struct Matrix
 // scratch of the assembly pipeline (reused across calls)
 struct AssemblyScratch
 {
-    DBuf<int32_t> row_count, row_start, row_fill, uniq_count;
+    DBuf<int32_t> row_count, row_start, uniq_count;
     DBuf<int2>    bucket;  // (column, source) of the kept triplets, bucketed by row
     DBuf<int32_t> sorted_col, sorted_src;
     DBuf<int32_t> run_start;  // [U+1] sorted position of each unique block's first source
-    DBuf<int32_t> long_rows;  // [1 + nb]: count, then the rows too long for one warp
+    DBuf<int32_t> long_rows;  // [nb] the rows too long for one warp
     DBuf<int32_t> long_runs;  // [1 + U]: count, then the blocks whose run is summed by a warp
     DBuf<int32_t> scan_tmp;
     DBuf<int>     err;
