@@ -33,14 +33,11 @@
 // BF16 tiles. A pivot that is not positive even in FP64 (an indefinite
 // cluster) is replaced by the diagonal entry it started from.
 #include "b2s_internal.cuh"
-#include "b2s_tma.cuh"
 
 #include <algorithm>
 
 namespace b2s
 {
-int* device_error_flag(b2s_solver* s);
-
 namespace
 {
 constexpr int    NI                = BANK * 3;  // 48 rows per cluster
@@ -68,24 +65,23 @@ __constant__ SymPairs c_sym_pairs = make_sym_pairs();
 
 // shared-memory geometry per type: row stride of the 48x48 matrix and of the
 // temporary tile (16-byte aligned rows, conflict-free 2x4 tile accesses),
-// warps per CTA
+// warps per CTA, CTAs per SM
 template <typename T>
 struct InvGeom;
 template <>
 struct InvGeom<float>
 {
-    static constexpr int LD = 52, TLD = 20, WARPS = 2;
+    static constexpr int LD = 52, TLD = 20, WARPS = 2, CTAS = 8;
 };
 template <>
 struct InvGeom<double>
 {
-    static constexpr int LD = 50, TLD = 18, WARPS = 1;
+    static constexpr int LD = 50, TLD = 18, WARPS = 1, CTAS = 8;
 };
 
 template <typename T>
 struct __align__(16) InvWarpSmem
 {
-    double stage[SYM * 9];     // the next cluster's FP64 Galerkin blocks (bulk copy)
     T S[NI * InvGeom<T>::LD];  // the cluster matrix, full symmetric storage
     T Tt[16 * InvGeom<T>::TLD];  // one temporary 16x16 tile
     T dinv[NI];                  // 1 / d_k of the factorisation
@@ -271,31 +267,42 @@ __constant__ TileOp c_xops[6] = {
 // Factorise and invert one cluster (the whole warp). Returns true when the
 // cluster is stiff (a pivot ratio below STIFF_PIVOT_RATIO, or a pivot that
 // is not positive).
-template <typename T, typename AfterScatter>
-__device__ bool invert_cluster(float* __restrict__ out, InvWarpSmem<T>& sm, const SymPairs& pairs, int lane,
-                               AfterScatter after_scatter)
+template <typename T>
+__device__ bool invert_cluster(const double* __restrict__ H, float* __restrict__ out, InvWarpSmem<T>& sm,
+                               const SymPairs& pairs, int lane)
 {
     constexpr int LD = InvGeom<T>::LD, TLD = InvGeom<T>::TLD;
     T*            S  = sm.S;
     auto          tile = [&](int I, int J) -> T* { return S + (16 * I) * LD + 16 * J; };
     const TileOwn own(lane);
 
-    // 0. scatter the staged blocks: block (a, b), a <= b, column-major
-    // component q = pb * 3 + pa is entry (3a + pa, 3b + pb); mirrored below
-    // the diagonal for a < b
-    const double* H = sm.stage;
-    for(int e = lane; e < SYM * 9; e += 32)
+    // 0. scatter the blocks: block (a, b), a <= b, column-major component
+    // q = pb * 3 + pa is entry (3a + pa, 3b + pb); mirrored below the diagonal
+    // for a < b
+    constexpr int LOADS = 8;  // loads in flight per lane
+#pragma unroll 1
+    for(int e0 = lane; e0 < SYM * 9; e0 += 32 * LOADS)
     {
-        const int    blk = e / 9, q = e - 9 * blk;
-        const int    a = pairs.r[blk], b = pairs.c[blk];
-        const int    row = 3 * a + q % 3, col = 3 * b + q / 3;
-        const double v = H[e];
-        S[row * LD + col] = (T)v;
-        if(a != b)
-            S[col * LD + row] = (T)v;
+        double v[LOADS];
+#pragma unroll
+        for(int j = 0; j < LOADS; ++j)
+            v[j] = e0 + 32 * j < SYM * 9 ? __ldcs(H + e0 + 32 * j) : 0.0;
+#pragma unroll
+        for(int j = 0; j < LOADS; ++j)
+        {
+            const int e = e0 + 32 * j;
+            if(e < SYM * 9)
+            {
+                const int blk = e / 9, q = e - 9 * blk;
+                const int a = pairs.r[blk], b = pairs.c[blk];
+                const int row = 3 * a + q % 3, col = 3 * b + q / 3;
+                S[row * LD + col] = (T)v[j];
+                if(a != b)
+                    S[col * LD + row] = (T)v[j];
+            }
+        }
     }
     __syncwarp();
-    after_scatter();  // the stage is free: the next cluster's copy may start
     for(int i = lane; i < NI; i += 32)
     {
         T d = S[i * LD + i];
@@ -433,68 +440,43 @@ __device__ bool invert_cluster(float* __restrict__ out, InvWarpSmem<T>& sm, cons
 // One warp per cluster. list == nullptr: every cluster (grid-stride), the
 // stiffness flag of each written and, with `queue`, the stiff ones appended
 // to stiff_list for the FP64 pass. Otherwise the clusters list[0 ..
-// *list_count) (the FP64 pass over the stiff clusters). Each warp brings its
-// next cluster's Galerkin blocks (9,792 B) into shared memory by a bulk copy
-// (TMA) while it factorises the current one; a copy wait that runs out sets
-// DERR_TMA_TIMEOUT and the warp stops.
+// *list_count) (the FP64 pass over the stiff clusters). Bound by the latency of
+// the shuffle-and-reciprocal chain of the diagonal tiles, so by the warps per
+// SM: a cluster takes 11.7 KB of shared memory (FP32) and its blocks are read
+// straight into it, the next cluster's prefetched to L2 meanwhile. With the
+// blocks staged in shared memory (9.8 KB more) 10 warps fit an SM instead of
+// 16: 733 us for 37,388 clusters, against 598.
 template <typename T>
-__global__ void __launch_bounds__(InvGeom<T>::WARPS * 32)
+__global__ void __launch_bounds__(InvGeom<T>::WARPS * 32, InvGeom<T>::CTAS)
     k_cluster_inverse(int clusters, const double* __restrict__ hess, float* __restrict__ inv,
                       const int32_t* __restrict__ list, const int32_t* __restrict__ list_count,
                       uint8_t* __restrict__ stiff, int32_t* __restrict__ stiff_list, int32_t* __restrict__ stiff_count,
-                      int queue, int* err)
+                      int queue)
 {
-    constexpr uint32_t BYTES = SYM * 9 * sizeof(double);  // 9,792, a multiple of 16
+    constexpr int BYTES = SYM * 9 * sizeof(double);  // 9,792
     __shared__ InvWarpSmem<T> sm[InvGeom<T>::WARPS];
     __shared__ SymPairs       pairs;
-    __shared__ uint64_t       bar[InvGeom<T>::WARPS];
     for(int i = threadIdx.x; i < SYM; i += blockDim.x)
     {
         pairs.r[i] = c_sym_pairs.r[i];
         pairs.c[i] = c_sym_pairs.c[i];
     }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if(lane == 0)
-    {
-        mbar_init(&bar[w], 1);
-        mbar_fence_init();
-    }
     __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int gw = blockIdx.x * InvGeom<T>::WARPS + w;
     const int W  = gridDim.x * InvGeom<T>::WARPS;
     const int n  = list ? *list_count : clusters;
     auto cluster_at = [&](int i) { return list ? list[i] : i; };
-    if(gw < n && lane == 0)
-    {
-        mbar_arrive_expect_tx(&bar[w], BYTES);
-        bulk_copy_g2s(sm[w].stage, hess + (size_t)cluster_at(gw) * SYM * 9, BYTES, &bar[w]);
-    }
-    uint32_t phase = 0;
     for(int i = gw; i < n; i += W)
     {
-        const int  cl = cluster_at(i);
-        const bool ok = mbar_wait(&bar[w], phase, err, DERR_TMA_TIMEOUT);
-        phase ^= 1u;
-        if(!__all_sync(0xffffffffu, ok))
+        const int cl = cluster_at(i);
+        if(i + W < n)
         {
-            if(lane == 0)  // drain the copy that may still be in flight (bounded)
-                mbar_wait(&bar[w], phase ^ 1u, nullptr, 0);
-            __syncwarp();
-            return;
+            const char* next = reinterpret_cast<const char*>(hess + (size_t)cluster_at(i + W) * SYM * 9);
+            for(int o = 128 * lane; o < BYTES; o += 32 * 128)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(next + o));
         }
-        // invert_cluster reads the staged blocks first; the next copy goes
-        // out once they are in S (ordered by its first __syncwarp)
-        const bool st = invert_cluster<T>(inv + (size_t)cl * SYM * 9, sm[w], pairs, lane, [&]
-                                          {
-                                              if(lane == 0 && i + W < n)
-                                              {
-                                                  fence_proxy_async_smem();
-                                                  mbar_arrive_expect_tx(&bar[w], BYTES);
-                                                  bulk_copy_g2s(sm[w].stage,
-                                                                hess + (size_t)cluster_at(i + W) * SYM * 9, BYTES,
-                                                                &bar[w]);
-                                              }
-                                          });
+        const bool st = invert_cluster<T>(hess + (size_t)cl * SYM * 9, inv + (size_t)cl * SYM * 9, sm[w], pairs, lane);
         if(lane == 0 && !list)
         {
             stiff[cl] = st ? 1 : 0;
@@ -528,7 +510,6 @@ void mas_invert_clusters(b2s_solver* s, int mode)
     MasState&    M   = s->mas;
     cudaStream_t st  = s->stream;
     const int    C   = M.clusters;
-    int*         err = device_error_flag(s);
     M.stiff.resize(std::max(C, 1));
     M.stiff_list.resize(std::max(C, 1));
     M.stiff_count.resize(1);
@@ -539,13 +520,13 @@ void mas_invert_clusters(b2s_solver* s, int mode)
     {
         k_cluster_inverse<double><<<inverse_grid<double>(C), InvGeom<double>::WARPS * 32, 0, st>>>(
             C, M.hess.data(), M.inv.data(), nullptr, nullptr, M.stiff.data(), M.stiff_list.data(),
-            M.stiff_count.data(), 1, err);
+            M.stiff_count.data(), 1);
         B2S_CHECK_LAUNCH();
         return;
     }
     k_cluster_inverse<float><<<inverse_grid<float>(C), InvGeom<float>::WARPS * 32, 0, st>>>(
         C, M.hess.data(), M.inv.data(), nullptr, nullptr, M.stiff.data(), M.stiff_list.data(), M.stiff_count.data(),
-        1, err);
+        1);
     B2S_CHECK_LAUNCH();
     if(mode == B2S_INVERT_F32_ONLY)
         return;
@@ -553,7 +534,7 @@ void mas_invert_clusters(b2s_solver* s, int mode)
     // a small fixed grid walks the list (it returns at once when it is empty)
     const int grid = std::min(inverse_grid<double>(C), 2 * NUM_SMS_HINT);
     k_cluster_inverse<double><<<grid, InvGeom<double>::WARPS * 32, 0, st>>>(
-        C, M.hess.data(), M.inv.data(), M.stiff_list.data(), M.stiff_count.data(), nullptr, nullptr, nullptr, 0, err);
+        C, M.hess.data(), M.inv.data(), M.stiff_list.data(), M.stiff_count.data(), nullptr, nullptr, nullptr, 0);
     B2S_CHECK_LAUNCH();
 }
 }  // namespace b2s
