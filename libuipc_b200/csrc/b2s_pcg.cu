@@ -52,11 +52,13 @@ int vec_grid(int64_t n)
 __device__ __forceinline__ bool frozen(const PcgScalars* sc) { return sc && sc->converged != 0; }
 
 // 3x3 block Jacobi inverses (row-major), identity where the diagonal block is
-// missing or singular
-__global__ void k_diag_inverse(int32_t nb, const int32_t* diag_index, const double* vals, int64_t U, double* dinv)
+// missing or singular. With r2p (MAS on rows off .. off + vn): only the rows
+// outside its partition, the others' inverses are never applied
+__global__ void k_diag_inverse(int32_t nb, const int32_t* diag_index, const double* vals, int64_t U, double* dinv,
+                               const int32_t* __restrict__ r2p, int off, int vn)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= nb)
+    if(i >= nb || (r2p && i >= off && i < off + vn && r2p[i - off] >= 0))
         return;
     const int k = diag_index[i];
     double*   o = dinv + (size_t)i * 9;
@@ -520,17 +522,17 @@ void precond_assemble(b2s_solver* s, int kind, int invert_mode)
     cudaStream_t st = s->stream;
     const Matrix& A = s->A;
     s->dinv.resize((size_t)std::max(A.nb, 1) * 9);
+    const bool mas = kind == B2S_PRECOND_MAS;
+    B2S_REQUIRE(!mas || s->mas.initialized, B2S_ERR_STATE, "MAS preconditioner requested before b2s_mas_init");
     if(A.nb > 0)
     {
         k_diag_inverse<<<grid_for(A.nb, 256), 256, 0, st>>>(A.nb, A.diag_index.data(), A.vals.data(), A.stride,
-                                                            s->dinv.data());
+                                                            s->dinv.data(), mas ? s->mas.r2p.data() : nullptr,
+                                                            s->mas.offset, s->mas.vn);
         B2S_CHECK_LAUNCH();
     }
-    if(kind == B2S_PRECOND_MAS)
-    {
-        B2S_REQUIRE(s->mas.initialized, B2S_ERR_STATE, "MAS preconditioner requested before b2s_mas_init");
+    if(mas)
         mas_assemble(s, invert_mode);
-    }
     if(s->abd_n > 0)
     {
         B2S_REQUIRE(s->abd_offset + 4 * (int64_t)s->abd_n <= A.nb, B2S_ERR_ARGUMENT,
