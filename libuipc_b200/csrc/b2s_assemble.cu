@@ -251,17 +251,21 @@ __device__ __forceinline__ bool key_less(int32_t ca, int32_t sa, int32_t cb, int
     return ca < cb || (ca == cb && sa < sb);
 }
 
-// One warp per row: rank every (col, src) pair of the row by counting the
-// pairs that order before it, write the sorted row and its unique-column count.
+// One warp per row: the row's (col, src) pairs sorted; out go the sources in
+// that order (sorted_src) and, in place of the row's pairs from its first on,
+// each distinct column with the position of its first source, and their number
+// (uniq_count). The columns of all pairs are not written: marking the
+// runs from them in a second pass cost 126 MB out and in on 31 M triplets
+// (sort + mark 544 us; 454 now).
 __global__ void __launch_bounds__(ASM_BLOCK) k_sort_rows(int32_t nb, const int32_t* __restrict__ row_start,
-                                                         const int2* __restrict__ bucket,
-                                                         int32_t* __restrict__ sorted_col,
+                                                         int2* bucket,
                                                          int32_t* __restrict__ sorted_src,
                                                          int32_t* __restrict__ uniq_count, int32_t* long_rows,
                                                          int32_t* n_long)
 {
     __shared__ int32_t s_col[ASM_BLOCK / 32][ROW_CAP];
     __shared__ int32_t s_src[ASM_BLOCK / 32][ROW_CAP];
+    __shared__ int32_t s_sorted[ASM_BLOCK / 32][ROW_CAP];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int warps_total = gridDim.x * (ASM_BLOCK / 32);
     for(int32_t r = blockIdx.x * (ASM_BLOCK / 32) + w; r < nb; r += warps_total)
@@ -288,12 +292,13 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_sort_rows(int32_t nb, const int32
                     key = keep_min ? (key < other ? key : other) : (key < other ? other : key);
                 }
             const uint64_t prev = __shfl_up_sync(0xffffffffu, key, 1);
+            const bool     head = lane < L && (lane == 0 || (prev >> 32) != (key >> 32));
+            const unsigned hm   = __ballot_sync(0xffffffffu, head);
             if(lane < L)
-            {
-                sorted_col[beg + lane] = (int32_t)(key >> 32);
                 sorted_src[beg + lane] = (int32_t)(key & 0xFFFFFFFFull);
-                uniq = (lane == 0 || (prev >> 32) != (key >> 32)) ? 1 : 0;
-            }
+            if(head)
+                bucket[beg + __popc(hm & ((1u << lane) - 1u))] = make_int2((int32_t)(key >> 32), beg + lane);
+            uniq = __popc(hm);
         }
         else if(L <= 64)
         {
@@ -345,12 +350,13 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_sort_rows(int32_t nb, const int32
                 const int      p    = j * 32 + lane;
                 const uint64_t up1  = __shfl_up_sync(0xffffffffu, key[j], 1);
                 const uint64_t prev = lane > 0 ? up1 : (j == 1 ? last0 : ~0ull);
+                const bool     head = p < L && (p == 0 || (prev >> 32) != (key[j] >> 32));
+                const unsigned hm   = __ballot_sync(0xffffffffu, head);
                 if(p < L)
-                {
-                    sorted_col[beg + p] = (int32_t)(key[j] >> 32);
                     sorted_src[beg + p] = (int32_t)(key[j] & 0xFFFFFFFFull);
-                    uniq += (p == 0 || (prev >> 32) != (key[j] >> 32)) ? 1 : 0;
-                }
+                if(head)
+                    bucket[beg + uniq + __popc(hm & ((1u << lane) - 1u))] = make_int2((int32_t)(key[j] >> 32), beg + p);
+                uniq += __popc(hm);
             }
         }
         else if(L <= ROW_CAP)
@@ -365,17 +371,21 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_sort_rows(int32_t nb, const int32
             for(int k = lane; k < L; k += 32)
             {
                 const int32_t c = s_col[w][k], sr = s_src[w][k];
-                int rank = 0, head = 1;
+                int           rank = 0;
                 for(int q = 0; q < L; ++q)
-                {
-                    const int32_t cq = s_col[w][q], sq = s_src[w][q];
-                    rank += key_less(cq, sq, c, sr) ? 1 : 0;
-                    if(cq == c && sq < sr)
-                        head = 0;
-                }
-                sorted_col[beg + rank] = c;
+                    rank += key_less(s_col[w][q], s_src[w][q], c, sr) ? 1 : 0;
                 sorted_src[beg + rank] = sr;
-                uniq += head;
+                s_sorted[w][rank]      = c;
+            }
+            __syncwarp();
+            for(int base = 0; base < L; base += 32)
+            {
+                const int      p    = base + lane;
+                const bool     head = p < L && (p == 0 || s_sorted[w][p] != s_sorted[w][p - 1]);
+                const unsigned hm   = __ballot_sync(0xffffffffu, head);
+                if(head)
+                    bucket[beg + uniq + __popc(hm & ((1u << lane) - 1u))] = make_int2(s_sorted[w][p], beg + p);
+                uniq += __popc(hm);
             }
             __syncwarp();
         }
@@ -386,9 +396,6 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_sort_rows(int32_t nb, const int32
                 long_rows[atomicAdd(n_long, 1)] = (int32_t)r;
             continue;
         }
-#pragma unroll
-        for(int o = 16; o > 0; o >>= 1)
-            uniq += __shfl_xor_sync(0xffffffffu, uniq, o);
         if(lane == 0)
             uniq_count[r] = uniq;
     }
@@ -519,131 +526,103 @@ __global__ void __launch_bounds__(LONG_THREADS) k_sort_long_rows(const int32_t* 
                     }
             }
         __syncthreads();  // the sorted row is visible to the CTA
-        // the row's number of distinct columns
-        int heads = 0;
-        for(int i = threadIdx.x; i < L; i += LONG_THREADS)
-            heads += (i == 0 || sorted_col[beg + i] != sorted_col[beg + i - 1]) ? 1 : 0;
-#pragma unroll
-        for(int o = 16; o > 0; o >>= 1)
-            heads += __shfl_xor_sync(0xffffffffu, heads, o);
-        if((threadIdx.x & 31) == 0)
-            s_heads[threadIdx.x >> 5] = heads;
-        __syncthreads();
-        if(threadIdx.x < 32)
+        // the row's distinct columns, in order
+        int before = 0;
+        for(int base = 0; base < L; base += LONG_THREADS)
         {
-            int h = s_heads[threadIdx.x];
+            const int      i    = base + (int)threadIdx.x;
+            const int32_t  c    = i < L ? sorted_col[beg + i] : 0;
+            const bool     head = i < L && (i == 0 || sorted_col[beg + i - 1] != c);
+            const unsigned hm   = __ballot_sync(0xffffffffu, head);
+            __syncthreads();  // s_heads of the previous round is read
+            if((threadIdx.x & 31) == 0)
+                s_heads[threadIdx.x >> 5] = __popc(hm);
+            __syncthreads();
+            int mine = before;
 #pragma unroll
-            for(int o = 16; o > 0; o >>= 1)
-                h += __shfl_xor_sync(0xffffffffu, h, o);
-            if(threadIdx.x == 0)
-                uniq_count[r] = h;
+            for(int q = 0; q < LONG_THREADS / 32; ++q)
+            {
+                mine += q < (int)(threadIdx.x >> 5) ? s_heads[q] : 0;
+                before += s_heads[q];
+            }
+            if(head)
+                bucket[beg + mine + __popc(hm & ((1u << (threadIdx.x & 31)) - 1u))] = make_int2(c, beg + i);
         }
+        if(threadIdx.x == 0)
+            uniq_count[r] = before;
         __syncthreads();  // s_heads and s_key are free for the next row
     }
 }
 
-// One warp per row: every run of equal columns becomes one slot of the
-// block-upper BSR: its row, column and the position of its first source in
-// the sorted order (run_start; run_start[U] = the kept triplets). The stream's
-// padding past U gets row -1 / column 0 (never used: every reader checks).
+// One warp per row: the row's runs become slots of the block-upper BSR: row,
+// column and the position of the first source in the sorted order (run_start;
+// run_start[U] = the kept triplets). The stream's padding past U gets row -1 /
+// column 0 (never used: every reader checks). Rows of more than ROW_CAP pairs,
+// which may have thousands of blocks, are k_mark_long_rows's.
 __global__ void __launch_bounds__(ASM_BLOCK) k_mark_runs(int32_t nb, int64_t U, int64_t S,
                                                          const int32_t* __restrict__ row_start,
-                                                         const int32_t* __restrict__ sorted_col,
+                                                         const int2* __restrict__ runs,
                                                          const int32_t* __restrict__ rowptr,
                                                          int32_t* __restrict__ out_rows, int32_t* __restrict__ out_cols,
                                                          int32_t* __restrict__ run_start,
                                                          int32_t* __restrict__ diag_index)
 {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int warps_total = gridDim.x * (ASM_BLOCK / 32);
+    // eight lanes per row: a mesh row has about eight blocks
+    constexpr int LANES = 8;
+    const int     lane = threadIdx.x % LANES, groups = gridDim.x * (ASM_BLOCK / LANES);
     if(blockIdx.x == 0 && threadIdx.x < 32)
     {
-        if(U + lane < S)
+        if(U + threadIdx.x < S)
         {
-            out_rows[U + lane] = -1;
-            out_cols[U + lane] = 0;
+            out_rows[U + threadIdx.x] = -1;
+            out_cols[U + threadIdx.x] = 0;
         }
-        if(lane == 0)
+        if(threadIdx.x == 0)
             run_start[U] = row_start[nb];
     }
-    for(int32_t r = blockIdx.x * (ASM_BLOCK / 32) + w; r < nb; r += warps_total)
+    for(int32_t r = blockIdx.x * (ASM_BLOCK / LANES) + threadIdx.x / LANES; r < nb; r += groups)
     {
-        const int32_t beg = row_start[r], L = row_start[r + 1] - beg;
-        if(L > ROW_CAP)
-            continue;  // k_mark_long_rows
-        const int32_t obeg = rowptr[r];
-        int           heads_before = 0;
-        for(int base = 0; base < L; base += 32)
+        const int32_t beg = row_start[r], o = rowptr[r], n = rowptr[r + 1] - o;
+        if(row_start[r + 1] - beg > ROW_CAP)
+            continue;
+        int32_t c0 = -1;
+        for(int k = lane; k < n; k += LANES)
         {
-            const int k = base + lane;
-            bool head = false;
-            int32_t c = 0;
-            if(k < L)
-            {
-                c    = sorted_col[beg + k];
-                head = (k == 0) || (sorted_col[beg + k - 1] != c);
-            }
-            const unsigned hm   = __ballot_sync(0xffffffffu, head);
-            const int      slot = heads_before + __popc(hm & ((1u << lane) - 1u));
-            if(head)
-            {
-                const int64_t o = (int64_t)obeg + slot;
-                out_rows[o]  = r;
-                out_cols[o]  = c;
-                run_start[o] = beg + k;
-            }
-            heads_before += __popc(hm);
+            const int2 q     = runs[beg + k];
+            out_rows[o + k]  = r;
+            out_cols[o + k]  = q.x;
+            run_start[o + k] = q.y;
+            if(k == 0)
+                c0 = q.x;
         }
         if(lane == 0)
-            diag_index[r] = (L > 0 && sorted_col[beg] == r) ? obeg : -1;
+            diag_index[r] = c0 == r ? o : -1;
     }
 }
 
-// the same for the rows listed by k_sort_rows, one CTA per row: a warp stepping
-// through 20,000 pairs 32 at a time is a chain of 640 dependent rounds
+// the rows listed by k_sort_rows, one CTA per row
 __global__ void __launch_bounds__(LONG_THREADS) k_mark_long_rows(const int32_t* __restrict__ long_rows,
                                                                  const int32_t* __restrict__ n_rows,
                                                                  const int32_t* __restrict__ row_start,
-                                                                 const int32_t* __restrict__ sorted_col,
+                                                                 const int2* __restrict__ runs,
                                                                  const int32_t* __restrict__ rowptr,
                                                                  int32_t* __restrict__ out_rows,
                                                                  int32_t* __restrict__ out_cols,
                                                                  int32_t* __restrict__ run_start,
                                                                  int32_t* __restrict__ diag_index)
 {
-    __shared__ int s_warp[LONG_THREADS / 32];
-    const int      n_long = *n_rows, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int n_long = *n_rows;
     for(int e = blockIdx.x; e < n_long; e += gridDim.x)
     {
-        const int32_t r = long_rows[e], beg = row_start[r], L = row_start[r + 1] - beg;
-        int64_t       o0 = rowptr[r];
-        if(threadIdx.x == 0)
-            diag_index[r] = sorted_col[beg] == r ? (int32_t)o0 : -1;
-        for(int base = 0; base < L; base += LONG_THREADS)
+        const int32_t r = long_rows[e], beg = row_start[r], o = rowptr[r], n = rowptr[r + 1] - o;
+        for(int k = threadIdx.x; k < n; k += LONG_THREADS)
         {
-            const int     k    = base + (int)threadIdx.x;
-            const int32_t c    = k < L ? sorted_col[beg + k] : 0;
-            const bool    head = k < L && (k == 0 || sorted_col[beg + k - 1] != c);
-            const unsigned hm  = __ballot_sync(0xffffffffu, head);
-            __syncthreads();  // s_warp of the previous round is read
-            if(lane == 0)
-                s_warp[w] = __popc(hm);
-            __syncthreads();
-            int before = 0, all = 0;
-#pragma unroll
-            for(int q = 0; q < LONG_THREADS / 32; ++q)
-            {
-                before += q < w ? s_warp[q] : 0;
-                all += s_warp[q];
-            }
-            if(head)
-            {
-                const int64_t o = o0 + before + __popc(hm & ((1u << lane) - 1u));
-                out_rows[o]     = r;
-                out_cols[o]     = c;
-                run_start[o]    = beg + k;
-            }
-            o0 += all;
+            const int2 q     = runs[beg + k];
+            out_rows[o + k]  = r;
+            out_cols[o + k]  = q.x;
+            run_start[o + k] = q.y;
+            if(k == 0)
+                diag_index[r] = q.x == r ? o : -1;
         }
     }
 }
@@ -911,8 +890,8 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
     {
         w.long_rows.resize((size_t)nb, 1.25);
         k_sort_rows<<<asm_grid((int64_t)nb * 32, ASM_BLOCK), ASM_BLOCK, 0, st>>>(
-            nb, w.row_start.data(), w.bucket.data(), w.sorted_col.data(),
-            w.sorted_src.data(), w.uniq_count.data(), w.long_rows.data(), n_long_dev);
+            nb, w.row_start.data(), w.bucket.data(), w.sorted_src.data(), w.uniq_count.data(), w.long_rows.data(),
+            n_long_dev);
         B2S_CHECK_LAUNCH();
         // the long rows (their number is read on the device)
         k_sort_long_rows<<<NUM_SMS_HINT * 2, LONG_THREADS, 0, st>>>(w.long_rows.data(), n_long_dev, w.row_start.data(),
@@ -944,15 +923,15 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
     {
         // slots of the runs, then their sums (values as planes with stride M.stride)
         w.run_start.resize((size_t)U + 1, 1.2);
-        k_mark_runs<<<asm_grid((int64_t)nb * 32, ASM_BLOCK), ASM_BLOCK, 0, st>>>(
-            nb, U, M.stride, w.row_start.data(), w.sorted_col.data(), M.rowptr.data(), M.rows.data(), M.cols.data(),
+        k_mark_runs<<<asm_grid((int64_t)nb * 8, ASM_BLOCK), ASM_BLOCK, 0, st>>>(
+            nb, U, M.stride, w.row_start.data(), w.bucket.data(), M.rowptr.data(), M.rows.data(), M.cols.data(),
             w.run_start.data(), M.diag_index.data());
         B2S_CHECK_LAUNCH();
         if(n_long > 0)
         {
             k_mark_long_rows<<<std::min(n_long, NUM_SMS_HINT * 2), LONG_THREADS, 0, st>>>(
-                w.long_rows.data(), n_long_dev, w.row_start.data(), w.sorted_col.data(), M.rowptr.data(),
-                M.rows.data(), M.cols.data(), w.run_start.data(), M.diag_index.data());
+                w.long_rows.data(), n_long_dev, w.row_start.data(), w.bucket.data(), M.rowptr.data(), M.rows.data(),
+                M.cols.data(), w.run_start.data(), M.diag_index.data());
             B2S_CHECK_LAUNCH();
         }
         if(U > 0)

@@ -141,8 +141,8 @@ struct Matrix
 struct AssemblyScratch
 {
     DBuf<int32_t> row_count, row_start, uniq_count;
-    DBuf<int2>    bucket;  // (column, source) of the kept triplets, bucketed by row
-    DBuf<int32_t> sorted_col, sorted_src;
+    DBuf<int2>    bucket;  // (column, source) of the kept triplets by row; once sorted, (column, first position) of its runs
+    DBuf<int32_t> sorted_col, sorted_src;  // (columns of the long rows only)
     DBuf<int32_t> run_start;  // [U+1] sorted position of each unique block's first source
     DBuf<int32_t> long_rows;  // [nb] the rows too long for one warp
     DBuf<int32_t> long_runs;  // [1 + U]: count, then the blocks whose run is summed by a warp
