@@ -125,6 +125,8 @@ int b2s_destroy(b2s_solver* s)
         cudaFreeHost(s->pcg.h_sc);
     if(s->asmb.h_info)
         cudaFreeHost(s->asmb.h_info);
+    if(s->h_back)
+        cudaFreeHost(s->h_back);
     if(s->ev_begin)
         cudaEventDestroy(s->ev_begin);
     if(s->ev_end)
@@ -242,11 +244,7 @@ int b2s_spmv(b2s_solver* s, const double* x, double* y, double* h_dot)
                        B2S_REQUIRE(x && y, B2S_ERR_ARGUMENT, "null vector");
                        s->dot_out.resize(4);
                        b2s::spmv_f64(s, s->A, x, y, h_dot ? s->dot_out.data() : nullptr);
-                       b2s::check_device_errors(s);
-                       if(h_dot)
-                           B2S_CUDA(cudaMemcpyAsync(h_dot, s->dot_out.data(), sizeof(double), cudaMemcpyDeviceToHost,
-                                                    s->stream));
-                       B2S_CUDA(cudaStreamSynchronize(s->stream));
+                       b2s::read_back(s, s->dot_out.data(), h_dot ? 1 : 0, h_dot);
                    });
 }
 
@@ -259,10 +257,7 @@ int b2s_spmv_mixed(b2s_solver* s, const float* x, float* y, double* h_dot)
                        B2S_REQUIRE(x && y, B2S_ERR_ARGUMENT, "null vector");
                        s->dot_out.resize(4);
                        b2s::spmv_mixed(s, x, y, s->dot_out.data());
-                       if(h_dot)
-                           B2S_CUDA(cudaMemcpyAsync(h_dot, s->dot_out.data(), sizeof(double), cudaMemcpyDeviceToHost,
-                                                    s->stream));
-                       B2S_CUDA(cudaStreamSynchronize(s->stream));
+                       b2s::read_back(s, s->dot_out.data(), h_dot ? 1 : 0, h_dot);
                    });
 }
 

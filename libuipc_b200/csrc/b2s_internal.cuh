@@ -212,6 +212,14 @@ struct PcgScalars
     long long max_iter;
 };
 
+// scalars on their way to the host (pinned, written by the device)
+constexpr int READ_BACK = 64;
+struct ReadBack
+{
+    double v[READ_BACK];
+    int    err;
+};
+
 struct Reduction
 {
     DBuf<double>       partials;  // [2 * grid]
@@ -259,6 +267,7 @@ struct b2s_solver
     b2s::DBuf<double>    dot_out;
     b2s::Reduction       red;
     b2s::DBuf<int>       dev_err;  // DeviceError bits raised by kernels
+    b2s::ReadBack*       h_back = nullptr;  // pinned: the last read_back
     // the MAS apply's second stream: the coarse levels run on it beside the
     // fine level's products (forked from `stream` and joined back by events)
     cudaStream_t             mas_side = nullptr;
@@ -320,6 +329,9 @@ void precond_apply_mixed(b2s_solver* s, const float* r, float* z);
 void spmv_mixed(b2s_solver* s, const float* x, float* y, double* d_dot);
 double spmv_mixed_timing(b2s_solver* s, int launches);
 void check_device_errors(b2s_solver* s);
+// n <= READ_BACK doubles from the device into h, with the stream's work done
+// and its device errors raised
+void read_back(b2s_solver* s, const double* d, int n, double* h);
 
 // message of the last failed call made without a solver handle (read back
 // through b2s_last_error(NULL))

@@ -1419,8 +1419,7 @@ void ws_predict(b2s_solver* s, int mode, const double* b, int n_hist, const doub
         dp.a[k] = dp.b[k] = b;
         launch_dots(s, n, dp, k + 1, W.dots.data() + 48);
         double hd[64];
-        B2S_CUDA(cudaMemcpyAsync(hd, W.dots.data(), sizeof(hd), cudaMemcpyDeviceToHost, st));
-        B2S_CUDA(cudaStreamSynchronize(st));
+        read_back(s, W.dots.data(), 64, hd);
         double G[WS_MAXC * WS_MAXC], gv[WS_MAXC], alpha[WS_MAXC] = {};
         for(int i = 0, q = 0; i < k; ++i)
         {
@@ -1468,8 +1467,7 @@ void ws_predict(b2s_solver* s, int mode, const double* b, int n_hist, const doub
             dc.b[2] = zb;
             launch_dots(s, n, dc, 3, W.dots.data() + 60);
             double h3[3];
-            B2S_CUDA(cudaMemcpyAsync(h3, W.dots.data() + 60, sizeof(h3), cudaMemcpyDeviceToHost, st));
-            B2S_CUDA(cudaStreamSynchronize(st));
+            read_back(s, W.dots.data() + 60, 3, h3);
             const double rr = h3[0], rz = h3[1], bz = h3[2];
             out.rel_res_tried = std::sqrt(rr / bb);
             out.rz_ratio    = bz > 0 ? rz / bz : INFINITY;

@@ -439,10 +439,15 @@ __global__ void k_residual_f32(int32_t nb, const double* __restrict__ b, const d
 }
 
 // between the 3-per-node FP32 vectors of the ABI and the padded ones
-__global__ void k_pad4(int32_t nb, const float* __restrict__ a, float* __restrict__ b)
+// (with `zero`, that padded vector is cleared in the same pass)
+__global__ void k_pad4(int32_t nb, const float* __restrict__ a, float* __restrict__ b, float* __restrict__ zero)
 {
     for(int64_t i = (int64_t)blockIdx.x * VEC_BLOCK + threadIdx.x; i < nb; i += (int64_t)gridDim.x * VEC_BLOCK)
+    {
         reinterpret_cast<float4*>(b)[i] = make_float4(a[3 * i], a[3 * i + 1], a[3 * i + 2], 0.0f);
+        if(zero)
+            reinterpret_cast<float4*>(zero)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
 }
 __global__ void k_unpad4(int32_t nb, const float* __restrict__ a, float* __restrict__ b)
 {
@@ -587,8 +592,7 @@ void precond_apply(b2s_solver* s, const double* r, double* z)
 {
     B2S_REQUIRE(s->precond_kind >= 0, B2S_ERR_STATE, "precond_apply before b2s_precond_assemble");
     precond_launch(s, s->precond_kind, r, z, nullptr, s->red);
-    check_device_errors(s);
-    B2S_CUDA(cudaStreamSynchronize(s->stream));
+    read_back(s, nullptr, 0, nullptr);
 }
 
 // z = P r queued on the solver's stream (no synchronisation, no error check)
@@ -714,8 +718,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
     launch_dot(s, P.r.data(), P.r.data(), n, s->dot_out.data() + 1);
     launch_dot(s, b, b, n, s->dot_out.data() + 2);
     double h3[3];
-    B2S_CUDA(cudaMemcpyAsync(h3, s->dot_out.data(), sizeof(h3), cudaMemcpyDeviceToHost, st));
-    B2S_CUDA(cudaStreamSynchronize(st));
+    read_back(s, s->dot_out.data(), 3, h3);
     double rz0 = h3[0];
     const double rr0 = h3[1], bb = h3[2];
     B2S_REQUIRE(std::isfinite(rr0) && std::isfinite(bb), B2S_ERR_NUMERIC,
@@ -740,8 +743,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
                                                             s->red.counter.data(), s->dot_out.data());
         B2S_CHECK_LAUNCH();
         double h2[2];
-        B2S_CUDA(cudaMemcpyAsync(h2, s->dot_out.data(), sizeof(h2), cudaMemcpyDeviceToHost, st));
-        B2S_CUDA(cudaStreamSynchronize(st));
+        read_back(s, s->dot_out.data(), 2, h2);
         return h2[1] > 0 ? std::sqrt(h2[0] / h2[1]) : 0.0;
     };
 
@@ -875,10 +877,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
             B2S_CHECK_LAUNCH();
             precond_launch(s, kind, P.r.data(), P.z.data(), nullptr, s->red);
             launch_dot(s, P.r.data(), P.z.data(), n, s->dot_out.data());
-            double rz;
-            B2S_CUDA(cudaMemcpyAsync(&rz, s->dot_out.data(), sizeof(double), cudaMemcpyDeviceToHost, st));
-            B2S_CUDA(cudaStreamSynchronize(st));
-            h.rz = rz;
+            read_back(s, s->dot_out.data(), 1, &h.rz);
             done = false;
         }
     }
@@ -966,10 +965,10 @@ void spmv_mixed(b2s_solver* s, const float* x, float* y, double* d_dot)
     ensure_reduction(P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
     P.p32.resize(4 * (size_t)nb, 1.1);
     P.Ap32.resize(4 * (size_t)nb, 1.1);
-    k_pad4<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, x, P.p32.data());
+    k_pad4<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, x, P.p32.data(), P.Ap32.data());
     B2S_CHECK_LAUNCH();
-    B2S_CUDA(cudaMemsetAsync(P.Ap32.data(), 0, sizeof(float) * 4 * (size_t)nb, st));
-    B2S_CUDA(cudaMemsetAsync(d_dot, 0, sizeof(double), st));  // stays 0 for an empty matrix
+    if(A.nnz == 0)
+        B2S_CUDA(cudaMemsetAsync(d_dot, 0, sizeof(double), st));
     spmv_f32_launch(s, A, P.p32.data(), P.Ap32.data(), P.red, d_dot, nullptr);
     k_unpad4<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, P.Ap32.data(), y);
     B2S_CHECK_LAUNCH();
@@ -1018,12 +1017,12 @@ void precond_apply_mixed(b2s_solver* s, const float* r, float* z)
     PcgState&     P  = s->pcg;
     P.r32.resize(4 * (size_t)nb, 1.1);
     P.z32.resize(4 * (size_t)nb, 1.1);
-    k_pad4<<<vec_grid(nb), VEC_BLOCK, 0, s->stream>>>(nb, r, P.r32.data());
+    k_pad4<<<vec_grid(nb), VEC_BLOCK, 0, s->stream>>>(nb, r, P.r32.data(), nullptr);
     B2S_CHECK_LAUNCH();
     precond_launch_f32(s, s->precond_kind, P.r32.data(), P.z32.data(), nullptr, s->red);
     k_unpad4<<<vec_grid(nb), VEC_BLOCK, 0, s->stream>>>(nb, P.z32.data(), z);
     B2S_CHECK_LAUNCH();
-    check_device_errors(s);
+    read_back(s, nullptr, 0, nullptr);
 }
 
 static void pcg_iteration_mixed(b2s_solver* s, int kind, double* x, int slot)
@@ -1105,6 +1104,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
     k_residual_f32<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, b, P.tmp.data(), P.r32.data());
     B2S_CHECK_LAUNCH();
 
+    double bb = 0.0;  // b.b (dot_out[2])
     auto restart_from_r = [&](int k) -> double
     {
         // z = P r, p = z; returns r.z (FP64 sum); also leaves r.r in dot_out[1]
@@ -1113,14 +1113,12 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
                                                             s->red.counter.data(), s->dot_out.data());
         B2S_CHECK_LAUNCH();
         B2S_CUDA(cudaMemcpyAsync(P.p32.data(), P.z32.data(), sizeof(float) * n4, cudaMemcpyDeviceToDevice, st));
-        double h2[2];
-        B2S_CUDA(cudaMemcpyAsync(h2, s->dot_out.data(), sizeof(h2), cudaMemcpyDeviceToHost, st));
-        B2S_CUDA(cudaStreamSynchronize(st));
-        return h2[0];
+        double h3[3];
+        read_back(s, s->dot_out.data(), 3, h3);
+        bb = h3[2];
+        return h3[0];
     };
     launch_dot(s, b, b, n, s->dot_out.data() + 2);
-    double bb = 0.0;
-    B2S_CUDA(cudaMemcpyAsync(&bb, s->dot_out.data() + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
     double rz0 = restart_from_r(kind);
     B2S_REQUIRE(std::isfinite(bb), B2S_ERR_NUMERIC, "non-finite right-hand side");
     bool bypass = false;
@@ -1140,8 +1138,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
                                                             s->red.counter.data(), s->dot_out.data());
         B2S_CHECK_LAUNCH();
         double h2[2];
-        B2S_CUDA(cudaMemcpyAsync(h2, s->dot_out.data(), sizeof(h2), cudaMemcpyDeviceToHost, st));
-        B2S_CUDA(cudaStreamSynchronize(st));
+        read_back(s, s->dot_out.data(), 2, h2);
         return h2[1] > 0 ? std::sqrt(h2[0] / h2[1]) : 0.0;
     };
     auto replace_residual = [&]()
