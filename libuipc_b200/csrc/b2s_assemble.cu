@@ -965,13 +965,16 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
     }
     M.has_trank = false;
     if(spmv_tiles && U > 0)
-    {
-        M.trank.resize(M.stride, 1.2);
-        k_tile_rank<<<(unsigned)((U + SPMV_TILE - 1) / SPMV_TILE), RANK_THREADS, 0, st>>>(U, M.cols.data(),
-                                                                                     M.trank.data());
-        B2S_CHECK_LAUNCH();
-        M.has_trank = true;
-    }
+        build_tile_ranks(s, M);
     M.valid = true;
+}
+
+void build_tile_ranks(b2s_solver* s, Matrix& M)
+{
+    M.trank.resize(M.stride, 1.2);
+    k_tile_rank<<<(unsigned)((M.nnz + SPMV_TILE - 1) / SPMV_TILE), RANK_THREADS, 0, s->stream>>>(
+        M.nnz, M.cols.data(), M.trank.data());
+    B2S_CHECK_LAUNCH();
+    M.has_trank = true;
 }
 }  // namespace b2s

@@ -168,7 +168,7 @@ struct MasState
     DBuf<int32_t> p2r, r2p;        // [N], [vn]
     DBuf<int32_t> ctable;          // [vn * (L-1)] global node at levels 1..L-1
     DBuf<int32_t> node1;           // [vn] global level-1 node of each vertex (-1: none)
-    DBuf<int32_t> anc;             // [level_count[1] * (L-2)] global slots of each level-1 node's ancestors
+    DBuf<int4>    anc;             // [level_count[1]] global slots of each level-1 node's ancestors (levels 2-5)
     DBuf<int32_t> cst;             // [L * vn] local id of vertex v at level l+1
     DBuf<uint16_t> comp_mask[MAX_LEVELS];  // per level: component lane mask of each node
     DBuf<int32_t>  new_local[MAX_LEVELS];  // per level: local id of each node at the next level
@@ -185,11 +185,12 @@ struct MasState
     Matrix        coarse[MAX_LEVELS];
     DBuf<int32_t> trip_rows, trip_cols;
     DBuf<double>  trip_vals;
-    // apply buffers (FP32, 3 per node slot); after an apply the level-1 slots
-    // of Z hold the folded prolongation Z_1 + Z_2[parent] + ...
+    // apply buffers (FP32, 3 per node slot)
     DBuf<float>   R, Z;
+    DBuf<double>  R64;  // sums of the restriction at the levels above 1 (zero between applies)
     // host copies for introspection
     std::vector<int32_t> h_ctable;
+    long long     generation = 0;  // bumped by every initialisation
 };
 
 // ---------------------------------------------------------------------------
@@ -226,8 +227,27 @@ struct Reduction
     DBuf<unsigned int> counter;
 };
 
+// The row order of a PCG with the MAS preconditioner: the partition slots
+// first (16 per bank, so a bank's residuals are contiguous), then the rows
+// outside the MAS. The matrix is copied into it once per assembly; a slot
+// without a vertex, like a row without blocks, holds one zero diagonal block.
+struct PcgOrder
+{
+    int32_t       n = 0;      // rows in this order (0: not built)
+    int32_t       slots = 0;  // MAS slots, the first rows
+    int32_t       nb = 0;     // rows of the matrix
+    DBuf<int32_t> row_of;     // [n] block row of each row (-1: padding slot)
+    DBuf<int32_t> pos;        // [nb] its inverse
+    DBuf<int32_t> node1;      // [slots] global level-1 node of each slot (-1: none)
+    Matrix        A;          // the matrix in this order
+    long long     mas_generation = -1;  // MAS initialisation it was built from
+    long long     f64_generation = -1, f32_generation = -1;  // assembly whose FP64 / FP32 values A holds
+};
+
 struct PcgState
 {
+    PcgOrder     ord;
+    DBuf<double> xs;  // the solution in PCG order
     DBuf<double> r, z, p, Ap, tmp;
     DBuf<PcgScalars> sc;
     Reduction        red;
@@ -268,10 +288,6 @@ struct b2s_solver
     b2s::Reduction       red;
     b2s::DBuf<int>       dev_err;  // DeviceError bits raised by kernels
     b2s::ReadBack*       h_back = nullptr;  // pinned: the last read_back
-    // the MAS apply's second stream: the coarse levels run on it beside the
-    // fine level's products (forked from `stream` and joined back by events)
-    cudaStream_t             mas_side = nullptr;
-    cudaEvent_t              mas_fork = nullptr, mas_join = nullptr;
     // stage timers (CUDA events on `stream`)
     bool                     timing = false;
     b2s_timers               timers{};
@@ -342,6 +358,13 @@ void mas_assemble(b2s_solver* s, int invert_mode);
 void mas_apply(b2s_solver* s, const double* r, double* z);
 // host: recursive graph bisection into parts of at most max_part vertices
 void partition_graph(int32_t n, const int32_t* xadj, const int32_t* adj, int32_t max_part, int32_t* part_ids);
+
+// Z of every MAS node from the restriction's R_0, R_1 and coarse sums (queued)
+void mas_apply_all(b2s_solver* s, const int* converged, bool bf16);
+// the per-tile column ranks of the FP64 SpMV, and the row-start groups of the
+// FP32 one when every row has a block
+void build_tile_ranks(b2s_solver* s, Matrix& M);
+void build_row_groups_full(b2s_solver* s, Matrix& A);
 
 // PCG
 void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options& o, b2s_pcg_stats& st);

@@ -1,0 +1,392 @@
+// Device code of the MAS apply: the restriction to the coarse levels, products
+// of one bank's inverse with its residuals, and the streams of banks.
+#pragma once
+#include "b2s_internal.cuh"
+#include "b2s_tma.cuh"
+
+#include <cuda_bf16.h>
+
+namespace b2s
+{
+__host__ __device__ __forceinline__ int sym_index(int row, int col)
+{
+    return BANK * row - row * (row + 1) / 2 + col;
+}
+
+// ---------------------------------------------------------------------------
+// apply: one warp per bank, persistent over banks. The bank's inverse is
+// brought into shared memory by bulk asynchronous copies (TMA), NST deep per
+// warp, so later banks' copies are in flight while this one computes. The
+// residual of the next bank (and, at level 0, the part_to_real index of the
+// bank after it) is loaded into registers one bank ahead, so the dependent
+// part_to_real -> r gather never stalls the product.
+//
+// FP32 inverses (4,896 B: the 136 upper 3x3 blocks, column-major) are applied
+// on the CUDA cores: lanes 0-15 own the bank's nodes and the 48x48 product is
+// split over the two half-warps (columns 0-7 / 8-15).
+//
+// BF16 inverses (mixed precision) are applied on the tensor cores. Per cluster:
+// the FP32 factor D = diag(M)^1/2 (48 floats, 192 B), then the six upper 16x16
+// tiles (I <= J) of the 48x48 matrix D^-1 M D^-1 in BF16 (6 x 512 B), 3,264 B
+// in all. Tile rows are 32 B; the two 16-B halves of row R are swapped when
+// bit 2 of R is set, so each 8-row ldmatrix phase touches all 32 banks once.
+// z = D (M_s (D r)) by mma.m16n8k16 (BF16 operands, FP32 accumulation): A is
+// tile (I, J), for J < I the stored tile (J, I) loaded transposed; B column 0
+// is BF16(D r) and column 1 its BF16 rounding remainder, so the FP32 residual
+// enters with ~16 significant bits and the stored inverse is the only 8-bit
+// rounding. (A 48x48 matrix times one vector is an HBM-bound GEMV; the tensor
+// cores are used to cut the instruction count per byte, not for FLOPs.)
+// ---------------------------------------------------------------------------
+constexpr int APPLY_WARPS = 4;
+constexpr uint32_t INV_BYTES = SYM * 9 * sizeof(float);  // 4896, a multiple of 16
+constexpr uint32_t INV16_SCALE_BYTES = BANK * 3 * sizeof(float);                    // 192
+constexpr uint32_t INV16_TILE_BYTES  = 16 * 16 * 2;                                 // 512
+constexpr uint32_t INV16_BYTES       = INV16_SCALE_BYTES + 6 * INV16_TILE_BYTES;  // 3264
+constexpr int APPLY_STAGES_F32  = 2;
+constexpr int APPLY_STAGES_BF16 = 2;
+
+// index of the upper tile (I, J), I <= J: (0,0) (0,1) (0,2) (1,1) (1,2) (2,2)
+__host__ __device__ __forceinline__ int tile_id(int I, int J) { return I * 3 - I * (I + 1) / 2 + J; }
+// byte offset of 16-B half `half` of row `row` inside a tile
+__host__ __device__ __forceinline__ uint32_t tile_off(int row, int half)
+{
+    return (uint32_t)row * 32u + ((uint32_t)(half ^ ((row >> 2) & 1)) << 4);
+}
+
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& a0, uint32_t& a1, uint32_t& a2, uint32_t& a3)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3)
+                 : "r"(addr));
+}
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t& a0, uint32_t& a1, uint32_t& a2, uint32_t& a3)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3)
+                 : "r"(addr));
+}
+// c += A (16x16, row) * B (16x8, col), BF16 in, FP32 accumulate
+__device__ __forceinline__ void mma_bf16_16816(float& c0, float& c1, float& c2, float& c3, uint32_t a0, uint32_t a1,
+                                               uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%0, %1, %2, %3};"
+        : "+f"(c0), "+f"(c1), "+f"(c2), "+f"(c3)
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack_bf16x2(__nv_bfloat16 lo, __nv_bfloat16 hi)
+{
+    return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+}
+
+// Zb[0..48) = D M_s D r for one cluster; r48: the bank's residual (node-major)
+__device__ __forceinline__ void cluster_product_mma(const unsigned char* slot, const float* r48, int lane,
+                                                    float* __restrict__ Zb)
+{
+    const float*   D     = reinterpret_cast<const float*>(slot);
+    const uint32_t tiles = smem_addr(slot + INV16_SCALE_BYTES);
+    const int      g = lane >> 2, t = lane & 3;
+    uint32_t       b[3][2];
+#pragma unroll
+    for(int J = 0; J < 3; ++J)
+    {
+#pragma unroll
+        for(int h = 0; h < 2; ++h)
+        {
+            const int           k  = J * 16 + 2 * t + 8 * h;
+            const float         x0 = r48[k] * D[k], x1 = r48[k + 1] * D[k + 1];
+            const __nv_bfloat16 h0 = __float2bfloat16_rn(x0), h1 = __float2bfloat16_rn(x1);
+            uint32_t            v  = 0;
+            if(g == 0)
+                v = pack_bf16x2(h0, h1);
+            else if(g == 1)
+                v = pack_bf16x2(__float2bfloat16_rn(x0 - __bfloat162float(h0)),
+                                __float2bfloat16_rn(x1 - __bfloat162float(h1)));
+            b[J][h] = v;
+        }
+    }
+    // row address this lane gives ldmatrix: matrix q = lane / 8 of the four
+    // 8x8 quarters, row lane % 8 of it
+    const int      q = lane >> 3, rr = lane & 7;
+    const uint32_t offN = tile_off(rr + ((q & 1) << 3), q >> 1);
+    const uint32_t offT = tile_off(rr + ((q >> 1) << 3), q & 1);
+#pragma unroll
+    for(int I = 0; I < 3; ++I)
+    {
+        float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
+#pragma unroll
+        for(int J = 0; J < 3; ++J)
+        {
+            uint32_t a0, a1, a2, a3;
+            if(J >= I)
+                ldsm_x4(tiles + tile_id(I, J) * INV16_TILE_BYTES + offN, a0, a1, a2, a3);
+            else
+                ldsm_x4_trans(tiles + tile_id(J, I) * INV16_TILE_BYTES + offT, a0, a1, a2, a3);
+            mma_bf16_16816(c0, c1, c2, c3, a0, a1, a2, a3, b[J][0], b[J][1]);
+        }
+        if(t == 0)
+        {
+            const int k0 = I * 16 + g, k1 = k0 + 8;
+            Zb[k0] = (c0 + c1) * D[k0];
+            Zb[k1] = (c2 + c3) * D[k1];
+        }
+    }
+}
+
+__device__ __forceinline__ void cluster_product(const float* M, const float (*r)[3], int lane, float out[3])
+{
+    // lanes 0..15: row node `lane`, columns 0..7; lanes 16..31: row node lane-16, columns 8..15
+    const int rn = lane & 15, c0 = (lane >> 4) * 8;
+    float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f;
+#pragma unroll
+    for(int cc = 0; cc < 8; ++cc)
+    {
+        const int cn = c0 + cc;
+        const float x0 = r[cn][0], x1 = r[cn][1], x2 = r[cn][2];
+        if(cn >= rn)
+        {
+            const float* B = M + sym_index(rn, cn) * 9;  // column-major
+            acc0 = __fmaf_rn(B[0], x0, acc0); acc0 = __fmaf_rn(B[3], x1, acc0); acc0 = __fmaf_rn(B[6], x2, acc0);
+            acc1 = __fmaf_rn(B[1], x0, acc1); acc1 = __fmaf_rn(B[4], x1, acc1); acc1 = __fmaf_rn(B[7], x2, acc1);
+            acc2 = __fmaf_rn(B[2], x0, acc2); acc2 = __fmaf_rn(B[5], x1, acc2); acc2 = __fmaf_rn(B[8], x2, acc2);
+        }
+        else
+        {
+            const float* B = M + sym_index(cn, rn) * 9;  // use B^T
+            acc0 = __fmaf_rn(B[0], x0, acc0); acc0 = __fmaf_rn(B[1], x1, acc0); acc0 = __fmaf_rn(B[2], x2, acc0);
+            acc1 = __fmaf_rn(B[3], x0, acc1); acc1 = __fmaf_rn(B[4], x1, acc1); acc1 = __fmaf_rn(B[5], x2, acc1);
+            acc2 = __fmaf_rn(B[6], x0, acc2); acc2 = __fmaf_rn(B[7], x1, acc2); acc2 = __fmaf_rn(B[8], x2, acc2);
+        }
+    }
+    acc0 += __shfl_down_sync(0xffffffffu, acc0, 16);
+    acc1 += __shfl_down_sync(0xffffffffu, acc1, 16);
+    acc2 += __shfl_down_sync(0xffffffffu, acc2, 16);
+    out[0] = acc0;
+    out[1] = acc1;
+    out[2] = acc2;
+}
+
+// Every bank's residual slice (16 nodes x 3 floats, 192 B, contiguous) and its
+// inverse come into shared memory by bulk copies (TMA) on one barrier, NST
+// banks ahead per warp, so a warp never waits on a dependent gather. BF: BF16
+// tiles on the tensor cores (INV16_BYTES per cluster), otherwise FP32
+// (INV_BYTES); a stiff cluster (inverted in FP64) is applied from its FP32
+// inverse in HBM in the BF16 path.
+constexpr uint32_t R_BYTES = BANK * 3 * sizeof(float);  // 192
+
+template <bool BF>
+__host__ __device__ constexpr uint32_t stage_bytes()
+{
+    return (BF ? INV16_BYTES : INV_BYTES) + R_BYTES;
+}
+
+// what the apply reads and writes
+struct ApplyArgs
+{
+    const unsigned char* inv;    // packed inverses of all clusters (FP32 or BF16)
+    const float*         inv32;  // FP32 inverses (stiff clusters of the BF16 path)
+    const uint8_t*       stiff;  // [clusters], null in the FP32 path
+    float*               R;
+    float*               Z;
+    double*              R64;  // sums of the levels above 1 (from slot 16 g2 on)
+    int*                 err;
+    int                  n0, n1, n2;  // banks of level 0, of level 1, of the levels above
+    int                  g1, g2;      // first bank of level 1 and of level 2
+};
+
+// the bank's inverse and, with `with_r`, its residual slice, on one barrier
+template <bool BF>
+__device__ __forceinline__ void issue_bank_copy(unsigned char* stage, uint64_t* bar, const ApplyArgs& A, int64_t gbank,
+                                                bool with_r)
+{
+    constexpr uint32_t CB = BF ? INV16_BYTES : INV_BYTES;
+    mbar_arrive_expect_tx(bar, CB + (with_r ? R_BYTES : 0u));
+    bulk_copy_g2s(stage, A.inv + (size_t)gbank * CB, CB, bar);
+    if(with_r)
+        bulk_copy_g2s(stage + CB, A.R + (size_t)gbank * (BANK * 3), R_BYTES, bar);
+}
+
+// Z of one bank from its staged inverse and residual (the whole warp)
+template <bool BF>
+__device__ __forceinline__ void bank_product(const ApplyArgs& A, unsigned char* stage, int64_t gbank, bool use32, int lane)
+{
+    constexpr uint32_t CB = BF ? INV16_BYTES : INV_BYTES;
+    const float(*s_r)[3] = reinterpret_cast<const float(*)[3]>(stage + CB);
+    float* Zb            = A.Z + gbank * (BANK * 3);
+    if(BF && !use32)
+        cluster_product_mma(stage, &s_r[0][0], lane, Zb);
+    else
+    {
+        float        out[3];
+        const float* Mc = use32 ? A.inv32 + (size_t)gbank * SYM * 9 : reinterpret_cast<const float*>(stage);
+        cluster_product(Mc, s_r, lane, out);
+        if(lane < 16)
+        {
+            Zb[3 * lane]     = out[0];
+            Zb[3 * lane + 1] = out[1];
+            Zb[3 * lane + 2] = out[2];
+        }
+    }
+}
+
+// The residual of a coarse bank (level 2 up) from its FP64 sums: to R and the
+// staged slice in FP32, the sums cleared for the next restriction.
+__device__ __forceinline__ void take_coarse(const ApplyArgs& A, int64_t gbank, float* s_r, int lane)
+{
+    double* q = A.R64 + (gbank - A.g2) * (BANK * 3);
+    for(int e = lane; e < BANK * 3; e += 32)
+    {
+        const float v = (float)__ldcg(q + e);
+        q[e]          = 0.0;
+        s_r[e]        = v;
+        A.R[gbank * (BANK * 3) + e] = v;
+    }
+    __syncwarp();
+}
+
+// The banks handled by one warp (warp gw of W). The list: the coarse banks
+// from level 2 up (global banks g2 ..), then level 0, then level 1 (from g1).
+// A copy wait that runs out sets the error flag, drains the warp's copies in
+// flight and ends the warp.
+template <bool BF, int NST>
+__device__ __forceinline__ void apply_banks(int gw, int W, int lane, const ApplyArgs& A, unsigned char* s_stage,
+                                            uint64_t* s_bar)
+{
+    constexpr uint32_t SB   = stage_bytes<BF>();
+    constexpr uint32_t CB   = BF ? INV16_BYTES : INV_BYTES;
+    const int          n    = A.n2 + A.n0 + A.n1;
+    const int          mine = gw < n ? (n - 1 - gw) / W + 1 : 0;
+    auto               bank_of = [&](int j) -> int64_t
+    {
+        const int i = gw + j * W - A.n2;
+        return i < 0 ? (int64_t)A.g2 + i + A.n2 : (i < A.n0 ? i : (int64_t)A.g1 + (i - A.n0));
+    };
+    auto issue = [&](int j, int slot)
+    { issue_bank_copy<BF>(s_stage + slot * SB, &s_bar[slot], A, bank_of(j), gw + j * W >= A.n2); };
+    if(lane == 0)
+        for(int j = 0; j < mine && j < NST; ++j)
+            issue(j, j);
+    __syncwarp();
+    int j = 0;
+    for(; j < mine; ++j)
+    {
+        const int64_t  gbank = bank_of(j);
+        const int      slot  = j % NST;
+        const bool     use32 = BF && A.stiff != nullptr && A.stiff[gbank] != 0;
+        unsigned char* stage = s_stage + slot * SB;
+        if(gw + j * W < A.n2)
+            take_coarse(A, gbank, reinterpret_cast<float*>(stage + CB), lane);
+        const bool ok = mbar_wait(&s_bar[slot], (uint32_t)((j / NST) & 1), A.err, DERR_TMA_TIMEOUT);
+        if(!__all_sync(0xffffffffu, ok))
+            break;
+        bank_product<BF>(A, stage, gbank, use32, lane);
+        __syncwarp();
+        if(lane == 0 && j + NST < mine)
+        {
+            fence_proxy_async_smem();
+            issue(j + NST, slot);
+        }
+    }
+    if(j < mine && lane == 0)
+        for(int q = j; q < mine && q < j + NST; ++q)
+            mbar_wait(&s_bar[q % NST], (uint32_t)((q / NST) & 1), nullptr, 0);
+    __syncwarp();
+}
+
+// The level-1 sums of a block of rows (in slot order; thread t's slot is its
+// row) and their part of the sums of the levels above. s_r: the residuals
+// [threads][3]; cm, nl: component mask and level-1 index of the thread's slot
+// (cm = 0: none); anc: its level-1 node's ancestors, needed by the components'
+// lowest lanes. R_1 in FP32, summed by the lowest lane in lane order. The
+// levels above, whose nodes collect from many blocks, are summed in FP64 by
+// reductions in L2 (their order moves the last bits of an FP64 sum that is then
+// rounded to FP32): every level is complete when the kernel is. A chain of
+// restrictions from level to level inside the apply took 25 us (88,641
+// vertices) to 43 us (551,368, behind the fine level's traffic) where the apply
+// now takes 8.8 and 26.8 us. Whole block;
+// s_lead: [threads][3] floats, s_anc: [threads] int4, s_n: [warps].
+template <int THREADS>
+__device__ __forceinline__ void restrict_coarse(const float (*s_r)[3], uint32_t cm, int nl, int4 anc, int begin1,
+                                                float* __restrict__ R, double* __restrict__ R64, int begin2,
+                                                float (*s_lead)[3], int4* s_anc, int* s_n)
+{
+    const int      t = threadIdx.x, lane = t & 31, w = t >> 5, sub = t & 15;
+    const bool     lead = cm != 0 && (cm & ((1u << sub) - 1u)) == 0;
+    const unsigned all  = __ballot_sync(0xffffffffu, lead);
+    if(lane == 0)
+        s_n[w] = __popc(all);
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+    if(lead)
+    {
+        const float(*b)[3] = s_r + (t & ~15);
+        for(uint32_t m = cm; m; m &= m - 1)
+        {
+            const int l = __ffs(m) - 1;
+            s0 += b[l][0];
+            s1 += b[l][1];
+            s2 += b[l][2];
+        }
+        const int64_t g = (int64_t)begin1 + nl;
+        R[3 * g]     = s0;
+        R[3 * g + 1] = s1;
+        R[3 * g + 2] = s2;
+    }
+    __syncthreads();
+    int at = __popc(all & ((1u << lane) - 1u)), n = 0;
+#pragma unroll
+    for(int q = 0; q < THREADS / 32; ++q)
+    {
+        at += q < w ? s_n[q] : 0;
+        n += s_n[q];
+    }
+    if(lead)
+    {
+        s_lead[at][0] = s0;
+        s_lead[at][1] = s1;
+        s_lead[at][2] = s2;
+        s_anc[at]     = anc;
+    }
+    __syncthreads();
+    // warp lv: level 2 + lv. The block's components have one or two ancestors
+    // there: one sum over the warp and one reduction per entry for each
+    static_assert(THREADS >= 128, "a warp per level above 1");
+    if(w >= 4)
+        return;
+    for(int base = 0; base < n; base += 32)
+    {
+        const int k    = base + lane;
+        int       node = k < n ? reinterpret_cast<const int*>(s_anc + k)[w] : -1;
+        float     v[3] = {0.f, 0.f, 0.f};
+        if(k < n)
+#pragma unroll
+            for(int c = 0; c < 3; ++c)
+                v[c] = s_lead[k][c];
+        while(true)
+        {
+            const int best = (int)__reduce_min_sync(0xffffffffu, (unsigned)node);  // -1: the largest
+            if(best < 0)
+                break;
+            const bool in = node == best;
+            double     a[3];
+#pragma unroll
+            for(int c = 0; c < 3; ++c)
+                a[c] = in ? (double)v[c] : 0.0;
+#pragma unroll
+            for(int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for(int c = 0; c < 3; ++c)
+                    a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
+            if(lane < 3)
+                asm volatile("red.global.add.f64 [%0], %1;" ::"l"(R64 + 3 * ((int64_t)best - begin2) + lane),
+                             "d"(lane == 0 ? a[0] : (lane == 1 ? a[1] : a[2]))
+                             : "memory");
+            if(in)
+                node = -1;
+        }
+    }
+}
+
+// the arguments of an apply from the current build (b2s_mas.cu)
+ApplyArgs mas_apply_args(b2s_solver* s, bool bf16);
+}  // namespace b2s

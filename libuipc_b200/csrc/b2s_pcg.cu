@@ -13,12 +13,15 @@
 // replayed from one CUDA graph and checked once by the host, as the
 // reference's graph block replay does (:1923-1998).
 #include "b2s_internal.cuh"
+#include "b2s_mas_apply.cuh"
+#include "b2s_pcg.cuh"
 #include "b2s_reduce.cuh"
 
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 namespace b2s
 {
@@ -193,18 +196,6 @@ __global__ void __launch_bounds__(ABD_WARPS * 32) k_abd_inverse(int n_bodies, in
             out[(size_t)b * 144 + i * 12 + lane - 12] = ok ? a[i] : (lane - 12 == i ? 1.0 : 0.0);
 }
 
-struct MasView
-{
-    int            active;  // MAS present
-    int            off, vn, L;
-    int            abd_off, abd_n;  // affine-body range: block rows abd_off .. abd_off + 4 abd_n
-    const double*  abd_inv;         // [abd_n * 144]
-    const int32_t* r2p;
-    const int32_t* node1;  // [vn] level-1 node of each vertex (its Z slot holds the folded coarse sum)
-    int            T;      // coarse levels (L-1)
-    const float*   Z;      // node values by slot
-};
-
 // node i's three entries of r: NS = 3 values per node (FP64 vectors), or 4
 // (the padded FP32 vectors of the mixed PCG: one 16-byte load)
 template <typename VT, int NS>
@@ -225,15 +216,55 @@ __device__ __forceinline__ void load_r(const VT* r, int64_t i, double& a, double
     }
 }
 
+// the MAS value of slot p with level-1 node n1 (-1: none): the fine level's Z
+// of the slot plus its coarse nodes' (level 1 up; neighbours mostly share
+// them, so these are broadcast hits in L1)
+__device__ __forceinline__ void mas_value(const MasView& mv, int p, int n1, double z[3])
+{
+    float c0 = mv.Z[3 * (int64_t)p], c1 = mv.Z[3 * (int64_t)p + 1], c2 = mv.Z[3 * (int64_t)p + 2];
+    if(n1 >= 0)
+    {
+        const int4 a  = mv.anc[n1 - mv.begin1];
+        float      w0 = mv.Z[3 * (int64_t)n1], w1 = mv.Z[3 * (int64_t)n1 + 1], w2 = mv.Z[3 * (int64_t)n1 + 2];
+        const int  up[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for(int k = 0; k < 4; ++k)
+            if(up[k] >= 0)
+            {
+                w0 += mv.Z[3 * (int64_t)up[k]];
+                w1 += mv.Z[3 * (int64_t)up[k] + 1];
+                w2 += mv.Z[3 * (int64_t)up[k] + 2];
+            }
+        c0 += w0;
+        c1 += w1;
+        c2 += w2;
+    }
+    z[0] = (double)c0;
+    z[1] = (double)c1;
+    z[2] = (double)c2;
+}
+
 // z_i for block row i: MAS (partitioned vertices of its range), else 3x3
-// block Jacobi (kind 1 / 2), else identity (kind 0); r_i is returned in rr
-template <typename VT, int NS>
+// block Jacobi (kind 1 / 2), else identity (kind 0); r_i is returned in rr.
+// ORD: r and i are in PCG order (the slots, then the other rows)
+template <typename VT, int NS, bool ORD>
 __device__ __forceinline__ void precond_row(int kind, const MasView& mv, const double* dinv, const VT* r, int i,
                                             double z[3], double rr[3])
 {
     load_r<VT, NS>(r, i, rr[0], rr[1], rr[2]);
     const double r0 = rr[0], r1 = rr[1], r2 = rr[2];
-    if(kind == B2S_PRECOND_MAS && mv.active)
+    int          row = i;  // the matrix's row
+    if constexpr(ORD)
+    {
+        if(kind == B2S_PRECOND_MAS && i < mv.slots)
+        {
+            mas_value(mv, i, mv.T > 0 ? mv.slot_node1[i] : -1, z);
+            return;
+        }
+        if(kind != B2S_PRECOND_NONE)
+            row = mv.row_of[i];
+    }
+    else if(kind == B2S_PRECOND_MAS && mv.active)
     {
         const int v = i - mv.off;
         if(v >= 0 && v < mv.vn)
@@ -241,19 +272,7 @@ __device__ __forceinline__ void precond_row(int kind, const MasView& mv, const d
             const int p = mv.r2p[v];
             if(p >= 0)
             {
-                // the fine level's Z of the vertex's slot plus the coarse
-                // levels' sum folded into its level-1 node
-                const int n1 = mv.T > 0 ? mv.node1[v] : -1;
-                float     c0 = mv.Z[3 * (int64_t)p], c1 = mv.Z[3 * (int64_t)p + 1], c2 = mv.Z[3 * (int64_t)p + 2];
-                if(n1 >= 0)
-                {
-                    c0 += mv.Z[3 * (int64_t)n1];
-                    c1 += mv.Z[3 * (int64_t)n1 + 1];
-                    c2 += mv.Z[3 * (int64_t)n1 + 2];
-                }
-                z[0] = (double)c0;
-                z[1] = (double)c1;
-                z[2] = (double)c2;
+                mas_value(mv, p, mv.T > 0 ? mv.node1[v] : -1, z);
                 return;
             }
         }
@@ -265,12 +284,12 @@ __device__ __forceinline__ void precond_row(int kind, const MasView& mv, const d
         z[2] = r2;
         return;
     }
-    if(mv.abd_n > 0 && i >= mv.abd_off && i < mv.abd_off + 4 * mv.abd_n)
+    if(mv.abd_n > 0 && row >= mv.abd_off && row < mv.abd_off + 4 * mv.abd_n)
     {
         // row l of body b: z = (H_b^-1)[3l .. 3l+2][0 .. 11] r_b
-        const int     b = (i - mv.abd_off) >> 2, l = (i - mv.abd_off) & 3;
+        const int     b = (row - mv.abd_off) >> 2, l = (row - mv.abd_off) & 3;
         const double* Hi = mv.abd_inv + (size_t)b * 144 + 36 * l;
-        const int64_t n0 = (int64_t)mv.abd_off + 4 * b;  // the body's first node
+        const int64_t n0 = (int64_t)i - l;  // the body's first node (its rows stay together in either order)
         double        a0 = 0.0, a1 = 0.0, a2 = 0.0;
         for(int j = 0; j < 12; ++j)
         {
@@ -284,7 +303,7 @@ __device__ __forceinline__ void precond_row(int kind, const MasView& mv, const d
         z[2] = a2;
         return;
     }
-    const double* D = dinv + (size_t)i * 9;
+    const double* D = dinv + (size_t)row * 9;
     z[0] = D[0] * r0 + D[1] * r1 + D[2] * r2;
     z[1] = D[3] * r0 + D[4] * r1 + D[5] * r2;
     z[2] = D[6] * r0 + D[7] * r1 + D[8] * r2;
@@ -295,7 +314,7 @@ __device__ __forceinline__ void precond_row(int kind, const MasView& mv, const d
 // 32 registers, so the whole reduction grid (8 CTAs per SM) is resident at
 // once (with 40 the last quarter of the grid ran as a second wave: the MAS
 // apply with this finish measured 77.4 -> 73.8 us on 551 k vertices).
-template <typename VT, int NS>
+template <typename VT, int NS, bool ORD>
 __global__ void __launch_bounds__(RED_BLOCK, 8) k_precond_finish(int32_t nb, int kind, MasView mv,
                                                               const double* __restrict__ dinv,
                                                               const VT* __restrict__ r, VT* __restrict__ z,
@@ -308,7 +327,7 @@ __global__ void __launch_bounds__(RED_BLOCK, 8) k_precond_finish(int32_t nb, int
     for(int i = blockIdx.x * RED_BLOCK + threadIdx.x; i < nb; i += gridDim.x * RED_BLOCK)
     {
         double zi[3], ri[3];
-        precond_row<VT, NS>(kind, mv, dinv, r, i, zi, ri);
+        precond_row<VT, NS, ORD>(kind, mv, dinv, r, i, zi, ri);
         const VT z0 = (VT)zi[0], z1 = (VT)zi[1], z2 = (VT)zi[2];
         if constexpr(NS == 4)
             *reinterpret_cast<float4*>(z + 4 * (int64_t)i) = make_float4(z0, z1, z2, 0.0f);
@@ -406,7 +425,106 @@ __global__ void k_update_xr_mixed4(int32_t nb, PcgScalars* sc, double* __restric
     }
 }
 
-// p = z + beta p over the padded vectors (n = 4 nb; pads stay zero)
+// The same update in PCG order with the MAS restriction in the pass: the
+// first `slots` rows are the partition slots, 16 per bank, so the half-warp
+// that updates a bank's residuals also writes them as R_0 (FP32), and the
+// block their sums at the coarse levels (restrict_coarse). In the vertices'
+// own order the restriction was a launch of its own that gathered r through
+// the partition: 20.3 us for update and restriction of 551,368 vertices (mixed),
+// 16.7 here with the sums of every coarse level. NS: entries per node (3: FP64
+// vectors, Ap zeroed here; 4: padded FP32). UPDATE = false: only the restriction of r.
+template <typename VT, int NS, bool UPDATE>
+__global__ void __launch_bounds__(VEC_BLOCK)
+    k_update_restrict(int32_t n, int32_t slots, PcgScalars* sc, double* __restrict__ x, const VT* __restrict__ p,
+                      VT* __restrict__ r, VT* __restrict__ Ap, const uint16_t* __restrict__ comp_mask,
+                      const int32_t* __restrict__ new_local, const int4* __restrict__ anc, int begin1, int begin2,
+                      int push, float* __restrict__ R, double* __restrict__ R64)
+{
+    if(UPDATE && frozen(sc))
+        return;
+    __shared__ float s_r[VEC_BLOCK][3];
+    __shared__ float s_p[VEC_BLOCK][3];  // p (NS = 4), then the components' sums
+    __shared__ int4  s_anc[VEC_BLOCK];
+    __shared__ int   s_n[VEC_BLOCK / 32];
+    const int        t = threadIdx.x, i = blockIdx.x * VEC_BLOCK + t, sub = t & 15;
+    const int64_t    e0 = 3 * (int64_t)blockIdx.x * VEC_BLOCK;  // the block's first entry of 3 per node
+    uint32_t         cm = 0;
+    int              nl = 0;
+    int4             an = make_int4(-1, -1, -1, -1);
+    if(i < slots && push)
+    {
+        cm = comp_mask[i];
+        nl = new_local[i];
+        if(cm != 0 && (cm & ((1u << sub) - 1u)) == 0)
+            an = anc[nl];
+    }
+    double alpha = 0.0;
+    if constexpr(UPDATE)
+        alpha = sc->rz / sc->pAp;
+    float* fr = &s_r[0][0];
+    if constexpr(NS == 4)
+    {
+        if(i < n)
+        {
+            float4 rr = reinterpret_cast<const float4*>(r)[i];
+            if constexpr(UPDATE)
+            {
+                const float  af = (float)alpha;
+                const float4 ap = reinterpret_cast<const float4*>(Ap)[i];
+                const float4 pp = reinterpret_cast<const float4*>(p)[i];
+                rr.x = __fmaf_rn(-af, ap.x, rr.x);
+                rr.y = __fmaf_rn(-af, ap.y, rr.y);
+                rr.z = __fmaf_rn(-af, ap.z, rr.z);
+                reinterpret_cast<float4*>(r)[i] = rr;
+                s_p[t][0] = pp.x;
+                s_p[t][1] = pp.y;
+                s_p[t][2] = pp.z;
+            }
+            s_r[t][0] = rr.x;
+            s_r[t][1] = rr.y;
+            s_r[t][2] = rr.z;
+        }
+        __syncthreads();
+    }
+    // the arrays of 3 per node, entry by entry (consecutive lanes on
+    // consecutive entries: thread by node, each access spread over 3 times the
+    // lines)
+#pragma unroll
+    for(int j = 0; j < 3; ++j)
+    {
+        const int     f = t + j * VEC_BLOCK;
+        const int64_t e = e0 + f;
+        if(e >= 3 * (int64_t)n)
+            continue;
+        if constexpr(NS == 4)
+        {
+            if constexpr(UPDATE)
+                x[e] += alpha * (double)(&s_p[0][0])[f];
+        }
+        else
+        {
+            double q = r[e];
+            if constexpr(UPDATE)
+            {
+                x[e] += alpha * p[e];
+                q -= alpha * Ap[e];
+                r[e]  = q;
+                Ap[e] = 0.0;
+            }
+            fr[f] = (float)q;
+        }
+        if(e < 3 * (int64_t)slots)
+            R[e] = fr[f];
+    }
+    if(UPDATE && i == 0)
+        sc->alpha = alpha;
+    if(push)
+    {
+        __syncthreads();  // s_r is complete, s_p is free
+        restrict_coarse<VEC_BLOCK>(s_r, cm, nl, an, begin1, R, R64, begin2, s_p, s_anc, s_n);
+    }
+}
+
 // p = z + beta p over the padded vectors (nb nodes), and Ap = 0 for the
 // SpMV that follows: zeroed here rather than after its last reader, so the
 // zero lines are still in L2 when the SpMV's reductions reach them
@@ -436,6 +554,138 @@ __global__ void k_residual_f32(int32_t nb, const double* __restrict__ b, const d
     for(int64_t i = (int64_t)blockIdx.x * VEC_BLOCK + threadIdx.x; i < nb; i += (int64_t)gridDim.x * VEC_BLOCK)
         reinterpret_cast<float4*>(r)[i] = make_float4((float)(b[3 * i] - Ax[3 * i]), (float)(b[3 * i + 1] - Ax[3 * i + 1]),
                                                       (float)(b[3 * i + 2] - Ax[3 * i + 2]), 0.0f);
+}
+
+// r = b - Ax in PCG order (b, Ax in the matrix's order; Ax null: r = b), zero in
+// padding slots; NS = 4: FP32, padded
+template <typename VT, int NS>
+__global__ void k_residual_ord(int32_t n, const int32_t* __restrict__ row_of, const double* __restrict__ b,
+                               const double* __restrict__ Ax, VT* __restrict__ r)
+{
+    for(int i = blockIdx.x * VEC_BLOCK + threadIdx.x; i < n; i += gridDim.x * VEC_BLOCK)
+    {
+        const int64_t o = 3 * (int64_t)row_of[i];
+        double        v[3] = {0.0, 0.0, 0.0};
+        if(o >= 0)
+#pragma unroll
+            for(int c = 0; c < 3; ++c)
+                v[c] = Ax ? b[o + c] - Ax[o + c] : b[o + c];
+        if constexpr(NS == 4)
+            reinterpret_cast<float4*>(r)[i] = make_float4((float)v[0], (float)v[1], (float)v[2], 0.0f);
+        else
+#pragma unroll
+            for(int c = 0; c < 3; ++c)
+                r[3 * (int64_t)i + c] = v[c];
+    }
+}
+
+// FP64 vector between the matrix's order and PCG order
+__global__ void k_to_ord(int32_t n, const int32_t* __restrict__ row_of, const double* __restrict__ x,
+                         double* __restrict__ xs)
+{
+    for(int i = blockIdx.x * VEC_BLOCK + threadIdx.x; i < n; i += gridDim.x * VEC_BLOCK)
+    {
+        const int64_t o = 3 * (int64_t)row_of[i];
+#pragma unroll
+        for(int c = 0; c < 3; ++c)
+            xs[3 * (int64_t)i + c] = o >= 0 ? x[o + c] : 0.0;
+    }
+}
+__global__ void k_from_ord(int32_t nb, const int32_t* __restrict__ pos, const double* __restrict__ xs,
+                           double* __restrict__ x)
+{
+    for(int r = blockIdx.x * VEC_BLOCK + threadIdx.x; r < nb; r += gridDim.x * VEC_BLOCK)
+    {
+        const int64_t i = 3 * (int64_t)pos[r];
+#pragma unroll
+        for(int c = 0; c < 3; ++c)
+            x[3 * (int64_t)r + c] = xs[i + c];
+    }
+}
+
+// the order: 1 for the rows outside the MAS slots, then their places
+__global__ void k_ord_other(int32_t nb, int off, int vn, const int32_t* __restrict__ r2p, int32_t* __restrict__ other)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if(i < nb)
+        other[i] = (i < off || i >= off + vn || r2p[i - off] < 0) ? 1 : 0;
+}
+__global__ void k_ord_pos(int32_t nb, int off, int vn, int slots, const int32_t* __restrict__ r2p,
+                          const int32_t* __restrict__ rank, int32_t* __restrict__ pos, int32_t* __restrict__ row_of)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if(i >= nb)
+        return;
+    const int p = (i >= off && i < off + vn) ? r2p[i - off] : -1;
+    const int q = p >= 0 ? p : slots + rank[i];
+    pos[i]      = q;
+    row_of[q]   = i;
+}
+__global__ void k_ord_node1(int slots, int begin1, const int32_t* __restrict__ new_local, int32_t* __restrict__ node1)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if(p < slots)
+        node1[p] = new_local[p] >= 0 ? begin1 + new_local[p] : -1;
+}
+
+// the matrix in that order: blocks per row (one at least), the rows' blocks
+// moved together (columns renumbered, the order inside a row kept; row and
+// column may swap sides, which a symmetric product does not mind), and the
+// zero diagonal blocks of the empty rows
+__global__ void k_ord_count(int32_t n, const int32_t* __restrict__ row_of, const int32_t* __restrict__ rowptr,
+                            int32_t* __restrict__ cnt)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if(i >= n)
+        return;
+    const int r = row_of[i];
+    cnt[i]      = r >= 0 ? max(rowptr[r + 1] - rowptr[r], 1) : 1;
+}
+template <typename VT>
+__global__ void k_ord_fill(int64_t U, int64_t S, int64_t So, const int32_t* __restrict__ pos,
+                           const int32_t* __restrict__ rowptr, const int32_t* __restrict__ rows,
+                           const int32_t* __restrict__ cols, const double* __restrict__ vals,
+                           const int32_t* __restrict__ rowptr_o, int32_t* __restrict__ rows_o,
+                           int32_t* __restrict__ cols_o, VT* __restrict__ vals_o)
+{
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if(k >= U)
+        return;
+    const int     r = rows[k], i = pos[r];
+    const int64_t d = (int64_t)rowptr_o[i] + (k - rowptr[r]);
+    rows_o[d]       = i;
+    cols_o[d]       = pos[cols[k]];
+#pragma unroll
+    for(int q = 0; q < 9; ++q)
+        vals_o[q * So + d] = (VT)vals[q * S + k];
+}
+template <typename VT>
+__global__ void k_ord_empty(int32_t n, int64_t So, const int32_t* __restrict__ row_of,
+                            const int32_t* __restrict__ rowptr, const int32_t* __restrict__ rowptr_o,
+                            int32_t* __restrict__ rows_o, int32_t* __restrict__ cols_o, VT* __restrict__ vals_o)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if(i >= n)
+        return;
+    const int     r = row_of[i];
+    const int64_t d = rowptr_o[i];
+    if(r < 0 || rowptr[r + 1] == rowptr[r])
+    {
+        rows_o[d] = i;
+        cols_o[d] = i;
+#pragma unroll
+        for(int q = 0; q < 9; ++q)
+            vals_o[q * So + d] = (VT)0;
+    }
+    if(i == n - 1)  // the padding of the stream
+        for(int64_t e = rowptr_o[n]; e < So; ++e)
+        {
+            rows_o[e] = -1;
+            cols_o[e] = 0;
+#pragma unroll
+            for(int q = 0; q < 9; ++q)
+                vals_o[q * So + e] = (VT)0;
+        }
 }
 
 // between the 3-per-node FP32 vectors of the ABI and the padded ones
@@ -554,7 +804,7 @@ void precond_assemble(b2s_solver* s, int kind, int invert_mode)
     B2S_CUDA(cudaStreamSynchronize(st));
 }
 
-static MasView mas_view(b2s_solver* s)
+MasView mas_view(b2s_solver* s)
 {
     MasView mv{};
     const MasState& M = s->mas;
@@ -567,9 +817,133 @@ static MasView mas_view(b2s_solver* s)
     mv.L      = M.L;
     mv.r2p    = M.r2p.data();
     mv.node1  = M.node1.data();
+    mv.anc    = M.anc.data();
+    mv.begin1 = M.L > 1 ? M.level_begin[1] : 0;
     mv.T      = M.L <= 1 ? 0 : M.L - 1;
     mv.Z      = M.Z.data();
+    mv.row_of     = s->pcg.ord.row_of.data();
+    mv.slot_node1 = s->pcg.ord.node1.data();
+    mv.slots      = s->pcg.ord.slots;
     return mv;
+}
+
+// the PCG order of the current MAS and matrix, and the matrix in it
+static void ensure_order(b2s_solver* s, bool f32)
+{
+    PcgOrder&       O  = s->pcg.ord;
+    const MasState& M  = s->mas;
+    const Matrix&   A  = s->A;
+    cudaStream_t    st = s->stream;
+    const int       TB = 256;
+    AssemblyScratch& w = s->asmb;
+    if(O.mas_generation != M.generation || O.nb != A.nb)
+    {
+        O.mas_generation = -1;
+        O.f64_generation = O.f32_generation = -1;
+        w.row_count.resize((size_t)A.nb + 1, 1.25);
+        w.row_start.resize((size_t)A.nb + 1, 1.25);
+        k_ord_other<<<grid_for(A.nb, TB), TB, 0, st>>>(A.nb, M.offset, M.vn, M.r2p.data(), w.row_count.data());
+        B2S_CHECK_LAUNCH();
+        exclusive_scan(s, w.row_count.data(), w.row_start.data(), A.nb, w.scan_tmp);
+        int32_t others = 0;
+        B2S_CUDA(cudaMemcpyAsync(&others, w.row_start.data() + A.nb, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        B2S_CUDA(cudaStreamSynchronize(st));
+        O.slots = M.N;
+        O.nb    = A.nb;
+        O.n     = M.N + others;
+        O.row_of.resize(O.n);
+        O.pos.resize(A.nb);
+        B2S_CUDA(cudaMemsetAsync(O.row_of.data(), 0xff, O.row_of.bytes(), st));
+        k_ord_pos<<<grid_for(A.nb, TB), TB, 0, st>>>(A.nb, M.offset, M.vn, M.N, M.r2p.data(), w.row_start.data(),
+                                                     O.pos.data(), O.row_of.data());
+        B2S_CHECK_LAUNCH();
+        O.node1.resize(M.N);
+        k_ord_node1<<<grid_for(M.N, TB), TB, 0, st>>>(M.N, M.L > 1 ? M.level_begin[1] : 0, M.new_local[0].data(),
+                                                      O.node1.data());
+        B2S_CHECK_LAUNCH();
+        O.mas_generation = M.generation;
+    }
+    if((f32 ? O.f32_generation : O.f64_generation) == A.generation)
+        return;
+    Matrix& P = O.A;
+    if(O.f32_generation != A.generation && O.f64_generation != A.generation)
+    {
+        w.row_count.resize((size_t)O.n + 1, 1.25);
+        P.rowptr.resize((size_t)O.n + 1, 1.25);
+        k_ord_count<<<grid_for(O.n, TB), TB, 0, st>>>(O.n, O.row_of.data(), A.rowptr.data(), w.row_count.data());
+        B2S_CHECK_LAUNCH();
+        exclusive_scan(s, w.row_count.data(), P.rowptr.data(), O.n, w.scan_tmp);
+        int32_t nnz = 0;
+        B2S_CUDA(cudaMemcpyAsync(&nnz, P.rowptr.data() + O.n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        B2S_CUDA(cudaStreamSynchronize(st));
+        P.nb     = O.n;
+        P.nnz    = nnz;
+        P.stride = (P.nnz + 15) / 16 * 16;
+        P.rows.resize(P.stride, 1.2);
+        P.cols.resize(P.stride, 1.2);
+        P.has_trank = P.has_groups = false;
+    }
+    auto fill = [&](auto* vals)
+    {
+        using VT = std::remove_pointer_t<decltype(vals)>;
+        if(A.nnz > 0)
+        {
+            k_ord_fill<VT><<<grid_for(A.nnz, TB), TB, 0, st>>>(A.nnz, A.stride, P.stride, O.pos.data(),
+                                                               A.rowptr.data(), A.rows.data(), A.cols.data(),
+                                                               A.vals.data(), P.rowptr.data(), P.rows.data(),
+                                                               P.cols.data(), vals);
+            B2S_CHECK_LAUNCH();
+        }
+        k_ord_empty<VT><<<grid_for(O.n, TB), TB, 0, st>>>(O.n, P.stride, O.row_of.data(), A.rowptr.data(),
+                                                          P.rowptr.data(), P.rows.data(), P.cols.data(), vals);
+        B2S_CHECK_LAUNCH();
+    };
+    if(f32)
+    {
+        P.vals32.resize((size_t)9 * P.stride, 1.2);
+        fill(P.vals32.data());
+        if(!P.has_groups)
+            build_row_groups_full(s, P);
+        O.f32_generation = A.generation;
+    }
+    else
+    {
+        P.vals.resize((size_t)9 * P.stride, 1.2);
+        fill(P.vals.data());
+        if(!P.has_trank)
+            build_tile_ranks(s, P);
+        O.f64_generation = A.generation;
+    }
+}
+
+// the restriction in PCG order, with the x, r update of the iteration
+// (UPDATE). Without an apply to follow (kind other than MAS) nothing is
+// restricted: the apply clears the coarse sums.
+template <typename VT, int NS, bool UPDATE>
+static void update_restrict_launch(b2s_solver* s, int kind, PcgScalars* sc, double* xs, const VT* p, VT* r, VT* Ap)
+{
+    const PcgOrder& O = s->pcg.ord;
+    MasState&       M = s->mas;
+    k_update_restrict<VT, NS, UPDATE><<<grid_for(O.n, VEC_BLOCK), VEC_BLOCK, 0, s->stream>>>(
+        O.n, O.slots, sc, xs, p, r, Ap, M.comp_mask[0].data(), M.new_local[0].data(), M.anc.data(),
+        M.L > 1 ? M.level_begin[1] : 0, M.L > 2 ? M.level_begin[2] : 0,
+        kind == B2S_PRECOND_MAS && M.L > 1 ? 1 : 0, M.R.data(), M.R64.data());
+    B2S_CHECK_LAUNCH();
+}
+
+// z = P r in PCG order from R_0 and R_1 (update_restrict_launch first), with
+// the dots and the scalar update of the iteration when `sc` is given
+template <typename VT, int NS>
+static void precond_launch_ord(b2s_solver* s, int kind, bool bf16, const VT* r, VT* z, PcgScalars* sc, Reduction& red)
+{
+    const int32_t n = s->pcg.ord.n;
+    if(kind == B2S_PRECOND_MAS)
+        mas_apply_all(s, sc ? &sc->converged : nullptr, bf16);
+    const int grid = reduction_grid(n);
+    ensure_reduction(red, grid, 2);
+    k_precond_finish<VT, NS, true><<<grid, RED_BLOCK, 0, s->stream>>>(n, kind, mas_view(s), s->dinv.data(), r, z, sc,
+                                                                     red.partials.data(), red.counter.data());
+    B2S_CHECK_LAUNCH();
 }
 
 // z = P r, optionally fused with the dots + scalar update of a PCG iteration
@@ -583,7 +957,7 @@ static void precond_launch(b2s_solver* s, int kind, const double* r, double* z, 
         mas_apply_levels(s, r, sc ? &sc->converged : nullptr);
     const int grid = reduction_grid(nb);
     ensure_reduction(red, grid, 2);
-    k_precond_finish<double, 3><<<grid, RED_BLOCK, 0, st>>>(nb, kind, mas_view(s), s->dinv.data(), r, z, sc,
+    k_precond_finish<double, 3, false><<<grid, RED_BLOCK, 0, st>>>(nb, kind, mas_view(s), s->dinv.data(), r, z, sc,
                                                  red.partials.data(), red.counter.data());
     B2S_CHECK_LAUNCH();
 }
@@ -609,7 +983,7 @@ namespace
 {
 struct GraphKey
 {
-    const void* ptrs[10];
+    const void* ptrs[14];
     int64_t     ints[6];
     bool operator==(const GraphKey& o) const { return std::memcmp(this, &o, sizeof(GraphKey)) == 0; }
 };
@@ -628,11 +1002,11 @@ static cudaError_t record_timing_event(cudaEvent_t ev, cudaStream_t st)
 }
 
 // one PCG iteration; with timing on, `slot` selects the 4 events that
-// bracket its SpMV and its preconditioner apply
-static void pcg_iteration(b2s_solver* s, int kind, double* x, int slot)
+// bracket its SpMV and its preconditioner apply. ord: in PCG order (MAS)
+static void pcg_iteration(b2s_solver* s, int kind, bool ord, double* x, int slot)
 {
     PcgState&     P  = s->pcg;
-    const Matrix& A  = s->A;
+    const Matrix& A  = ord ? P.ord.A : s->A;
     cudaStream_t  st = s->stream;
     const int64_t n  = 3 * (int64_t)A.nb;
     cudaEvent_t*  ev = s->timing ? &s->iter_events[(size_t)slot * 4] : nullptr;
@@ -641,11 +1015,19 @@ static void pcg_iteration(b2s_solver* s, int kind, double* x, int slot)
     spmv_f64_launch(s, A, P.p.data(), P.Ap.data(), P.red, &P.sc.data()->pAp, &P.sc.data()->converged);
     if(ev)
         B2S_CUDA(record_timing_event(ev[1], st));
-    k_update_xr<<<vec_grid(n), VEC_BLOCK, 0, st>>>(n, P.sc.data(), x, P.p.data(), P.r.data(), P.Ap.data());
-    B2S_CHECK_LAUNCH();
+    if(ord)
+        update_restrict_launch<double, 3, true>(s, kind, P.sc.data(), x, P.p.data(), P.r.data(), P.Ap.data());
+    else
+    {
+        k_update_xr<<<vec_grid(n), VEC_BLOCK, 0, st>>>(n, P.sc.data(), x, P.p.data(), P.r.data(), P.Ap.data());
+        B2S_CHECK_LAUNCH();
+    }
     if(ev)
         B2S_CUDA(record_timing_event(ev[2], st));
-    precond_launch(s, kind, P.r.data(), P.z.data(), P.sc.data(), P.red);
+    if(ord)
+        precond_launch_ord<double, 3>(s, kind, false, P.r.data(), P.z.data(), P.sc.data(), P.red);
+    else
+        precond_launch(s, kind, P.r.data(), P.z.data(), P.sc.data(), P.red);
     if(ev)
         B2S_CUDA(record_timing_event(ev[3], st));
     k_update_p<<<vec_grid(n), VEC_BLOCK, 0, st>>>(n, P.sc.data(), P.z.data(), P.p.data());
@@ -676,47 +1058,88 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
     B2S_REQUIRE(o.tol > 0.0 && std::isfinite(o.tol), B2S_ERR_ARGUMENT, "tolerance must be positive");
     B2S_REQUIRE(o.stop_rule == B2S_STOP_RZ || o.stop_rule == B2S_STOP_RELRES, B2S_ERR_ARGUMENT, "unknown stop rule");
     cudaStream_t  st = s->stream;
-    const Matrix& A  = s->A;
     PcgState&     P  = s->pcg;
-    const int64_t n  = 3 * (int64_t)A.nb;
+    const int64_t n0 = 3 * (int64_t)s->A.nb;  // b and x
     std::memset(&st_out, 0, sizeof(st_out));
-    if(n == 0)
+    if(n0 == 0)
     {
         st_out.converged = 1;
         return;
     }
+    B2S_REQUIRE(s->A.nnz == 0 || s->A.has_trank, B2S_ERR_STATE, "matrix lacks the SpMV tile ranks");
+    // with the MAS the recursion runs in its slot order (see PcgOrder)
+    const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized;
+    if(ord)
+        ensure_order(s, false);
+    const PcgOrder& O  = P.ord;
+    const Matrix&   A  = ord ? O.A : s->A;
+    const int64_t   n  = 3 * (int64_t)A.nb;  // the recursion's vectors
+    double*         xi = x;                  // the iterate
     P.r.resize(n, 1.1);
     P.z.resize(n, 1.1);
     P.p.resize(n, 1.1);
     P.Ap.resize(n, 1.1);
-    P.tmp.resize(n, 1.1);
+    P.tmp.resize(n0, 1.1);
+    if(ord)
+    {
+        P.xs.resize(n, 1.1);
+        xi = P.xs.data();
+    }
     P.sc.resize(1);
     if(!P.h_sc)
         B2S_CUDA(cudaMallocHost(&P.h_sc, sizeof(PcgScalars)));
     ensure_reduction(P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
     device_error_flag(s);  // allocated before any graph capture
-    B2S_REQUIRE(A.nnz == 0 || A.has_trank, B2S_ERR_STATE, "matrix lacks the SpMV tile ranks");
     s->dot_out.resize(4);
     const int ci = o.check_interval > 0 ? o.check_interval : 1;
-    const int64_t max_iter = o.max_iter > 0 ? o.max_iter : std::max<int64_t>(2 * n, 1);
+    const int64_t max_iter = o.max_iter > 0 ? o.max_iter : std::max<int64_t>(2 * n0, 1);
 
-    // r = b - A x0
-    if(o.x0_given)
+    // r = b - A x (x0 = 0: r = b), z = P r
+    auto residual = [&](bool zero)
     {
-        spmv_f64(s, A, x, P.tmp.data(), nullptr);
-        k_residual<<<vec_grid(n), VEC_BLOCK, 0, st>>>(n, b, P.tmp.data(), P.r.data());
+        if(!zero)
+            spmv_f64(s, s->A, x, P.tmp.data(), nullptr);
+        if(ord)
+            k_residual_ord<double, 3><<<vec_grid(A.nb), VEC_BLOCK, 0, st>>>(A.nb, O.row_of.data(), b,
+                                                                            zero ? nullptr : P.tmp.data(), P.r.data());
+        else if(!zero)
+            k_residual<<<vec_grid(n), VEC_BLOCK, 0, st>>>(n, b, P.tmp.data(), P.r.data());
+        else
+        {
+            B2S_CUDA(cudaMemcpyAsync(P.r.data(), b, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
+            return;
+        }
         B2S_CHECK_LAUNCH();
-    }
-    else
+    };
+    auto apply = [&](int k)
     {
-        B2S_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, st));
-        B2S_CUDA(cudaMemcpyAsync(P.r.data(), b, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
+        if(!ord)
+        {
+            precond_launch(s, k, P.r.data(), P.z.data(), nullptr, s->red);
+            return;
+        }
+        if(k == B2S_PRECOND_MAS)
+            update_restrict_launch<double, 3, false>(s, k, nullptr, nullptr, nullptr, P.r.data(), nullptr);
+        precond_launch_ord<double, 3>(s, k, false, P.r.data(), P.z.data(), nullptr, s->red);
+    };
+    if(!o.x0_given)
+        B2S_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n0, st));
+    residual(!o.x0_given);
+    if(ord)
+    {
+        if(o.x0_given)
+        {
+            k_to_ord<<<vec_grid(A.nb), VEC_BLOCK, 0, st>>>(A.nb, O.row_of.data(), x, xi);
+            B2S_CHECK_LAUNCH();
+        }
+        else
+            B2S_CUDA(cudaMemsetAsync(xi, 0, sizeof(double) * n, st));
     }
     int kind = s->precond_kind;
-    precond_launch(s, kind, P.r.data(), P.z.data(), nullptr, s->red);
+    apply(kind);
     launch_dot(s, P.r.data(), P.z.data(), n, s->dot_out.data());
     launch_dot(s, P.r.data(), P.r.data(), n, s->dot_out.data() + 1);
-    launch_dot(s, b, b, n, s->dot_out.data() + 2);
+    launch_dot(s, b, b, n0, s->dot_out.data() + 2);
     double h3[3];
     read_back(s, s->dot_out.data(), 3, h3);
     double rz0 = h3[0];
@@ -738,8 +1161,8 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
 
     auto true_residual = [&]() -> double
     {
-        spmv_f64(s, A, x, P.tmp.data(), nullptr);
-        k_res_norms<<<reduction_grid(n), RED_BLOCK, 0, st>>>(n, b, P.tmp.data(), s->red.partials.data(),
+        spmv_f64(s, s->A, x, P.tmp.data(), nullptr);
+        k_res_norms<<<reduction_grid(n0), RED_BLOCK, 0, st>>>(n0, b, P.tmp.data(), s->red.partials.data(),
                                                             s->red.counter.data(), s->dot_out.data());
         B2S_CHECK_LAUNCH();
         double h2[2];
@@ -780,7 +1203,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         if(use_graph)
         {
             GraphKey key{};
-            key.ptrs[0] = x;
+            key.ptrs[0] = xi;
             key.ptrs[1] = A.vals.data();
             key.ptrs[2] = A.rows.data();
             key.ptrs[3] = P.r.data();
@@ -789,13 +1212,17 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
             key.ptrs[6] = P.red.partials.data();
             key.ptrs[7] = s->mas.Z.data();
             key.ptrs[8] = A.cols.data();
-            key.ptrs[9] = b;
+            key.ptrs[9] = P.z.data();
+            key.ptrs[10] = P.p.data();
+            key.ptrs[11] = P.Ap.data();
+            key.ptrs[12] = A.trank.data();
+            key.ptrs[13] = O.row_of.data();
             key.ints[0] = A.nnz;
             key.ints[1] = A.nb;
             key.ints[2] = kind;
             key.ints[3] = ci;
             key.ints[4] = s->mas.initialized ? s->mas.total : -1;
-            key.ints[5] = s->mas.L + (s->timing ? 1000 : 0);
+            key.ints[5] = s->mas.generation * 2 + (s->timing ? 1 : 0);
             size_t hk = 1469598103934665603ull;
             const unsigned char* kb = reinterpret_cast<const unsigned char*>(&key);
             for(size_t q = 0; q < sizeof(key); ++q)
@@ -811,7 +1238,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
                 const long long before = g_kernel_launches;
                 B2S_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
                 for(int it = 0; it < ci; ++it)
-                    pcg_iteration(s, kind, x, it);
+                    pcg_iteration(s, kind, ord, xi, it);
                 B2S_CUDA(cudaStreamEndCapture(st, &g));
                 P.graph_kernels = g_kernel_launches - before;
                 g_kernel_launches = before;
@@ -837,7 +1264,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
             }
             else
                 for(int it = 0; it < ci; ++it)
-                    pcg_iteration(s, kind, x, it);
+                    pcg_iteration(s, kind, ord, xi, it);
             B2S_CUDA(cudaMemcpyAsync(P.h_sc, P.sc.data(), sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
             B2S_CUDA(cudaStreamSynchronize(st));
             if(s->timing)
@@ -861,6 +1288,11 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         }
         const PcgScalars r = *P.h_sc;
         iter_total         = r.iter;
+        if(ord)
+        {
+            k_from_ord<<<vec_grid(O.nb), VEC_BLOCK, 0, st>>>(O.nb, O.pos.data(), xi, x);
+            B2S_CHECK_LAUNCH();
+        }
         if(r.converged == 3)
             throw Error(B2S_ERR_NUMERIC, "PCG breakdown: r.z became non-finite at iteration " + std::to_string(r.iter));
         st_out.iterations_exact = r.converged == 1 ? r.iter_conv : r.iter;
@@ -872,10 +1304,8 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         {
             // the recursive residual drifted from b - A x: replace it and continue
             ++replacements;
-            spmv_f64(s, A, x, P.tmp.data(), nullptr);
-            k_residual<<<vec_grid(n), VEC_BLOCK, 0, st>>>(n, b, P.tmp.data(), P.r.data());
-            B2S_CHECK_LAUNCH();
-            precond_launch(s, kind, P.r.data(), P.z.data(), nullptr, s->red);
+            residual(false);
+            apply(kind);
             launch_dot(s, P.r.data(), P.z.data(), n, s->dot_out.data());
             read_back(s, s->dot_out.data(), 1, &h.rz);
             done = false;
@@ -926,7 +1356,7 @@ static void precond_launch_f32(b2s_solver* s, int kind, const float* r, float* z
         mas_apply_levels_f32(s, r, sc ? &sc->converged : nullptr, mixed_inverse_bf16());
     const int grid = reduction_grid(nb);
     ensure_reduction(red, grid, 2);
-    k_precond_finish<float, 4><<<grid, RED_BLOCK, 0, s->stream>>>(nb, kind, mas_view(s), s->dinv.data(), r, z, sc,
+    k_precond_finish<float, 4, false><<<grid, RED_BLOCK, 0, s->stream>>>(nb, kind, mas_view(s), s->dinv.data(), r, z, sc,
                                                                red.partials.data(), red.counter.data());
     B2S_CHECK_LAUNCH();
 }
@@ -1025,10 +1455,10 @@ void precond_apply_mixed(b2s_solver* s, const float* r, float* z)
     read_back(s, nullptr, 0, nullptr);
 }
 
-static void pcg_iteration_mixed(b2s_solver* s, int kind, double* x, int slot)
+static void pcg_iteration_mixed(b2s_solver* s, int kind, bool ord, double* x, int slot)
 {
     PcgState&     P  = s->pcg;
-    const Matrix& A  = s->A;
+    const Matrix& A  = ord ? P.ord.A : s->A;
     cudaStream_t  st = s->stream;
     const int32_t nb = A.nb;
     cudaEvent_t*  ev = s->timing ? &s->iter_events[(size_t)slot * 4] : nullptr;
@@ -1037,12 +1467,20 @@ static void pcg_iteration_mixed(b2s_solver* s, int kind, double* x, int slot)
     spmv_f32_launch(s, A, P.p32.data(), P.Ap32.data(), P.red, &P.sc.data()->pAp, &P.sc.data()->converged);
     if(ev)
         B2S_CUDA(record_timing_event(ev[1], st));
-    k_update_xr_mixed4<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, P.sc.data(), x, P.p32.data(), P.r32.data(),
-                                                           P.Ap32.data());
-    B2S_CHECK_LAUNCH();
+    if(ord)
+        update_restrict_launch<float, 4, true>(s, kind, P.sc.data(), x, P.p32.data(), P.r32.data(), P.Ap32.data());
+    else
+    {
+        k_update_xr_mixed4<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, P.sc.data(), x, P.p32.data(), P.r32.data(),
+                                                               P.Ap32.data());
+        B2S_CHECK_LAUNCH();
+    }
     if(ev)
         B2S_CUDA(record_timing_event(ev[2], st));
-    precond_launch_f32(s, kind, P.r32.data(), P.z32.data(), P.sc.data(), P.red);
+    if(ord)
+        precond_launch_ord<float, 4>(s, kind, mixed_inverse_bf16(), P.r32.data(), P.z32.data(), P.sc.data(), P.red);
+    else
+        precond_launch_f32(s, kind, P.r32.data(), P.z32.data(), P.sc.data(), P.red);
     if(ev)
         B2S_CUDA(record_timing_event(ev[3], st));
     k_update_p_mixed4<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, P.sc.data(), P.z32.data(), P.p32.data(),
@@ -1061,17 +1499,33 @@ static void pcg_iteration_mixed(b2s_solver* s, int kind, double* x, int slot)
 void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_options& o, b2s_pcg_stats& st_out)
 {
     cudaStream_t st = s->stream;
-    Matrix&      A  = s->A;
     PcgState&    P  = s->pcg;
-    const int64_t n = 3 * (int64_t)A.nb;
+    const int64_t n = 3 * (int64_t)s->A.nb;  // b and x
     std::memset(&st_out, 0, sizeof(st_out));
     if(n == 0)
     {
         st_out.converged = 1;
         return;
     }
-    const int32_t nb = A.nb;
-    const int64_t n4 = 4 * (int64_t)nb;  // padded FP32 vectors
+    B2S_REQUIRE(s->A.nnz == 0 || s->A.has_trank, B2S_ERR_STATE, "matrix lacks the SpMV tile ranks");
+    // FP32 matrix planes (in the MAS slot order with the MAS, see PcgOrder) and
+    // BF16 inverses: once per assembly / build
+    const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized;
+    if(ord)
+        ensure_order(s, true);
+    else
+        ensure_f32_planes(s);
+    ensure_bf16_inverses(s);
+    const PcgOrder& O  = P.ord;
+    const Matrix&   A  = ord ? O.A : s->A;
+    const int32_t   nb = A.nb;               // the recursion's rows
+    const int64_t   n4 = 4 * (int64_t)nb;  // padded FP32 vectors
+    double*         xi = x;                    // the iterate
+    if(ord)
+    {
+        P.xs.resize(3 * (size_t)nb, 1.1);
+        xi = P.xs.data();
+    }
     P.r32.resize(n4, 1.1);
     P.z32.resize(n4, 1.1);
     P.p32.resize(n4, 1.1);
@@ -1084,31 +1538,59 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
     ensure_reduction(s->red, reduction_grid(), 2);
     device_error_flag(s);
     s->dot_out.resize(4);
-    B2S_REQUIRE(A.nnz == 0 || A.has_trank, B2S_ERR_STATE, "matrix lacks the SpMV tile ranks");
     const int     ci       = o.check_interval > 0 ? o.check_interval : 1;
     const int64_t max_iter = o.max_iter > 0 ? o.max_iter : std::max<int64_t>(2 * n, 1);
     int           kind     = s->precond_kind;
 
-    // FP32 matrix planes, BF16 MAS inverses (once per assembly / build)
-    ensure_f32_planes(s);
-    ensure_bf16_inverses(s);
-
-    // r = b - A x0 (FP64), stored FP32
-    if(o.x0_given)
-        spmv_f64(s, A, x, P.tmp.data(), nullptr);
-    else
+    // r = b - A x (FP64; x0 = 0: r = b), stored FP32
+    auto residual = [&](bool zero)
     {
+        if(!zero)
+            spmv_f64(s, s->A, x, P.tmp.data(), nullptr);
+        if(ord)
+            k_residual_ord<float, 4><<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, O.row_of.data(), b,
+                                                                         zero ? nullptr : P.tmp.data(), P.r32.data());
+        else
+        {
+            if(zero)
+                B2S_CUDA(cudaMemsetAsync(P.tmp.data(), 0, sizeof(double) * n, st));
+            k_residual_f32<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, b, P.tmp.data(), P.r32.data());
+        }
+        B2S_CHECK_LAUNCH();
+    };
+    auto store_x = [&]()
+    {
+        if(!ord)
+            return;
+        k_from_ord<<<vec_grid(O.nb), VEC_BLOCK, 0, st>>>(O.nb, O.pos.data(), xi, x);
+        B2S_CHECK_LAUNCH();
+    };
+    if(!o.x0_given)
         B2S_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, st));
-        B2S_CUDA(cudaMemsetAsync(P.tmp.data(), 0, sizeof(double) * n, st));
+    residual(!o.x0_given);
+    if(ord)
+    {
+        if(o.x0_given)
+        {
+            k_to_ord<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, O.row_of.data(), x, xi);
+            B2S_CHECK_LAUNCH();
+        }
+        else
+            B2S_CUDA(cudaMemsetAsync(xi, 0, sizeof(double) * 3 * (size_t)nb, st));
     }
-    k_residual_f32<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, b, P.tmp.data(), P.r32.data());
-    B2S_CHECK_LAUNCH();
 
     double bb = 0.0;  // b.b (dot_out[2])
     auto restart_from_r = [&](int k) -> double
     {
         // z = P r, p = z; returns r.z (FP64 sum); also leaves r.r in dot_out[1]
-        precond_launch_f32(s, k, P.r32.data(), P.z32.data(), nullptr, s->red);
+        if(ord)
+        {
+            if(k == B2S_PRECOND_MAS)
+                update_restrict_launch<float, 4, false>(s, k, nullptr, nullptr, nullptr, P.r32.data(), nullptr);
+            precond_launch_ord<float, 4>(s, k, mixed_inverse_bf16(), P.r32.data(), P.z32.data(), nullptr, s->red);
+        }
+        else
+            precond_launch_f32(s, k, P.r32.data(), P.z32.data(), nullptr, s->red);
         k_dot2_f32<<<reduction_grid(n4), RED_BLOCK, 0, st>>>(n4, P.r32.data(), P.z32.data(), s->red.partials.data(),
                                                             s->red.counter.data(), s->dot_out.data());
         B2S_CHECK_LAUNCH();
@@ -1133,19 +1615,13 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
     const double bnorm = std::sqrt(bb);
     auto true_residual = [&]() -> double
     {
-        spmv_f64(s, A, x, P.tmp.data(), nullptr);
+        spmv_f64(s, s->A, x, P.tmp.data(), nullptr);
         k_res_norms<<<reduction_grid(n), RED_BLOCK, 0, st>>>(n, b, P.tmp.data(), s->red.partials.data(),
                                                             s->red.counter.data(), s->dot_out.data());
         B2S_CHECK_LAUNCH();
         double h2[2];
         read_back(s, s->dot_out.data(), 2, h2);
         return h2[1] > 0 ? std::sqrt(h2[0] / h2[1]) : 0.0;
-    };
-    auto replace_residual = [&]()
-    {
-        spmv_f64(s, A, x, P.tmp.data(), nullptr);
-        k_residual_f32<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, b, P.tmp.data(), P.r32.data());
-        B2S_CHECK_LAUNCH();
     };
     if(rz0 == 0.0 || bb == 0.0)
     {
@@ -1174,11 +1650,12 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
             ensure_iter_events(s, ci);
         if(use_graph)
         {
-            const void*   ptrs[12] = {x,          A.vals32.data(), A.rows.data(),     P.r32.data(),
+            const void*   ptrs[15] = {xi,         A.vals32.data(), A.rows.data(),     P.r32.data(),
                                       s->mas.inv16.data(), s->dinv.data(), P.red.partials.data(), s->mas.Z.data(),
-                                      A.cols.data(), P.p32.data(), P.Ap32.data(), P.z32.data()};
+                                      A.cols.data(), P.p32.data(), P.Ap32.data(), P.z32.data(),
+                                      A.grp_row.data(), A.grp_mask.data(), O.row_of.data()};
             const int64_t ints[6]  = {A.nnz, A.nb, kind, ci, s->mas.initialized ? s->mas.total : -1,
-                                      s->mas.L + (s->timing ? 1000 : 0)};
+                                      s->mas.generation * 2 + (s->timing ? 1 : 0)};
             size_t hk = 1469598103934665603ull;
             for(const void* q : ptrs)
                 hk = (hk ^ (size_t)q) * 1099511628211ull;
@@ -1195,7 +1672,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
                 const long long before = g_kernel_launches;
                 B2S_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
                 for(int it = 0; it < ci; ++it)
-                    pcg_iteration_mixed(s, kind, x, it);
+                    pcg_iteration_mixed(s, kind, ord, xi, it);
                 B2S_CUDA(cudaStreamEndCapture(st, &g));
                 P.graph_mixed_kernels = g_kernel_launches - before;
                 g_kernel_launches     = before;
@@ -1221,7 +1698,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
             }
             else
                 for(int it = 0; it < ci; ++it)
-                    pcg_iteration_mixed(s, kind, x, it);
+                    pcg_iteration_mixed(s, kind, ord, xi, it);
             B2S_CUDA(cudaMemcpyAsync(P.h_sc, P.sc.data(), sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
             B2S_CUDA(cudaStreamSynchronize(st));
             if(s->timing)
@@ -1244,13 +1721,15 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
             if(o.replace_every > 0 && P.h_sc->iter - last_replace >= o.replace_every)
             {
                 // reliable update: FP64 residual of the FP64 iterate, p and r.z kept
-                replace_residual();
+                store_x();
+                residual(false);
                 ++replacements;
                 last_replace = P.h_sc->iter;
             }
         }
         const PcgScalars r = *P.h_sc;
         iter_total         = r.iter;
+        store_x();
         if(r.converged == 3)
             throw Error(B2S_ERR_NUMERIC, "mixed PCG breakdown: r.z non-finite at iteration " + std::to_string(r.iter));
         st_out.iterations_exact = r.converged == 1 ? r.iter_conv : r.iter;
@@ -1262,7 +1741,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
         {
             // the FP32 recursion claimed a stop the FP64 residual does not
             // confirm: continue from the true residual
-            replace_residual();
+            residual(false);
             ++replacements;
             last_replace = iter_total;
             h.rz         = restart_from_r(kind);

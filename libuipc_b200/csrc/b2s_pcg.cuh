@@ -1,0 +1,26 @@
+// What the PCG's kernels share: the preconditioner as they read it.
+#pragma once
+#include "b2s_internal.cuh"
+
+namespace b2s
+{
+struct MasView
+{
+    int            active;  // MAS present
+    int            off, vn, L;
+    int            abd_off, abd_n;  // affine-body range: block rows abd_off .. abd_off + 4 abd_n
+    const double*  abd_inv;         // [abd_n * 144]
+    const int32_t* r2p;
+    const int32_t* node1;  // [vn] level-1 node of each vertex (global slot)
+    const int4*    anc;    // per level-1 node: its ancestors' slots (-1: none)
+    int            begin1;  // first level-1 slot
+    int            T;      // coarse levels (L-1)
+    const float*   Z;      // node values by slot
+    // rows in PCG order (null: the matrix's own order)
+    const int32_t* row_of;
+    const int32_t* slot_node1;  // [slots]
+    int            slots;
+};
+
+MasView mas_view(b2s_solver* s);
+}  // namespace b2s

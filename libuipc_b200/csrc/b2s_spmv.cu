@@ -585,6 +585,20 @@ void build_row_groups(b2s_solver* s, Matrix& A)
     A.has_groups = h == 0;
 }
 
+// the same for a matrix whose rows all hold a block: no gap to look for, and
+// nothing for the host to wait for
+void build_row_groups_full(b2s_solver* s, Matrix& A)
+{
+    const int64_t G = (A.nnz + 127) / 128;
+    A.grp_row.resize(G, 1.2);
+    A.grp_mask.resize(G, 1.2);
+    s->asmb.err.resize(1);
+    k_row_groups<<<(unsigned)((G + 7) / 8), 256, 0, s->stream>>>(A.nnz, G, A.rows.data(), A.grp_row.data(),
+                                                                 A.grp_mask.data(), s->asmb.err.data());
+    B2S_CHECK_LAUNCH();
+    A.has_groups = true;
+}
+
 // ---------------------------------------------------------------------------
 // plain dot product (deterministic)
 // ---------------------------------------------------------------------------

@@ -1,0 +1,103 @@
+"""The PCG in MAS slot order against direct solves: padded parts, vertices left
+out of the partition, block rows outside the MAS range on both sides, an empty
+row, affine bodies, x0 given or not, FP64 and mixed, graph and stream-ordered;
+the same handle used again with another partition and another matrix size."""
+import numpy as np
+import pytest
+
+from conftest import to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(rng, n, before, after, bodies):
+    """SPD block system: 4*bodies body rows, `before` rows, n mesh rows, `after`
+    rows, the last of them empty; a random mesh graph with couplings out of it."""
+    nb = 4 * bodies + before + n + after
+    off = 4 * bodies + before
+    edges = {(min(a, b), max(a, b)) for a in range(n) for b in (a + 1, a + 2, a + 5, a + 11) if b < n}
+    rows, cols, vals = [], [], []
+
+    def add(i, j, B):
+        if i > j:
+            i, j, B = j, i, B.T
+        rows.append(i), cols.append(j), vals.append(B.T.ravel())
+
+    last = nb - 1 if after else nb
+    links = [(off + a, off + b) for a, b in sorted(edges)]
+    links += [(int(rng.integers(0, off)), off + int(rng.integers(0, n))) for _ in range(n // 8 if off else 0)]
+    links += [(off + int(rng.integers(0, n)), int(rng.integers(off + n, last))) for _ in range(n // 8 if last > off + n else 0)]
+    for i, j in links:
+        Q = rng.normal(size=(3, 3))
+        K = Q @ Q.T + 0.1 * np.eye(3)
+        add(i, i, K), add(j, j, K), add(i, j, -K)
+    for i in range(last):
+        add(i, i, 0.3 * np.eye(3))
+    for b in range(bodies):
+        Q = rng.normal(size=(12, 12))
+        M = Q @ Q.T + np.eye(12)
+        for i in range(4):
+            for j in range(4):
+                add(4 * b + i, 4 * b + j, M[3 * i:3 * i + 3, 3 * j:3 * j + 3]) if i <= j else None
+    rows, cols, vals = np.array(rows, np.int32), np.array(cols, np.int32), np.array(vals)
+    A = np.zeros((3 * nb, 3 * nb))
+    for i, j, v in zip(rows, cols, vals):
+        B = v.reshape(3, 3).T
+        A[3 * i:3 * i + 3, 3 * j:3 * j + 3] += B
+        if i != j:
+            A[3 * j:3 * j + 3, 3 * i:3 * i + 3] += B.T
+    e = np.array(sorted(edges) + [(b, a) for a, b in sorted(edges)])
+    e = e[np.lexsort((e[:, 1], e[:, 0]))]
+    start = np.zeros(n + 1, np.int32)
+    start[1:] = np.cumsum(np.bincount(e[:, 0], minlength=n))
+    return nb, off, rows, cols, vals, A, last, start, e[:, 1].astype(np.int32)
+
+
+def _maps(rng, n, part, skip):
+    """Parts of `part` consecutive vertices padded to 16, holes anywhere in a
+    bank, `skip` vertices unpartitioned."""
+    out = rng.permutation(n)[:skip]
+    keep = np.setdiff1d(np.arange(n), out)
+    p2r = []
+    for k in range(0, keep.size, part):
+        lanes = np.full(16, -1)
+        vs = keep[k:k + part]
+        lanes[np.sort(rng.permutation(16)[:vs.size])] = vs
+        p2r.append(lanes)
+    p2r = np.concatenate(p2r).astype(np.int32)
+    r2p = np.full(n, -1, np.int32)
+    r2p[p2r[p2r >= 0]] = np.nonzero(p2r >= 0)[0]
+    return p2r, r2p
+
+
+@pytest.mark.parametrize("n,before,after,bodies,part,skip", [
+    (16, 0, 0, 0, 16, 0), (40, 0, 0, 0, 13, 0), (130, 5, 0, 0, 16, 7), (333, 0, 9, 0, 11, 0), (300, 3, 4, 3, 16, 40)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_pcg_in_slot_order(solver, cuda, n, before, after, bodies, part, skip, precision):
+    import torch
+
+    rng = np.random.default_rng(n + precision)
+    for again in range(2):  # a second matrix and partition on the same handle
+        nb, off, rows, cols, vals, A, last, start, lst = _system(rng, n - again, before, after, bodies)
+        m = n - again
+        solver.assemble(nb, to_dev(rows, cuda), to_dev(cols, cuda), to_dev(vals, cuda))
+        solver.abd_init(0, 0)
+        solver.mas_init(off, m, start, lst, *_maps(rng, m, part, skip))
+        solver.abd_init(0, bodies)
+        solver.precond_assemble(2)
+        b = rng.normal(size=3 * nb)
+        b[3 * last:] = 0.0
+        ref = np.zeros(3 * nb)
+        ref[:3 * last] = np.linalg.solve(A[:3 * last, :3 * last], b[:3 * last])
+        bd = to_dev(b, cuda)
+        for given, graph in ((False, True), (True, True), (True, False)):
+            x = to_dev(ref + 0.1 * rng.normal(size=3 * nb) * (np.arange(3 * nb) < 3 * last), cuda)
+            st = solver.pcg(bd, x, tol=1e-11, stop_rule=1, x0_given=given, precision=precision, use_graph=graph,
+                            replace_every=10 if precision and graph else 0)
+            assert st["converged"] == 1 and st["bypassed"] == 0
+            # |dx| <= |A^-1| |r|, |r| <= 1e-11 |b|
+            lim = 1e-11 * np.linalg.norm(b) * np.linalg.norm(np.linalg.inv(A[:3 * last, :3 * last]), 2) * 1.01
+            assert np.linalg.norm(x.cpu().numpy() - ref) <= lim + 1e-13 * np.linalg.norm(ref)
+        x = torch.full((3 * nb,), 7.0, dtype=torch.float64, device=cuda)
+        st = solver.pcg(bd, x, tol=1e-11, stop_rule=1, precision=precision, max_iter=3)
+        assert st["converged"] == 0 and bool(torch.isfinite(x).all())
