@@ -42,6 +42,7 @@ SOLVE_SOURCES = [
     "b2s_mas.cu",
     "b2s_mas_invert.cu",
     "b2s_pcg.cu",
+    "b2s_pcg_small.cu",
     "b2s_learned.cu",
     "b2s_generate.cu",
     "b2s_generate_shell.cu",

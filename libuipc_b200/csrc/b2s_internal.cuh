@@ -247,6 +247,8 @@ struct PcgOrder
 struct PcgState
 {
     PcgOrder     ord;
+    DBuf<double>   small_partials;  // one-launch loop: block sums, barrier counter
+    DBuf<unsigned> small_bar;
     DBuf<double> xs;  // the solution in PCG order
     DBuf<double> r, z, p, Ap, tmp;
     DBuf<PcgScalars> sc;

@@ -981,6 +981,9 @@ void precond_launch(b2s_solver* s, const double* r, double* z)
 // ---------------------------------------------------------------------------
 namespace
 {
+// iterations per launch of the one-launch loop at most (bounds its duration)
+constexpr long long SMALL_LOOP = 1 << 14;
+
 struct GraphKey
 {
     const void* ptrs[14];
@@ -1198,9 +1201,11 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
 
         // CUDA graph of `ci` iterations (re-captured when anything it bakes in changes)
         bool use_graph = o.use_graph && st != nullptr;
+        // small systems: the whole loop in one launch
+        const bool small = use_graph && !s->timing && pcg_small_fits(s, A, kind, ord, false);
         if(s->timing)
             ensure_iter_events(s, ci);
-        if(use_graph)
+        if(use_graph && !small)
         {
             GraphKey key{};
             key.ptrs[0] = xi;
@@ -1257,7 +1262,9 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         long long iter_before = h.iter;
         while(true)
         {
-            if(use_graph)
+            if(small)
+                pcg_small_launch(s, A, kind, ord, SMALL_LOOP, xi);
+            else if(use_graph)
             {
                 B2S_CUDA(cudaGraphLaunch(P.graph, st));
                 g_kernel_launches += P.graph_kernels;
@@ -1646,9 +1653,12 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
         B2S_CUDA(cudaMemcpyAsync(P.sc.data(), &h, sizeof(h), cudaMemcpyHostToDevice, st));
         B2S_CUDA(cudaMemsetAsync(P.Ap32.data(), 0, sizeof(float) * n4, st));
         bool use_graph = o.use_graph && st != nullptr;
+        // small systems: the loop in one launch, up to the next replacement
+        const bool small = use_graph && !s->timing && (kind != B2S_PRECOND_MAS || mixed_inverse_bf16())
+                           && pcg_small_fits(s, A, kind, ord, true);
         if(s->timing)
             ensure_iter_events(s, ci);
-        if(use_graph)
+        if(use_graph && !small)
         {
             const void*   ptrs[15] = {xi,         A.vals32.data(), A.rows.data(),     P.r32.data(),
                                       s->mas.inv16.data(), s->dinv.data(), P.red.partials.data(), s->mas.Z.data(),
@@ -1691,7 +1701,14 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
         long long iter_before = h.iter;
         while(true)
         {
-            if(use_graph)
+            if(small)
+            {
+                // whole blocks of check_interval, as the replacements are counted
+                const long long due = o.replace_every > 0 ? std::max<long long>(last_replace + o.replace_every - iter_before, 1) :
+                                                            SMALL_LOOP;
+                pcg_small_launch_f32(s, A, kind, ord, std::min<long long>((due + ci - 1) / ci * ci, SMALL_LOOP), xi);
+            }
+            else if(use_graph)
             {
                 B2S_CUDA(cudaGraphLaunch(P.graph_mixed, st));
                 g_kernel_launches += P.graph_mixed_kernels;

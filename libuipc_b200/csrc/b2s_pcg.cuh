@@ -1,4 +1,5 @@
-// What the PCG's kernels share: the preconditioner as they read it.
+// What the PCG's kernels share: the preconditioner as they read it, and the
+// one-launch loop of small systems.
 #pragma once
 #include "b2s_internal.cuh"
 
@@ -23,4 +24,11 @@ struct MasView
 };
 
 MasView mas_view(b2s_solver* s);
+
+// One launch for up to `iterations` PCG iterations (b2s_pcg_small.cu): A and
+// the vectors in PCG order with the MAS (`ord`), r, p and x set by the caller,
+// Ap zero, the scalars in s->pcg.sc (read and written back).
+bool pcg_small_fits(b2s_solver* s, const Matrix& A, int kind, bool ord, bool f32);
+void pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x);
+void pcg_small_launch_f32(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x);
 }  // namespace b2s
