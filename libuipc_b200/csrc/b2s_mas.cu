@@ -327,6 +327,160 @@ __global__ void k_g_extract(int64_t U, const int32_t* rows, const int32_t* cols,
         dst[q] = vals[(int64_t)q * S + k];
 }
 
+// The last coarse levels in one CTA: while a level's matrix has at most
+// TAIL_BLOCKS blocks, every further level -- restriction, sort by (row, column,
+// source), sums in source order, extraction of the clusters -- is a few
+// microseconds of work that the general assembly spreads over a dozen launches
+// and a wait of the host (about 50 us per level whatever its size). Same order
+// of the sums as there.
+constexpr int TAIL_BLOCKS  = 2048;
+constexpr int TAIL_THREADS = 1024;
+struct TailLevel
+{
+    int            begin;  // first node slot
+    const int32_t* map;    // node of the level below -> node of this level
+    int32_t*       rows;
+    int32_t*       cols;
+    double*        vals;  // planes of TAIL_BLOCKS
+};
+struct TailArgs
+{
+    int            first, L;
+    int            U;  // blocks of level first - 1
+    const int32_t* rows;
+    const int32_t* cols;
+    const double*  vals;
+    int64_t        S;
+    TailLevel      lv[MAX_LEVELS];
+    double*        hess;
+};
+constexpr size_t TAIL_SMEM = (size_t)TAIL_BLOCKS * (9 * sizeof(double) + sizeof(uint64_t));
+
+__global__ void __launch_bounds__(TAIL_THREADS) k_coarse_tail(TailArgs A)
+{
+    extern __shared__ double s_val[];  // [TAIL_BLOCKS][9], then the keys
+    uint64_t*      s_key = reinterpret_cast<uint64_t*>(s_val + 9 * TAIL_BLOCKS);
+    __shared__ int s_start[TAIL_BLOCKS + 1], s_warp[TAIL_THREADS / 32];
+    const int      tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    int            n = A.U;
+    const int32_t* rows = A.rows;
+    const int32_t* cols = A.cols;
+    const double*  vals = A.vals;
+    int64_t        S    = A.S;
+    for(int l = A.first; l < A.L; ++l)
+    {
+        const TailLevel& T = A.lv[l];
+        int              n2 = 32;
+        while(n2 < n)
+            n2 <<= 1;
+        // keys (row << 38 | column << 12 | source) and values as restricted
+        for(int k = tid; k < n2; k += TAIL_THREADS)
+        {
+            uint64_t key = ~0ull;
+            if(k < n)
+            {
+                const int a = rows[k], b = cols[k], ca = T.map[a], cb = T.map[b];
+                if(ca >= 0 && cb >= 0)
+                {
+                    const int lo = ca < cb ? ca : cb, hi = ca < cb ? cb : ca;
+                    key = ((uint64_t)lo << 38) | ((uint64_t)hi << 12) | (uint64_t)k;
+                    double B[9];
+#pragma unroll
+                    for(int q = 0; q < 9; ++q)
+                        B[q] = vals[q * S + k];
+#pragma unroll
+                    for(int q = 0; q < 9; ++q)
+                    {
+                        const double t = B[(q % 3) * 3 + q / 3];
+                        s_val[9 * k + q] = ca < cb || a == b ? B[q] : (ca > cb ? t : B[q] + t);
+                    }
+                }
+            }
+            s_key[k] = key;
+        }
+        __syncthreads();
+        for(int size = 2; size <= n2; size <<= 1)
+            for(int stride = size >> 1; stride > 0; stride >>= 1)
+            {
+                for(int i = tid; i < n2 / 2; i += TAIL_THREADS)
+                {
+                    const int      lo = 2 * i - (i & (stride - 1));
+                    const int      hi = lo + stride;
+                    const bool     up = (lo & size) == 0;
+                    const uint64_t x = s_key[lo], y = s_key[hi];
+                    if((x > y) == up)
+                    {
+                        s_key[lo] = y;
+                        s_key[hi] = x;
+                    }
+                }
+                __syncthreads();
+            }
+        // run starts: two consecutive positions per thread
+        bool head[2], end[2];
+#pragma unroll
+        for(int j = 0; j < 2; ++j)
+        {
+            const int p = 2 * tid + j;
+            const bool in = p < n2 && s_key[p] != ~0ull;
+            head[j] = in && (p == 0 || (s_key[p - 1] >> 12) != (s_key[p] >> 12));
+            end[j]  = in && (p + 1 == n2 || s_key[p + 1] == ~0ull);
+        }
+        int v = (int)head[0] + (int)head[1], incl = v;
+#pragma unroll
+        for(int o = 1; o < 32; o <<= 1)
+        {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            incl += lane >= o ? t : 0;
+        }
+        if(lane == 31)
+            s_warp[w] = incl;
+        __syncthreads();
+        int slot = incl - v, U = 0;
+#pragma unroll
+        for(int q = 0; q < TAIL_THREADS / 32; ++q)
+        {
+            slot += q < w ? s_warp[q] : 0;
+            U += s_warp[q];
+        }
+#pragma unroll
+        for(int j = 0; j < 2; ++j)
+        {
+            if(head[j])
+                s_start[slot++] = 2 * tid + j;
+            if(end[j])
+                s_start[U] = 2 * tid + j + 1;
+        }
+        __syncthreads();
+        for(int e = tid; e < 9 * U; e += TAIL_THREADS)
+        {
+            const int      o = e / 9, q = e - 9 * o, b = s_start[o], f = s_start[o + 1];
+            const uint64_t key = s_key[b];
+            const int      r = (int)(key >> 38), c = (int)((key >> 12) & 0x3FFFFFFu);
+            double         acc = s_val[9 * (int)(key & 0xFFFu) + q];
+            for(int k = b + 1; k < f; ++k)
+                acc += s_val[9 * (int)(s_key[k] & 0xFFFu) + q];
+            T.vals[(int64_t)q * TAIL_BLOCKS + o] = acc;
+            if(r / BANK == c / BANK)
+            {
+                const int gr = T.begin + r, gc = T.begin + c;
+                A.hess[((size_t)(gr / BANK) * SYM + sym_index(gr % BANK, gc % BANK)) * 9 + q] = acc;
+            }
+            if(q == 0)
+            {
+                T.rows[o] = r;
+                T.cols[o] = c;
+            }
+        }
+        __syncthreads();  // the level's matrix is visible to the CTA, the shared arrays are free
+        n    = U;
+        rows = T.rows;
+        cols = T.cols;
+        vals = T.vals;
+        S    = TAIL_BLOCKS;
+    }
+}
+
 // pack the FP32 inverse M of every cluster as D (FP32) + the BF16 tiles of
 // D^-1 M D^-1, D = diag(M)^1/2: the stored matrix has a unit diagonal, so BF16
 // rounds every entry relative to O(1), and M = D (D^-1 M D^-1) D is recovered
@@ -699,6 +853,33 @@ void mas_assemble(b2s_solver* s, int invert_mode)
     {
         const int64_t T = prev->nnz;
         Matrix&       C = M.coarse[level];
+        if(level > 1 && T <= TAIL_BLOCKS)
+        {
+            if(T == 0)
+                break;
+            TailArgs a{};
+            a.first = level;
+            a.L     = M.L;
+            a.U     = (int)T;
+            a.rows  = prev->rows.data();
+            a.cols  = prev->cols.data();
+            a.vals  = prev->vals.data();
+            a.S     = prev->stride;
+            a.hess  = M.hess.data();
+            for(int l = level; l < M.L; ++l)
+            {
+                Matrix& D = M.coarse[l];
+                D.rows.resize(TAIL_BLOCKS);
+                D.cols.resize(TAIL_BLOCKS);
+                D.vals.resize((size_t)9 * TAIL_BLOCKS);
+                a.lv[l] = TailLevel{M.level_begin[l], X.new_local[l - 1].data(), D.rows.data(), D.cols.data(),
+                                    D.vals.data()};
+            }
+            B2S_CUDA(cudaFuncSetAttribute(k_coarse_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM));
+            k_coarse_tail<<<1, TAIL_THREADS, TAIL_SMEM, st>>>(a);
+            B2S_CHECK_LAUNCH();
+            break;
+        }
         M.trip_rows.resize(std::max<int64_t>(T, 1), 1.2);
         M.trip_cols.resize(std::max<int64_t>(T, 1), 1.2);
         M.trip_vals.resize((size_t)9 * std::max<int64_t>(T, 1), 1.2);
