@@ -162,7 +162,7 @@ int b2s_assemble(b2s_solver* s, int32_t nb, int64_t T, const int32_t* rows, cons
                        B2S_REQUIRE(T == 0 || (rows && cols && vals), B2S_ERR_ARGUMENT, "null triplet array");
                        B2S_REQUIRE(nb <= INT32_MAX / 3, B2S_ERR_ARGUMENT, "too many block rows");
                        timed_stage(s, &b2s_timers::assemble_ms,
-                                   [&] { b2s::assemble_triplets(s, s->A, nb, T, rows, cols, vals, true); });
+                                   [&] { b2s::assemble_triplets(s, s->A, nb, T, rows, cols, vals); });
                        s->precond_kind = -1;  // any preconditioner must be rebuilt
                        B2S_CUDA(cudaStreamSynchronize(s->stream));
                    });
@@ -237,6 +237,9 @@ int b2s_spmv(b2s_solver* s, const double* x, double* y, double* h_dot)
                        B2S_REQUIRE(s->A.valid, B2S_ERR_STATE, "no assembled matrix");
                        B2S_REQUIRE(x && y, B2S_ERR_ARGUMENT, "null vector");
                        s->dot_out.resize(4);
+                       // a second product is a loop of them: worth the tile ranks
+                       if(++s->A.products == 2)
+                           b2s::ensure_tile_ranks(s, s->A);
                        b2s::spmv_f64(s, s->A, x, y, h_dot ? s->dot_out.data() : nullptr);
                        b2s::read_back(s, s->dot_out.data(), h_dot ? 1 : 0, h_dot);
                    });

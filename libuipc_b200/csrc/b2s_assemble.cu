@@ -853,7 +853,7 @@ void copy_blocks_out(b2s_solver* s, const Matrix& A, double* out)
 }
 
 void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const int32_t* rows, const int32_t* cols,
-                       const double* vals, bool spmv_tiles)
+                       const double* vals)
 {
     B2S_REQUIRE(nb >= 0 && T >= 0, B2S_ERR_ARGUMENT, "negative matrix size");
     B2S_REQUIRE(T < (int64_t)INT32_MAX, B2S_ERR_ARGUMENT, "more than 2^31-1 triplets");
@@ -963,10 +963,9 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
         B2S_CUDA(cudaMemsetAsync(M.rows.data(), 0xff, sizeof(int32_t) * M.stride, st));
         B2S_CUDA(cudaMemsetAsync(M.cols.data(), 0, sizeof(int32_t) * M.stride, st));
     }
-    M.has_trank = false;
-    if(spmv_tiles && U > 0)
-        build_tile_ranks(s, M);
-    M.valid = true;
+    M.has_trank = false;  // built when the FP64 SpMV is to run more than once or twice
+    M.products  = 0;
+    M.valid     = true;
 }
 
 void build_tile_ranks(b2s_solver* s, Matrix& M)

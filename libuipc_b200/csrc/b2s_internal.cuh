@@ -126,6 +126,7 @@ struct Matrix
     // in shared memory and merges equal columns before its reductions
     DBuf<uint16_t> trank;    // [stride]
     bool           has_trank = false;
+    int            products = 0;  // FP64 products a caller has asked for since the assembly
     DBuf<int32_t>  diag_index;  // [nb] position of block (i,i), -1 if absent
     // row starts of the FP32 SpMV, per group of 128 blocks: the first block's
     // row and a 128-bit mask of the blocks that start a row (no row ids read)
@@ -309,10 +310,9 @@ namespace b2s
 void exclusive_scan(b2s_solver* s, const int32_t* in, int32_t* out, int64_t n, DBuf<int32_t>& tmp);
 
 // assembly of raw triplets into a block-upper matrix (shared by the global
-// matrix and the MAS coarse levels); `spmv_tiles` also computes the per-tile
-// column ranks the SpMV uses
+// matrix and the MAS coarse levels)
 void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const int32_t* rows,
-                       const int32_t* cols, const double* vals, bool spmv_tiles);
+                       const int32_t* cols, const double* vals);
 
 // the first nnz blocks of A as 9 doubles each (column-major) to `out`, host or
 // device memory, on the solver's stream
@@ -366,6 +366,7 @@ void mas_apply_all(b2s_solver* s, const int* converged, bool bf16);
 // the per-tile column ranks of the FP64 SpMV, and the row-start groups of the
 // FP32 one when every row has a block
 void build_tile_ranks(b2s_solver* s, Matrix& M);
+void ensure_tile_ranks(b2s_solver* s, Matrix& M);
 void build_row_groups_full(b2s_solver* s, Matrix& A);
 
 // PCG

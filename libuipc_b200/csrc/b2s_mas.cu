@@ -891,8 +891,7 @@ void mas_assemble(b2s_solver* s, int invert_mode)
                 M.r2p.data(), map, M.trip_rows.data(), M.trip_cols.data(), M.trip_vals.data(), M.hess.data());
             B2S_CHECK_LAUNCH();
         }
-        assemble_triplets(s, C, M.level_count[level], T, M.trip_rows.data(), M.trip_cols.data(), M.trip_vals.data(),
-                          false);
+        assemble_triplets(s, C, M.level_count[level], T, M.trip_rows.data(), M.trip_cols.data(), M.trip_vals.data());
         if(C.nnz > 0)
         {
             k_g_extract<<<grid_for(C.nnz, TB), TB, 0, st>>>(C.nnz, C.rows.data(), C.cols.data(), C.vals.data(),

@@ -910,8 +910,6 @@ static void ensure_order(b2s_solver* s, bool f32)
     {
         P.vals.resize((size_t)9 * P.stride, 1.2);
         fill(P.vals.data());
-        if(!P.has_trank)
-            build_tile_ranks(s, P);
         O.f64_generation = A.generation;
     }
 }
@@ -1069,7 +1067,6 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         st_out.converged = 1;
         return;
     }
-    B2S_REQUIRE(s->A.nnz == 0 || s->A.has_trank, B2S_ERR_STATE, "matrix lacks the SpMV tile ranks");
     // with the MAS the recursion runs in its slot order (see PcgOrder)
     const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized;
     if(ord)
@@ -1203,6 +1200,8 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         bool use_graph = o.use_graph && st != nullptr;
         // small systems: the whole loop in one launch
         const bool small = use_graph && !s->timing && pcg_small_fits(s, A, kind, ord, false);
+        if(!small)
+            ensure_tile_ranks(s, ord ? P.ord.A : s->A);
         if(s->timing)
             ensure_iter_events(s, ci);
         if(use_graph && !small)
@@ -1514,7 +1513,6 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
         st_out.converged = 1;
         return;
     }
-    B2S_REQUIRE(s->A.nnz == 0 || s->A.has_trank, B2S_ERR_STATE, "matrix lacks the SpMV tile ranks");
     // FP32 matrix planes (in the MAS slot order with the MAS, see PcgOrder) and
     // BF16 inverses: once per assembly / build
     const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized;

@@ -375,6 +375,83 @@ __global__ void __launch_bounds__(DIRECT_THREADS, DIRECT_CTAS_SM)
     }
 }
 
+// FP64 values without tile ranks, two blocks per thread straight into
+// registers as k_spmv_direct does it: for a matrix that is multiplied once or
+// twice (the residual that confirms a mixed solve, a warm start), where the
+// ranks k_spmv_tile reads would cost more than they save (4.3 M blocks: 97 us
+// against 83, and 146 for the ranks). f64 has no vector reduction, so every
+// transposed half costs three.
+constexpr int D64_BPT = 2;
+template <bool WITH_DOT>
+__global__ void __launch_bounds__(DIRECT_THREADS)
+    k_spmv_direct64(int64_t S, int64_t U, const int32_t* __restrict__ rows, const int32_t* __restrict__ cols,
+                    const double* __restrict__ vals, const double* __restrict__ x, double* y, double* partials,
+                    unsigned int* counter, double* dot_out, const int* stop)
+{
+    if(stop && *stop)
+        return;
+    const int64_t n_chunks = S / D64_BPT;
+    double        dot      = 0.0;
+    for(int64_t c = (int64_t)blockIdx.x * DIRECT_THREADS + threadIdx.x; c < n_chunks;
+        c += (int64_t)gridDim.x * DIRECT_THREADS)
+    {
+        const int64_t e0 = c * D64_BPT;
+        const int2    r2 = __ldcs(reinterpret_cast<const int2*>(rows + e0));
+        const int2    c2 = __ldcs(reinterpret_cast<const int2*>(cols + e0));
+        const int32_t r[2] = {r2.x, r2.y}, cc[2] = {c2.x, c2.y};
+        double        b[9][2];
+#pragma unroll
+        for(int q = 0; q < 9; ++q)
+        {
+            const double2 v = __ldcs(reinterpret_cast<const double2*>(vals + (int64_t)q * S + e0));
+            b[q][0] = v.x; b[q][1] = v.y;
+        }
+        int32_t cur = -1;
+        double  a0 = 0, a1 = 0, a2 = 0, xi0 = 0, xi1 = 0, xi2 = 0;
+#pragma unroll
+        for(int k = 0; k < D64_BPT; ++k)
+        {
+            if(r[k] < 0)
+                break;
+            const int32_t ck = cc[k];
+            double        xj0, xj1, xj2;
+            load_node<double, false>(x, ck, xj0, xj1, xj2);
+            if(r[k] != cur)
+            {
+                if(cur >= 0)
+                    red_node<double, false>(y, cur, a0, a1, a2);
+                cur = r[k];
+                a0 = a1 = a2 = 0;
+                load_node<double, false>(x, cur, xi0, xi1, xi2);
+            }
+            const double y0 = b[0][k] * xj0 + b[3][k] * xj1 + b[6][k] * xj2;
+            const double y1 = b[1][k] * xj0 + b[4][k] * xj1 + b[7][k] * xj2;
+            const double y2 = b[2][k] * xj0 + b[5][k] * xj1 + b[8][k] * xj2;
+            a0 += y0;
+            a1 += y1;
+            a2 += y2;
+            const bool off = cur != ck;
+            if(WITH_DOT)
+            {
+                const double d = xi0 * y0 + xi1 * y1 + xi2 * y2;
+                dot += off ? 2.0 * d : d;
+            }
+            if(off)
+                red_node<double, false>(y, ck, b[0][k] * xi0 + b[1][k] * xi1 + b[2][k] * xi2,
+                                        b[3][k] * xi0 + b[4][k] * xi1 + b[5][k] * xi2,
+                                        b[6][k] * xi0 + b[7][k] * xi1 + b[8][k] * xi2);
+        }
+        if(cur >= 0)
+            red_node<double, false>(y, cur, a0, a1, a2);
+    }
+    if(WITH_DOT)
+    {
+        double v[1] = {dot}, tot[1];
+        if(grid_sum<1>(v, partials, counter, tot))
+            *dot_out = tot[0];
+    }
+}
+
 // persistent grid: the CTAs that fit on the SMs at once, capped by the tiles
 // (and by spmv_grid, which sizes the reduction partials)
 template <typename K>
@@ -404,7 +481,7 @@ void launch_stream(cudaStream_t st, int64_t U, int64_t S, const int32_t* rows, c
 // the largest grid any SpMV kernel launches for U blocks (sizes the dot partials)
 int spmv_grid(int64_t U)
 {
-    const int64_t t = (U + SPMV_BPT * DIRECT_THREADS - 1) / (SPMV_BPT * DIRECT_THREADS);
+    const int64_t t = (U + D64_BPT * DIRECT_THREADS - 1) / (D64_BPT * DIRECT_THREADS);
     return (int)std::max<int64_t>(1, std::min<int64_t>(t, (int64_t)NUM_SMS_HINT * 8));
 }
 
@@ -466,6 +543,12 @@ void check_device_errors(b2s_solver* s)
         read_back(s, nullptr, 0, nullptr);
 }
 
+void ensure_tile_ranks(b2s_solver* s, Matrix& A)
+{
+    if(!A.has_trank && A.nnz > 0)
+        build_tile_ranks(s, A);
+}
+
 // y = A x; y is overwritten. d_dot (device) receives x.(A x) when non-null.
 void spmv_f64(b2s_solver* s, const Matrix& A, const double* x, double* y, double* d_dot)
 {
@@ -477,8 +560,21 @@ void spmv_f64(b2s_solver* s, const Matrix& A, const double* x, double* y, double
             B2S_CUDA(cudaMemsetAsync(d_dot, 0, sizeof(double), st));
         return;
     }
-    B2S_REQUIRE(A.has_trank, B2S_ERR_STATE, "matrix lacks the SpMV tile ranks");
     ensure_reduction(s->red, spmv_grid(A.nnz), 1);
+    if(!A.has_trank)
+    {
+        auto k   = d_dot ? k_spmv_direct64<true> : k_spmv_direct64<false>;
+        int  occ = 0;
+        if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, DIRECT_THREADS, 0) != cudaSuccess || occ < 1)
+            occ = 1;
+        const int64_t ctas = (A.stride / D64_BPT + DIRECT_THREADS - 1) / DIRECT_THREADS;
+        const int     grid = (int)std::max<int64_t>(
+            1, std::min<int64_t>({ctas, (int64_t)NUM_SMS_HINT * std::min(occ, 8), (int64_t)spmv_grid(A.nnz)}));
+        k<<<grid, DIRECT_THREADS, 0, st>>>(A.stride, A.nnz, A.rows.data(), A.cols.data(), A.vals.data(), x, y,
+                                           s->red.partials.data(), s->red.counter.data(), d_dot, nullptr);
+        B2S_CHECK_LAUNCH();
+        return;
+    }
     if(d_dot)
         launch_stream<double, double, true>(st, A.nnz, A.stride, A.rows.data(), A.cols.data(), A.trank.data(), A.vals.data(), x, y,
                                             &s->red, d_dot, nullptr);
