@@ -914,6 +914,30 @@ static void ensure_order(b2s_solver* s, bool f32)
     }
 }
 
+// ensure_order, or false (the recursion then runs in the matrix's own order)
+// when the device has no room for the second copy of the matrix
+static bool try_order(b2s_solver* s, bool f32)
+{
+    try
+    {
+        ensure_order(s, f32);
+        return true;
+    }
+    catch(const Error&)
+    {
+        if(cudaGetLastError() != cudaErrorMemoryAllocation)
+            throw;
+        PcgOrder& O = s->pcg.ord;
+        O.A.vals.release();
+        O.A.vals32.release();
+        O.A.rows.release();
+        O.A.cols.release();
+        O.A.trank.release();
+        O.f64_generation = O.f32_generation = -1;
+        return false;
+    }
+}
+
 // the restriction in PCG order, with the x, r update of the iteration
 // (UPDATE). Without an apply to follow (kind other than MAS) nothing is
 // restricted: the apply clears the coarse sums.
@@ -1068,9 +1092,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         return;
     }
     // with the MAS the recursion runs in its slot order (see PcgOrder)
-    const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized;
-    if(ord)
-        ensure_order(s, false);
+    const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized && try_order(s, false);
     const PcgOrder& O  = P.ord;
     const Matrix&   A  = ord ? O.A : s->A;
     const int64_t   n  = 3 * (int64_t)A.nb;  // the recursion's vectors
@@ -1515,10 +1537,8 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
     }
     // FP32 matrix planes (in the MAS slot order with the MAS, see PcgOrder) and
     // BF16 inverses: once per assembly / build
-    const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized;
-    if(ord)
-        ensure_order(s, true);
-    else
+    const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized && try_order(s, true);
+    if(!ord)
         ensure_f32_planes(s);
     ensure_bf16_inverses(s);
     const PcgOrder& O  = P.ord;

@@ -661,9 +661,9 @@ void launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterat
 // the barriers, not the streams, bound the iteration.
 bool pcg_small_fits(b2s_solver* s, const Matrix& A, int kind, bool ord, bool f32)
 {
-    if(A.nnz == 0 || (ord && kind == B2S_PRECOND_JACOBI))
+    const bool mas = kind == B2S_PRECOND_MAS;
+    if(A.nnz == 0 || (mas && !ord) || (ord && kind == B2S_PRECOND_JACOBI))
         return false;
-    const bool   mas  = kind == B2S_PRECOND_MAS;
     const void*  k    = f32 ? (mas ? (const void*)k_pcg_small<float, true> : (const void*)k_pcg_small<float, false>) :
                               (mas ? (const void*)k_pcg_small<double, true> : (const void*)k_pcg_small<double, false>);
     const size_t smem = f32 ? small_smem<float>(mas) : small_smem<double>(mas);
