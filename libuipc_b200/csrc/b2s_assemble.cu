@@ -171,7 +171,7 @@ void exclusive_scan(b2s_solver* s, const int32_t* in, int32_t* out, int64_t n, D
 namespace
 {
 constexpr int ASM_BLOCK = 256;
-constexpr int ROW_CAP   = 256;  // (col, src) pairs per row held in shared memory
+constexpr int ROW_CAP   = 256;  // (col, src) pairs per row that one warp sorts in registers
 
 // The triplets of a warp mostly come from one or two elements, so few
 // distinct rows: the lanes holding the same row (__match_any_sync) add their
@@ -246,9 +246,77 @@ __global__ void k_scatter_rows(const int32_t* __restrict__ rows, const int32_t* 
     }
 }
 
-__device__ __forceinline__ bool key_less(int32_t ca, int32_t sa, int32_t cb, int32_t sb)
+// One row of at most 32 K pairs by one warp, K keys per lane (positions
+// j * 32 + lane): bitonic sort in registers, partners 32 apart or more in the
+// same lane, the others by shuffles; padding = max key. Then the sources in
+// order and the runs over the row's pairs. Returns the number of runs.
+template <int K>
+__device__ __forceinline__ int sort_row(int2* bucket, int32_t* __restrict__ sorted_src, int32_t beg, int32_t L, int lane)
 {
-    return ca < cb || (ca == cb && sa < sb);
+    uint64_t key[K];
+#pragma unroll
+    for(int j = 0; j < K; ++j)
+    {
+        const int p = j * 32 + lane;
+        key[j]      = ~0ull;
+        if(p < L)
+        {
+            const int2 q = bucket[beg + p];
+            key[j]       = ((uint64_t)(uint32_t)q.x << 32) | (uint64_t)(uint32_t)q.y;
+        }
+    }
+#pragma unroll
+    for(int k = 2; k <= 32 * K; k <<= 1)
+#pragma unroll
+        for(int s = k >> 1; s > 0; s >>= 1)
+        {
+            if(s >= 32)
+            {
+#pragma unroll
+                for(int j = 0; j < K; ++j)
+                {
+                    const int o = j ^ (s / 32);
+                    if(o > j)
+                    {
+                        const bool     up = ((j * 32) & k) == 0;  // k > s >= 32: the lane does not matter
+                        const uint64_t lo = key[j] < key[o] ? key[j] : key[o];
+                        const uint64_t hi = key[j] < key[o] ? key[o] : key[j];
+                        key[j]            = up ? lo : hi;
+                        key[o]            = up ? hi : lo;
+                    }
+                }
+            }
+            else
+            {
+#pragma unroll
+                for(int j = 0; j < K; ++j)
+                {
+                    const int      p     = j * 32 + lane;
+                    const uint64_t other = __shfl_xor_sync(0xffffffffu, key[j], s);
+                    const bool     keep_min = ((p & s) == 0) == ((p & k) == 0);
+                    key[j] = keep_min ? (key[j] < other ? key[j] : other) : (key[j] < other ? other : key[j]);
+                }
+            }
+        }
+    __syncwarp();  // every lane holds its pairs: the runs may replace them
+    int      uniq = 0;
+    uint64_t last = ~0ull;  // key at the position before this group's first
+#pragma unroll
+    for(int j = 0; j < K; ++j)
+    {
+        const int      p    = j * 32 + lane;
+        const uint64_t up1  = __shfl_up_sync(0xffffffffu, key[j], 1);
+        const uint64_t prev = lane > 0 ? up1 : last;
+        last                = __shfl_sync(0xffffffffu, key[j], 31);
+        const bool     head = p < L && (p == 0 || (prev >> 32) != (key[j] >> 32));
+        const unsigned hm   = __ballot_sync(0xffffffffu, head);
+        if(p < L)
+            sorted_src[beg + p] = (int32_t)(key[j] & 0xFFFFFFFFull);
+        if(head)
+            bucket[beg + uniq + __popc(hm & ((1u << lane) - 1u))] = make_int2((int32_t)(key[j] >> 32), beg + p);
+        uniq += __popc(hm);
+    }
+    return uniq;
 }
 
 // One warp per row: the row's (col, src) pairs sorted; out go the sources in
@@ -256,144 +324,35 @@ __device__ __forceinline__ bool key_less(int32_t ca, int32_t sa, int32_t cb, int
 // each distinct column with the position of its first source, and their number
 // (uniq_count). The columns of all pairs are not written: marking the
 // runs from them in a second pass cost 126 MB out and in on 31 M triplets
-// (sort + mark 544 us; 454 now).
+// (sort + mark 544 us; 454 now). Rows of more than 64 pairs are only listed
+// here: four or eight keys per lane would cost the common rows registers (the
+// whole assembly of the 31 M triplets 1.66 -> 1.68 ms).
 __global__ void __launch_bounds__(ASM_BLOCK) k_sort_rows(int32_t nb, const int32_t* __restrict__ row_start,
                                                          int2* bucket,
                                                          int32_t* __restrict__ sorted_src,
                                                          int32_t* __restrict__ uniq_count, int32_t* long_rows,
-                                                         int32_t* n_long)
+                                                         int32_t* n_long, int32_t* n_mid)
 {
-    __shared__ int32_t s_col[ASM_BLOCK / 32][ROW_CAP];
-    __shared__ int32_t s_src[ASM_BLOCK / 32][ROW_CAP];
-    __shared__ int32_t s_sorted[ASM_BLOCK / 32][ROW_CAP];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int warps_total = gridDim.x * (ASM_BLOCK / 32);
     for(int32_t r = blockIdx.x * (ASM_BLOCK / 32) + w; r < nb; r += warps_total)
     {
         const int32_t beg = row_start[r], L = row_start[r + 1] - beg;
-        int           uniq = 0;
+        int           uniq;
         if(L <= 32)
-        {
-            // one key per lane (column << 32 | source), bitonic sort across
-            // the warp, padding = max key
-            uint64_t key = ~0ull;
-            if(lane < L)
-            {
-                const int2 q = bucket[beg + lane];
-                key          = ((uint64_t)(uint32_t)q.x << 32) | (uint64_t)(uint32_t)q.y;
-            }
-#pragma unroll
-            for(int k = 2; k <= 32; k <<= 1)
-#pragma unroll
-                for(int s = k >> 1; s > 0; s >>= 1)
-                {
-                    const uint64_t other    = __shfl_xor_sync(0xffffffffu, key, s);
-                    const bool     keep_min = ((lane & s) == 0) == ((lane & k) == 0);
-                    key = keep_min ? (key < other ? key : other) : (key < other ? other : key);
-                }
-            const uint64_t prev = __shfl_up_sync(0xffffffffu, key, 1);
-            const bool     head = lane < L && (lane == 0 || (prev >> 32) != (key >> 32));
-            const unsigned hm   = __ballot_sync(0xffffffffu, head);
-            if(lane < L)
-                sorted_src[beg + lane] = (int32_t)(key & 0xFFFFFFFFull);
-            if(head)
-                bucket[beg + __popc(hm & ((1u << lane) - 1u))] = make_int2((int32_t)(key >> 32), beg + lane);
-            uniq = __popc(hm);
-        }
+            uniq = sort_row<1>(bucket, sorted_src, beg, L, lane);
         else if(L <= 64)
-        {
-            // bitonic sort of the (column << 32 | source) keys in registers,
-            // two per lane (positions lane and lane + 32), padding = max key
-            uint64_t key[2];
-#pragma unroll
-            for(int j = 0; j < 2; ++j)
-            {
-                const int p = j * 32 + lane;
-                if(p < L)
-                {
-                    const int2 q = bucket[beg + p];
-                    key[j]       = ((uint64_t)(uint32_t)q.x << 32) | (uint64_t)(uint32_t)q.y;
-                }
-                else
-                    key[j] = ~0ull;
-            }
-#pragma unroll
-            for(int k = 2; k <= 64; k <<= 1)
-#pragma unroll
-                for(int s = k >> 1; s > 0; s >>= 1)
-                {
-                    if(s == 32)
-                    {
-                        // k = 64: ascending; the partner is this lane's other key
-                        const uint64_t lo = key[0] < key[1] ? key[0] : key[1];
-                        const uint64_t hi = key[0] < key[1] ? key[1] : key[0];
-                        key[0]            = lo;
-                        key[1]            = hi;
-                    }
-                    else
-                    {
-#pragma unroll
-                        for(int j = 0; j < 2; ++j)
-                        {
-                            const int      p     = j * 32 + lane;
-                            const uint64_t other = __shfl_xor_sync(0xffffffffu, key[j], s);
-                            const bool     up    = (p & k) == 0;
-                            const bool     keep_min = ((p & s) == 0) == up;
-                            key[j] = keep_min ? (key[j] < other ? key[j] : other) : (key[j] < other ? other : key[j]);
-                        }
-                    }
-                }
-            const uint64_t last0 = __shfl_sync(0xffffffffu, key[0], 31);
-#pragma unroll
-            for(int j = 0; j < 2; ++j)
-            {
-                const int      p    = j * 32 + lane;
-                const uint64_t up1  = __shfl_up_sync(0xffffffffu, key[j], 1);
-                const uint64_t prev = lane > 0 ? up1 : (j == 1 ? last0 : ~0ull);
-                const bool     head = p < L && (p == 0 || (prev >> 32) != (key[j] >> 32));
-                const unsigned hm   = __ballot_sync(0xffffffffu, head);
-                if(p < L)
-                    sorted_src[beg + p] = (int32_t)(key[j] & 0xFFFFFFFFull);
-                if(head)
-                    bucket[beg + uniq + __popc(hm & ((1u << lane) - 1u))] = make_int2((int32_t)(key[j] >> 32), beg + p);
-                uniq += __popc(hm);
-            }
-        }
-        else if(L <= ROW_CAP)
-        {
-            for(int k = lane; k < L; k += 32)
-            {
-                const int2 q = bucket[beg + k];
-                s_col[w][k]  = q.x;
-                s_src[w][k]  = q.y;
-            }
-            __syncwarp();
-            for(int k = lane; k < L; k += 32)
-            {
-                const int32_t c = s_col[w][k], sr = s_src[w][k];
-                int           rank = 0;
-                for(int q = 0; q < L; ++q)
-                    rank += key_less(s_col[w][q], s_src[w][q], c, sr) ? 1 : 0;
-                sorted_src[beg + rank] = sr;
-                s_sorted[w][rank]      = c;
-            }
-            __syncwarp();
-            for(int base = 0; base < L; base += 32)
-            {
-                const int      p    = base + lane;
-                const bool     head = p < L && (p == 0 || s_sorted[w][p] != s_sorted[w][p - 1]);
-                const unsigned hm   = __ballot_sync(0xffffffffu, head);
-                if(head)
-                    bucket[beg + uniq + __popc(hm & ((1u << lane) - 1u))] = make_int2(s_sorted[w][p], beg + p);
-                uniq += __popc(hm);
-            }
-            __syncwarp();
-        }
+            uniq = sort_row<2>(bucket, sorted_src, beg, L, lane);
         else
         {
-            // longer than a warp's shared memory: sorted by k_sort_long_rows
+            // more keys per lane, or a CTA per row: k_sort_long_rows
             if(lane == 0)
-                long_rows[atomicAdd(n_long, 1)] = (int32_t)r;
+            {
+                if(L > ROW_CAP)
+                    long_rows[atomicAdd(n_long, 1)] = (int32_t)r;
+                else
+                    long_rows[nb - 1 - atomicAdd(n_mid, 1)] = (int32_t)r;
+            }
             continue;
         }
         if(lane == 0)
@@ -401,8 +360,11 @@ __global__ void __launch_bounds__(ASM_BLOCK) k_sort_rows(int32_t nb, const int32
     }
 }
 
-// Rows longer than ROW_CAP pairs (e.g. an affine body touched by thousands of
-// cloth vertices), listed by k_sort_rows: one CTA per row (persistent over the
+// The rows listed by k_sort_rows. Up to ROW_CAP pairs, most rows of a coarse
+// MAS level: a warp per row, four or eight keys per lane (ranked before by
+// counting the smaller pairs of the row for every pair; MAS build of 551,368
+// vertices 1.72 -> 1.64 ms). Longer (e.g. an affine body touched by
+// thousands of cloth vertices): one CTA per row (persistent over the
 // list). The keys (column << 32 | source; unique) are sorted LONG_TILE at a
 // time in shared memory (bitonic); with several tiles every key's rank is its
 // place in its tile plus a binary search in each of the others. Counting the
@@ -445,14 +407,25 @@ __device__ __forceinline__ void sort_tile(uint64_t* s_key, int n)
         }
 }
 
-__global__ void __launch_bounds__(LONG_THREADS) k_sort_long_rows(const int32_t* __restrict__ long_rows,
+__global__ void __launch_bounds__(LONG_THREADS) k_sort_long_rows(int32_t nb, const int32_t* __restrict__ long_rows,
                                                                  const int32_t* __restrict__ n_rows,
+                                                                 const int32_t* __restrict__ n_mid,
                                                                  const int32_t* __restrict__ row_start, int2* bucket,
                                                                  int32_t* sorted_col, int32_t* sorted_src,
                                                                  int32_t* __restrict__ uniq_count)
 {
     __shared__ uint64_t s_key[LONG_TILE];
     __shared__ int      s_heads[LONG_THREADS / 32];
+    // the rows of 65 to 256 pairs (listed from the end), a warp each
+    const int lane = threadIdx.x & 31, mid = *n_mid;
+    for(int e = blockIdx.x * (LONG_THREADS / 32) + (threadIdx.x >> 5); e < mid; e += gridDim.x * (LONG_THREADS / 32))
+    {
+        const int32_t r = long_rows[nb - 1 - e], beg = row_start[r], L = row_start[r + 1] - beg;
+        const int     u = L <= 128 ? sort_row<4>(bucket, sorted_src, beg, L, lane) :
+                                     sort_row<8>(bucket, sorted_src, beg, L, lane);
+        if(lane == 0)
+            uniq_count[r] = u;
+    }
     const int n_long = *n_rows;
     for(int e = blockIdx.x; e < n_long; e += gridDim.x)
     {
@@ -862,15 +835,17 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
     M.valid             = false;
     M.generation += 1;
     M.nb                = nb;
-    // row counts, then the error bits and the number of long rows: one fill
-    w.row_count.resize((size_t)nb + 3, 1.25);
+    // row counts, then the error bits and the numbers of long and of mid rows:
+    // one fill
+    w.row_count.resize((size_t)nb + 4, 1.25);
     w.row_start.resize((size_t)nb + 1, 1.25);
     int* const     err    = w.row_count.data() + nb + 1;
     int32_t* const n_long_dev = w.row_count.data() + nb + 2;
+    int32_t* const n_mid_dev  = w.row_count.data() + nb + 3;
     w.uniq_count.resize((size_t)nb + 1, 1.25);
     M.rowptr.resize((size_t)nb + 1, 1.25);
     M.diag_index.resize((size_t)std::max(nb, 1), 1.25);
-    B2S_CUDA(cudaMemsetAsync(w.row_count.data(), 0, sizeof(int32_t) * ((size_t)nb + 3), st));
+    B2S_CUDA(cudaMemsetAsync(w.row_count.data(), 0, sizeof(int32_t) * ((size_t)nb + 4), st));
     if(T > 0)
     {
         w.bucket.resize(T, 1.25);
@@ -891,12 +866,12 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
         w.long_rows.resize((size_t)nb, 1.25);
         k_sort_rows<<<asm_grid((int64_t)nb * 32, ASM_BLOCK), ASM_BLOCK, 0, st>>>(
             nb, w.row_start.data(), w.bucket.data(), w.sorted_src.data(), w.uniq_count.data(), w.long_rows.data(),
-            n_long_dev);
+            n_long_dev, n_mid_dev);
         B2S_CHECK_LAUNCH();
-        // the long rows (their number is read on the device)
-        k_sort_long_rows<<<NUM_SMS_HINT * 2, LONG_THREADS, 0, st>>>(w.long_rows.data(), n_long_dev, w.row_start.data(),
-                                                                    w.bucket.data(), w.sorted_col.data(),
-                                                                    w.sorted_src.data(), w.uniq_count.data());
+        // the mid and the long rows (their numbers are read on the device)
+        k_sort_long_rows<<<NUM_SMS_HINT * 2, LONG_THREADS, 0, st>>>(
+            nb, w.long_rows.data(), n_long_dev, n_mid_dev, w.row_start.data(), w.bucket.data(), w.sorted_col.data(),
+            w.sorted_src.data(), w.uniq_count.data());
         B2S_CHECK_LAUNCH();
     }
     exclusive_scan(s, w.uniq_count.data(), M.rowptr.data(), nb, w.scan_tmp);

@@ -145,7 +145,7 @@ struct AssemblyScratch
     DBuf<int2>    bucket;  // (column, source) of the kept triplets by row; once sorted, (column, first position) of its runs
     DBuf<int32_t> sorted_col, sorted_src;  // (columns of the long rows only)
     DBuf<int32_t> run_start;  // [U+1] sorted position of each unique block's first source
-    DBuf<int32_t> long_rows;  // [nb] the rows too long for one warp
+    DBuf<int32_t> long_rows;  // [nb] rows of more than ROW_CAP pairs from the front, of more than 64 from the back
     DBuf<int32_t> long_runs;  // [1 + U]: count, then the blocks whose run is summed by a warp
     DBuf<int32_t> scan_tmp;
     DBuf<int>     err;
