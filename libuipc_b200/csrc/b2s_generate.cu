@@ -117,7 +117,7 @@ __device__ __forceinline__ int slot_r(int k) { return (0x3323213210ull >> (4 * k
 // Hessian blocks (b2s_snh.cuh: closed form, everything in registers). Bound by
 // the FP64 pipe and the 800 B of triplets written per tet. A 9x9 Jacobi per
 // tet, its two 648-byte arrays in local memory, took the whole system of
-// 480,000 tets 11.1 ms; with this kernel it takes 0.21 ms (1.9 TB/s). The
+// 480,000 tets 11.1 ms; with this kernel it takes 0.19 ms (2.1 TB/s). The
 // blocks go through shared memory, five slots at a time, so that a warp's
 // stores cover whole 360-byte runs: written thread by thread every 8-byte
 // store of a warp would touch 32 sectors. 46 KB and at most 128 registers:

@@ -27,6 +27,14 @@ struct Projected
     double m[3][3], p[3], q[3];
 };
 
+__host__ __device__ inline double inv_sqrt(double x)
+{
+#ifdef __CUDA_ARCH__
+    return rsqrt(x);
+#else
+    return 1.0 / sqrt(x);
+#endif
+}
 __host__ __device__ inline double dot3(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 __host__ __device__ inline void cross3(const double* a, const double* b, double* c)
 {
@@ -44,9 +52,10 @@ __host__ __device__ inline bool rotate_columns(double a[3][3], double v[3][3])
     const double al = dot3(a[P], a[P]), be = dot3(a[Q], a[Q]), ga = dot3(a[P], a[Q]);
     if(!(ga * ga > 1e-31 * (al * be)))
         return false;
-    const double z = (be - al) / (2.0 * ga);
-    const double t = (z >= 0.0 ? 1.0 : -1.0) / (fabs(z) + sqrt(z * z + 1.0));
-    const double c = 1.0 / sqrt(t * t + 1.0), s = c * t;
+    // t = sign(z) / (|z| + sqrt(z^2 + 1)) of z = d / g without forming z
+    const double d = be - al, g = 2.0 * ga;
+    const double t = (d >= 0.0 ? g : -g) / (fabs(d) + sqrt(d * d + g * g));
+    const double c = inv_sqrt(t * t + 1.0), s = c * t;
     for(int r = 0; r < 3; ++r)
     {
         const double ap = a[P][r], aq = a[Q][r], vp = v[P][r], vq = v[Q][r];
@@ -65,7 +74,7 @@ __host__ __device__ inline void any_orthogonal(const double* u, double* w)
     const double e[3] = {x <= y && x <= z ? 1.0 : 0.0, !(x <= y && x <= z) && y <= z ? 1.0 : 0.0,
                          !(x <= y && x <= z) && !(y <= z) ? 1.0 : 0.0};
     cross3(u, e, w);
-    const double n = 1.0 / sqrt(dot3(w, w));
+    const double n = inv_sqrt(dot3(w, w));
     for(int r = 0; r < 3; ++r)
         w[r] *= n;
 }
@@ -110,13 +119,13 @@ __host__ __device__ inline void rotation_svd(const double F[9], double u[3][3], 
     n1 = s0 ? n2 : (s1 ? t0 : t1);
     if(n0 > 0.0)
     {
-        const double i0 = 1.0 / sqrt(n0);
+        const double i0 = inv_sqrt(n0);
         for(int r = 0; r < 3; ++r)
             u[0][r] = a[0][r] * i0;
     }
     else if(n1 > 0.0)
     {
-        const double i1 = 1.0 / sqrt(n1);
+        const double i1 = inv_sqrt(n1);
         double       w[3];
         for(int r = 0; r < 3; ++r)
             w[r] = a[1][r] * i1;
@@ -129,7 +138,7 @@ __host__ __device__ inline void rotation_svd(const double F[9], double u[3][3], 
     const double nw = dot3(w1, w1);
     if(nw > 1e-30 * n0 && nw > 0.0)
     {
-        const double iw = 1.0 / sqrt(nw);
+        const double iw = inv_sqrt(nw);
         for(int r = 0; r < 3; ++r)
             u[1][r] = w1[r] * iw;
     }
