@@ -1111,6 +1111,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
     if(!P.h_sc)
         B2S_CUDA(cudaMallocHost(&P.h_sc, sizeof(PcgScalars)));
     ensure_reduction(P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
+    ensure_reduction(s->red, reduction_grid(), 2);  // the largest grid: the sums below run over rows and over entries
     device_error_flag(s);  // allocated before any graph capture
     s->dot_out.resize(4);
     const int ci = o.check_interval > 0 ? o.check_interval : 1;
@@ -1198,7 +1199,6 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         st_out.rel_res   = true_residual();
         return;
     }
-    ensure_reduction(s->red, reduction_grid(), 2);
 
     // device scalars
     PcgScalars h{};

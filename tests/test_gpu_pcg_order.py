@@ -101,3 +101,19 @@ def test_pcg_in_slot_order(solver, cuda, n, before, after, bodies, part, skip, p
         x = torch.full((3 * nb,), 7.0, dtype=torch.float64, device=cuda)
         st = solver.pcg(bd, x, tol=1e-11, stop_rule=1, precision=precision, max_iter=3)
         assert st["converged"] == 0 and bool(torch.isfinite(x).all())
+
+
+@pytest.mark.parametrize("nb", [1, 300, 120000])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_zero_right_hand_side_on_a_new_handle(solver, cuda, nb, precision):
+    """b = 0 stops before the loop: the residual's sums run over more blocks
+    than any sum before them on this handle."""
+    import torch
+
+    idx = torch.arange(nb, dtype=torch.int32, device=cuda)
+    vals = torch.eye(3, dtype=torch.float64, device=cuda).reshape(1, 9).expand(nb, 9).contiguous()
+    solver.assemble(nb, idx, idx, vals)
+    solver.precond_assemble(1)
+    x = torch.full((3 * nb,), 3.0, dtype=torch.float64, device=cuda)
+    st = solver.pcg(torch.zeros_like(x), x, precision=precision)
+    assert st["converged"] == 1 and st["rel_res"] == 0.0 and not x.any()
