@@ -16,10 +16,7 @@ __host__ __device__ __forceinline__ int sym_index(int row, int col)
 // ---------------------------------------------------------------------------
 // apply: one warp per bank, persistent over banks. The bank's inverse is
 // brought into shared memory by bulk asynchronous copies (TMA), NST deep per
-// warp, so later banks' copies are in flight while this one computes. The
-// residual of the next bank (and, at level 0, the part_to_real index of the
-// bank after it) is loaded into registers one bank ahead, so the dependent
-// part_to_real -> r gather never stalls the product.
+// warp, so later banks' copies are in flight while this one computes.
 //
 // FP32 inverses (4,896 B: the 136 upper 3x3 blocks, column-major) are applied
 // on the CUDA cores: lanes 0-15 own the bank's nodes and the 48x48 product is

@@ -17,6 +17,7 @@
 // (column, index) order; after a barrier each thread merges its SPMV_BPT
 // consecutive slots, so runs of equal columns also leave as one reduction
 // each (~0.62 of the measured HBM bandwidth on 4.25 M blocks).
+// A matrix multiplied only once or twice is not given ranks (k_spmv_direct64).
 // FP32 values (k_spmv_direct, mixed precision): the same row runs, but every
 // transposed half leaves as one vector reduction of the padded node and the
 // kernel holds no shared memory and no barrier (~0.77).
@@ -378,7 +379,7 @@ __global__ void __launch_bounds__(DIRECT_THREADS, DIRECT_CTAS_SM)
 // FP64 values without tile ranks, two blocks per thread straight into
 // registers as k_spmv_direct does it: for a matrix that is multiplied once or
 // twice (the residual that confirms a mixed solve, a warm start), where the
-// ranks k_spmv_tile reads would cost more than they save (4.3 M blocks: 97 us
+// ranks k_spmv_tile reads would cost more than they save (4.3 M blocks: 104 us
 // against 83, and 146 for the ranks). f64 has no vector reduction, so every
 // transposed half costs three.
 constexpr int D64_BPT = 2;
