@@ -444,6 +444,7 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
                     }
                     for(int e = lane; e < BANK * 3; e += 32)
                         s_r1[e] = __ldcg(a.A.R + g * (BANK * 3) + e);
+                    __syncwarp();  // every lane's entries, for the others in bank_product
                     const bool ok = mbar_wait(bar, (uint32_t)((u1 / SM_COARSE) & 1), a.A.err, DERR_TMA_TIMEOUT);
                     underway      = false;
                     if(!__all_sync(0xffffffffu, ok))
