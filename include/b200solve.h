@@ -243,6 +243,13 @@ int b2s_set_timing(b2s_solver* s, int enable);
 int b2s_get_timers(const b2s_solver* s, b2s_timers* out);
 int b2s_reset_timers(b2s_solver* s);
 
+/* ---- failure injection ----------------------------------------------------------------
+ * For tests of the error paths: a wait of this handle's kernels gives up early.
+ * Nothing faults or hangs; the affected call returns the status it returns when
+ * the same happens by itself. */
+#define B2S_INJECT_WAIT_POLLS 0 /* a grid barrier of the one-launch PCG gives up after `value` polls (-1: the default, seconds) */
+int b2s_inject_failure(b2s_solver* s, int what, int64_t value);
+
 /* ---- learned PCG warm start ------------------------------------------------------------
  * No counterpart in the reference (its PCG starts from x0 = 0,
  * linear_fused_pcg.cu:1782-2005). A small MLP on MAS level-1 aggregates

@@ -20,6 +20,7 @@ B2S_INVERT_F32_ONLY = 2
 
 B2S_STOP_RZ = 0
 B2S_STOP_RELRES = 1
+B2S_INJECT_WAIT_POLLS = 0
 
 B2S_PRECISION_FP64 = 0
 B2S_PRECISION_MIXED = 1
@@ -137,6 +138,7 @@ SIGNATURES = {
     "b2s_set_timing": (C.c_int, [vp, C.c_int]),
     "b2s_get_timers": (C.c_int, [vp, C.POINTER(Timers)]),
     "b2s_reset_timers": (C.c_int, [vp]),
+    "b2s_inject_failure": (C.c_int, [vp, C.c_int, i64]),
     "b2s_ws_init": (C.c_int, [vp, i32, C.c_uint64]),
     "b2s_ws_add_sample": (C.c_int, [vp, vp, i32, vp, vp]),
     "b2s_ws_num_samples": (C.c_int, [vp, i32p, i64p]),

@@ -474,6 +474,17 @@ int b2s_reset_timers(b2s_solver* s)
     return B2S_OK;
 }
 
+int b2s_inject_failure(b2s_solver* s, int what, int64_t value)
+{
+    return guarded(s,
+                   [&]
+                   {
+                       B2S_REQUIRE(what == B2S_INJECT_WAIT_POLLS, B2S_ERR_ARGUMENT, "unknown failure");
+                       B2S_REQUIRE(value >= -1 && value <= INT32_MAX, B2S_ERR_ARGUMENT, "value out of range");
+                       s->inject_polls = value;
+                   });
+}
+
 // ---------------------------------------------------------------------------
 // partition utilities (host)
 // ---------------------------------------------------------------------------

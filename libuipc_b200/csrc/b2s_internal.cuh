@@ -297,6 +297,7 @@ struct b2s_solver
     cudaEvent_t              ev_begin = nullptr, ev_end = nullptr;
     std::vector<cudaEvent_t> iter_events;  // 4 per iteration of a graph block
     b2s::LearnedState*       ws = nullptr;  // learned warm start, created on first use
+    int64_t                  inject_polls = -1;  // B2S_INJECT_WAIT_POLLS
     // triplet arrays owned by the solver (b2s_triplet_buffers): producers
     // write the raw triplets here, b2s_assemble_owned reads them in place
     b2s::DBuf<int32_t>       own_rows, own_cols;
@@ -347,6 +348,10 @@ void precond_apply_mixed(b2s_solver* s, const float* r, float* z);
 void spmv_mixed(b2s_solver* s, const float* x, float* y, double* d_dot);
 double spmv_mixed_timing(b2s_solver* s, int launches);
 void check_device_errors(b2s_solver* s);
+// pinned memory for scalars on their way to the host
+void ensure_read_back(b2s_solver* s);
+// throws when the error bits e (already cleared on the device) are not zero
+void raise_device_errors(b2s_solver* s, int e);
 // n <= READ_BACK doubles from the device into h, with the stream's work done
 // and its device errors raised
 void read_back(b2s_solver* s, const double* d, int n, double* h);

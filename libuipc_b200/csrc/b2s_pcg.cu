@@ -730,6 +730,13 @@ __global__ void __launch_bounds__(RED_BLOCK) k_dot2_f32(int64_t n, const float* 
     }
 }
 
+// scalars and error bits (cleared) into pinned host memory
+__global__ void k_scalars_out(const PcgScalars* sc, int* err, PcgScalars* out, ReadBack* back)
+{
+    *out      = *sc;
+    back->err = atomicExch(err, 0);
+}
+
 // FP32 copy of the value planes (mixed-precision SpMV)
 __global__ void k_planes_f32(int64_t count, const double* __restrict__ src, float* __restrict__ dst)
 {
@@ -1059,6 +1066,20 @@ static void pcg_iteration(b2s_solver* s, int kind, bool ord, double* x, int slot
     B2S_CHECK_LAUNCH();
 }
 
+// The loop's scalars and the device's error bits to the host, in one wait.
+// Throws when a wait on the device has run out (the one-launch loop then leaves
+// the scalars as they were) or when the iterations launched since `iter_before`
+// did nothing: the host's loop ends with every launch that does not advance.
+static void read_scalars(b2s_solver* s, long long iter_before)
+{
+    PcgState& P = s->pcg;
+    k_scalars_out<<<1, 1, 0, s->stream>>>(P.sc.data(), s->dev_err.data(), P.h_sc, s->h_back);
+    B2S_CHECK_LAUNCH();
+    B2S_CUDA(cudaStreamSynchronize(s->stream));
+    raise_device_errors(s, s->h_back->err);
+    B2S_REQUIRE(P.h_sc->converged != 0 || P.h_sc->iter > iter_before, B2S_ERR_CUDA, "the PCG made no progress");
+}
+
 static void ensure_iter_events(b2s_solver* s, int ci)
 {
     while((int)s->iter_events.size() < 4 * ci)
@@ -1110,6 +1131,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
     P.sc.resize(1);
     if(!P.h_sc)
         B2S_CUDA(cudaMallocHost(&P.h_sc, sizeof(PcgScalars)));
+    ensure_read_back(s);
     ensure_reduction(P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
     ensure_reduction(s->red, reduction_grid(), 2);  // the largest grid: the sums below run over rows and over entries
     device_error_flag(s);  // allocated before any graph capture
@@ -1293,8 +1315,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
             else
                 for(int it = 0; it < ci; ++it)
                     pcg_iteration(s, kind, ord, xi, it);
-            B2S_CUDA(cudaMemcpyAsync(P.h_sc, P.sc.data(), sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
-            B2S_CUDA(cudaStreamSynchronize(st));
+            read_scalars(s, iter_before);
             if(s->timing)
             {
                 // the iterations of this block that did work (the rest were frozen)
@@ -1559,6 +1580,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
     P.sc.resize(1);
     if(!P.h_sc)
         B2S_CUDA(cudaMallocHost(&P.h_sc, sizeof(PcgScalars)));
+    ensure_read_back(s);
     ensure_reduction(P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
     ensure_reduction(s->red, reduction_grid(), 2);
     device_error_flag(s);
@@ -1734,8 +1756,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
             else
                 for(int it = 0; it < ci; ++it)
                     pcg_iteration_mixed(s, kind, ord, xi, it);
-            B2S_CUDA(cudaMemcpyAsync(P.h_sc, P.sc.data(), sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
-            B2S_CUDA(cudaStreamSynchronize(st));
+            read_scalars(s, iter_before);
             if(s->timing)
             {
                 const long long live = std::min<long long>(P.h_sc->iter - iter_before, ci);

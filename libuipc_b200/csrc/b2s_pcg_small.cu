@@ -15,7 +15,9 @@
 // barrier whose arrival releases and whose wait acquires at device scope. The
 // bulk copies (TMA) only read inverses, which the launch never writes. Every
 // wait is bounded: a barrier or a copy that runs out sets the error flag and
-// the block leaves; the others' barriers then run out too.
+// the block leaves, its copies in flight waited for; the others' barriers then
+// run out too. The scalars stay as they were, and the host, which reads the
+// flag with them after every launch, ends the call with an error.
 #include "b2s_mas_apply.cuh"
 #include "b2s_pcg.cuh"
 
@@ -58,11 +60,13 @@ struct SmallArgs
     const uint16_t* comp_mask;  // of the slots
     const int32_t*  new_local;
     long long      iterations;
+    unsigned       polls;  // of a barrier, before it gives up
 };
 
 // grid barrier: false when it runs out, or when a warp of this block has given
 // up (*s_dead: the block does not arrive)
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned& epoch, int* err, const int* s_dead)
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned& epoch, unsigned polls, int* err,
+                                             const int* s_dead)
 {
     __shared__ int s_ok;
     epoch += gridDim.x;
@@ -74,7 +78,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned& epoch, int
         if(!dead)
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         int ok = 0;
-        for(unsigned i = 0; i < SM_SPINS && !dead; ++i)
+        for(unsigned i = 0; i < polls && !dead; ++i)
         {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
@@ -281,7 +285,7 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
     // every block leaves the loop through here when a barrier runs out
     auto barrier = [&]() -> bool
     {
-        const bool ok = grid_barrier(a.bar, epoch, a.A.err, &s_dead);
+        const bool ok = grid_barrier(a.bar, epoch, a.polls, a.A.err, &s_dead);
         if(MAS && !ok && underway)
             mbar_wait(&s_bar[SM_WARPS + u1 % SM_COARSE], (uint32_t)((u1 / SM_COARSE) & 1), nullptr, 0);
         return ok;
@@ -307,6 +311,8 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
         }
         __syncthreads();
         const bool here = bank0 >= n0 || mbar_wait(&s_bar[w], 0, a.A.err, DERR_TMA_TIMEOUT);
+        if(!here)  // once more, for the copy to end before the block does
+            mbar_wait(&s_bar[w], 0, nullptr, 0);
         if(!__syncthreads_and(here))
             return;  // the others' first barrier runs out
         if(a.A.stiff)
@@ -646,6 +652,7 @@ void launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterat
     }
     a.A.err      = device_error_flag(s);
     a.iterations = iterations;
+    a.polls      = s->inject_polls < 0 ? SM_SPINS : (unsigned)s->inject_polls;
     P.small_partials.resize(3 * (size_t)grid);
     P.small_bar.resize(1);
     a.partials = P.small_partials.data();

@@ -522,19 +522,32 @@ __global__ void k_read_back(const double* __restrict__ d, int n, int* err, ReadB
 // memory, then one wait for the stream: a copy to pageable memory waits by
 // itself, ~9 us each, and an entry point that read its error flag and then its
 // dot did so twice.
-void read_back(b2s_solver* s, const double* d, int n, double* h)
+void ensure_read_back(b2s_solver* s)
 {
     if(!s->h_back)
         B2S_CUDA(cudaMallocHost(&s->h_back, sizeof(ReadBack)));
+}
+
+void raise_device_errors(b2s_solver* s, int e)
+{
+    if(e == 0)
+        return;
+    // an apply that stopped halfway has left sums for the next one
+    if(s->mas.R64.size() > 0)
+        B2S_CUDA(cudaMemsetAsync(s->mas.R64.data(), 0, s->mas.R64.bytes(), s->stream));
+    throw Error(B2S_ERR_CUDA, std::string("device error flag ") + std::to_string(e)
+                                  + ((e & DERR_TMA_TIMEOUT) ? ": a bulk-copy or barrier wait timed out" : ""));
+}
+
+void read_back(b2s_solver* s, const double* d, int n, double* h)
+{
+    ensure_read_back(s);
     k_read_back<<<1, 32, 0, s->stream>>>(d, n, s->dev_err.size() ? s->dev_err.data() : nullptr, s->h_back);
     B2S_CHECK_LAUNCH();
     B2S_CUDA(cudaStreamSynchronize(s->stream));
     for(int i = 0; i < n; ++i)
         h[i] = s->h_back->v[i];
-    const int e = s->h_back->err;
-    if(e != 0)
-        throw Error(B2S_ERR_CUDA, std::string("device error flag ") + std::to_string(e)
-                                      + ((e & DERR_TMA_TIMEOUT) ? ": a bulk-copy or barrier wait timed out" : ""));
+    raise_device_errors(s, s->h_back->err);
 }
 
 // raise (and clear) the error bits kernels left in the device flag

@@ -9,6 +9,8 @@
 * Iteration cap (LinearPCG::pcg, linear_pcg.cu:420-435): with max_iter = 3 the
   solve stops unconverged and reports it.
 * Warm start refused by its FP64 check: x0 = 0 (the plain start).
+* A device wait that runs out (b2s_inject_failure shortens it): the call ends
+  with B2S_ERR_CUDA and the handle solves again.
 """
 import numpy as np
 import pytest
@@ -135,3 +137,32 @@ def test_warm_start_refused_by_its_check_is_zero(solver, cuda, cube5):
     xz = torch.zeros_like(b)
     st0 = solver.pcg(b, xz, tol=1e-4, stop_rule=_abi.B2S_STOP_RELRES)
     assert st["iterations_exact"] == st0["iterations_exact"]
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("kind", [_abi.B2S_PRECOND_JACOBI, _abi.B2S_PRECOND_MAS])
+@pytest.mark.parametrize("polls", [0, 1])
+def test_a_barrier_that_runs_out_ends_the_call(solver, cuda, cube10, kind, precision, polls):
+    """The one-launch PCG (1,331 rows) with barriers that give up after `polls`
+    polls: the call returns an error, and the same handle, with the same build
+    and with the default limit again, solves as it did before."""
+    import torch
+
+    b = _setup(solver, cube10, cuda, kind)
+    args = dict(tol=1e-8, stop_rule=_abi.B2S_STOP_RELRES, precision=precision, replace_every=50)
+    x0 = torch.zeros_like(b)
+    st0 = solver.pcg(b, x0, **args)
+    assert st0["converged"] == 1
+    solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_WAIT_POLLS, polls))
+    for _ in range(2):
+        with pytest.raises(B200SolveError) as e:
+            solver.pcg(b, torch.zeros_like(b), **args)
+        assert e.value.code == _abi.B2S_ERR_CUDA and "timed out" in str(e.value)
+    solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_WAIT_POLLS, -1))
+    x = torch.zeros_like(b)
+    st = solver.pcg(b, x, **args)
+    # the two solves differ in the order of the SpMV's reductions only: the stop
+    # may move by a few iterations, the answers by the tolerance's own error
+    # (3e-7 of the solution on a cube at this tolerance)
+    assert st["converged"] == 1 and abs(st["iterations_exact"] - st0["iterations_exact"]) <= 5
+    assert float((x - x0).norm()) <= 1e-5 * float(x0.norm())
