@@ -289,11 +289,13 @@ __device__ __forceinline__ void precond_row(int kind, const MasView& mv, const d
         // row l of body b: z = (H_b^-1)[3l .. 3l+2][0 .. 11] r_b
         const int     b = (row - mv.abd_off) >> 2, l = (row - mv.abd_off) & 3;
         const double* Hi = mv.abd_inv + (size_t)b * 144 + 36 * l;
-        const int64_t n0 = (int64_t)i - l;  // the body's first node (its rows stay together in either order)
         double        a0 = 0.0, a1 = 0.0, a2 = 0.0;
         for(int j = 0; j < 12; ++j)
         {
-            const double rj = r[NS * (n0 + j / 3) + j % 3];
+            // in PCG order a body's rows need not follow one another: a caller
+            // may have put some of them into the MAS partition
+            const int64_t n  = ORD ? mv.pos[row - l + j / 3] : row - l + j / 3;
+            const double  rj = r[NS * n + j % 3];
             a0 += Hi[j] * rj;
             a1 += Hi[12 + j] * rj;
             a2 += Hi[24 + j] * rj;
@@ -829,6 +831,7 @@ MasView mas_view(b2s_solver* s)
     mv.T      = M.L <= 1 ? 0 : M.L - 1;
     mv.Z      = M.Z.data();
     mv.row_of     = s->pcg.ord.row_of.data();
+    mv.pos        = s->pcg.ord.pos.data();
     mv.slot_node1 = s->pcg.ord.node1.data();
     mv.slots      = s->pcg.ord.slots;
     return mv;

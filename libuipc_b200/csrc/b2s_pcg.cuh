@@ -19,6 +19,7 @@ struct MasView
     const float*   Z;      // node values by slot
     // rows in PCG order (null: the matrix's own order)
     const int32_t* row_of;
+    const int32_t* pos;  // its inverse
     const int32_t* slot_node1;  // [slots]
     int            slots;
 };

@@ -338,8 +338,8 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
         load_vec(a.p, i, p);
         load_vec(a.x, i, x);
     }
-    // block Jacobi rows
-    const int  row = (MAS && live && !in_bank) ? a.mv.row_of[i] : i;
+    // the matrix's row (-1: padding slot); a body's rows may lie anywhere in PCG order
+    const int  row = (MAS && live) ? a.mv.row_of[i] : i;
     const bool body = a.mv.abd_n > 0 && row >= a.mv.abd_off && row < a.mv.abd_off + 4 * a.mv.abd_n;
     PcgScalars sc   = *a.sc;
     double*    part0 = a.partials;
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
                 for(int q = 0; q < 4; ++q)
                 {
                     VT rq[3];
-                    load_vec(a.r, (int64_t)i - l + q, rq);
+                    load_vec(a.r, MAS ? a.mv.pos[row - l + q] : row - l + q, rq);
 #pragma unroll
                     for(int c = 0; c < 3; ++c)
 #pragma unroll

@@ -173,3 +173,53 @@ def test_banks_of_many_components(solver, cuda, n, part, edges, precision):
     # the same recursion; the sums' order moves the stop by a few iterations,
     # and in FP32 the restarts from the true residual with it
     assert abs(its[0] - its[1]) <= (3 if precision == 0 else 0.2 * its[1])
+
+
+@pytest.mark.parametrize("first", [56, 58, 72, 76])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_body_rows_inside_the_mas_range(solver, cuda, first, precision):
+    """An affine body whose rows a later b2s_mas_init covers, some of them in
+    the partition and some not: rows of the partition take the MAS, the others
+    the body's inverse with the residual of all four rows. The recursion in
+    slot order follows the operator b2s_precond_apply shows, in one launch, in
+    a graph and launch by launch."""
+    import torch
+
+    rng = np.random.default_rng(first)
+    nb, off, rows, cols, vals, A, last, start, lst = _system(rng, 80, 0, 0, 0)
+    p2r, r2p = _maps(rng, nb, 16, 0)
+    out = np.arange(first + 1, first + 4, 2)  # two of the body's rows leave the partition
+    p2r[r2p[out]] = -1
+    r2p[out] = -1
+    solver.assemble(nb, to_dev(rows, cuda), to_dev(cols, cuda), to_dev(vals, cuda))
+    solver.abd_init(first, 1)
+    solver.mas_init(0, nb, start, lst, p2r, r2p)
+    solver.precond_assemble(2)
+    n = 3 * nb
+    z = torch.zeros(n, dtype=torch.float64 if precision == 0 else torch.float32, device=cuda)
+    apply = solver.precond_apply if precision == 0 else solver.precond_apply_mixed
+    P = np.zeros((n, n))
+    for k in range(n):
+        e = torch.zeros_like(z)
+        e[k] = 1.0
+        apply(e, z)
+        P[:, k] = z.cpu().numpy()
+    b = rng.normal(size=n)
+    x, r = np.zeros(n), b.copy()
+    p = s = P @ r
+    rz0 = rz = r @ s
+    for _ in range(4):
+        a = rz / (p @ A @ p)
+        x, r = x + a * p, r - a * (A @ p)
+        s = P @ r
+        p, rz = s + (r @ s) / rz * p, r @ s
+    assert np.linalg.norm(P - P.T) > 1e-3 * np.linalg.norm(P)  # not the operator of any other reading of the range
+    for graph, timing in ((True, False), (True, True), (False, False)):
+        solver.set_timing(timing)
+        xd = torch.zeros(n, dtype=torch.float64, device=cuda)
+        st = solver.pcg(to_dev(b, cuda), xd, tol=1e-30, max_iter=5, precision=precision, use_graph=graph)
+        # FP32 inverses and Z, or BF16 tiles with FP32 vectors whose residual
+        # enters with 16 bits: 2^-24 and 2^-16 per apply, times the growth over four steps
+        tol = 1e-5 if precision == 0 else 1e-2
+        assert st["bypassed"] == 0 and abs(st["rz0"] - rz0) <= tol * rz0
+        assert np.linalg.norm(xd.cpu().numpy() - x) <= tol * np.linalg.norm(x)
