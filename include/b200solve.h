@@ -244,10 +244,11 @@ int b2s_get_timers(const b2s_solver* s, b2s_timers* out);
 int b2s_reset_timers(b2s_solver* s);
 
 /* ---- failure injection ----------------------------------------------------------------
- * For tests of the error paths: a wait of this handle's kernels gives up early.
- * Nothing faults or hangs; the affected call returns the status it returns when
- * the same happens by itself. */
+ * For tests of the error paths: a wait of this handle's kernels gives up early,
+ * or the host sees a launch refused. Nothing faults or hangs; the affected call
+ * does what it does when the same happens by itself. */
 #define B2S_INJECT_WAIT_POLLS 0 /* a grid barrier of the one-launch PCG gives up after `value` polls (-1: the default, seconds) */
+#define B2S_INJECT_LAUNCH 1     /* the next `value` cooperative launches are refused, as for a stream with too few SMs */
 int b2s_inject_failure(b2s_solver* s, int what, int64_t value);
 
 /* ---- learned PCG warm start ------------------------------------------------------------

@@ -21,6 +21,7 @@ B2S_INVERT_F32_ONLY = 2
 B2S_STOP_RZ = 0
 B2S_STOP_RELRES = 1
 B2S_INJECT_WAIT_POLLS = 0
+B2S_INJECT_LAUNCH = 1
 
 B2S_PRECISION_FP64 = 0
 B2S_PRECISION_MIXED = 1

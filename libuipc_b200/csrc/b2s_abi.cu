@@ -479,9 +479,11 @@ int b2s_inject_failure(b2s_solver* s, int what, int64_t value)
     return guarded(s,
                    [&]
                    {
-                       B2S_REQUIRE(what == B2S_INJECT_WAIT_POLLS, B2S_ERR_ARGUMENT, "unknown failure");
-                       B2S_REQUIRE(value >= -1 && value <= INT32_MAX, B2S_ERR_ARGUMENT, "value out of range");
-                       s->inject_polls = value;
+                       B2S_REQUIRE(what == B2S_INJECT_WAIT_POLLS || what == B2S_INJECT_LAUNCH, B2S_ERR_ARGUMENT,
+                                   "unknown failure");
+                       B2S_REQUIRE(value >= (what == B2S_INJECT_WAIT_POLLS ? -1 : 0) && value <= INT32_MAX,
+                                   B2S_ERR_ARGUMENT, "value out of range");
+                       (what == B2S_INJECT_WAIT_POLLS ? s->inject_polls : s->inject_launch) = value;
                    });
 }
 

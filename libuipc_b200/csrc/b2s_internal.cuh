@@ -298,6 +298,7 @@ struct b2s_solver
     std::vector<cudaEvent_t> iter_events;  // 4 per iteration of a graph block
     b2s::LearnedState*       ws = nullptr;  // learned warm start, created on first use
     int64_t                  inject_polls = -1;  // B2S_INJECT_WAIT_POLLS
+    int64_t                  inject_launch = 0;  // B2S_INJECT_LAUNCH
     // triplet arrays owned by the solver (b2s_triplet_buffers): producers
     // write the raw triplets here, b2s_assemble_owned reads them in place
     b2s::DBuf<int32_t>       own_rows, own_cols;

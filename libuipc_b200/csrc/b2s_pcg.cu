@@ -1243,16 +1243,18 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         B2S_CUDA(cudaMemcpyAsync(P.p.data(), P.z.data(), sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
         B2S_CUDA(cudaMemsetAsync(P.Ap.data(), 0, sizeof(double) * n, st));
 
-        // CUDA graph of `ci` iterations (re-captured when anything it bakes in changes)
         bool use_graph = o.use_graph && st != nullptr;
         // small systems: the whole loop in one launch
-        const bool small = use_graph && !s->timing && pcg_small_fits(s, A, kind, ord, false);
-        if(!small)
-            ensure_tile_ranks(s, ord ? P.ord.A : s->A);
+        bool small = use_graph && !s->timing && pcg_small_fits(s, A, kind, ord, false);
         if(s->timing)
             ensure_iter_events(s, ci);
-        if(use_graph && !small)
+        // else launch by launch, from a CUDA graph of `ci` iterations
+        // (re-captured when anything it bakes in changes)
+        auto prepare_steps = [&]()
         {
+            ensure_tile_ranks(s, ord ? P.ord.A : s->A);
+            if(!use_graph)
+                return;
             GraphKey key{};
             key.ptrs[0] = xi;
             key.ptrs[1] = A.vals.data();
@@ -1304,18 +1306,23 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
                 else
                     P.graph_key = hk;
             }
-        }
+        };
+        if(!small)
+            prepare_steps();
         long long iter_before = h.iter;
         while(true)
         {
-            if(small)
-                pcg_small_launch(s, A, kind, ord, SMALL_LOOP, xi);
-            else if(use_graph)
+            if(small && !pcg_small_launch(s, A, kind, ord, SMALL_LOOP, xi))
+            {
+                small = false;
+                prepare_steps();
+            }
+            if(!small && use_graph)
             {
                 B2S_CUDA(cudaGraphLaunch(P.graph, st));
                 g_kernel_launches += P.graph_kernels;
             }
-            else
+            else if(!small)
                 for(int it = 0; it < ci; ++it)
                     pcg_iteration(s, kind, ord, xi, it);
             read_scalars(s, iter_before);
@@ -1697,12 +1704,15 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
         B2S_CUDA(cudaMemsetAsync(P.Ap32.data(), 0, sizeof(float) * n4, st));
         bool use_graph = o.use_graph && st != nullptr;
         // small systems: the loop in one launch, up to the next replacement
-        const bool small = use_graph && !s->timing && (kind != B2S_PRECOND_MAS || mixed_inverse_bf16())
-                           && pcg_small_fits(s, A, kind, ord, true);
+        bool small = use_graph && !s->timing && (kind != B2S_PRECOND_MAS || mixed_inverse_bf16())
+                     && pcg_small_fits(s, A, kind, ord, true);
         if(s->timing)
             ensure_iter_events(s, ci);
-        if(use_graph && !small)
+        // else launch by launch (graph as in pcg_solve)
+        auto prepare_steps = [&]()
         {
+            if(!use_graph)
+                return;
             const void*   ptrs[15] = {xi,         A.vals32.data(), A.rows.data(),     P.r32.data(),
                                       s->mas.inv16.data(), s->dinv.data(), P.red.partials.data(), s->mas.Z.data(),
                                       A.cols.data(), P.p32.data(), P.Ap32.data(), P.z32.data(),
@@ -1740,7 +1750,9 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
                 else
                     P.graph_mixed_key = hk;
             }
-        }
+        };
+        if(!small)
+            prepare_steps();
         long long iter_before = h.iter;
         while(true)
         {
@@ -1749,14 +1761,18 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
                 // whole blocks of check_interval, as the replacements are counted
                 const long long due = o.replace_every > 0 ? std::max<long long>(last_replace + o.replace_every - iter_before, 1) :
                                                             SMALL_LOOP;
-                pcg_small_launch_f32(s, A, kind, ord, std::min<long long>((due + ci - 1) / ci * ci, SMALL_LOOP), xi);
+                if(!pcg_small_launch_f32(s, A, kind, ord, std::min<long long>((due + ci - 1) / ci * ci, SMALL_LOOP), xi))
+                {
+                    small = false;
+                    prepare_steps();
+                }
             }
-            else if(use_graph)
+            if(!small && use_graph)
             {
                 B2S_CUDA(cudaGraphLaunch(P.graph_mixed, st));
                 g_kernel_launches += P.graph_mixed_kernels;
             }
-            else
+            else if(!small)
                 for(int it = 0; it < ci; ++it)
                     pcg_iteration_mixed(s, kind, ord, xi, it);
             read_scalars(s, iter_before);

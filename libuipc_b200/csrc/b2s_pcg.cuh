@@ -28,8 +28,10 @@ MasView mas_view(b2s_solver* s);
 
 // One launch for up to `iterations` PCG iterations (b2s_pcg_small.cu): A and
 // the vectors in PCG order with the MAS (`ord`), r, p and x set by the caller,
-// Ap zero, the scalars in s->pcg.sc (read and written back).
+// Ap zero, the scalars in s->pcg.sc (read and written back). The launch returns
+// false, with nothing done, when the device refuses it (fewer SMs than the
+// device has: a shared or partitioned GPU): the caller launches step by step.
 bool pcg_small_fits(b2s_solver* s, const Matrix& A, int kind, bool ord, bool f32);
-void pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x);
-void pcg_small_launch_f32(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x);
+bool pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x);
+bool pcg_small_launch_f32(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x);
 }  // namespace b2s

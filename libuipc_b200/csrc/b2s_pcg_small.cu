@@ -622,7 +622,7 @@ int small_grid(const Matrix& A)
 }
 
 template <typename VT>
-void launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x, const VT* vals, VT* r,
+bool launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x, const VT* vals, VT* r,
             VT* p, VT* Ap)
 {
     PcgState&     P   = s->pcg;
@@ -662,8 +662,19 @@ void launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterat
     const size_t smem = small_smem<VT>(mas);
     B2S_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void* args[] = {&a};
-    B2S_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(SM_THREADS), args, smem, s->stream));
+    cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
+    if(s->inject_launch > 0)
+        --s->inject_launch;
+    else
+        e = cudaLaunchCooperativeKernel(k, dim3(grid), dim3(SM_THREADS), args, smem, s->stream);
+    if(e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported)
+    {
+        cudaGetLastError();
+        return false;
+    }
+    B2S_CUDA(e);
     B2S_CHECK_LAUNCH();
+    return true;
 }
 }  // namespace
 
@@ -693,14 +704,14 @@ bool pcg_small_fits(b2s_solver* s, const Matrix& A, int kind, bool ord, bool f32
     return (int64_t)small_grid(A) <= (int64_t)occ * sms && A.nnz <= 16ll * SM_THREADS * occ * sms;
 }
 
-void pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x)
+bool pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x)
 {
     PcgState& P = s->pcg;
-    launch<double>(s, A, kind, ord, iterations, x, A.vals.data(), P.r.data(), P.p.data(), P.Ap.data());
+    return launch<double>(s, A, kind, ord, iterations, x, A.vals.data(), P.r.data(), P.p.data(), P.Ap.data());
 }
-void pcg_small_launch_f32(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x)
+bool pcg_small_launch_f32(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x)
 {
     PcgState& P = s->pcg;
-    launch<float>(s, A, kind, ord, iterations, x, A.vals32.data(), P.r32.data(), P.p32.data(), P.Ap32.data());
+    return launch<float>(s, A, kind, ord, iterations, x, A.vals32.data(), P.r32.data(), P.p32.data(), P.Ap32.data());
 }
 }  // namespace b2s

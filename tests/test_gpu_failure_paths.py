@@ -166,3 +166,29 @@ def test_a_barrier_that_runs_out_ends_the_call(solver, cuda, cube10, kind, preci
     # (3e-7 of the solution on a cube at this tolerance)
     assert st["converged"] == 1 and abs(st["iterations_exact"] - st0["iterations_exact"]) <= 5
     assert float((x - x0).norm()) <= 1e-5 * float(x0.norm())
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("kind", [_abi.B2S_PRECOND_JACOBI, _abi.B2S_PRECOND_MAS])
+@pytest.mark.parametrize("replace_every", [0, 20])
+def test_a_refused_cooperative_launch_takes_the_steps(solver, cuda, cube10, kind, precision, replace_every):
+    """Where the device refuses the one-launch PCG's grid, the same call runs
+    launch by launch (the captured graph, in slot order with the MAS)."""
+    import torch
+
+    b = _setup(solver, cube10, cuda, kind)
+    args = dict(tol=1e-8, stop_rule=_abi.B2S_STOP_RELRES, precision=precision, replace_every=replace_every)
+    x0, x1 = torch.zeros_like(b), torch.zeros_like(b)
+    solver.reset_timers()
+    st0 = solver.pcg(b, x0, **args)
+    one = solver.timers()["kernel_launches"]
+    solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_LAUNCH, 1000))
+    solver.reset_timers()
+    st1 = solver.pcg(b, x1, **args)
+    steps = solver.timers()["kernel_launches"]
+    solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_LAUNCH, 0))
+    assert st0["converged"] == st1["converged"] == 1
+    assert steps >= 4 * st1["iterations_exact"] > one  # it did take the steps
+    # as for the barriers above: rounding order only
+    assert abs(st0["iterations_exact"] - st1["iterations_exact"]) <= 5
+    assert float((x0 - x1).norm()) <= 1e-5 * float(x0.norm())
