@@ -188,7 +188,11 @@ struct MasState
     DBuf<double>  trip_vals;
     // apply buffers (FP32, 3 per node slot)
     DBuf<float>   R, Z;
-    DBuf<double>  R64;  // sums of the restriction at the levels above 1 (zero between applies)
+    // the restriction to the levels above 1: FP64 sums of a block of slots, one
+    // entry per node and block that has a component under it, a node's in block order
+    DBuf<double>  part;        // [3 * entries], written by every restriction
+    DBuf<int32_t> part_start;  // [nodes above level 1 + 1] first entry of each node
+    DBuf<int4>    part_dst;    // [level_count[1]] entries of each level-1 node at levels 2-5: 2 entry + (not its first), -1: none
     // host copies for introspection
     std::vector<int32_t> h_ctable;
     long long     generation = 0;  // bumped by every initialisation
@@ -352,7 +356,7 @@ void check_device_errors(b2s_solver* s);
 // pinned memory for scalars on their way to the host
 void ensure_read_back(b2s_solver* s);
 // throws when the error bits e (already cleared on the device) are not zero
-void raise_device_errors(b2s_solver* s, int e);
+void raise_device_errors(int e);
 // n <= READ_BACK doubles from the device into h, with the stream's work done
 // and its device errors raised
 void read_back(b2s_solver* s, const double* d, int n, double* h);

@@ -19,8 +19,9 @@
 // Galerkin matrices are built level by level as sparse matrices with the same
 // deterministic triplet assembly as the global matrix (A_{l+1} from A_l), so
 // no FP64 atomics pile onto the few clusters of the top levels; the apply
-// restricts to level 1 in one launch and does every level in a second one
-// (one warp per bank; fixed summation order, bit-reproducible).
+// restricts to every coarse level in one launch (above level 1 as partial sums
+// per block of slots) and does every level in a second one (one warp per bank);
+// every sum has a fixed order, so an apply is bit-reproducible.
 #include "b2s_internal.cuh"
 #include "b2s_reduce.cuh"
 #include "b2s_mas_apply.cuh"
@@ -537,7 +538,7 @@ __global__ void __launch_bounds__(PACK_THREADS) k_pack_inverse_bf16(int clusters
 }
 
 // Every level in one launch: the restriction has left R_0, R_1 and the FP64
-// sums of the levels above, so no bank waits for another. One launch per level
+// partial sums of the levels above, so no bank waits for another. One launch per level
 // (level 1 on the whole GPU, the others on a side stream beside the fine level,
 // then a fold of the prolongation) left systems below ~100,000 vertices
 // waiting for a chain of six 4-5 us launches: the level launches and the fold
@@ -546,8 +547,6 @@ __global__ void __launch_bounds__(PACK_THREADS) k_pack_inverse_bf16(int clusters
 template <bool BF, int NST>
 __global__ void __launch_bounds__(APPLY_WARPS * 32, BF ? 7 : 5) k_apply_all(ApplyArgs A, const int* converged)
 {
-    if(converged && *converged)
-        return;
     constexpr uint32_t SB = stage_bytes<BF>();
     __shared__ __align__(128) unsigned char s_stage[APPLY_WARPS][NST][SB];
     __shared__ uint64_t s_bar[APPLY_WARPS][NST];
@@ -559,31 +558,40 @@ __global__ void __launch_bounds__(APPLY_WARPS * 32, BF ? 7 : 5) k_apply_all(Appl
         mbar_fence_init();
     }
     __syncwarp();
-    apply_banks<BF, NST>(blockIdx.x * APPLY_WARPS + w, gridDim.x * APPLY_WARPS, lane, A, &s_stage[w][0][0], s_bar[w]);
+    __shared__ double s_sum[BANK * APPLY_WARPS * 3];
+    int gw = ((int)blockIdx.x - A.heavy) * APPLY_WARPS + w;
+    if((int)blockIdx.x < A.heavy)
+    {
+        heavy_bank<BF, APPLY_WARPS>(A, (int64_t)A.g4 + blockIdx.x, converged, &s_stage[0][0][0], s_bar[0], s_sum);
+        if(w == 0)
+            return;
+        // its other warps join the rest, last in the order
+        gw = ((int)gridDim.x - A.heavy) * APPLY_WARPS + (int)blockIdx.x * (APPLY_WARPS - 1) + w - 1;
+    }
+    apply_banks<BF, NST>(gw, (int)gridDim.x * APPLY_WARPS - A.heavy, lane, A, converged, &s_stage[w][0][0], s_bar[w]);
 }
 
 // The fine residual in partition order and the sums of every coarse level, a
 // thread per slot: R_0 (FP32, zero in padding slots) is the only gather of r
 // through part_to_real, so the fine level streams its banks' residuals with
 // their inverses.
-constexpr int RESTRICT_THREADS = 256;
 template <typename VT>
 __global__ void __launch_bounds__(RESTRICT_THREADS)
     k_restrict_fine(int n_slots, const int32_t* __restrict__ p2r, const VT* __restrict__ r, int roff,
                     const uint16_t* __restrict__ comp_mask, const int32_t* __restrict__ new_local,
-                    const int4* __restrict__ anc, int begin1, int begin2, int push, float* __restrict__ R,
-                    double* __restrict__ R64, const int* converged)
+                    const int4* __restrict__ dst, int begin1, int push, float* __restrict__ R,
+                    double* __restrict__ part, const int* converged)
 {
     if(converged && *converged)
         return;
     __shared__ float s_r[RESTRICT_THREADS][3], s_lead[RESTRICT_THREADS][3];
-    __shared__ int4  s_anc[RESTRICT_THREADS];
+    __shared__ int4  s_dst[RESTRICT_THREADS];
     __shared__ int   s_n[RESTRICT_THREADS / 32];
     const int t = threadIdx.x, p = blockIdx.x * RESTRICT_THREADS + t, sub = t & 15;
     float     n0 = 0.f, n1 = 0.f, n2 = 0.f;
     uint32_t  cm = 0;
     int       nl = 0;
-    int4      an = make_int4(-1, -1, -1, -1);
+    int4      to = make_int4(-1, -1, -1, -1);
     if(p < n_slots)
     {
         const int v = p2r[p];
@@ -594,7 +602,7 @@ __global__ void __launch_bounds__(RESTRICT_THREADS)
                 cm = comp_mask[p];
                 nl = new_local[p];
                 if(cm != 0 && (cm & ((1u << sub) - 1u)) == 0)
-                    an = anc[nl];
+                    to = dst[nl];
             }
             if constexpr(sizeof(VT) == 4)
             {
@@ -619,7 +627,7 @@ __global__ void __launch_bounds__(RESTRICT_THREADS)
     s_r[t][2] = n2;
     __syncthreads();
     if(push)
-        restrict_coarse<RESTRICT_THREADS>(s_r, cm, nl, an, begin1, R, R64, begin2, s_lead, s_anc, s_n);
+        restrict_coarse<RESTRICT_THREADS>(s_r, cm, nl, to, begin1, R, part, s_lead, s_dst, s_n);
 }
 
 // the ancestors of the level-1 nodes, four per node (levels 2-5; -1: none):
@@ -644,11 +652,81 @@ __global__ void k_h_ancestors(int cnt1, int L, LevelIds ids, int4* anc)
     anc[c] = make_int4(a[0], a[1], a[2], a[3]);
 }
 
+// the block of slots of every level-1 node
+__global__ void k_h_block(int n_slots, const int32_t* __restrict__ new_local, int32_t* __restrict__ block)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if(p < n_slots && new_local[p] >= 0)
+        block[new_local[p]] = p / RESTRICT_THREADS;  // the same from every slot of the node
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+
+// The entries of the partial sums above level 1 (MasState::part): for every
+// node there, one per block of RESTRICT_THREADS slots with a level-1 node under
+// it, in block order; every level-1 node learns its entries. Level-1 nodes are
+// numbered bank by bank, so their blocks ascend.
+static void place_partials(b2s_solver* s)
+{
+    MasState&     M    = s->mas;
+    const int     cnt1 = M.level_count[1], begin2 = M.level_begin[2], nodes = M.total - begin2;
+    cudaStream_t  st   = s->stream;
+    DBuf<int32_t> d_block;
+    d_block.resize(std::max(cnt1, 1));
+    std::vector<int32_t> block(cnt1), start(nodes + 1, 0), last(nodes, -1);
+    std::vector<int4>    dst(cnt1);
+    if(cnt1 > 0)
+    {
+        k_h_block<<<grid_for(M.N, 256), 256, 0, st>>>(M.N, M.new_local[0].data(), d_block.data());
+        B2S_CHECK_LAUNCH();
+        B2S_CUDA(cudaMemcpyAsync(block.data(), d_block.data(), sizeof(int32_t) * cnt1, cudaMemcpyDeviceToHost, st));
+        B2S_CUDA(cudaMemcpyAsync(dst.data(), M.anc.data(), sizeof(int4) * cnt1, cudaMemcpyDeviceToHost, st));
+        B2S_CUDA(cudaStreamSynchronize(st));
+    }
+    // dst: the ancestors, then 2 (place among the node's entries) + (not the
+    // entry's first); start[m + 1]: the node's entries
+    for(int c = 0; c < cnt1; ++c)
+        for(int32_t* a : {&dst[c].x, &dst[c].y, &dst[c].z, &dst[c].w})
+            if(*a >= 0)
+            {
+                const int  m     = *a - begin2;
+                const bool first = last[m] != block[c];
+                last[m]          = block[c];
+                start[m + 1] += first ? 1 : 0;
+            }
+    int64_t entries = 0;
+    for(int m = 0; m < nodes; ++m)
+    {
+        entries += start[m + 1];
+        B2S_REQUIRE(entries < INT32_MAX / 2, B2S_ERR_ARGUMENT, "MAS hierarchy too large");
+        start[m + 1] = (int32_t)entries;
+        last[m]      = -1;
+    }
+    std::vector<int32_t> next(start.begin(), start.end() - 1);  // the entry after the node's current one
+    for(int c = 0; c < cnt1; ++c)
+        for(int32_t* a : {&dst[c].x, &dst[c].y, &dst[c].z, &dst[c].w})
+            if(*a >= 0)
+            {
+                const int  m     = *a - begin2;
+                const bool first = last[m] != block[c];
+                last[m]          = block[c];
+                next[m] += first ? 1 : 0;
+                *a = 2 * (next[m] - 1) + (first ? 0 : 1);
+            }
+    M.part.resize(std::max<size_t>(3 * (size_t)entries, 1));
+    M.part_start.resize(nodes + 1);
+    M.part_dst.resize(std::max(cnt1, 1));
+    B2S_CUDA(cudaMemcpyAsync(M.part_start.data(), start.data(), sizeof(int32_t) * (nodes + 1), cudaMemcpyHostToDevice,
+                             st));
+    if(cnt1 > 0)
+        B2S_CUDA(cudaMemcpyAsync(M.part_dst.data(), dst.data(), sizeof(int4) * cnt1, cudaMemcpyHostToDevice, st));
+    B2S_CUDA(cudaStreamSynchronize(st));
+}
+
 void mas_init(b2s_solver* s, int32_t offset, int32_t vn, const int32_t* adj_start, const int32_t* adj_list, int32_t N,
               const int32_t* p2r, const int32_t* r2p)
 {
@@ -791,8 +869,6 @@ void mas_init(b2s_solver* s, int32_t offset, int32_t vn, const int32_t* adj_star
     }
     M.hess.resize((size_t)M.clusters * SYM * 9);
     M.inv.resize((size_t)M.clusters * SYM * 9);
-    M.R64.resize(std::max<size_t>(3 * (size_t)(M.total - (L > 2 ? M.level_begin[2] : M.total)), 1));
-    B2S_CUDA(cudaMemsetAsync(M.R64.data(), 0, M.R64.bytes(), st));  // an apply leaves it zero
     M.R.resize((size_t)M.total * 3 + 3);
     M.Z.resize((size_t)M.total * 3 + 3);
     B2S_CUDA(cudaMemsetAsync(M.R.data(), 0, M.R.bytes(), st));
@@ -810,6 +886,8 @@ void mas_init(b2s_solver* s, int32_t offset, int32_t vn, const int32_t* adj_star
         k_h_ancestors<<<grid_for(M.level_count[1], TB), TB, 0, st>>>(M.level_count[1], L, ids, M.anc.data());
         B2S_CHECK_LAUNCH();
     }
+    if(L > 1)
+        place_partials(s);
     // level-1 node of every vertex, contiguous (the finish reads it per vertex)
     M.node1.resize(std::max(vn, 1));
     if(L > 1)
@@ -836,7 +914,6 @@ void mas_assemble(b2s_solver* s, int invert_mode)
     const int    TB = 256;
     const Matrix& A = s->A;
     B2S_CUDA(cudaMemsetAsync(M.hess.data(), 0, M.hess.bytes(), st));
-    B2S_CUDA(cudaMemsetAsync(M.R64.data(), 0, M.R64.bytes(), st));  // whatever an apply that failed has left
     if(A.nnz > 0 && M.L <= 1)
     {
         k_g_restrict<true><<<grid_for(A.nnz, GAL_BLOCKS), GAL_BLOCKS, 0, st>>>(
@@ -915,29 +992,42 @@ ApplyArgs mas_apply_args(b2s_solver* s, bool bf16)
     A.stiff = bf16 ? M.stiff.data() : nullptr;
     A.R     = M.R.data();
     A.Z     = M.Z.data();
-    A.R64   = M.R64.data();
+    A.part       = M.part.data();
+    A.part_start = M.part_start.data();
     A.err   = device_error_flag(s);
     A.n0    = M.N / BANK;
     A.n1    = M.L > 1 ? (M.level_count[1] + BANK - 1) / BANK : 0;
     A.g1    = M.L > 1 ? M.level_begin[1] / BANK : 0;
     A.g2    = M.L > 2 ? M.level_begin[2] / BANK : M.clusters;
+    A.g3    = M.L > 3 ? M.level_begin[3] / BANK : M.clusters;
     A.n2    = M.clusters - A.g2;
+    A.n3    = M.clusters - A.g3;
+    A.g4    = M.L > 4 ? M.level_begin[4] / BANK : M.clusters;
+    A.n4    = M.clusters - A.g4;
+    A.heavy = A.own = 0;
     return A;
 }
 
-// Z of every node from R_0, R_1 and the sums of the levels above
+// Z of every node from R_0, R_1 and the partial sums of the levels above
 void mas_apply_all(b2s_solver* s, const int* converged, bool bf16)
 {
-    const ApplyArgs A = mas_apply_args(s, bf16);
-    const int       n = A.n0 + A.n1 + A.n2;
+    ApplyArgs A = mas_apply_args(s, bf16);
+    const int n = A.n0 + A.n1 + A.n2;
     if(n == 0)
         return;
     auto k   = bf16 ? k_apply_all<true, APPLY_STAGES_BF16> : k_apply_all<false, APPLY_STAGES_F32>;
     int  occ = 0;
     if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, APPLY_WARPS * 32, 0) != cudaSuccess || occ < 1)
         occ = 1;
-    // persistent: the CTAs that fit at once, at most one warp per bank
+    // persistent: the CTAs that fit at once, at most one warp per bank; the banks
+    // of level 4 up each get a CTA to begin with, while those are an eighth at most
     const int grid = std::min((n + APPLY_WARPS - 1) / APPLY_WARPS, NUM_SMS_HINT * occ);
+    if(8 * A.n4 <= grid)
+        A.heavy = A.n4;
+    // the level-3 banks get warps of their own unless that costs the others another round
+    const int left = n - A.heavy, warps = grid * APPLY_WARPS - A.heavy, own = A.n3 - A.heavy;
+    if(4 * own <= warps && (left - own + warps - own - 1) / (warps - own) <= (left + warps - 1) / warps)
+        A.own = own;
     k<<<grid, APPLY_WARPS * 32, 0, s->stream>>>(A, converged);
     B2S_CHECK_LAUNCH();
 }
@@ -953,9 +1043,8 @@ static void apply_levels_t(b2s_solver* s, const VT* r, const int* converged, boo
     // element offset of the range's first vertex in r (FP32: 4 per node)
     const int off = (sizeof(VT) == 4 ? 4 : 3) * M.offset;
     k_restrict_fine<VT><<<grid_for(M.N, RESTRICT_THREADS), RESTRICT_THREADS, 0, st>>>(
-        M.N, M.p2r.data(), r, off, M.comp_mask[0].data(), M.new_local[0].data(), M.anc.data(),
-        M.L > 1 ? M.level_begin[1] : 0, M.L > 2 ? M.level_begin[2] : 0, M.L > 1 ? 1 : 0, M.R.data(), M.R64.data(),
-        converged);
+        M.N, M.p2r.data(), r, off, M.comp_mask[0].data(), M.new_local[0].data(), M.part_dst.data(),
+        M.L > 1 ? M.level_begin[1] : 0, M.L > 1 ? 1 : 0, M.R.data(), M.part.data(), converged);
     B2S_CHECK_LAUNCH();
     mas_apply_all(s, converged, bf16);
 }

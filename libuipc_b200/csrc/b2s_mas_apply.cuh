@@ -186,10 +186,13 @@ struct ApplyArgs
     const uint8_t*       stiff;  // [clusters], null in the FP32 path
     float*               R;
     float*               Z;
-    double*              R64;  // sums of the levels above 1 (from slot 16 g2 on)
+    const double*        part;        // partial sums of the levels above 1 (MasState::part)
+    const int32_t*       part_start;  // [node from slot 16 g2 on] its first entry
     int*                 err;
-    int                  n0, n1, n2;  // banks of level 0, of level 1, of the levels above
-    int                  g1, g2;      // first bank of level 1 and of level 2
+    int                  n0, n1, n2, n3, n4;  // banks of level 0, of level 1, of all levels from 2, 3, 4 up
+    int                  g1, g2, g3, g4;      // first bank of level 1, 2, 3 and 4
+    int                  heavy;  // n4 when the first n4 CTAs take those banks, else 0
+    int                  own;    // then the next banks that are their warp's only one
 };
 
 // the bank's inverse and, with `with_r`, its residual slice, on one barrier
@@ -227,40 +230,176 @@ __device__ __forceinline__ void bank_product(const ApplyArgs& A, unsigned char* 
     }
 }
 
-// The residual of a coarse bank (level 2 up) from its FP64 sums: to R and the
-// staged slice in FP32, the sums cleared for the next restriction.
-__device__ __forceinline__ void take_coarse(const ApplyArgs& A, int64_t gbank, float* s_r, int lane)
+// a[c] = the sum of the entries b, b + step, .. < e, in that order, AHEAD of
+// them fetched together
+template <int AHEAD>
+__device__ __forceinline__ void sum_entries(const double* part, int b, int e, int step, double a[3])
 {
-    double* q = A.R64 + (gbank - A.g2) * (BANK * 3);
-    for(int e = lane; e < BANK * 3; e += 32)
+    a[0] = a[1] = a[2] = 0.0;
+    for(int k = b; k < e; k += AHEAD * step)
     {
-        const float v = (float)__ldcg(q + e);
-        q[e]          = 0.0;
-        s_r[e]        = v;
-        A.R[gbank * (BANK * 3) + e] = v;
+        double v[AHEAD][3];
+#pragma unroll
+        for(int j = 0; j < AHEAD; ++j)
+#pragma unroll
+            for(int c = 0; c < 3; ++c)
+                v[j][c] = k + j * step < e ? __ldcg(part + 3 * (int64_t)(k + j * step) + c) : 0.0;
+#pragma unroll
+        for(int j = 0; j < AHEAD; ++j)
+#pragma unroll
+            for(int c = 0; c < 3; ++c)
+                a[c] += v[j][c];
+    }
+}
+
+__device__ __forceinline__ void warp_sum3(double a[3])
+{
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for(int c = 0; c < 3; ++c)
+            a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
+}
+
+// the entries of a coarse bank's nodes: lanes 2n and 2n + 1 get node n's
+__device__ __forceinline__ int2 bank_entries(const ApplyArgs& A, int64_t gbank, int lane)
+{
+    const int32_t* st = A.part_start + (gbank - A.g2) * BANK + (lane >> 1);
+    return make_int2(__ldg(st), __ldg(st + 1));
+}
+
+// The residual of a coarse bank (level 2 up) from the blocks' partial sums, in
+// a fixed order, to R and the staged slice in FP32. A node has one entry per
+// 256 slots under it: about 1 at level 2, 16 at level 3, 256 at level 4. Two
+// lanes per node while no node has more than 32, else the warp node by node.
+// be: bank_entries. AHEAD: 9 where the registers are there (half of a level-3
+// node's 16 or 17 entries in one go)
+template <int AHEAD>
+__device__ __forceinline__ void take_coarse(const ApplyArgs& A, int64_t gbank, int2 be, float* s_r, int lane)
+{
+    double a[3];
+    auto   put = [&](int node)
+    {
+#pragma unroll
+        for(int c = 0; c < 3; ++c)
+        {
+            const float v       = (float)a[c];
+            s_r[3 * node + c] = v;
+            A.R[gbank * (BANK * 3) + 3 * node + c] = v;
+        }
+    };
+    if(__reduce_max_sync(0xffffffffu, be.y - be.x) <= 32)
+    {
+        sum_entries<AHEAD>(A.part, be.x + (lane & 1), be.y, 2, a);
+#pragma unroll
+        for(int c = 0; c < 3; ++c)
+            a[c] += __shfl_xor_sync(0xffffffffu, a[c], 1);
+        if((lane & 1) == 0)
+            put(lane >> 1);
+    }
+    else
+    {
+        const int nodes = __popc(__ballot_sync(0xffffffffu, be.x < be.y)) / 2;  // the level's last bank may not be full
+        for(int i = 3 * nodes + lane; i < BANK * 3; i += 32)
+            s_r[i] = 0.0f;
+        for(int node = 0; node < nodes; ++node)
+        {
+            const int b = __shfl_sync(0xffffffffu, be.x, 2 * node), e = __shfl_sync(0xffffffffu, be.y, 2 * node);
+            sum_entries<AHEAD>(A.part, b + lane, e, 32, a);
+            warp_sum3(a);
+            if(lane == 0)
+                put(node);
+        }
     }
     __syncwarp();
 }
 
-// The banks handled by one warp (warp gw of W). The list: the coarse banks
-// from level 2 up (global banks g2 ..), then level 0, then level 1 (from g1).
-// A copy wait that runs out sets the error flag, drains the warp's copies in
+// A bank of level 4 up with its sums by a whole CTA: its few nodes have an entry
+// per 256 slots of tens of thousands each, and one warp's loads in flight take
+// longer than the rest of the apply does (a warp per such bank: 3.7 us more per
+// iteration on 88,641 vertices, 4.6 on 551,368). A warp per node, or the CTA node
+// by node when there are fewer than four; the product by warp 0, the others
+// return. s_sum: [16][WARPS][3] doubles.
+template <bool BF, int WARPS>
+__device__ __forceinline__ void heavy_bank(const ApplyArgs& A, int64_t gbank, const int* stop, unsigned char* stage,
+                                           uint64_t* bar, double* s_sum)
+{
+    constexpr uint32_t CB = BF ? INV16_BYTES : INV_BYTES;
+    const int          lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int2         be = bank_entries(A, gbank, lane);  // on its way with the flag
+    if(stop && *stop)
+        return;
+    if(threadIdx.x == 0)
+        issue_bank_copy<BF>(stage, bar, A, gbank, false);
+    const int  nodes   = __popc(__ballot_sync(0xffffffffu, be.x < be.y)) / 2;
+    const bool by_warp = nodes >= WARPS;
+    for(int node = by_warp ? w : 0; node < nodes; node += by_warp ? WARPS : 1)
+    {
+        const int b = __shfl_sync(0xffffffffu, be.x, 2 * node), e = __shfl_sync(0xffffffffu, be.y, 2 * node);
+        double    a[3];
+        sum_entries<4>(A.part, by_warp ? b + lane : b + (int)threadIdx.x, e, by_warp ? 32 : WARPS * 32, a);
+        warp_sum3(a);
+        if(lane < WARPS * 3)  // one warp's sum: the others' places hold zero
+        {
+            const int q = lane / 3, c = lane - 3 * q;
+            if(by_warp || q == w)
+                s_sum[(node * WARPS + q) * 3 + c] = q == w ? (c == 0 ? a[0] : (c == 1 ? a[1] : a[2])) : 0.0;
+        }
+    }
+    __syncthreads();
+    if(w != 0)
+        return;
+    float* s_r = reinterpret_cast<float*>(stage + CB);
+    for(int i = lane; i < BANK * 3; i += 32)
+    {
+        const int node = i / 3, c = i - 3 * node;
+        double    t    = 0.0;
+        if(node < nodes)
+#pragma unroll
+            for(int q = 0; q < WARPS; ++q)
+                t += s_sum[(node * WARPS + q) * 3 + c];
+        s_r[i]                            = (float)t;
+        A.R[gbank * (BANK * 3) + i] = (float)t;
+    }
+    const bool ok = mbar_wait(bar, 0, A.err, DERR_TMA_TIMEOUT);
+    if(!__all_sync(0xffffffffu, ok))
+    {
+        mbar_wait(bar, 0, nullptr, 0);
+        return;
+    }
+    __syncwarp();
+    bank_product<BF>(A, stage, gbank, BF && A.stiff != nullptr && A.stiff[gbank] != 0, lane);
+}
+
+// The banks handled by one warp (warp gw of W). The list: the banks from level
+// 4 up (global banks g4 ..; skipped when CTAs of their own have them), of level 3
+// (from g3), of level 2, of level 0, of level 1. The first `own` of the list, with
+// longer sums to take, are their warps' only ones. A copy wait that runs out sets the error flag, drains the warp's copies in
 // flight and ends the warp.
 template <bool BF, int NST>
-__device__ __forceinline__ void apply_banks(int gw, int W, int lane, const ApplyArgs& A, unsigned char* s_stage,
-                                            uint64_t* s_bar)
+__device__ __forceinline__ void apply_banks(int gw, int W, int lane, const ApplyArgs& A, const int* stop,
+                                            unsigned char* s_stage, uint64_t* s_bar)
 {
     constexpr uint32_t SB   = stage_bytes<BF>();
     constexpr uint32_t CB   = BF ? INV16_BYTES : INV_BYTES;
-    const int          n    = A.n2 + A.n0 + A.n1;
-    const int          mine = gw < n ? (n - 1 - gw) / W + 1 : 0;
+    const int          n    = A.n2 + A.n0 + A.n1 - A.heavy;
+    const int          V    = W - A.own;
+    const int          mine = gw >= n ? 0 : (gw < A.own ? 1 : (n - 1 - gw) / V + 1);
     auto               bank_of = [&](int j) -> int64_t
     {
-        const int i = gw + j * W - A.n2;
-        return i < 0 ? (int64_t)A.g2 + i + A.n2 : (i < A.n0 ? i : (int64_t)A.g1 + (i - A.n0));
+        const int i = A.heavy + gw + j * V;
+        if(i >= A.n2)
+            return i - A.n2 < A.n0 ? i - A.n2 : (int64_t)A.g1 + (i - A.n2 - A.n0);
+        return i < A.n4 ? (int64_t)A.g4 + i : (i < A.n3 ? (int64_t)A.g3 + i - A.n4 : (int64_t)A.g2 + i - A.n3);
     };
+    auto coarse = [&](int j) { return A.heavy + gw + j * V < A.n2; };
     auto issue = [&](int j, int slot)
-    { issue_bank_copy<BF>(s_stage + slot * SB, &s_bar[slot], A, bank_of(j), gw + j * W >= A.n2); };
+    { issue_bank_copy<BF>(s_stage + slot * SB, &s_bar[slot], A, bank_of(j), !coarse(j)); };
+    int2 be = make_int2(0, 0);  // of a coarse bank: the first one's on its way with the flag
+    if(mine > 0 && coarse(0))
+        be = bank_entries(A, bank_of(0), lane);
+    if(stop && *stop)
+        return;
     if(lane == 0)
         for(int j = 0; j < mine && j < NST; ++j)
             issue(j, j);
@@ -272,8 +411,12 @@ __device__ __forceinline__ void apply_banks(int gw, int W, int lane, const Apply
         const int      slot  = j % NST;
         const bool     use32 = BF && A.stiff != nullptr && A.stiff[gbank] != 0;
         unsigned char* stage = s_stage + slot * SB;
-        if(gw + j * W < A.n2)
-            take_coarse(A, gbank, reinterpret_cast<float*>(stage + CB), lane);
+        if(coarse(j))
+        {
+            if(j > 0)
+                be = bank_entries(A, gbank, lane);
+            take_coarse<BF ? 4 : 9>(A, gbank, be, reinterpret_cast<float*>(stage + CB), lane);
+        }
         const bool ok = mbar_wait(&s_bar[slot], (uint32_t)((j / NST) & 1), A.err, DERR_TMA_TIMEOUT);
         if(!__all_sync(0xffffffffu, ok))
             break;
@@ -294,20 +437,23 @@ __device__ __forceinline__ void apply_banks(int gw, int W, int lane, const Apply
 // The level-1 sums of a block of rows (in slot order; thread t's slot is its
 // row) and their part of the sums of the levels above. s_r: the residuals
 // [threads][3]; cm, nl: component mask and level-1 index of the thread's slot
-// (cm = 0: none); anc: its level-1 node's ancestors, needed by the components'
-// lowest lanes. R_1 in FP32, summed by the lowest lane in lane order. The
-// levels above, whose nodes collect from many blocks, are summed in FP64 by
-// reductions in L2 (their order moves the last bits of an FP64 sum that is then
-// rounded to FP32): every level is complete when the kernel is. A chain of
-// restrictions from level to level inside the apply took 25 us (88,641
-// vertices) to 43 us (551,368, behind the fine level's traffic) where the apply
-// now takes 8.8 and 26.8 us. Whole block;
-// s_lead: [threads][3] floats, s_anc: [threads] int4, s_n: [warps].
+// (cm = 0: none); dst: its level-1 node's entries (MasState::part_dst), needed by
+// the components' lowest lanes. R_1 in FP32, summed by the lowest lane in lane
+// order. The levels above, whose nodes collect from many blocks, get one FP64
+// partial sum per node and block, in a fixed order like the apply's sums of them
+// (take_coarse): every level is complete when the kernel is, the same in every
+// run. FP64 reductions in L2 (`red`) in their place left the last bits to the
+// order of the blocks. A chain of restrictions from level to level inside the
+// apply took 25 us (88,641 vertices) to 43 us (551,368, behind the fine level's
+// traffic). Whole block; s_lead: [threads][3] floats, s_dst: [threads] int4,
+// s_n: [warps].
+constexpr int RESTRICT_THREADS = 256;  // slots per block: the entries' unit
 template <int THREADS>
-__device__ __forceinline__ void restrict_coarse(const float (*s_r)[3], uint32_t cm, int nl, int4 anc, int begin1,
-                                                float* __restrict__ R, double* __restrict__ R64, int begin2,
-                                                float (*s_lead)[3], int4* s_anc, int* s_n)
+__device__ __forceinline__ void restrict_coarse(const float (*s_r)[3], uint32_t cm, int nl, int4 dst, int begin1,
+                                                float* __restrict__ R, double* __restrict__ part, float (*s_lead)[3],
+                                                int4* s_dst, int* s_n)
 {
+    static_assert(THREADS == RESTRICT_THREADS, "the entries are those of blocks of RESTRICT_THREADS slots");
     const int      t = threadIdx.x, lane = t & 31, w = t >> 5, sub = t & 15;
     const bool     lead = cm != 0 && (cm & ((1u << sub) - 1u)) == 0;
     const unsigned all  = __ballot_sync(0xffffffffu, lead);
@@ -342,18 +488,19 @@ __device__ __forceinline__ void restrict_coarse(const float (*s_r)[3], uint32_t 
         s_lead[at][0] = s0;
         s_lead[at][1] = s1;
         s_lead[at][2] = s2;
-        s_anc[at]     = anc;
+        s_dst[at]     = dst;
     }
     __syncthreads();
     // warp lv: level 2 + lv. The block's components have one or two ancestors
-    // there: one sum over the warp and one reduction per entry for each
+    // there: one sum over the warp for each. Beyond 32 components an entry may
+    // come up again; the same lanes then add to it.
     static_assert(THREADS >= 128, "a warp per level above 1");
     if(w >= 4)
         return;
     for(int base = 0; base < n; base += 32)
     {
-        const int k    = base + lane;
-        int       node = k < n ? reinterpret_cast<const int*>(s_anc + k)[w] : -1;
+        const int k = base + lane;
+        int       e = k < n ? reinterpret_cast<const int*>(s_dst + k)[w] : -1;
         float     v[3] = {0.f, 0.f, 0.f};
         if(k < n)
 #pragma unroll
@@ -361,10 +508,10 @@ __device__ __forceinline__ void restrict_coarse(const float (*s_r)[3], uint32_t 
                 v[c] = s_lead[k][c];
         while(true)
         {
-            const int best = (int)__reduce_min_sync(0xffffffffu, (unsigned)node);  // -1: the largest
+            const int best = (int)__reduce_min_sync(0xffffffffu, (unsigned)e);  // -1: the largest
             if(best < 0)
                 break;
-            const bool in = node == best;
+            const bool in = e >= 0 && (e >> 1) == (best >> 1);  // best: its first component of the block, if here
             double     a[3];
 #pragma unroll
             for(int c = 0; c < 3; ++c)
@@ -375,11 +522,15 @@ __device__ __forceinline__ void restrict_coarse(const float (*s_r)[3], uint32_t 
                 for(int c = 0; c < 3; ++c)
                     a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
             if(lane < 3)
-                asm volatile("red.global.add.f64 [%0], %1;" ::"l"(R64 + 3 * ((int64_t)best - begin2) + lane),
-                             "d"(lane == 0 ? a[0] : (lane == 1 ? a[1] : a[2]))
-                             : "memory");
+            {
+                double* q = part + 3 * (int64_t)(best >> 1) + lane;
+                double  d = lane == 0 ? a[0] : (lane == 1 ? a[1] : a[2]);
+                if(best & 1)
+                    d += *q;
+                *q = d;
+            }
             if(in)
-                node = -1;
+                e = -1;
         }
     }
 }

@@ -439,26 +439,26 @@ template <typename VT, int NS, bool UPDATE>
 __global__ void __launch_bounds__(VEC_BLOCK)
     k_update_restrict(int32_t n, int32_t slots, PcgScalars* sc, double* __restrict__ x, const VT* __restrict__ p,
                       VT* __restrict__ r, VT* __restrict__ Ap, const uint16_t* __restrict__ comp_mask,
-                      const int32_t* __restrict__ new_local, const int4* __restrict__ anc, int begin1, int begin2,
-                      int push, float* __restrict__ R, double* __restrict__ R64)
+                      const int32_t* __restrict__ new_local, const int4* __restrict__ dst, int begin1, int push,
+                      float* __restrict__ R, double* __restrict__ part)
 {
     if(UPDATE && frozen(sc))
         return;
     __shared__ float s_r[VEC_BLOCK][3];
     __shared__ float s_p[VEC_BLOCK][3];  // p (NS = 4), then the components' sums
-    __shared__ int4  s_anc[VEC_BLOCK];
+    __shared__ int4  s_dst[VEC_BLOCK];
     __shared__ int   s_n[VEC_BLOCK / 32];
     const int        t = threadIdx.x, i = blockIdx.x * VEC_BLOCK + t, sub = t & 15;
     const int64_t    e0 = 3 * (int64_t)blockIdx.x * VEC_BLOCK;  // the block's first entry of 3 per node
     uint32_t         cm = 0;
     int              nl = 0;
-    int4             an = make_int4(-1, -1, -1, -1);
+    int4             to = make_int4(-1, -1, -1, -1);
     if(i < slots && push)
     {
         cm = comp_mask[i];
         nl = new_local[i];
         if(cm != 0 && (cm & ((1u << sub) - 1u)) == 0)
-            an = anc[nl];
+            to = dst[nl];
     }
     double alpha = 0.0;
     if constexpr(UPDATE)
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(VEC_BLOCK)
     if(push)
     {
         __syncthreads();  // s_r is complete, s_p is free
-        restrict_coarse<VEC_BLOCK>(s_r, cm, nl, an, begin1, R, R64, begin2, s_p, s_anc, s_n);
+        restrict_coarse<VEC_BLOCK>(s_r, cm, nl, to, begin1, R, part, s_p, s_dst, s_n);
     }
 }
 
@@ -950,16 +950,15 @@ static bool try_order(b2s_solver* s, bool f32)
 
 // the restriction in PCG order, with the x, r update of the iteration
 // (UPDATE). Without an apply to follow (kind other than MAS) nothing is
-// restricted: the apply clears the coarse sums.
+// restricted.
 template <typename VT, int NS, bool UPDATE>
 static void update_restrict_launch(b2s_solver* s, int kind, PcgScalars* sc, double* xs, const VT* p, VT* r, VT* Ap)
 {
     const PcgOrder& O = s->pcg.ord;
     MasState&       M = s->mas;
     k_update_restrict<VT, NS, UPDATE><<<grid_for(O.n, VEC_BLOCK), VEC_BLOCK, 0, s->stream>>>(
-        O.n, O.slots, sc, xs, p, r, Ap, M.comp_mask[0].data(), M.new_local[0].data(), M.anc.data(),
-        M.L > 1 ? M.level_begin[1] : 0, M.L > 2 ? M.level_begin[2] : 0,
-        kind == B2S_PRECOND_MAS && M.L > 1 ? 1 : 0, M.R.data(), M.R64.data());
+        O.n, O.slots, sc, xs, p, r, Ap, M.comp_mask[0].data(), M.new_local[0].data(), M.part_dst.data(),
+        M.L > 1 ? M.level_begin[1] : 0, kind == B2S_PRECOND_MAS && M.L > 1 ? 1 : 0, M.R.data(), M.part.data());
     B2S_CHECK_LAUNCH();
 }
 
@@ -1079,7 +1078,7 @@ static void read_scalars(b2s_solver* s, long long iter_before)
     k_scalars_out<<<1, 1, 0, s->stream>>>(P.sc.data(), s->dev_err.data(), P.h_sc, s->h_back);
     B2S_CHECK_LAUNCH();
     B2S_CUDA(cudaStreamSynchronize(s->stream));
-    raise_device_errors(s, s->h_back->err);
+    raise_device_errors(s->h_back->err);
     B2S_REQUIRE(P.h_sc->converged != 0 || P.h_sc->iter > iter_before, B2S_ERR_CUDA, "the PCG made no progress");
 }
 

@@ -59,6 +59,8 @@ struct SmallArgs
     ApplyArgs      A;
     const uint16_t* comp_mask;  // of the slots
     const int32_t*  new_local;
+    const int4*     part_dst;
+    double*         part;
     long long      iterations;
     unsigned       polls;  // of a barrier, before it gives up
 };
@@ -265,7 +267,7 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
     __shared__ int      s_dead;  // a warp of this block gave up waiting
     __shared__ float    s_z[MAS ? SM_WARPS : 1][2 * BANK * 3];
     __shared__ float    s_rr[MAS ? SM_THREADS : 1][3], s_lead[MAS ? SM_THREADS : 1][3];
-    __shared__ int4     s_anc[MAS ? SM_THREADS : 1];
+    __shared__ int4     s_dst[MAS ? SM_THREADS : 1];
     __shared__ int      s_n[SM_WARPS];
     const int  lane = threadIdx.x & 31, w = threadIdx.x >> 5, sub = lane & 15;
     const int  i = blockIdx.x * SM_THREADS + threadIdx.x;  // this thread's row
@@ -276,7 +278,7 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
     int        u1 = 0, u2 = 0;  // copies run through the level-1 / level-2 stages
     uint32_t   cm = 0;
     int        nl = 0, n1 = -1;
-    int4       an = make_int4(-1, -1, -1, -1);
+    int4       an = make_int4(-1, -1, -1, -1), to = an;
     bool       stiff[2] = {false, false};
     unsigned char* own = s_dyn + (size_t)2 * w * SB;
     bool           underway = false;  // level-1 warp: its first copy of the iteration is not waited for yet
@@ -326,10 +328,17 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
                 nl = a.new_local[i];
                 n1 = a.mv.slot_node1[i];
                 if(n1 >= 0)
+                {
                     an = a.mv.anc[n1 - a.mv.begin1];
+                    to = a.part_dst[n1 - a.mv.begin1];
+                }
             }
         }
     }
+    int2 be2 = make_int2(0, 0);  // level-2 warp: the entries of its first bank
+    if constexpr(MAS)
+        if(w == SM_L2_WARP && (int)(gridDim.x - 1 - blockIdx.x) < a.A.n2)
+            be2 = bank_entries(a.A, (int64_t)a.A.g2 + (gridDim.x - 1 - blockIdx.x), lane);
     VT     r[3] = {0, 0, 0}, p[3] = {0, 0, 0}, z[3];
     double x[3] = {0, 0, 0};
     if(live)
@@ -402,8 +411,7 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
                 s_rr[threadIdx.x][c] = (float)r[c];
             __syncthreads();
             if(a.mv.T > 0)
-                restrict_coarse<SM_THREADS>(s_rr, cm, nl, an, a.mv.begin1, a.A.R, a.A.R64, a.A.g2 * BANK, s_lead,
-                                            s_anc, s_n);
+                restrict_coarse<SM_THREADS>(s_rr, cm, nl, to, a.mv.begin1, a.A.R, a.part, s_lead, s_dst, s_n);
             // their products, before the barrier that publishes R_1
 #pragma unroll
             for(int k = 0; k < 2; ++k)
@@ -482,7 +490,8 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
                         fence_proxy_async_smem();
                         issue_bank_copy<BF>(st, bar, a.A, g, false);
                     }
-                    take_coarse(a.A, g, reinterpret_cast<float*>(st + CB), lane);
+                    take_coarse<4>(a.A, g, b < (int)gridDim.x ? be2 : bank_entries(a.A, g, lane),
+                                reinterpret_cast<float*>(st + CB), lane);
                     const bool ok = mbar_wait(bar, (uint32_t)((u2 / SM_COARSE) & 1), a.A.err, DERR_TMA_TIMEOUT);
                     if(!__all_sync(0xffffffffu, ok))
                     {
@@ -649,6 +658,8 @@ bool launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterat
         a.A         = mas_apply_args(s, sizeof(VT) == 4);
         a.comp_mask = s->mas.comp_mask[0].data();
         a.new_local = s->mas.new_local[0].data();
+        a.part_dst  = s->mas.part_dst.data();
+        a.part      = s->mas.part.data();
     }
     a.A.err      = device_error_flag(s);
     a.iterations = iterations;

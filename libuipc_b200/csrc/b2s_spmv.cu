@@ -528,13 +528,10 @@ void ensure_read_back(b2s_solver* s)
         B2S_CUDA(cudaMallocHost(&s->h_back, sizeof(ReadBack)));
 }
 
-void raise_device_errors(b2s_solver* s, int e)
+void raise_device_errors(int e)
 {
     if(e == 0)
         return;
-    // an apply that stopped halfway has left sums for the next one
-    if(s->mas.R64.size() > 0)
-        B2S_CUDA(cudaMemsetAsync(s->mas.R64.data(), 0, s->mas.R64.bytes(), s->stream));
     throw Error(B2S_ERR_CUDA, std::string("device error flag ") + std::to_string(e)
                                   + ((e & DERR_TMA_TIMEOUT) ? ": a bulk-copy or barrier wait timed out" : ""));
 }
@@ -547,7 +544,7 @@ void read_back(b2s_solver* s, const double* d, int n, double* h)
     B2S_CUDA(cudaStreamSynchronize(s->stream));
     for(int i = 0; i < n; ++i)
         h[i] = s->h_back->v[i];
-    raise_device_errors(s, s->h_back->err);
+    raise_device_errors(s->h_back->err);
 }
 
 // raise (and clear) the error bits kernels left in the device flag
