@@ -559,16 +559,20 @@ __global__ void __launch_bounds__(APPLY_WARPS * 32, BF ? 7 : 5) k_apply_all(Appl
     }
     __syncwarp();
     __shared__ double s_sum[BANK * APPLY_WARPS * 3];
-    int gw = ((int)blockIdx.x - A.heavy) * APPLY_WARPS + w;
+    const int         rest = (int)gridDim.x - A.heavy;
+    int               gw = ((int)blockIdx.x - A.heavy) * APPLY_WARPS + w, W = rest * APPLY_WARPS;
+    if(A.join)
+        W += A.heavy * (APPLY_WARPS - 1);
     if((int)blockIdx.x < A.heavy)
     {
-        heavy_bank<BF, APPLY_WARPS>(A, (int64_t)A.g4 + blockIdx.x, converged, &s_stage[0][0][0], s_bar[0], s_sum);
-        if(w == 0)
+        static_assert(NST >= 2 && SB % 16 == 0, "a barrier and room for the entries");
+        heavy_bank<BF, APPLY_WARPS>(A, (int64_t)A.g3 + blockIdx.x, converged, &s_stage[0][0][0], &s_stage[0][1][0],
+                                    (APPLY_WARPS * NST - 1) * SB, s_bar[0], s_sum);
+        if(w == 0 || !A.join)
             return;
-        // its other warps join the rest, last in the order
-        gw = ((int)gridDim.x - A.heavy) * APPLY_WARPS + (int)blockIdx.x * (APPLY_WARPS - 1) + w - 1;
+        gw = rest * APPLY_WARPS + (int)blockIdx.x * (APPLY_WARPS - 1) + w - 1;  // last in the order
     }
-    apply_banks<BF, NST>(gw, (int)gridDim.x * APPLY_WARPS - A.heavy, lane, A, converged, &s_stage[w][0][0], s_bar[w]);
+    apply_banks<BF, NST>(gw, W, lane, A, converged, &s_stage[w][0][0], s_bar[w]);
 }
 
 // The fine residual in partition order and the sums of every coarse level, a
@@ -717,7 +721,7 @@ static void place_partials(b2s_solver* s)
                 next[m] += first ? 1 : 0;
                 *a = 2 * (next[m] - 1) + (first ? 0 : 1);
             }
-    M.part.resize(std::max<size_t>(3 * (size_t)entries, 1));
+    M.part.resize(3 * (size_t)entries + 3);  // one more: copies end at even entries
     M.part_start.resize(nodes + 1);
     M.part_dst.resize(std::max(cnt1, 1));
     B2S_CUDA(cudaMemcpyAsync(M.part_start.data(), start.data(), sizeof(int32_t) * (nodes + 1), cudaMemcpyHostToDevice,
@@ -1002,9 +1006,7 @@ ApplyArgs mas_apply_args(b2s_solver* s, bool bf16)
     A.g3    = M.L > 3 ? M.level_begin[3] / BANK : M.clusters;
     A.n2    = M.clusters - A.g2;
     A.n3    = M.clusters - A.g3;
-    A.g4    = M.L > 4 ? M.level_begin[4] / BANK : M.clusters;
-    A.n4    = M.clusters - A.g4;
-    A.heavy = A.own = 0;
+    A.heavy = A.join = 0;
     return A;
 }
 
@@ -1020,14 +1022,13 @@ void mas_apply_all(b2s_solver* s, const int* converged, bool bf16)
     if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, APPLY_WARPS * 32, 0) != cudaSuccess || occ < 1)
         occ = 1;
     // persistent: the CTAs that fit at once, at most one warp per bank; the banks
-    // of level 4 up each get a CTA to begin with, while those are an eighth at most
-    const int grid = std::min((n + APPLY_WARPS - 1) / APPLY_WARPS, NUM_SMS_HINT * occ);
-    if(8 * A.n4 <= grid)
-        A.heavy = A.n4;
-    // the level-3 banks get warps of their own unless that costs the others another round
-    const int left = n - A.heavy, warps = grid * APPLY_WARPS - A.heavy, own = A.n3 - A.heavy;
-    if(4 * own <= warps && (left - own + warps - own - 1) / (warps - own) <= (left + warps - 1) / warps)
-        A.own = own;
+    // of level 3 up have a CTA each, while those are an eighth at most. Its other
+    // warps are late for the rest: they join it when it takes four banks a warp
+    const int most = NUM_SMS_HINT * occ;
+    if(8 * A.n3 <= std::min((n + APPLY_WARPS - 1) / APPLY_WARPS, most))
+        A.heavy = A.n3;
+    const int grid = std::min(A.heavy + (n - A.heavy + APPLY_WARPS - 1) / APPLY_WARPS, most);
+    A.join         = n >= 4 * APPLY_WARPS * grid;
     k<<<grid, APPLY_WARPS * 32, 0, s->stream>>>(A, converged);
     B2S_CHECK_LAUNCH();
 }

@@ -189,10 +189,10 @@ struct ApplyArgs
     const double*        part;        // partial sums of the levels above 1 (MasState::part)
     const int32_t*       part_start;  // [node from slot 16 g2 on] its first entry
     int*                 err;
-    int                  n0, n1, n2, n3, n4;  // banks of level 0, of level 1, of all levels from 2, 3, 4 up
-    int                  g1, g2, g3, g4;      // first bank of level 1, 2, 3 and 4
-    int                  heavy;  // n4 when the first n4 CTAs take those banks, else 0
-    int                  own;    // then the next banks that are their warp's only one
+    int                  n0, n1, n2, n3;  // banks of level 0, of level 1, of all levels from 2, 3 up
+    int                  g1, g2, g3;      // first bank of level 1, 2 and 3
+    int                  heavy;  // n3 when the first n3 CTAs take those banks, else 0
+    int                  join;   // 1: their other warps then join the rest
 };
 
 // the bank's inverse and, with `with_r`, its residual slice, on one barrier
@@ -232,9 +232,9 @@ __device__ __forceinline__ void bank_product(const ApplyArgs& A, unsigned char* 
 
 // a[c] = the sum of the entries b, b + step, .. < e, in that order, AHEAD of
 // them fetched together
-template <int AHEAD>
 __device__ __forceinline__ void sum_entries(const double* part, int b, int e, int step, double a[3])
 {
+    constexpr int AHEAD = 4;
     a[0] = a[1] = a[2] = 0.0;
     for(int k = b; k < e; k += AHEAD * step)
     {
@@ -252,15 +252,6 @@ __device__ __forceinline__ void sum_entries(const double* part, int b, int e, in
     }
 }
 
-__device__ __forceinline__ void warp_sum3(double a[3])
-{
-#pragma unroll
-    for(int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for(int c = 0; c < 3; ++c)
-            a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
-}
-
 // the entries of a coarse bank's nodes: lanes 2n and 2n + 1 get node n's
 __device__ __forceinline__ int2 bank_entries(const ApplyArgs& A, int64_t gbank, int lane)
 {
@@ -270,16 +261,24 @@ __device__ __forceinline__ int2 bank_entries(const ApplyArgs& A, int64_t gbank, 
 
 // The residual of a coarse bank (level 2 up) from the blocks' partial sums, in
 // a fixed order, to R and the staged slice in FP32. A node has one entry per
-// 256 slots under it: about 1 at level 2, 16 at level 3, 256 at level 4. Two
-// lanes per node while no node has more than 32, else the warp node by node.
-// be: bank_entries. AHEAD: 9 where the registers are there (half of a level-3
-// node's 16 or 17 entries in one go)
-template <int AHEAD>
+// 256 slots under it: about 1 at level 2, 16 at level 3, 256 at level 4. All
+// nodes at once, two lanes each in a full bank, up to the whole warp for a single
+// node (upper levels have few, with many entries). be: bank_entries
 __device__ __forceinline__ void take_coarse(const ApplyArgs& A, int64_t gbank, int2 be, float* s_r, int lane)
 {
-    double a[3];
-    auto   put = [&](int node)
-    {
+    const int nodes = __popc(__ballot_sync(0xffffffffu, be.x < be.y)) / 2;  // the level's last bank may not be full
+    const int lanes = nodes > 8 ? 2 : (nodes > 4 ? 4 : (nodes > 2 ? 8 : (nodes > 1 ? 16 : 32)));
+    const int node  = lane / lanes;
+    const int b = __shfl_sync(0xffffffffu, be.x, 2 * node), e = __shfl_sync(0xffffffffu, be.y, 2 * node);
+    double    a[3];
+    sum_entries(A.part, b + lane % lanes, e, lanes, a);
+    for(int o = lanes / 2; o > 0; o >>= 1)
+#pragma unroll
+        for(int c = 0; c < 3; ++c)
+            a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
+    for(int i = 3 * nodes + lane; i < BANK * 3; i += 32)
+        s_r[i] = 0.0f;
+    if(node < nodes && lane % lanes == 0)
 #pragma unroll
         for(int c = 0; c < 3; ++c)
         {
@@ -287,94 +286,111 @@ __device__ __forceinline__ void take_coarse(const ApplyArgs& A, int64_t gbank, i
             s_r[3 * node + c] = v;
             A.R[gbank * (BANK * 3) + 3 * node + c] = v;
         }
-    };
-    if(__reduce_max_sync(0xffffffffu, be.y - be.x) <= 32)
-    {
-        sum_entries<AHEAD>(A.part, be.x + (lane & 1), be.y, 2, a);
-#pragma unroll
-        for(int c = 0; c < 3; ++c)
-            a[c] += __shfl_xor_sync(0xffffffffu, a[c], 1);
-        if((lane & 1) == 0)
-            put(lane >> 1);
-    }
-    else
-    {
-        const int nodes = __popc(__ballot_sync(0xffffffffu, be.x < be.y)) / 2;  // the level's last bank may not be full
-        for(int i = 3 * nodes + lane; i < BANK * 3; i += 32)
-            s_r[i] = 0.0f;
-        for(int node = 0; node < nodes; ++node)
-        {
-            const int b = __shfl_sync(0xffffffffu, be.x, 2 * node), e = __shfl_sync(0xffffffffu, be.y, 2 * node);
-            sum_entries<AHEAD>(A.part, b + lane, e, 32, a);
-            warp_sum3(a);
-            if(lane == 0)
-                put(node);
-        }
-    }
     __syncwarp();
 }
 
-// A bank of level 4 up with its sums by a whole CTA: its few nodes have an entry
-// per 256 slots of tens of thousands each, and one warp's loads in flight take
-// longer than the rest of the apply does (a warp per such bank: 3.7 us more per
-// iteration on 88,641 vertices, 4.6 on 551,368). A warp per node, or the CTA node
-// by node when there are fewer than four; the product by warp 0, the others
-// return. s_sum: [16][WARPS][3] doubles.
+// A bank of level 3 up with its sums by a whole CTA: its entries, one per 256
+// slots under each node, come into shared memory by bulk copies of `room` bytes
+// at most and are added by 8 (16 nodes) to 128 threads (one node) per node. Beside
+// the fine level's copies, which fill the memory system from the first
+// microsecond, every dependent round of loads takes 2-4 us: with plain loads, 4 or
+// 9 ahead per lane of one warp, an iteration took 1.4 us (88,641 vertices) to 2.8
+// us (551,368) longer; with these the apply takes what it took with reductions
+// (10.6 us against 10.5, 88,641 vertices, caches flushed). The product is warp 0's; the others return at the end.
+// copies: two free barriers (the bank's inverse, the entries); stage: the bank's;
+// s_sum: [16][WARPS][3] doubles.
 template <bool BF, int WARPS>
 __device__ __forceinline__ void heavy_bank(const ApplyArgs& A, int64_t gbank, const int* stop, unsigned char* stage,
-                                           uint64_t* bar, double* s_sum)
+                                           unsigned char* entries, uint32_t room, uint64_t* copies, double* s_sum)
 {
     constexpr uint32_t CB = BF ? INV16_BYTES : INV_BYTES;
-    const int          lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr uint32_t ENTRY = 3 * sizeof(double);
+    const int          t = threadIdx.x, lane = t & 31, w = t >> 5;
     const int2         be = bank_entries(A, gbank, lane);  // on its way with the flag
     if(stop && *stop)
         return;
-    if(threadIdx.x == 0)
-        issue_bank_copy<BF>(stage, bar, A, gbank, false);
-    const int  nodes   = __popc(__ballot_sync(0xffffffffu, be.x < be.y)) / 2;
-    const bool by_warp = nodes >= WARPS;
-    for(int node = by_warp ? w : 0; node < nodes; node += by_warp ? WARPS : 1)
+    const int nodes = __popc(__ballot_sync(0xffffffffu, be.x < be.y)) / 2;
+    int       pow2 = 1;
+    while(pow2 < nodes)
+        pow2 <<= 1;
+    const int G = WARPS * 32 / pow2, node = t / G, sub = t % G;  // threads of a node
+    const int b = __shfl_sync(0xffffffffu, be.x, 2 * node), e = __shfl_sync(0xffffffffu, be.y, 2 * node);
+    const int first = __shfl_sync(0xffffffffu, be.x, 0) & ~1;  // (copies start and end at even entries: 16 bytes)
+    const int last  = __shfl_sync(0xffffffffu, be.y, 2 * max(nodes - 1, 0));
+    const int step  = (int)(room / ENTRY) & ~1;
+    auto      issue = [&](int c)
     {
-        const int b = __shfl_sync(0xffffffffu, be.x, 2 * node), e = __shfl_sync(0xffffffffu, be.y, 2 * node);
-        double    a[3];
-        sum_entries<4>(A.part, by_warp ? b + lane : b + (int)threadIdx.x, e, by_warp ? 32 : WARPS * 32, a);
-        warp_sum3(a);
-        if(lane < WARPS * 3)  // one warp's sum: the others' places hold zero
+        const uint32_t bytes = ENTRY * (uint32_t)min(step, (last - c + 1) & ~1);
+        mbar_arrive_expect_tx(&copies[1], bytes);
+        bulk_copy_g2s(entries, A.part + 3 * (int64_t)c, bytes, &copies[1]);
+    };
+    if(t == 0)
+    {
+        if(first < last)
+            issue(first);
+        issue_bank_copy<BF>(stage, &copies[0], A, gbank, false);
+    }
+    double a[3] = {0.0, 0.0, 0.0};
+    bool     ok   = true;
+    uint32_t phase = 0;
+    __syncthreads();  // the barriers of warp 0, initialised by its lane 0
+    for(int c = first; c < last; c += step, phase ^= 1u)
+    {
+        ok = __syncthreads_and(mbar_wait(&copies[1], phase, A.err, DERR_TMA_TIMEOUT));
+        if(!ok)  // once more, for the copy to end before the block goes on
         {
-            const int q = lane / 3, c = lane - 3 * q;
-            if(by_warp || q == w)
-                s_sum[(node * WARPS + q) * 3 + c] = q == w ? (c == 0 ? a[0] : (c == 1 ? a[1] : a[2])) : 0.0;
+            mbar_wait(&copies[1], phase, nullptr, 0);
+            break;
+        }
+        const double* p  = reinterpret_cast<const double*>(entries);
+        const int     to = min(e, c + step);
+        for(int k = b + sub + (c > b + sub ? (c - b - sub + G - 1) / G * G : 0); k < to; k += G)
+#pragma unroll
+            for(int q = 0; q < 3; ++q)
+                a[q] += p[3 * (k - c) + q];
+        __syncthreads();  // the entries are read
+        if(t == 0 && c + step < last)
+        {
+            fence_proxy_async_smem();
+            issue(c + step);
         }
     }
+    const int part = min(G, 32);
+    for(int o = part / 2; o > 0; o >>= 1)
+#pragma unroll
+        for(int q = 0; q < 3; ++q)
+            a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
+    if(node < nodes && lane % part == 0)
+#pragma unroll
+        for(int q = 0; q < 3; ++q)
+            s_sum[(node * WARPS + sub / 32) * 3 + q] = a[q];
+    fence_proxy_async_smem();  // the entries are read: the warps' own copies may follow
     __syncthreads();
     if(w != 0)
         return;
     float* s_r = reinterpret_cast<float*>(stage + CB);
     for(int i = lane; i < BANK * 3; i += 32)
     {
-        const int node = i / 3, c = i - 3 * node;
-        double    t    = 0.0;
-        if(node < nodes)
-#pragma unroll
-            for(int q = 0; q < WARPS; ++q)
-                t += s_sum[(node * WARPS + q) * 3 + c];
-        s_r[i]                            = (float)t;
-        A.R[gbank * (BANK * 3) + i] = (float)t;
+        const int m = i / 3, c = i - 3 * m;
+        double    v = 0.0;
+        if(m < nodes)
+            for(int q = 0; q < (G + 31) / 32; ++q)
+                v += s_sum[(m * WARPS + q) * 3 + c];
+        s_r[i]                      = (float)v;
+        A.R[gbank * (BANK * 3) + i] = (float)v;
     }
-    const bool ok = mbar_wait(bar, 0, A.err, DERR_TMA_TIMEOUT);
-    if(!__all_sync(0xffffffffu, ok))
-    {
-        mbar_wait(bar, 0, nullptr, 0);
+    const bool here = mbar_wait(&copies[0], 0, A.err, DERR_TMA_TIMEOUT);
+    if(!here)
+        mbar_wait(&copies[0], 0, nullptr, 0);
+    if(!__all_sync(0xffffffffu, here && ok))
         return;
-    }
-    __syncwarp();
+    __syncwarp();  // every lane's residuals, for the others in the product
     bank_product<BF>(A, stage, gbank, BF && A.stiff != nullptr && A.stiff[gbank] != 0, lane);
 }
 
 // The banks handled by one warp (warp gw of W). The list: the banks from level
-// 4 up (global banks g4 ..; skipped when CTAs of their own have them), of level 3
-// (from g3), of level 2, of level 0, of level 1. The first `own` of the list, with
-// longer sums to take, are their warps' only ones. A copy wait that runs out sets the error flag, drains the warp's copies in
+// 3 up (global banks g3 ..; skipped when CTAs of their own have them), of level 2,
+// of level 0, of level 1. A copy wait that runs out sets the error flag, drains the warp's copies in
 // flight and ends the warp.
 template <bool BF, int NST>
 __device__ __forceinline__ void apply_banks(int gw, int W, int lane, const ApplyArgs& A, const int* stop,
@@ -383,16 +399,15 @@ __device__ __forceinline__ void apply_banks(int gw, int W, int lane, const Apply
     constexpr uint32_t SB   = stage_bytes<BF>();
     constexpr uint32_t CB   = BF ? INV16_BYTES : INV_BYTES;
     const int          n    = A.n2 + A.n0 + A.n1 - A.heavy;
-    const int          V    = W - A.own;
-    const int          mine = gw >= n ? 0 : (gw < A.own ? 1 : (n - 1 - gw) / V + 1);
+    const int          mine = gw < n ? (n - 1 - gw) / W + 1 : 0;
     auto               bank_of = [&](int j) -> int64_t
     {
-        const int i = A.heavy + gw + j * V;
+        const int i = A.heavy + gw + j * W;
         if(i >= A.n2)
             return i - A.n2 < A.n0 ? i - A.n2 : (int64_t)A.g1 + (i - A.n2 - A.n0);
-        return i < A.n4 ? (int64_t)A.g4 + i : (i < A.n3 ? (int64_t)A.g3 + i - A.n4 : (int64_t)A.g2 + i - A.n3);
+        return i < A.n3 ? (int64_t)A.g3 + i : (int64_t)A.g2 + i - A.n3;
     };
-    auto coarse = [&](int j) { return A.heavy + gw + j * V < A.n2; };
+    auto coarse = [&](int j) { return A.heavy + gw + j * W < A.n2; };
     auto issue = [&](int j, int slot)
     { issue_bank_copy<BF>(s_stage + slot * SB, &s_bar[slot], A, bank_of(j), !coarse(j)); };
     int2 be = make_int2(0, 0);  // of a coarse bank: the first one's on its way with the flag
@@ -415,7 +430,7 @@ __device__ __forceinline__ void apply_banks(int gw, int W, int lane, const Apply
         {
             if(j > 0)
                 be = bank_entries(A, gbank, lane);
-            take_coarse<BF ? 4 : 9>(A, gbank, be, reinterpret_cast<float*>(stage + CB), lane);
+            take_coarse(A, gbank, be, reinterpret_cast<float*>(stage + CB), lane);
         }
         const bool ok = mbar_wait(&s_bar[slot], (uint32_t)((j / NST) & 1), A.err, DERR_TMA_TIMEOUT);
         if(!__all_sync(0xffffffffu, ok))

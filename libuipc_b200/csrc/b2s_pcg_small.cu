@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
                         fence_proxy_async_smem();
                         issue_bank_copy<BF>(st, bar, a.A, g, false);
                     }
-                    take_coarse<4>(a.A, g, b < (int)gridDim.x ? be2 : bank_entries(a.A, g, lane),
+                    take_coarse(a.A, g, b < (int)gridDim.x ? be2 : bank_entries(a.A, g, lane),
                                 reinterpret_cast<float*>(st + CB), lane);
                     const bool ok = mbar_wait(bar, (uint32_t)((u2 / SM_COARSE) & 1), a.A.err, DERR_TMA_TIMEOUT);
                     if(!__all_sync(0xffffffffu, ok))
