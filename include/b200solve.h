@@ -245,10 +245,11 @@ int b2s_reset_timers(b2s_solver* s);
 
 /* ---- failure injection ----------------------------------------------------------------
  * For tests of the error paths: a wait of this handle's kernels gives up early,
- * or the host sees a launch refused. Nothing faults or hangs; the affected call
+ * or the host sees a launch refused or an allocation fail. Nothing faults or hangs; the affected call
  * does what it does when the same happens by itself. */
 #define B2S_INJECT_WAIT_POLLS 0 /* a grid barrier of the one-launch PCG gives up after `value` polls (-1: the default, seconds) */
 #define B2S_INJECT_LAUNCH 1     /* the next `value` cooperative launches are refused, as for a stream with too few SMs */
+#define B2S_INJECT_ALLOC 2      /* the value-th device allocation of this thread from now on fails (0: none does) */
 int b2s_inject_failure(b2s_solver* s, int what, int64_t value);
 
 /* ---- learned PCG warm start ------------------------------------------------------------

@@ -22,6 +22,7 @@ B2S_STOP_RZ = 0
 B2S_STOP_RELRES = 1
 B2S_INJECT_WAIT_POLLS = 0
 B2S_INJECT_LAUNCH = 1
+B2S_INJECT_ALLOC = 2
 
 B2S_PRECISION_FP64 = 0
 B2S_PRECISION_MIXED = 1

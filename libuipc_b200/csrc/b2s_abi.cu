@@ -15,6 +15,7 @@ thread_local std::string g_create_error;
 namespace b2s
 {
 thread_local long long g_kernel_launches = 0;
+thread_local int64_t   g_inject_alloc    = 0;
 
 void set_handle_free_error(const std::string& msg) { g_create_error = msg; }
 }  // namespace b2s
@@ -479,11 +480,13 @@ int b2s_inject_failure(b2s_solver* s, int what, int64_t value)
     return guarded(s,
                    [&]
                    {
-                       B2S_REQUIRE(what == B2S_INJECT_WAIT_POLLS || what == B2S_INJECT_LAUNCH, B2S_ERR_ARGUMENT,
+                       B2S_REQUIRE(what >= B2S_INJECT_WAIT_POLLS && what <= B2S_INJECT_ALLOC, B2S_ERR_ARGUMENT,
                                    "unknown failure");
                        B2S_REQUIRE(value >= (what == B2S_INJECT_WAIT_POLLS ? -1 : 0) && value <= INT32_MAX,
                                    B2S_ERR_ARGUMENT, "value out of range");
-                       (what == B2S_INJECT_WAIT_POLLS ? s->inject_polls : s->inject_launch) = value;
+                       (what == B2S_INJECT_WAIT_POLLS ? s->inject_polls :
+                        what == B2S_INJECT_LAUNCH     ? s->inject_launch :
+                                                        b2s::g_inject_alloc) = value;
                    });
 }
 

@@ -806,10 +806,9 @@ void copy_blocks_out(b2s_solver* s, const Matrix& A, double* out)
     {
         tmp.resize((size_t)piece * 9);
     }
-    catch(const Error&)
+    catch(const OutOfMemory&)
     {
         // no room for the buffer: one strided copy per component
-        cudaGetLastError();
         for(int q = 0; q < 9; ++q)
             B2S_CUDA(cudaMemcpy2DAsync(out + q, 9 * sizeof(double), A.vals.data() + (size_t)q * A.stride,
                                        sizeof(double), sizeof(double), A.nnz, cudaMemcpyDefault, st));

@@ -30,6 +30,12 @@ struct Error : std::runtime_error
     }
 };
 
+// the device has no room (B2S_ERR_CUDA at the ABI)
+struct OutOfMemory : Error
+{
+    using Error::Error;
+};
+
 #define B2S_CUDA(call)                                                                       \
     do                                                                                       \
     {                                                                                        \
@@ -38,6 +44,9 @@ struct Error : std::runtime_error
             throw ::b2s::Error(B2S_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e__) \
                                                  + " (" + __FILE__ + ":" + std::to_string(__LINE__) + ")"); \
     } while(0)
+
+// B2S_INJECT_ALLOC: counts down to the failing allocation (0: off)
+extern thread_local int64_t g_inject_alloc;
 
 // kernels launched by this thread through the library (every launch site
 // goes through B2S_CHECK_LAUNCH; graph replays add their node count)
@@ -97,7 +106,17 @@ struct DBuf
                 want = count;
             if(want == 0)
                 want = 1;
-            B2S_CUDA(cudaMalloc(&ptr, want * sizeof(T)));
+            cudaError_t e = cudaErrorMemoryAllocation;
+            if(g_inject_alloc == 0 || --g_inject_alloc > 0)
+                e = cudaMalloc(&ptr, want * sizeof(T));
+            if(e == cudaErrorMemoryAllocation)
+            {
+                ptr = nullptr;
+                cudaGetLastError();
+                throw OutOfMemory(B2S_ERR_CUDA, "cudaMalloc of " + std::to_string(want * sizeof(T)) + " bytes: "
+                                                    + cudaGetErrorString(e));
+            }
+            B2S_CUDA(e);
             cap = want;
         }
         n = count;

@@ -924,25 +924,31 @@ static void ensure_order(b2s_solver* s, bool f32)
     }
 }
 
-// ensure_order, or false (the recursion then runs in the matrix's own order)
-// when the device has no room for the second copy of the matrix
-static bool try_order(b2s_solver* s, bool f32)
+// ensure_order and room(true), which allocates what the solve needs in that
+// order; false when the device has no room for the second copy of the matrix and
+// the longer vectors. They are given back then, and the recursion runs in the
+// matrix's own order.
+template <typename Room>
+static bool try_order(b2s_solver* s, bool f32, const Room& room)
 {
     try
     {
         ensure_order(s, f32);
+        room(true);
         return true;
     }
-    catch(const Error&)
+    catch(const OutOfMemory&)
     {
-        if(cudaGetLastError() != cudaErrorMemoryAllocation)
-            throw;
-        PcgOrder& O = s->pcg.ord;
-        O.A.vals.release();
-        O.A.vals32.release();
+        PcgState& P = s->pcg;
+        PcgOrder& O = P.ord;
+        for(DBuf<double>* d : {&O.A.vals, &P.xs, &P.r, &P.z, &P.p, &P.Ap})
+            d->release();
+        for(DBuf<float>* d : {&O.A.vals32, &P.r32, &P.z32, &P.p32, &P.Ap32})
+            d->release();
         O.A.rows.release();
         O.A.cols.release();
         O.A.trank.release();
+        O.A.has_trank    = false;
         O.f64_generation = O.f32_generation = -1;
         return false;
     }
@@ -1115,29 +1121,35 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         return;
     }
     // with the MAS the recursion runs in its slot order (see PcgOrder)
-    const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized && try_order(s, false);
+    int  kind      = s->precond_kind;
+    bool use_graph = o.use_graph && st != nullptr;
+    auto room      = [&](bool in_order)
+    {
+        Matrix&       M = in_order ? P.ord.A : s->A;
+        const int64_t m = 3 * (int64_t)M.nb;
+        for(DBuf<double>* d : {&P.r, &P.z, &P.p, &P.Ap})
+            d->resize(m, 1.1);
+        P.tmp.resize(n0, 1.1);
+        if(in_order)
+            P.xs.resize(m, 1.1);
+        P.sc.resize(1);
+        ensure_reduction(P.red, std::max(spmv_grid(M.nnz), reduction_grid()), 2);
+        ensure_reduction(s->red, reduction_grid(), 2);  // the largest grid: the sums below run over rows and over entries
+        device_error_flag(s);  // allocated before any graph capture
+        s->dot_out.resize(4);
+        if(!use_graph || s->timing || !pcg_small_fits(s, M, kind, in_order, false))
+            M.trank.resize(M.stride, 1.2);  // filled when the steps are prepared
+    };
+    const bool ord = kind == B2S_PRECOND_MAS && s->mas.initialized && try_order(s, false, room);
+    if(!ord)
+        room(false);
     const PcgOrder& O  = P.ord;
     const Matrix&   A  = ord ? O.A : s->A;
-    const int64_t   n  = 3 * (int64_t)A.nb;  // the recursion's vectors
-    double*         xi = x;                  // the iterate
-    P.r.resize(n, 1.1);
-    P.z.resize(n, 1.1);
-    P.p.resize(n, 1.1);
-    P.Ap.resize(n, 1.1);
-    P.tmp.resize(n0, 1.1);
-    if(ord)
-    {
-        P.xs.resize(n, 1.1);
-        xi = P.xs.data();
-    }
-    P.sc.resize(1);
+    const int64_t   n  = 3 * (int64_t)A.nb;         // the recursion's vectors
+    double*         xi = ord ? P.xs.data() : x;  // the iterate
     if(!P.h_sc)
         B2S_CUDA(cudaMallocHost(&P.h_sc, sizeof(PcgScalars)));
     ensure_read_back(s);
-    ensure_reduction(P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
-    ensure_reduction(s->red, reduction_grid(), 2);  // the largest grid: the sums below run over rows and over entries
-    device_error_flag(s);  // allocated before any graph capture
-    s->dot_out.resize(4);
     const int ci = o.check_interval > 0 ? o.check_interval : 1;
     const int64_t max_iter = o.max_iter > 0 ? o.max_iter : std::max<int64_t>(2 * n0, 1);
 
@@ -1182,7 +1194,6 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         else
             B2S_CUDA(cudaMemsetAsync(xi, 0, sizeof(double) * n, st));
     }
-    int kind = s->precond_kind;
     apply(kind);
     launch_dot(s, P.r.data(), P.z.data(), n, s->dot_out.data());
     launch_dot(s, P.r.data(), P.r.data(), n, s->dot_out.data() + 1);
@@ -1242,7 +1253,6 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         B2S_CUDA(cudaMemcpyAsync(P.p.data(), P.z.data(), sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
         B2S_CUDA(cudaMemsetAsync(P.Ap.data(), 0, sizeof(double) * n, st));
 
-        bool use_graph = o.use_graph && st != nullptr;
         // small systems: the whole loop in one launch
         bool small = use_graph && !s->timing && pcg_small_fits(s, A, kind, ord, false);
         if(s->timing)
@@ -1567,33 +1577,34 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
     }
     // FP32 matrix planes (in the MAS slot order with the MAS, see PcgOrder) and
     // BF16 inverses: once per assembly / build
-    const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized && try_order(s, true);
+    auto room = [&](bool in_order)
+    {
+        if(!in_order)
+            ensure_f32_planes(s);
+        ensure_bf16_inverses(s);
+        const Matrix& M = in_order ? P.ord.A : s->A;
+        for(DBuf<float>* d : {&P.r32, &P.z32, &P.p32, &P.Ap32})
+            d->resize(4 * (size_t)M.nb, 1.1);
+        P.tmp.resize(n, 1.1);
+        if(in_order)
+            P.xs.resize(3 * (size_t)M.nb, 1.1);
+        P.sc.resize(1);
+        ensure_reduction(P.red, std::max(spmv_grid(M.nnz), reduction_grid()), 2);
+        ensure_reduction(s->red, reduction_grid(), 2);
+        device_error_flag(s);
+        s->dot_out.resize(4);
+    };
+    const bool ord = s->precond_kind == B2S_PRECOND_MAS && s->mas.initialized && try_order(s, true, room);
     if(!ord)
-        ensure_f32_planes(s);
-    ensure_bf16_inverses(s);
+        room(false);
     const PcgOrder& O  = P.ord;
     const Matrix&   A  = ord ? O.A : s->A;
-    const int32_t   nb = A.nb;               // the recursion's rows
-    const int64_t   n4 = 4 * (int64_t)nb;  // padded FP32 vectors
-    double*         xi = x;                    // the iterate
-    if(ord)
-    {
-        P.xs.resize(3 * (size_t)nb, 1.1);
-        xi = P.xs.data();
-    }
-    P.r32.resize(n4, 1.1);
-    P.z32.resize(n4, 1.1);
-    P.p32.resize(n4, 1.1);
-    P.Ap32.resize(n4, 1.1);
-    P.tmp.resize(n, 1.1);
-    P.sc.resize(1);
+    const int32_t   nb = A.nb;                      // the recursion's rows
+    const int64_t   n4 = 4 * (int64_t)nb;           // padded FP32 vectors
+    double*         xi = ord ? P.xs.data() : x;  // the iterate
     if(!P.h_sc)
         B2S_CUDA(cudaMallocHost(&P.h_sc, sizeof(PcgScalars)));
     ensure_read_back(s);
-    ensure_reduction(P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
-    ensure_reduction(s->red, reduction_grid(), 2);
-    device_error_flag(s);
-    s->dot_out.resize(4);
     const int     ci       = o.check_interval > 0 ? o.check_interval : 1;
     const int64_t max_iter = o.max_iter > 0 ? o.max_iter : std::max<int64_t>(2 * n, 1);
     int           kind     = s->precond_kind;

@@ -30,7 +30,8 @@ MasView mas_view(b2s_solver* s);
 // the vectors in PCG order with the MAS (`ord`), r, p and x set by the caller,
 // Ap zero, the scalars in s->pcg.sc (read and written back). The launch returns
 // false, with nothing done, when the device refuses it (fewer SMs than the
-// device has: a shared or partitioned GPU): the caller launches step by step.
+// device has: a shared or partitioned GPU) or has no room for its sums: the
+// caller launches step by step.
 bool pcg_small_fits(b2s_solver* s, const Matrix& A, int kind, bool ord, bool f32);
 bool pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x);
 bool pcg_small_launch_f32(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x);

@@ -664,8 +664,15 @@ bool launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterat
     a.A.err      = device_error_flag(s);
     a.iterations = iterations;
     a.polls      = s->inject_polls < 0 ? SM_SPINS : (unsigned)s->inject_polls;
-    P.small_partials.resize(3 * (size_t)grid);
-    P.small_bar.resize(1);
+    try
+    {
+        P.small_partials.resize(3 * (size_t)grid);
+        P.small_bar.resize(1);
+    }
+    catch(const OutOfMemory&)
+    {
+        return false;
+    }
     a.partials = P.small_partials.data();
     a.bar      = P.small_bar.data();
     B2S_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned), s->stream));

@@ -192,3 +192,45 @@ def test_a_refused_cooperative_launch_takes_the_steps(solver, cuda, cube10, kind
     # as for the barriers above: rounding order only
     assert abs(st0["iterations_exact"] - st1["iterations_exact"]) <= 5
     assert float((x0 - x1).norm()) <= 1e-5 * float(x0.norm())
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("timing", [False, True])
+def test_no_room_for_the_slot_order(cuda, cube5, precision, timing):
+    """The MAS solve wants a copy of the matrix in slot order and vectors of that
+    length. Whichever of its allocations fails, the call gives them back and
+    solves in the matrix's own order; the next one has its copy again. timing:
+    launch by launch, with the FP64 SpMV's tile ranks."""
+    import torch
+
+    from libuipc_b200.linear_system import Solver
+
+    x0 = None
+    for k in range(0, 22):  # 0: none fails; the last ones lie past the solve's allocations
+        s = Solver(0)
+        try:
+            b = _setup(s, cube5, cuda, _abi.B2S_PRECOND_MAS)
+            s.set_timing(timing)
+            args = dict(tol=1e-8, stop_rule=_abi.B2S_STOP_RELRES, precision=precision, replace_every=50)
+            s._check(s.lib.b2s_inject_failure(s.h, _abi.B2S_INJECT_ALLOC, k))
+            x = torch.zeros_like(b)
+            st = s.pcg(b, x, **args)
+            s._check(s.lib.b2s_inject_failure(s.h, _abi.B2S_INJECT_ALLOC, 0))
+            assert st["converged"] == 1 and st["rel_res"] <= 1e-8
+            x0 = x if x0 is None else x0
+            again = torch.zeros_like(b)
+            assert s.pcg(b, again, **args)["converged"] == 1
+            for v in (x, again):  # both stop at 1e-8: as for the barriers above
+                assert float((v - x0).norm()) <= 1e-5 * float(x0.norm())
+        finally:
+            s.close()
+
+
+def test_an_allocation_that_fails_is_a_cuda_error(solver, cuda, cube5):
+    for k in (1, 2, 5):
+        solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_ALLOC, k))
+        with pytest.raises(B200SolveError) as e:
+            _setup(solver, cube5, cuda, _abi.B2S_PRECOND_JACOBI)
+        assert e.value.code == _abi.B2S_ERR_CUDA and "out of memory" in str(e.value)
+    solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_ALLOC, 0))
+    _setup(solver, cube5, cuda, _abi.B2S_PRECOND_JACOBI)
