@@ -121,8 +121,7 @@ int b2s_mas_get_clusters(b2s_solver* s, double* h_hess, float* h_inv);
 int b2s_mas_stiff_info(b2s_solver* s, int32_t* n_stiff, uint8_t* h_flags);
 /* Node buffers of the last MAS apply (FP32, 3 per node slot, total_nodes
  * slots): the restricted residual R of every coarse node and the local
- * solution Z of every node. (A PCG of a small system keeps the fine level's on
- * chip: call b2s_precond_apply to see those.) */
+ * solution Z of every node. */
 int b2s_mas_get_nodes(b2s_solver* s, float* h_R, float* h_Z);
 
 /* Partition utility (the caller-side step of FEMMASPreconditioner::do_init):

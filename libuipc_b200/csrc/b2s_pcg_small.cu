@@ -608,6 +608,14 @@ __global__ void __launch_bounds__(SM_THREADS, SM_CTAS) k_pcg_small(const __grid_
         store_vec(a.x, i, x);
         store_vec(a.r, i, r);
     }
+    // the fine level of the last apply (b2s_mas_get_nodes; the coarse levels are there)
+    if(in_bank)
+#pragma unroll
+        for(int c = 0; c < 3; ++c)
+        {
+            a.A.R[3 * (int64_t)i + c] = (float)r[c];
+            a.A.Z[3 * (int64_t)i + c] = s_z[w][(lane >> 4) * BANK * 3 + 3 * sub + c];
+        }
     if(i == 0)
         *a.sc = sc;
 }

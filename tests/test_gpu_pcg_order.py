@@ -223,3 +223,46 @@ def test_body_rows_inside_the_mas_range(solver, cuda, first, precision):
         tol = 1e-5 if precision == 0 else 1e-2
         assert st["bypassed"] == 0 and abs(st["rz0"] - rz0) <= tol * rz0
         assert np.linalg.norm(xd.cpu().numpy() - x) <= tol * np.linalg.norm(x)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_node_buffers_after_a_solve(solver, cuda, precision):
+    """b2s_mas_get_nodes shows the last apply of the PCG whichever loop ran: every
+    node's Z is its cluster's inverse times its R, and R_0 is the residual."""
+    import torch
+
+    rng = np.random.default_rng(5)
+    n = 700
+    rows, cols, vals, product = _wide_system(rng, n)
+    start = np.zeros(n + 1, np.int32)
+    v = np.arange(n - 1)
+    e = np.concatenate([np.stack([v, v + 1], 1), np.stack([v + 1, v], 1)])
+    e = e[np.lexsort((e[:, 1], e[:, 0]))]
+    start[1:] = np.cumsum(np.bincount(e[:, 0], minlength=n))
+    p2r, r2p = _maps(rng, n, 13, 0)
+    solver.assemble(n, to_dev(rows, cuda), to_dev(cols, cuda), to_dev(vals, cuda))
+    solver.mas_init(0, n, start, e[:, 1].astype(np.int32), p2r, r2p)
+    solver.precond_assemble(2)
+    b = rng.normal(size=3 * n)
+    for graph in (True, False):
+        for fresh in (0, 1):  # another solve: nothing of the first one may show
+            bb = b if fresh else rng.normal(size=3 * n)
+            x = torch.zeros(3 * n, dtype=torch.float64, device=cuda)
+            solver.pcg(to_dev(bb, cuda), x, tol=1e-30, max_iter=4, check_interval=1, precision=precision, use_graph=graph)
+        R, Z = solver.mas_nodes()
+        r = np.zeros((p2r.size, 3))
+        r[p2r >= 0] = (b - product(x.cpu().numpy())).reshape(n, 3)[p2r[p2r >= 0]]
+        # the recursive residual: FP64, or FP32 over three updates
+        assert np.abs(R[:p2r.size] - r).max() <= (1e-6 if precision == 0 else 1e-4) * np.abs(r).max()
+        _, inv = solver.mas_clusters()
+        M = np.zeros((len(inv), 16, 3, 16, 3))
+        for k, (i, j) in enumerate((i, j) for i in range(16) for j in range(i, 16)):
+            B = inv[:, k].reshape(-1, 3, 3).transpose(0, 2, 1)
+            M[:, i, :, j] = B
+            M[:, j, :, i] = B.transpose(0, 2, 1)
+        M = M.reshape(len(inv), 48, 48).astype(np.float64)
+        ref = np.einsum("cij,cj->ci", M, R.reshape(-1, 48).astype(np.float64))
+        # FP32 products of 48 terms, or BF16 entries of the scaled inverse (2^-9 each)
+        size = np.einsum("cij,cj->ci", np.abs(M), np.abs(R.reshape(-1, 48)).astype(np.float64))
+        lim = 50 * 2.0**-24 * size if precision == 0 else 2.0**-8 * np.linalg.norm(size, axis=1, keepdims=True)
+        assert (np.abs(Z.reshape(-1, 48) - ref) <= lim).all()
