@@ -100,7 +100,22 @@ int b2s_create(int device, b2s_solver** out)
             throw b2s::Error(B2S_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
         }
         s->stream = s->own_stream;
-        *out      = s;
+        try
+        {
+            // what every handle needs, so that no first call waits for it
+            B2S_CUDA(cudaMallocHost(&s->host, sizeof(b2s::HostScalars)));
+            b2s::device_error_flag(s);
+            s->dot_out.resize(4);
+            b2s::ensure_reduction(s, s->red, b2s::reduction_grid(), b2s::MAX_DOTS);
+            b2s::ensure_reduction(s, s->pcg.red, b2s::reduction_grid(), 2);
+            B2S_CUDA(cudaStreamSynchronize(s->stream));
+        }
+        catch(...)
+        {
+            b2s_destroy(s);
+            throw;
+        }
+        *out = s;
         return B2S_OK;
     }
     catch(const b2s::Error& e)
@@ -122,12 +137,8 @@ int b2s_destroy(b2s_solver* s)
     cudaSetDevice(s->device);
     cudaStreamSynchronize(s->stream);
     b2s::drop_graphs(s);
-    if(s->pcg.h_sc)
-        cudaFreeHost(s->pcg.h_sc);
-    if(s->asmb.h_info)
-        cudaFreeHost(s->asmb.h_info);
-    if(s->h_back)
-        cudaFreeHost(s->h_back);
+    if(s->host)
+        cudaFreeHost(s->host);
     if(s->ev_begin)
         cudaEventDestroy(s->ev_begin);
     if(s->ev_end)

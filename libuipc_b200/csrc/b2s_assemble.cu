@@ -877,13 +877,11 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
     // the sizes the host needs, written by the device straight into pinned host
     // memory (a copy to pageable memory is ~9 us each, and a MAS build assembles
     // five coarse levels)
-    if(!w.h_info)
-        B2S_CUDA(cudaMallocHost(&w.h_info, 3 * sizeof(int32_t)));
-    k_publish<<<1, 1, 0, st>>>(M.rowptr.data() + nb, err, n_long_dev, w.h_info);
+    k_publish<<<1, 1, 0, st>>>(M.rowptr.data() + nb, err, n_long_dev, s->host->info);
     B2S_CHECK_LAUNCH();
     B2S_CUDA(cudaStreamSynchronize(st));
-    const int32_t U = w.h_info[0], n_long = w.h_info[2];
-    const int     herr = w.h_info[1];
+    const int32_t U = s->host->info[0], n_long = s->host->info[2];
+    const int     herr = s->host->info[1];
     B2S_REQUIRE(!(herr & DERR_TRIPLET_INDEX), B2S_ERR_ARGUMENT,
                 "triplet column index outside [0, n_block_rows)");
     B2S_REQUIRE(!(herr & DERR_ROW_OVERFLOW), B2S_ERR_ARGUMENT,

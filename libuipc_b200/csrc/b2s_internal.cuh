@@ -168,7 +168,6 @@ struct AssemblyScratch
     DBuf<int32_t> long_runs;  // [1 + U]: count, then the blocks whose run is summed by a warp
     DBuf<int32_t> scan_tmp;
     DBuf<int>     err;
-    int32_t*      h_info = nullptr;  // pinned: blocks, error bits, long rows of the last assembly
 };
 
 // ---------------------------------------------------------------------------
@@ -203,6 +202,8 @@ struct MasState
     long long     inv16_generation = -1;  // assembly generation inv16 was packed from
     // coarse-level Galerkin matrices (upper BCOO per level, in level-local ids)
     Matrix        coarse[MAX_LEVELS];
+    DBuf<int32_t> tail_idx;   // rows and columns of the levels above 1 that k_coarse_tail makes
+    DBuf<double>  tail_vals;  // and their values
     DBuf<int32_t> trip_rows, trip_cols;
     DBuf<double>  trip_vals;
     // apply buffers (FP32, 3 per node slot)
@@ -245,6 +246,15 @@ struct ReadBack
     int    err;
 };
 
+// pinned memory of a handle, made with it: the first call that reads a scalar
+// would otherwise wait for the allocation
+struct HostScalars
+{
+    ReadBack   back;     // the last read_back
+    PcgScalars sc;       // of the PCG's host loop
+    int32_t    info[3];  // blocks, error bits, long rows of the last assembly
+};
+
 struct Reduction
 {
     DBuf<double>       partials;  // [2 * grid]
@@ -277,7 +287,6 @@ struct PcgState
     DBuf<double> r, z, p, Ap, tmp;
     DBuf<PcgScalars> sc;
     Reduction        red;
-    PcgScalars*      h_sc = nullptr;  // pinned mirror
     cudaGraphExec_t  graph = nullptr;
     size_t           graph_key = 0;
     long long        graph_kernels = 0;  // kernel nodes per graph launch
@@ -313,7 +322,7 @@ struct b2s_solver
     b2s::DBuf<double>    dot_out;
     b2s::Reduction       red;
     b2s::DBuf<int>       dev_err;  // DeviceError bits raised by kernels
-    b2s::ReadBack*       h_back = nullptr;  // pinned: the last read_back
+    b2s::HostScalars*    host = nullptr;
     // stage timers (CUDA events on `stream`)
     bool                     timing = false;
     b2s_timers               timers{};
@@ -362,7 +371,7 @@ struct DotPairs
 };
 void launch_dots(b2s_solver* s, int64_t n, const DotPairs& d, int m, double* d_out);
 // partial-sum storage of the grid reductions for `grid` blocks x `nv` values
-void ensure_reduction(Reduction& red, int grid, int nv);
+void ensure_reduction(b2s_solver* s, Reduction& red, int grid, int nv);
 
 // preconditioners
 void precond_assemble(b2s_solver* s, int kind, int invert_mode);
@@ -372,8 +381,7 @@ void precond_apply_mixed(b2s_solver* s, const float* r, float* z);
 void spmv_mixed(b2s_solver* s, const float* x, float* y, double* d_dot);
 double spmv_mixed_timing(b2s_solver* s, int launches);
 void check_device_errors(b2s_solver* s);
-// pinned memory for scalars on their way to the host
-void ensure_read_back(b2s_solver* s);
+int* device_error_flag(b2s_solver* s);
 // throws when the error bits e (already cleared on the device) are not zero
 void raise_device_errors(int e);
 // n <= READ_BACK doubles from the device into h, with the stream's work done

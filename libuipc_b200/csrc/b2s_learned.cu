@@ -1379,7 +1379,7 @@ void ws_predict(b2s_solver* s, int mode, const double* b, int n_hist, const doub
         W.dots.resize(64);
         const Matrix& A    = s->A;
         const int     grid = reduction_grid(A.nnz);
-        ensure_reduction(s->red, grid, WS_MAXC * (WS_MAXC + 1) / 2);
+        ensure_reduction(s, s->red, grid, WS_MAXC * (WS_MAXC + 1) / 2);
         Cands cs{};
         for(int i = 0; i < WS_MAXC; ++i)
             cs.c[i] = cand[i < k ? i : 0];

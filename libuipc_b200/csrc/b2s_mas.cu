@@ -30,7 +30,6 @@
 
 namespace b2s
 {
-int* device_error_flag(b2s_solver* s);
 void mas_invert_clusters(b2s_solver* s, int mode);
 
 namespace
@@ -721,6 +720,8 @@ static void place_partials(b2s_solver* s)
                 next[m] += first ? 1 : 0;
                 *a = 2 * (next[m] - 1) + (first ? 0 : 1);
             }
+    M.tail_idx.resize((size_t)2 * TAIL_BLOCKS * (M.L - 2));
+    M.tail_vals.resize((size_t)9 * TAIL_BLOCKS * (M.L - 2));
     M.part.resize(3 * (size_t)entries + 3);  // one more: copies end at even entries
     M.part_start.resize(nodes + 1);
     M.part_dst.resize(std::max(cnt1, 1));
@@ -949,12 +950,9 @@ void mas_assemble(b2s_solver* s, int invert_mode)
             a.hess  = M.hess.data();
             for(int l = level; l < M.L; ++l)
             {
-                Matrix& D = M.coarse[l];
-                D.rows.resize(TAIL_BLOCKS);
-                D.cols.resize(TAIL_BLOCKS);
-                D.vals.resize((size_t)9 * TAIL_BLOCKS);
-                a.lv[l] = TailLevel{M.level_begin[l], X.new_local[l - 1].data(), D.rows.data(), D.cols.data(),
-                                    D.vals.data()};
+                int32_t* idx = M.tail_idx.data() + (size_t)2 * TAIL_BLOCKS * (l - 2);
+                a.lv[l] = TailLevel{M.level_begin[l], X.new_local[l - 1].data(), idx, idx + TAIL_BLOCKS,
+                                    M.tail_vals.data() + (size_t)9 * TAIL_BLOCKS * (l - 2)};
             }
             B2S_CUDA(cudaFuncSetAttribute(k_coarse_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM));
             k_coarse_tail<<<1, TAIL_THREADS, TAIL_SMEM, st>>>(a);

@@ -27,10 +27,7 @@ namespace b2s
 {
 void spmv_f64_launch(b2s_solver* s, const Matrix& A, const double* x, double* y, Reduction& red, double* d_dot,
                      const int* stop);
-int* device_error_flag(b2s_solver* s);
-void check_device_errors(b2s_solver* s);
 int  spmv_grid(int64_t U);
-void ensure_reduction(Reduction& red, int grid, int nv);
 void mas_apply_levels(b2s_solver* s, const double* r, const int* converged);
 void mas_apply_levels_f32(b2s_solver* s, const float* r, const int* converged, bool bf16);
 void mas_pack_bf16(b2s_solver* s);
@@ -977,7 +974,7 @@ static void precond_launch_ord(b2s_solver* s, int kind, bool bf16, const VT* r, 
     if(kind == B2S_PRECOND_MAS)
         mas_apply_all(s, sc ? &sc->converged : nullptr, bf16);
     const int grid = reduction_grid(n);
-    ensure_reduction(red, grid, 2);
+    ensure_reduction(s, red, grid, 2);
     k_precond_finish<VT, NS, true><<<grid, RED_BLOCK, 0, s->stream>>>(n, kind, mas_view(s), s->dinv.data(), r, z, sc,
                                                                      red.partials.data(), red.counter.data());
     B2S_CHECK_LAUNCH();
@@ -993,7 +990,7 @@ static void precond_launch(b2s_solver* s, int kind, const double* r, double* z, 
     if(kind == B2S_PRECOND_MAS)
         mas_apply_levels(s, r, sc ? &sc->converged : nullptr);
     const int grid = reduction_grid(nb);
-    ensure_reduction(red, grid, 2);
+    ensure_reduction(s, red, grid, 2);
     k_precond_finish<double, 3, false><<<grid, RED_BLOCK, 0, st>>>(nb, kind, mas_view(s), s->dinv.data(), r, z, sc,
                                                  red.partials.data(), red.counter.data());
     B2S_CHECK_LAUNCH();
@@ -1081,11 +1078,11 @@ static void pcg_iteration(b2s_solver* s, int kind, bool ord, double* x, int slot
 static void read_scalars(b2s_solver* s, long long iter_before)
 {
     PcgState& P = s->pcg;
-    k_scalars_out<<<1, 1, 0, s->stream>>>(P.sc.data(), s->dev_err.data(), P.h_sc, s->h_back);
+    k_scalars_out<<<1, 1, 0, s->stream>>>(P.sc.data(), s->dev_err.data(), &s->host->sc, &s->host->back);
     B2S_CHECK_LAUNCH();
     B2S_CUDA(cudaStreamSynchronize(s->stream));
-    raise_device_errors(s->h_back->err);
-    B2S_REQUIRE(P.h_sc->converged != 0 || P.h_sc->iter > iter_before, B2S_ERR_CUDA, "the PCG made no progress");
+    raise_device_errors(s->host->back.err);
+    B2S_REQUIRE(s->host->sc.converged != 0 || s->host->sc.iter > iter_before, B2S_ERR_CUDA, "the PCG made no progress");
 }
 
 static void ensure_iter_events(b2s_solver* s, int ci)
@@ -1133,8 +1130,8 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         if(in_order)
             P.xs.resize(m, 1.1);
         P.sc.resize(1);
-        ensure_reduction(P.red, std::max(spmv_grid(M.nnz), reduction_grid()), 2);
-        ensure_reduction(s->red, reduction_grid(), 2);  // the largest grid: the sums below run over rows and over entries
+        ensure_reduction(s, P.red, std::max(spmv_grid(M.nnz), reduction_grid()), 2);
+        ensure_reduction(s, s->red, reduction_grid(), 2);  // the largest grid: the sums below run over rows and over entries
         device_error_flag(s);  // allocated before any graph capture
         s->dot_out.resize(4);
         if(!use_graph || s->timing || !pcg_small_fits(s, M, kind, in_order, false))
@@ -1147,9 +1144,6 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
     const Matrix&   A  = ord ? O.A : s->A;
     const int64_t   n  = 3 * (int64_t)A.nb;         // the recursion's vectors
     double*         xi = ord ? P.xs.data() : x;  // the iterate
-    if(!P.h_sc)
-        B2S_CUDA(cudaMallocHost(&P.h_sc, sizeof(PcgScalars)));
-    ensure_read_back(s);
     const int ci = o.check_interval > 0 ? o.check_interval : 1;
     const int64_t max_iter = o.max_iter > 0 ? o.max_iter : std::max<int64_t>(2 * n0, 1);
 
@@ -1338,7 +1332,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
             if(s->timing)
             {
                 // the iterations of this block that did work (the rest were frozen)
-                const long long live = std::min<long long>(P.h_sc->iter - iter_before, ci);
+                const long long live = std::min<long long>(s->host->sc.iter - iter_before, ci);
                 for(long long it = 0; it < live; ++it)
                 {
                     float a = 0.f, c = 0.f;
@@ -1350,11 +1344,11 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
                     s->timers.precond_apply_launches += 1;
                 }
             }
-            iter_before = P.h_sc->iter;
-            if(P.h_sc->converged != 0)
+            iter_before = s->host->sc.iter;
+            if(s->host->sc.converged != 0)
                 break;
         }
-        const PcgScalars r = *P.h_sc;
+        const PcgScalars r = s->host->sc;
         iter_total         = r.iter;
         if(ord)
         {
@@ -1423,7 +1417,7 @@ static void precond_launch_f32(b2s_solver* s, int kind, const float* r, float* z
     if(kind == B2S_PRECOND_MAS)
         mas_apply_levels_f32(s, r, sc ? &sc->converged : nullptr, mixed_inverse_bf16());
     const int grid = reduction_grid(nb);
-    ensure_reduction(red, grid, 2);
+    ensure_reduction(s, red, grid, 2);
     k_precond_finish<float, 4, false><<<grid, RED_BLOCK, 0, s->stream>>>(nb, kind, mas_view(s), s->dinv.data(), r, z, sc,
                                                                red.partials.data(), red.counter.data());
     B2S_CHECK_LAUNCH();
@@ -1460,7 +1454,7 @@ void spmv_mixed(b2s_solver* s, const float* x, float* y, double* d_dot)
     const int32_t nb = A.nb;
     cudaStream_t  st = s->stream;
     ensure_f32_planes(s);
-    ensure_reduction(P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
+    ensure_reduction(s, P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
     P.p32.resize(4 * (size_t)nb, 1.1);
     P.Ap32.resize(4 * (size_t)nb, 1.1);
     k_pad4<<<vec_grid(nb), VEC_BLOCK, 0, st>>>(nb, x, P.p32.data(), P.Ap32.data());
@@ -1483,7 +1477,7 @@ double spmv_mixed_timing(b2s_solver* s, int launches)
     cudaStream_t  st = s->stream;
     B2S_REQUIRE(launches > 0, B2S_ERR_ARGUMENT, "launch count must be positive");
     ensure_f32_planes(s);
-    ensure_reduction(P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
+    ensure_reduction(s, P.red, std::max(spmv_grid(A.nnz), reduction_grid()), 2);
     P.p32.resize(4 * (size_t)nb, 1.1);
     P.Ap32.resize(4 * (size_t)nb, 1.1);
     s->dot_out.resize(4);
@@ -1510,7 +1504,7 @@ void precond_apply_mixed(b2s_solver* s, const float* r, float* z)
 {
     B2S_REQUIRE(s->precond_kind >= 0, B2S_ERR_STATE, "precond_apply before b2s_precond_assemble");
     ensure_bf16_inverses(s);
-    ensure_reduction(s->red, reduction_grid(), 2);
+    ensure_reduction(s, s->red, reduction_grid(), 2);
     const int32_t nb = s->A.nb;
     PcgState&     P  = s->pcg;
     P.r32.resize(4 * (size_t)nb, 1.1);
@@ -1589,8 +1583,8 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
         if(in_order)
             P.xs.resize(3 * (size_t)M.nb, 1.1);
         P.sc.resize(1);
-        ensure_reduction(P.red, std::max(spmv_grid(M.nnz), reduction_grid()), 2);
-        ensure_reduction(s->red, reduction_grid(), 2);
+        ensure_reduction(s, P.red, std::max(spmv_grid(M.nnz), reduction_grid()), 2);
+        ensure_reduction(s, s->red, reduction_grid(), 2);
         device_error_flag(s);
         s->dot_out.resize(4);
     };
@@ -1602,9 +1596,6 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
     const int32_t   nb = A.nb;                      // the recursion's rows
     const int64_t   n4 = 4 * (int64_t)nb;           // padded FP32 vectors
     double*         xi = ord ? P.xs.data() : x;  // the iterate
-    if(!P.h_sc)
-        B2S_CUDA(cudaMallocHost(&P.h_sc, sizeof(PcgScalars)));
-    ensure_read_back(s);
     const int     ci       = o.check_interval > 0 ? o.check_interval : 1;
     const int64_t max_iter = o.max_iter > 0 ? o.max_iter : std::max<int64_t>(2 * n, 1);
     int           kind     = s->precond_kind;
@@ -1788,7 +1779,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
             read_scalars(s, iter_before);
             if(s->timing)
             {
-                const long long live = std::min<long long>(P.h_sc->iter - iter_before, ci);
+                const long long live = std::min<long long>(s->host->sc.iter - iter_before, ci);
                 for(long long it = 0; it < live; ++it)
                 {
                     float a = 0.f, c = 0.f;
@@ -1800,19 +1791,19 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
                     s->timers.precond_apply_launches += 1;
                 }
             }
-            iter_before = P.h_sc->iter;
-            if(P.h_sc->converged != 0)
+            iter_before = s->host->sc.iter;
+            if(s->host->sc.converged != 0)
                 break;
-            if(o.replace_every > 0 && P.h_sc->iter - last_replace >= o.replace_every)
+            if(o.replace_every > 0 && s->host->sc.iter - last_replace >= o.replace_every)
             {
                 // reliable update: FP64 residual of the FP64 iterate, p and r.z kept
                 store_x();
                 residual(false);
                 ++replacements;
-                last_replace = P.h_sc->iter;
+                last_replace = s->host->sc.iter;
             }
         }
-        const PcgScalars r = *P.h_sc;
+        const PcgScalars r = s->host->sc;
         iter_total         = r.iter;
         store_x();
         if(r.converged == 3)

@@ -26,7 +26,6 @@
 
 namespace b2s
 {
-int* device_error_flag(b2s_solver* s);
 
 namespace
 {

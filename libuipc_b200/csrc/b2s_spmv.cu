@@ -486,14 +486,14 @@ int spmv_grid(int64_t U)
     return (int)std::max<int64_t>(1, std::min<int64_t>(t, (int64_t)NUM_SMS_HINT * 8));
 }
 
-void ensure_reduction(Reduction& red, int grid, int nv)
+void ensure_reduction(b2s_solver* s, Reduction& red, int grid, int nv)
 {
     if(red.partials.size() < (size_t)grid * nv)
         red.partials.resize((size_t)grid * nv);
     if(red.counter.size() < 1)
     {
         red.counter.resize(1);
-        B2S_CUDA(cudaMemset(red.counter.data(), 0, sizeof(unsigned int)));
+        B2S_CUDA(cudaMemsetAsync(red.counter.data(), 0, sizeof(unsigned int), s->stream));
     }
 }
 
@@ -502,7 +502,7 @@ int* device_error_flag(b2s_solver* s)
     if(s->dev_err.size() < 1)
     {
         s->dev_err.resize(1);
-        B2S_CUDA(cudaMemset(s->dev_err.data(), 0, sizeof(int)));
+        B2S_CUDA(cudaMemsetAsync(s->dev_err.data(), 0, sizeof(int), s->stream));
     }
     return s->dev_err.data();
 }
@@ -522,12 +522,6 @@ __global__ void k_read_back(const double* __restrict__ d, int n, int* err, ReadB
 // memory, then one wait for the stream: a copy to pageable memory waits by
 // itself, ~9 us each, and an entry point that read its error flag and then its
 // dot did so twice.
-void ensure_read_back(b2s_solver* s)
-{
-    if(!s->h_back)
-        B2S_CUDA(cudaMallocHost(&s->h_back, sizeof(ReadBack)));
-}
-
 void raise_device_errors(int e)
 {
     if(e == 0)
@@ -538,13 +532,12 @@ void raise_device_errors(int e)
 
 void read_back(b2s_solver* s, const double* d, int n, double* h)
 {
-    ensure_read_back(s);
-    k_read_back<<<1, 32, 0, s->stream>>>(d, n, s->dev_err.size() ? s->dev_err.data() : nullptr, s->h_back);
+    k_read_back<<<1, 32, 0, s->stream>>>(d, n, s->dev_err.size() ? s->dev_err.data() : nullptr, &s->host->back);
     B2S_CHECK_LAUNCH();
     B2S_CUDA(cudaStreamSynchronize(s->stream));
     for(int i = 0; i < n; ++i)
-        h[i] = s->h_back->v[i];
-    raise_device_errors(s->h_back->err);
+        h[i] = s->host->back.v[i];
+    raise_device_errors(s->host->back.err);
 }
 
 // raise (and clear) the error bits kernels left in the device flag
@@ -571,7 +564,7 @@ void spmv_f64(b2s_solver* s, const Matrix& A, const double* x, double* y, double
             B2S_CUDA(cudaMemsetAsync(d_dot, 0, sizeof(double), st));
         return;
     }
-    ensure_reduction(s->red, spmv_grid(A.nnz), 1);
+    ensure_reduction(s, s->red, spmv_grid(A.nnz), 1);
     if(!A.has_trank)
     {
         auto k   = d_dot ? k_spmv_direct64<true> : k_spmv_direct64<false>;
@@ -748,7 +741,7 @@ void launch_dots(b2s_solver* s, int64_t n, const DotPairs& d, int m, double* d_o
     // with 1,038 of them that took longer than the products (20.7 us for 9
     // products of 265,923 entries)
     const int grid = std::min(reduction_grid(n), 2 * NUM_SMS_HINT);
-    ensure_reduction(s->red, grid, MAX_DOTS);
+    ensure_reduction(s, s->red, grid, MAX_DOTS);
     k_multi_dot<<<grid, RED_BLOCK, 0, s->stream>>>(n, m, d, s->red.partials.data(), s->red.counter.data(), d_out);
     B2S_CHECK_LAUNCH();
 }
@@ -768,7 +761,7 @@ int reduction_grid(int64_t items)
 void launch_dot(b2s_solver* s, const double* a, const double* b, int64_t n, double* d_out)
 {
     const int grid = reduction_grid(n);
-    ensure_reduction(s->red, grid, 1);
+    ensure_reduction(s, s->red, grid, 1);
     k_dot<<<grid, RED_BLOCK, 0, s->stream>>>(a, b, n, s->red.partials.data(), s->red.counter.data(), d_out);
     B2S_CHECK_LAUNCH();
 }
