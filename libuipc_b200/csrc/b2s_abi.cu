@@ -175,6 +175,7 @@ int b2s_assemble(b2s_solver* s, int32_t nb, int64_t T, const int32_t* rows, cons
                        B2S_REQUIRE(nb <= INT32_MAX / 3, B2S_ERR_ARGUMENT, "too many block rows");
                        timed_stage(s, &b2s_timers::assemble_ms,
                                    [&] { b2s::assemble_triplets(s, s->A, nb, T, rows, cols, vals); });
+                       s->A.trank.resize(s->A.stride, 1.2);  // room only: an allocation would cost a product ten times its time
                        s->precond_kind = -1;  // any preconditioner must be rebuilt
                        B2S_CUDA(cudaStreamSynchronize(s->stream));
                    });

@@ -234,3 +234,19 @@ def test_an_allocation_that_fails_is_a_cuda_error(solver, cuda, cube5):
         assert e.value.code == _abi.B2S_ERR_CUDA and "out of memory" in str(e.value)
     solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_ALLOC, 0))
     _setup(solver, cube5, cuda, _abi.B2S_PRECOND_JACOBI)
+
+
+def test_products_after_the_first_allocate_nothing(solver, cuda, cube10):
+    """The FP64 product builds its tile ranks from the second call of an assembly
+    on, in room the assembly has made."""
+    import torch
+
+    b = _setup(solver, cube10, cuda, _abi.B2S_PRECOND_JACOBI)
+    y = [torch.zeros_like(b) for _ in range(3)]
+    solver.spmv(b, y[0])
+    solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_ALLOC, 1))
+    solver.spmv(b, y[1], with_dot=True)
+    solver.spmv(b, y[2])
+    solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_ALLOC, 0))
+    for v in y[1:]:  # reductions in another order: a few ulp of the row sums
+        assert float((v - y[0]).abs().max()) <= 1e-13 * float(y[0].abs().max())
