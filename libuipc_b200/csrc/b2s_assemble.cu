@@ -743,6 +743,7 @@ __global__ void __launch_bounds__(RANK_THREADS) k_tile_rank(int64_t U, const int
 // Bound by HBM, 144 B per block. (One strided copy per component moved 8 bytes
 // at a time: 4.1 ms for 4.3 M blocks.)
 constexpr int OUT_BLOCKS = 256;
+constexpr int OUT_ROOM   = 4096;  // blocks that a read-back to host memory takes at a time, at least
 __global__ void __launch_bounds__(OUT_BLOCKS) k_blocks_out(int64_t k0, int64_t n, const double* __restrict__ vals,
                                                            int64_t S, double* __restrict__ out)
 {
@@ -799,29 +800,18 @@ void copy_blocks_out(b2s_solver* s, const Matrix& A, double* out)
         launch(0, A.nnz, out);
         return;
     }
-    // host (or another device's) memory: in pieces through a bounded buffer
-    const int64_t piece = std::min<int64_t>(A.nnz, 1 << 20);
-    DBuf<double>  tmp;
-    try
-    {
-        tmp.resize((size_t)piece * 9);
-    }
-    catch(const OutOfMemory&)
-    {
-        // no room for the buffer: one strided copy per component
-        for(int q = 0; q < 9; ++q)
-            B2S_CUDA(cudaMemcpy2DAsync(out + q, 9 * sizeof(double), A.vals.data() + (size_t)q * A.stride,
-                                       sizeof(double), sizeof(double), A.nnz, cudaMemcpyDefault, st));
-        B2S_CUDA(cudaStreamSynchronize(st));
-        return;
-    }
+    // host (or another device's) memory: in pieces through the assembly's scratch
+    // (8 bytes per triplet, OUT_ROOM blocks at least, idle between assemblies: a
+    // buffer made for the call took 600 us of a 20,000-block read-back to pinned
+    // memory, the nine strided copies before it 264)
+    double* const tmp   = reinterpret_cast<double*>(s->asmb.bucket.data());
+    const int64_t piece = std::min<int64_t>({A.nnz, (int64_t)(s->asmb.bucket.cap / 9), 1 << 20});
     for(int64_t k = 0; k < A.nnz; k += piece)
     {
         const int64_t n = std::min<int64_t>(piece, A.nnz - k);
-        launch(k, n, tmp.data());
-        B2S_CUDA(cudaMemcpyAsync(out + 9 * k, tmp.data(), sizeof(double) * 9 * (size_t)n, cudaMemcpyDefault, st));
+        launch(k, n, tmp);
+        B2S_CUDA(cudaMemcpyAsync(out + 9 * k, tmp, sizeof(double) * 9 * (size_t)n, cudaMemcpyDefault, st));
     }
-    B2S_CUDA(cudaStreamSynchronize(st));
 }
 
 void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const int32_t* rows, const int32_t* cols,
@@ -847,7 +837,7 @@ void assemble_triplets(b2s_solver* s, Matrix& M, int32_t nb, int64_t T, const in
     B2S_CUDA(cudaMemsetAsync(w.row_count.data(), 0, sizeof(int32_t) * ((size_t)nb + 4), st));
     if(T > 0)
     {
-        w.bucket.resize(T, 1.25);
+        w.bucket.resize(std::max<int64_t>(T, 9 * OUT_ROOM), 1.25);
         w.sorted_col.resize(T, 1.25);
         w.sorted_src.resize(T, 1.25);
         k_count_rows<<<asm_grid(T, ASM_BLOCK), ASM_BLOCK, 0, st>>>(rows, cols, T, nb, w.row_count.data(), err);

@@ -250,3 +250,20 @@ def test_products_after_the_first_allocate_nothing(solver, cuda, cube10):
     solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_ALLOC, 0))
     for v in y[1:]:  # reductions in another order: a few ulp of the row sums
         assert float((v - y[0]).abs().max()) <= 1e-13 * float(y[0].abs().max())
+
+
+@pytest.mark.parametrize("n_triplets", [1, 12, 10000, 10241, 60001])
+def test_read_back_allocates_nothing(solver, cuda, n_triplets):
+    """The blocks to host memory, in pieces through the assembly's scratch (5,120
+    blocks while there are fewer than 36,864 triplets, then a ninth of 1.25 times
+    those)."""
+    rng = np.random.default_rng(n_triplets)
+    idx = np.arange(n_triplets, dtype=np.int32) // 2  # two triplets per block
+    vals = rng.normal(size=(n_triplets, 9))
+    solver.assemble(n_triplets, to_dev(idx, cuda), to_dev(idx, cuda), to_dev(vals, cuda))
+    ref = vals[0::2].copy()
+    ref[:n_triplets // 2] += vals[1::2]
+    solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_ALLOC, 1))
+    _, col, v = solver.upper_bsr()
+    solver._check(solver.lib.b2s_inject_failure(solver.h, _abi.B2S_INJECT_ALLOC, 0))
+    assert np.array_equal(col, np.unique(idx)) and np.array_equal(v, ref)
