@@ -72,7 +72,7 @@ struct LearnedState
     // per-system scratch
     DBuf<float>  acc, feat, X, Y, H1, H2, dY, dH, loss_dev;
     DBuf<double> fields, d_mlp, Ac, x0, dots;
-    DBuf<double> inter;  // the candidates of a start, side by side per node
+    DBuf<double> inter;  // the candidates of a start, side by side per node (where the MAS build's scratch is too small)
     DBuf<__nv_bfloat16> w16;  // BF16 copy of the weights for inference
     long long    w16_version = -1, version = 0;
     cudaEvent_t  ev0 = nullptr, ev1 = nullptr;
@@ -747,11 +747,6 @@ __global__ void k_ws_lincomb(int64_t n, int nc, Cands cs, double* __restrict__ x
     }
 }
 
-// The Galerkin matrix of the candidate starts, G_ij = c_i . A c_j (i <= j,
-// row-major upper triangle), in one pass over the stored upper blocks with no
-// product vectors: with u_k = B c_k(col), a block B at (row, col) adds
-// c_i(row) . u_j and, off the diagonal (the transposed block), u_i . c_j(row).
-// FP64, fixed grid and order: deterministic.
 // the candidates of a node side by side: out[node][K padded to even][3], so a
 // gather of a node is one run of 16-byte loads instead of 3 K scattered ones
 // (blockIdx.y: the candidate)
@@ -768,9 +763,12 @@ __global__ void __launch_bounds__(WS_BLOCK) k_ws_interleave(int64_t n, Cands cs,
     }
 }
 
-// the k x k Galerkin matrix in one pass over the matrix (per block u = B c(col),
-// G_ij += c_i(row) . u_j + [off-diagonal] u_i . c_j(row)), the candidates
-// gathered from k_ws_interleave's copy. Bound by the gathers through L2 and by
+// The Galerkin matrix of the candidate starts, G_ij = c_i . A c_j (i <= j,
+// row-major upper triangle), in one pass over the stored upper blocks with no
+// product vectors: with u_k = B c_k(col), a block B at (row, col) adds
+// c_i(row) . u_j and, off the diagonal (the transposed block), u_i . c_j(row).
+// FP64, fixed grid and order: deterministic. The candidates are gathered from
+// k_ws_interleave's copy. Bound by the gathers through L2 and by
 // FP64: 8 candidates on 0.71 M blocks, 90 us with scattered gathers, 48 now.
 template <int K>
 __global__ void __launch_bounds__(RED_BLOCK) k_ws_gram(int64_t U, int64_t S, const int32_t* __restrict__ rows,
@@ -1386,15 +1384,23 @@ void ws_predict(b2s_solver* s, int mode, const double* b, int n_hist, const doub
         double* gram = W.dots.data();
         auto    gram_launch = [&](auto K) {
             constexpr int KK = decltype(K)::value;
-            W.inter.resize((size_t)A.nb * 3 * ((KK + 1) / 2 * 2), 1.1);
-            k_ws_interleave<KK><<<dim3(ws_grid(n), (KK + 1) / 2 * 2), WS_BLOCK, 0, st>>>(n, cs, W.inter.data());
+            // the MAS build's triplets are idle between builds and larger (9
+            // doubles per block): an allocation here made a first start 250 us longer
+            const size_t room  = (size_t)A.nb * 3 * ((KK + 1) / 2 * 2);
+            double*      inter = s->mas.trip_vals.data();
+            if(s->mas.trip_vals.cap < room)
+            {
+                W.inter.resize(room, 1.1);
+                inter = W.inter.data();
+            }
+            k_ws_interleave<KK><<<dim3(ws_grid(n), (KK + 1) / 2 * 2), WS_BLOCK, 0, st>>>(n, cs, inter);
             B2S_CHECK_LAUNCH();
             // a grid that fits at once: up to 45 sums are collected from every block
             int occ = 1;
             if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ws_gram<KK>, RED_BLOCK, 0) != cudaSuccess || occ < 1)
                 occ = 1;
             k_ws_gram<KK><<<std::min(grid, NUM_SMS_HINT * occ), RED_BLOCK, 0, st>>>(
-                A.nnz, A.stride, A.rows.data(), A.cols.data(), A.vals.data(), W.inter.data(), s->red.partials.data(),
+                A.nnz, A.stride, A.rows.data(), A.cols.data(), A.vals.data(), inter, s->red.partials.data(),
                 s->red.counter.data(), gram);
         };
         switch(k)
