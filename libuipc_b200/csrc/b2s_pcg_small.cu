@@ -1,6 +1,6 @@
 // The whole PCG loop of a small system in one cooperative launch.
 //
-// Below ~75,000 rows an iteration of the launch-per-step loop (b2s_pcg.cu) is
+// Below ~30,000 rows an iteration of the launch-per-step loop (b2s_pcg.cu) is
 // a chain of five launches that each do a microsecond of work, and the host
 // looks at the scalars every few iterations. Here the grid stays resident: a
 // thread owns one row of x, r, p and z in registers for the whole solve, a
@@ -704,8 +704,15 @@ bool launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterat
 }  // namespace
 
 // Whether the one-launch loop takes the system: every block resident at once
-// (148 x 2 blocks of 256 rows), and rows and blocks per thread low enough that
-// the barriers, not the streams, bound the iteration.
+// (148 x 2 blocks of 256 rows), and few enough blocks per thread (of one block
+// of threads per SM) that the barriers bound the iteration: its two-blocks-a-load
+// SpMV streams a matrix slower than the launches' kernels do. Measured, us per
+// iteration in one launch / launch by launch (graph), below and above each line:
+//   Jacobi, FP64 (6):  227,000 blocks 18.9 / 21.9 (tets), 237,000 31.0 / 29.3 (cloth)
+//   Jacobi, mixed (8): 301,000 blocks 17.0 / 19.4 (tets), 362,000 31.8 / 25.8 (cloth)
+//   MAS, FP64 (3):      43,000 blocks 20.4 / 25.3 (tets), 121,000 31.9 / 30.8 (cloth)
+//   MAS, mixed (5):    121,000 blocks 26.0 / 26.9 (cloth), 237,000 30.5 / 29.7 (cloth)
+// At 70,000 rows the launches win by a quarter (cloth 71.7 / 54.6, MAS, FP64).
 bool pcg_small_fits(b2s_solver* s, const Matrix& A, int kind, bool ord, bool f32)
 {
     const bool mas = kind == B2S_PRECOND_MAS;
@@ -714,6 +721,7 @@ bool pcg_small_fits(b2s_solver* s, const Matrix& A, int kind, bool ord, bool f32
     const void*  k    = f32 ? (mas ? (const void*)k_pcg_small<float, true> : (const void*)k_pcg_small<float, false>) :
                               (mas ? (const void*)k_pcg_small<double, true> : (const void*)k_pcg_small<double, false>);
     const size_t smem = f32 ? small_smem<float>(mas) : small_smem<double>(mas);
+    const int    per_thread = mas ? (f32 ? 5 : 3) : (f32 ? 8 : 6);
     if(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     {
         cudaGetLastError();
@@ -726,7 +734,7 @@ bool pcg_small_fits(b2s_solver* s, const Matrix& A, int kind, bool ord, bool f32
         cudaGetLastError();
         return false;
     }
-    return (int64_t)small_grid(A) <= (int64_t)occ * sms && A.nnz <= 16ll * SM_THREADS * occ * sms;
+    return (int64_t)small_grid(A) <= (int64_t)occ * sms && A.nnz <= (int64_t)per_thread * SM_THREADS * sms;
 }
 
 bool pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x)

@@ -119,10 +119,10 @@ def test_zero_right_hand_side_on_a_new_handle(solver, cuda, nb, precision):
     assert st["converged"] == 1 and st["rel_res"] == 0.0 and not x.any()
 
 
-def _wide_system(rng, n):
-    """n rows, couplings at distances 1, 3 and 41 (PSD per link) plus 0.3 I."""
-    i = np.concatenate([np.arange(n - d) for d in (1, 3, 41)])
-    j = i + np.repeat((1, 3, 41), (n - 1, n - 3, n - 41))
+def _wide_system(rng, n, far=(1, 3, 41)):
+    """n rows, couplings at the distances `far` (PSD per link) plus 0.3 I."""
+    i = np.concatenate([np.arange(n - d) for d in far])
+    j = i + np.repeat(far, [n - d for d in far])
     Q = rng.normal(size=(i.size, 3, 3))
     K = np.einsum("kab,kcb->kac", Q, Q)
     d = np.arange(n)
@@ -140,17 +140,20 @@ def _wide_system(rng, n):
     return rows, cols, vals, product
 
 
-@pytest.mark.parametrize("n,part,edges", [(40003, 16, 0), (52007, 13, 0), (61003, 16, 2), (75773, 16, 4), (75777, 16, 4)])
+@pytest.mark.parametrize("n,part,edges,far", [
+    (20003, 16, 0, (1, 3, 41)), (28001, 13, 2, (1, 3, 41)), (47003, 16, 4, (1, 3, 41)), (47900, 16, 4, (1, 3, 41)),
+    (52007, 13, 0, (5,)), (56000, 16, 0, (5,)), (75773, 16, 2, (1,)), (75777, 16, 2, (1,))])
 @pytest.mark.parametrize("precision", [0, 1])
-def test_banks_of_many_components(solver, cuda, n, part, edges, precision):
+def test_banks_of_many_components(solver, cuda, n, part, edges, far, precision):
     """A hierarchy whose banks fall into many components (mesh edges only inside
     runs of `edges` vertices), so every level has as many banks as blocks or
-    more and a block takes several of a level in turn; the last two sizes lie
-    on either side of what one launch holds."""
+    more and a block takes several of a level in turn; sizes on either side of
+    what the one-launch loop takes (3 or 5 blocks for each of 37,888 threads,
+    75,776 rows)."""
     import torch
 
     rng = np.random.default_rng(n + precision)
-    rows, cols, vals, product = _wide_system(rng, n)
+    rows, cols, vals, product = _wide_system(rng, n, far)
     v = np.arange(n)
     e = v[(v + 1 < n) & ((v + 1) % max(edges, 1) != 0)] if edges else v[:0]
     e = np.concatenate([np.stack([e, e + 1], 1), np.stack([e + 1, e], 1)])
