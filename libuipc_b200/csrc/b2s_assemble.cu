@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(const int32_t* __rest
 // beyond that the tile sums are scanned first.
 void exclusive_scan(b2s_solver* s, const int32_t* in, int32_t* out, int64_t n, DBuf<int32_t>& tmp)
 {
+    B2S_REQUIRE(n <= 0 || in + n <= out || out + n + 1 <= in, B2S_ERR_STATE, "exclusive_scan in place");
     cudaStream_t st = s->stream;
     if(n <= 0)
     {

@@ -339,8 +339,8 @@ struct b2s_solver
 
 namespace b2s
 {
-// device-wide exclusive scan of int32 (n elements, out may alias in); returns
-// the total (synchronises when want_total)
+// device-wide exclusive scan of n int32 into out[0 .. n], out[n] = the total;
+// queued on the solver's stream. in and out must not overlap
 void exclusive_scan(b2s_solver* s, const int32_t* in, int32_t* out, int64_t n, DBuf<int32_t>& tmp);
 
 // assembly of raw triplets into a block-upper matrix (shared by the global
