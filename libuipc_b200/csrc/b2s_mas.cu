@@ -267,11 +267,8 @@ __global__ void __launch_bounds__(GAL_BLOCKS)
         int       ca = -1, cb = -1, mode = 0, dst = -1;
         if(a >= 0 && a < n_in && b >= 0 && b < n_in)
         {
-            if(map)
-            {
-                ca = map[a];
-                cb = map[b];
-            }
+            ca = map[a];
+            cb = map[b];
             if constexpr(EXTRACT)
             {
                 const int pa = r2p[a], pb = r2p[b];
@@ -287,11 +284,8 @@ __global__ void __launch_bounds__(GAL_BLOCKS)
             mode |= ca < cb ? 1 : (ca > cb ? 2 : (a == b ? 1 : 3));
         else
             ca = cb = -1;
-        if(map)
-        {
-            out_rows[k] = ca < cb ? ca : cb;
-            out_cols[k] = ca < cb ? cb : ca;
-        }
+        out_rows[k] = ca < cb ? ca : cb;
+        out_cols[k] = ca < cb ? cb : ca;
         s_mode[t] = (unsigned char)mode;
         if constexpr(EXTRACT)
             s_dst[t] = dst;
@@ -919,13 +913,6 @@ void mas_assemble(b2s_solver* s, int invert_mode)
     const int    TB = 256;
     const Matrix& A = s->A;
     B2S_CUDA(cudaMemsetAsync(M.hess.data(), 0, M.hess.bytes(), st));
-    if(A.nnz > 0 && M.L <= 1)
-    {
-        k_g_restrict<true><<<grid_for(A.nnz, GAL_BLOCKS), GAL_BLOCKS, 0, st>>>(
-            A.nnz, A.rows.data(), A.cols.data(), A.vals.data(), A.stride, M.offset, M.vn, M.r2p.data(), nullptr,
-            nullptr, nullptr, nullptr, M.hess.data());
-        B2S_CHECK_LAUNCH();
-    }
     // coarse levels: A_1 from A (vertex ids -> level-1 ids), A_{l+1} from A_l
     const Matrix* prev     = &A;
     int           prev_off = M.offset;

@@ -820,7 +820,6 @@ MasView mas_view(b2s_solver* s)
     mv.abd_inv = s->abd_inv.data();
     mv.off    = M.offset;
     mv.vn     = M.vn;
-    mv.L      = M.L;
     mv.r2p    = M.r2p.data();
     mv.node1  = M.node1.data();
     mv.anc    = M.anc.data();
@@ -1315,7 +1314,7 @@ void pcg_solve(b2s_solver* s, const double* b, double* x, const b2s_pcg_options&
         long long iter_before = h.iter;
         while(true)
         {
-            if(small && !pcg_small_launch(s, A, kind, ord, SMALL_LOOP, xi))
+            if(small && !pcg_small_launch(s, A, kind, SMALL_LOOP, xi))
             {
                 small = false;
                 prepare_steps();
@@ -1762,7 +1761,7 @@ void pcg_solve_mixed(b2s_solver* s, const double* b, double* x, const b2s_pcg_op
                 // whole blocks of check_interval, as the replacements are counted
                 const long long due = o.replace_every > 0 ? std::max<long long>(last_replace + o.replace_every - iter_before, 1) :
                                                             SMALL_LOOP;
-                if(!pcg_small_launch_f32(s, A, kind, ord, std::min<long long>((due + ci - 1) / ci * ci, SMALL_LOOP), xi))
+                if(!pcg_small_launch_f32(s, A, kind, std::min<long long>((due + ci - 1) / ci * ci, SMALL_LOOP), xi))
                 {
                     small = false;
                     prepare_steps();

@@ -8,7 +8,7 @@ namespace b2s
 struct MasView
 {
     int            active;  // MAS present
-    int            off, vn, L;
+    int            off, vn;
     int            abd_off, abd_n;  // affine-body range: block rows abd_off .. abd_off + 4 abd_n
     const double*  abd_inv;         // [abd_n * 144]
     const int32_t* r2p;
@@ -33,6 +33,6 @@ MasView mas_view(b2s_solver* s);
 // device has: a shared or partitioned GPU) or has no room for its sums: the
 // caller launches step by step.
 bool pcg_small_fits(b2s_solver* s, const Matrix& A, int kind, bool ord, bool f32);
-bool pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x);
-bool pcg_small_launch_f32(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x);
+bool pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, long long iterations, double* x);
+bool pcg_small_launch_f32(b2s_solver* s, const Matrix& A, int kind, long long iterations, double* x);
 }  // namespace b2s

@@ -22,7 +22,6 @@
 #include "b2s_pcg.cuh"
 
 #include <algorithm>
-#include <cstdlib>
 
 namespace b2s
 {
@@ -41,8 +40,7 @@ struct SmallArgs
 {
     int32_t        n;  // rows
     int            kind;
-    int            ord;  // rows in PCG order (only then the MAS)
-    int64_t        U, S;
+    int64_t        S;
     const int32_t* rows;
     const int32_t* cols;
     const VT*      vals;  // planes
@@ -638,7 +636,7 @@ int small_grid(const Matrix& A)
 }
 
 template <typename VT>
-bool launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x, const VT* vals, VT* r,
+bool launch(b2s_solver* s, const Matrix& A, int kind, long long iterations, double* x, const VT* vals, VT* r,
             VT* p, VT* Ap)
 {
     PcgState&     P   = s->pcg;
@@ -647,8 +645,6 @@ bool launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterat
     SmallArgs<VT> a{};
     a.n    = A.nb;
     a.kind = kind;
-    a.ord  = ord ? 1 : 0;
-    a.U    = A.nnz;
     a.S    = A.stride;
     a.rows = A.rows.data();
     a.cols = A.cols.data();
@@ -737,14 +733,14 @@ bool pcg_small_fits(b2s_solver* s, const Matrix& A, int kind, bool ord, bool f32
     return (int64_t)small_grid(A) <= (int64_t)occ * sms && A.nnz <= (int64_t)per_thread * SM_THREADS * sms;
 }
 
-bool pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x)
+bool pcg_small_launch(b2s_solver* s, const Matrix& A, int kind, long long iterations, double* x)
 {
     PcgState& P = s->pcg;
-    return launch<double>(s, A, kind, ord, iterations, x, A.vals.data(), P.r.data(), P.p.data(), P.Ap.data());
+    return launch<double>(s, A, kind, iterations, x, A.vals.data(), P.r.data(), P.p.data(), P.Ap.data());
 }
-bool pcg_small_launch_f32(b2s_solver* s, const Matrix& A, int kind, bool ord, long long iterations, double* x)
+bool pcg_small_launch_f32(b2s_solver* s, const Matrix& A, int kind, long long iterations, double* x)
 {
     PcgState& P = s->pcg;
-    return launch<float>(s, A, kind, ord, iterations, x, A.vals32.data(), P.r32.data(), P.p32.data(), P.Ap32.data());
+    return launch<float>(s, A, kind, iterations, x, A.vals32.data(), P.r32.data(), P.p32.data(), P.Ap32.data());
 }
 }  // namespace b2s

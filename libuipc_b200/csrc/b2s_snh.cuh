@@ -15,7 +15,6 @@
 //   p[k], q[k]: half the sum and half the difference of the pair's clamped
 //   values: A_ab is weighted by p_k, its partner A_ba by q_k.
 #pragma once
-#include <cmath>
 
 namespace b2s
 {
@@ -27,16 +26,8 @@ struct Projected
     double m[3][3], p[3], q[3];
 };
 
-__host__ __device__ inline double inv_sqrt(double x)
-{
-#ifdef __CUDA_ARCH__
-    return rsqrt(x);
-#else
-    return 1.0 / sqrt(x);
-#endif
-}
-__host__ __device__ inline double dot3(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
-__host__ __device__ inline void cross3(const double* a, const double* b, double* c)
+__device__ inline double dot3(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
+__device__ inline void cross3(const double* a, const double* b, double* c)
 {
     c[0] = a[1] * b[2] - a[2] * b[1];
     c[1] = a[2] * b[0] - a[0] * b[2];
@@ -47,7 +38,7 @@ __host__ __device__ inline void cross3(const double* a, const double* b, double*
 // orthogonal; false when they already are (to rounding). A pair that is not
 // finite counts as orthogonal.
 template <int P, int Q>
-__host__ __device__ inline bool rotate_columns(double a[3][3], double v[3][3])
+__device__ inline bool rotate_columns(double a[3][3], double v[3][3])
 {
     const double al = dot3(a[P], a[P]), be = dot3(a[Q], a[Q]), ga = dot3(a[P], a[Q]);
     if(!(ga * ga > 1e-31 * (al * be)))
@@ -55,7 +46,7 @@ __host__ __device__ inline bool rotate_columns(double a[3][3], double v[3][3])
     // t = sign(z) / (|z| + sqrt(z^2 + 1)) of z = d / g without forming z
     const double d = be - al, g = 2.0 * ga;
     const double t = (d >= 0.0 ? g : -g) / (fabs(d) + sqrt(d * d + g * g));
-    const double c = inv_sqrt(t * t + 1.0), s = c * t;
+    const double c = rsqrt(t * t + 1.0), s = c * t;
     for(int r = 0; r < 3; ++r)
     {
         const double ap = a[P][r], aq = a[Q][r], vp = v[P][r], vq = v[Q][r];
@@ -68,13 +59,13 @@ __host__ __device__ inline bool rotate_columns(double a[3][3], double v[3][3])
 }
 
 // a unit vector orthogonal to the unit vector u
-__host__ __device__ inline void any_orthogonal(const double* u, double* w)
+__device__ inline void any_orthogonal(const double* u, double* w)
 {
     const double x = fabs(u[0]), y = fabs(u[1]), z = fabs(u[2]);
     const double e[3] = {x <= y && x <= z ? 1.0 : 0.0, !(x <= y && x <= z) && y <= z ? 1.0 : 0.0,
                          !(x <= y && x <= z) && !(y <= z) ? 1.0 : 0.0};
     cross3(u, e, w);
-    const double n = inv_sqrt(dot3(w, w));
+    const double n = rsqrt(dot3(w, w));
     for(int r = 0; r < 3; ++r)
         w[r] *= n;
 }
@@ -82,7 +73,7 @@ __host__ __device__ inline void any_orthogonal(const double* u, double* w)
 // F = U diag(sg) V^T by one-sided Jacobi: the columns of F V made orthogonal
 // (V a product of rotations), sg_2 the smallest in magnitude and signed so
 // that U is a rotation too
-__host__ __device__ inline void rotation_svd(const double F[9], double u[3][3], double v[3][3], double sg[3])
+__device__ inline void rotation_svd(const double F[9], double u[3][3], double v[3][3], double sg[3])
 {
     double a[3][3];
     for(int i = 0; i < 3; ++i)
@@ -119,13 +110,13 @@ __host__ __device__ inline void rotation_svd(const double F[9], double u[3][3], 
     n1 = s0 ? n2 : (s1 ? t0 : t1);
     if(n0 > 0.0)
     {
-        const double i0 = inv_sqrt(n0);
+        const double i0 = rsqrt(n0);
         for(int r = 0; r < 3; ++r)
             u[0][r] = a[0][r] * i0;
     }
     else if(n1 > 0.0)
     {
-        const double i1 = inv_sqrt(n1);
+        const double i1 = rsqrt(n1);
         double       w[3];
         for(int r = 0; r < 3; ++r)
             w[r] = a[1][r] * i1;
@@ -138,7 +129,7 @@ __host__ __device__ inline void rotation_svd(const double F[9], double u[3][3], 
     const double nw = dot3(w1, w1);
     if(nw > 1e-30 * n0 && nw > 0.0)
     {
-        const double iw = inv_sqrt(nw);
+        const double iw = rsqrt(nw);
         for(int r = 0; r < 3; ++r)
             u[1][r] = w1[r] * iw;
     }
@@ -151,7 +142,7 @@ __host__ __device__ inline void rotation_svd(const double F[9], double u[3][3], 
 
 // m = Q max(w, 0) Q^T of a symmetric 3x3 matrix; returned as it is when it is
 // safely positive definite (leading minors well above rounding)
-__host__ __device__ inline void clamp3(double m[3][3])
+__device__ inline void clamp3(double m[3][3])
 {
     const double d2 = m[0][0] * m[1][1] - m[0][1] * m[0][1];
     const double d3 = m[2][2] * d2 - m[0][2] * (m[0][2] * m[1][1] - m[0][1] * m[1][2])
@@ -198,7 +189,7 @@ __host__ __device__ inline void clamp3(double m[3][3])
 }
 
 // P = dPsi/dF and the projected Hessian's parts, all times `scale`
-__host__ __device__ inline void derivatives(const double F[9], double mu, double lambda, double scale, double P[9],
+__device__ inline void derivatives(const double F[9], double mu, double lambda, double scale, double P[9],
                                             Projected& h)
 {
     double g[9];
@@ -230,7 +221,7 @@ __host__ __device__ inline void derivatives(const double F[9], double mu, double
 // the 3x3 Hessian block (row-major) of two vertices whose shape gradients are
 // gq and gr in the V frame (V^T g): B[a][c] = sum gq_b gr_d H[(a,b),(c,d)] in
 // the U frame, rotated back
-__host__ __device__ inline void block(const Projected& h, const double gq[3], const double gr[3], double out[9])
+__device__ inline void block(const Projected& h, const double gq[3], const double gr[3], double out[9])
 {
     double B[3][3];
     for(int a = 0; a < 3; ++a)
