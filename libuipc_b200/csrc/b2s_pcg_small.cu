@@ -7,7 +7,7 @@
 // warp owns the two MAS banks of its 32 rows and keeps their inverses in
 // shared memory, and the steps are separated by grid barriers (three per
 // iteration with block Jacobi, five with the MAS). Only p (gathered by the
-// SpMV), Ap (its reductions) and the coarse nodes' R and Z go through L2.
+// SpMV), Ap (its reductions) and the coarse levels' sums and Z go through L2.
 // Same arithmetic per entry, stop rules and scalars as the launch-per-step
 // loop; the sums add per-block partials in a fixed order.
 //

@@ -1,5 +1,5 @@
 """Assembly at the edges of its row and run classes, bit-exact against numpy:
-rows around one warp's 32 / 64 pairs, the 256-pair shared-memory limit, one
+rows around one warp's 32 / 64 pairs, the 256-pair limit of a warp, one
 and several 4,096-pair tiles of the long-row sort; runs around the 64 sources
 that one thread sums; the matrix read back to device and to host memory."""
 import numpy as np
