@@ -389,9 +389,9 @@ __device__ __forceinline__ void heavy_bank(const ApplyArgs& A, int64_t gbank, co
 }
 
 // The banks handled by one warp (warp gw of W). The list: the banks from level
-// 3 up (global banks g3 ..; skipped when CTAs of their own have them), of level 2,
-// of level 0, of level 1. A copy wait that runs out sets the error flag, drains the warp's copies in
-// flight and ends the warp.
+// 3 up (global banks g3 ..; skipped when CTAs of their own have them), of level
+// 2, of level 0, of level 1. A copy wait that runs out sets the error flag,
+// drains the warp's copies in flight and ends the warp.
 template <bool BF, int NST>
 __device__ __forceinline__ void apply_banks(int gw, int W, int lane, const ApplyArgs& A, const int* stop,
                                             unsigned char* s_stage, uint64_t* s_bar)
